@@ -6,8 +6,8 @@
 // with a deterministic two-pass reduction through arena scratch (A^T x), 128-bit stores (x y^T).
 //
 // gemm_simt is the matrix multiply for everything the tensor-core path (gemm_tc.cu) does not
-// take: float64, shapes whose leading dimensions break TMA's 16-byte rule, and problems too
-// small to fill a 128-row tile. Row-major operands with leading dimensions, either operand
+// take: products of few columns, problems too small to fill a 128-row tile, operands whose splits do
+// not fit the arena; float64 goes on to gemm_f64.cu. Row-major operands with leading dimensions, either operand
 // transposed, batched with strides, the same fused epilogue as the tensor-core kernel.
 #include <algorithm>
 
@@ -384,6 +384,11 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(int transB, long long 
   }
 }
 
+// gemm_f64.cu
+int gemm_f64(b200_engine *e, int transA, int transB, long long M, long long N, long long K, const double *A,
+             long long lda, const double *B, long long ldb, double *C, long long ldc, long long batch,
+             long long strideA, long long strideB, long long strideC, const Epilogue &ep);
+
 int gemm_simt(b200_engine *e, int dtype, int transA, int transB, long long M, long long N, long long K,
               const void *A, long long lda, const void *B, long long ldb, void *C, long long ldc, long long batch,
               long long strideA, long long strideB, long long strideC, const Epilogue &ep) {
@@ -401,15 +406,13 @@ int gemm_simt(b200_engine *e, int dtype, int transA, int transB, long long M, lo
     B200_CHECK_LAUNCH(e, "gemm_skinny_kernel");
     return B200_OK;
   }
+  if (dtype == B200_F64)
+    return gemm_f64(e, transA, transB, M, N, K, (const double *)A, lda, (const double *)B, ldb, (double *)C, ldc,
+                    batch, strideA, strideB, strideC, ep);
   dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), (unsigned)batch);
-  if (dtype == B200_F32)
-    gemm_simt_kernel<float><<<grid, 256, 0, e->stream>>>(transA, transB, M, N, K, (const float *)A, lda,
-                                                        (const float *)B, ldb, (float *)C, ldc, strideA, strideB,
-                                                        strideC, ep);
-  else
-    gemm_simt_kernel<double><<<grid, 256, 0, e->stream>>>(transA, transB, M, N, K, (const double *)A, lda,
-                                                         (const double *)B, ldb, (double *)C, ldc, strideA, strideB,
-                                                         strideC, ep);
+  gemm_simt_kernel<float><<<grid, 256, 0, e->stream>>>(transA, transB, M, N, K, (const float *)A, lda,
+                                                      (const float *)B, ldb, (float *)C, ldc, strideA, strideB,
+                                                      strideC, ep);
   B200_CHECK_LAUNCH(e, "gemm_simt_kernel");
   return B200_OK;
 }
