@@ -235,45 +235,49 @@ __global__ void __launch_bounds__(256) maxpool2x2_any_kernel(const float *__rest
 
 // ---- im2col ------------------------------------------------------------------------------------
 // col[(b, oh, ow), (c, r, s)] = x[b, c, oh*sH - padH + r*dH, ow*sW - padW + s*dW], 0 outside.
-// One thread per column element; consecutive threads write consecutive (c, r, s), which makes
-// the big side (the col buffer) perfectly coalesced while reads of x hit L1/L2.
-// SPLIT: write the TF32 head and tail of each value instead (feeds the 3xTF32 matrix multiply
-// without a second pass over the col buffer); the row pitch `ld` may exceed C*kh*kw (padding = 0).
-__device__ __forceinline__ float to_tf32_rna(float v) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-  return __uint_as_float(r);
-}
-
-template <typename T, bool SPLIT>
-__global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T *__restrict__ col,
-                                                     T *__restrict__ col_lo, long long B, int C, int H, int W,
-                                                     int Ho, int Wo, int kh, int kw, int padH, int padW, int sH,
-                                                     int sW, int dH, int dW, int ld) {
-  const int crs = C * kh * kw;
-  const long long total = B * Ho * Wo * (long long)ld;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const int q = (int)(t % ld);
-    const long long row = t / ld;
-    T v = T(0);
-    if (q < crs) {
-      const int s = q % kw;
-      const int r = (q / kw) % kh;
-      const int c = q / (kw * kh);
-      const int ow = (int)(row % Wo);
-      const int oh = (int)((row / Wo) % Ho);
-      const long long b = row / ((long long)Wo * Ho);
+// A warp takes 32 consecutive entries q of a col row (one
+// (channel, tap) per lane, worked out once) and walks output positions of an image row, so the writes are
+// 128 contiguous bytes and nothing is divided per element; the reads of the 3.5 channels that 32 entries of
+// a 3x3 window span stay in L1 from one position to the next. Four positions are in flight per lane.
+// Bound by HBM (col is written once, nine times the image for 3x3); with an index division per element it
+// was bound by integer arithmetic: 100 x 32 x 14 x 14, 3x3 float32 57 -> 13 us.
+// grid: blockIdx.x walks groups of `rows` output rows of all images.
+template <typename T>
+__global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T *__restrict__ col, long long out_rows,
+                                                     int C, int H, int W, int Ho, int Wo, int kh, int kw, int padH,
+                                                     int padW, int sH, int sW, int dH, int dW, int rows) {
+  const int crs = C * kh * kw, pieces = (crs + 31) / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (long long g0 = (long long)blockIdx.x * rows; g0 < out_rows; g0 += (long long)gridDim.x * rows) {
+    const int here = (int)(out_rows - g0 < rows ? out_rows - g0 : rows);
+    for (int t = warp; t < pieces * here; t += 8) {
+      const int rr = t / pieces, q = (t - rr * pieces) * 32 + lane;
+      const long long row = g0 + rr, b = row / Ho;
+      const int oh = (int)(row - b * Ho);
+      if (q >= crs) continue;
+      const int c = q / (kh * kw), tap = q - c * kh * kw, r = tap / kw, s = tap - r * kw;
       const int ih = oh * sH - padH + r * dH;
-      const int iw = ow * sW - padW + s * dW;
-      if (ih >= 0 && ih < H && iw >= 0 && iw < W) v = x[((b * C + c) * H + ih) * (long long)W + iw];
-    }
-    if (SPLIT) {
-      const float h = to_tf32_rna((float)v);
-      col[t] = (T)h;
-      col_lo[t] = (T)to_tf32_rna(__fsub_rn((float)v, h));
-    } else {
-      col[t] = v;
+      int iw = s * dW - padW;
+      const T *in = x + ((b * C + c) * H + ih) * (long long)W;
+      T *out = col + row * Wo * (long long)crs + q;
+      const bool inside = ih >= 0 && ih < H;
+      int ow = 0;
+      for (; ow + 3 < Wo; ow += 4) {
+        T v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v[j] = inside && iw >= 0 && iw < W ? __ldg(in + iw) : T(0);
+          iw += sW;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) out[(long long)j * crs] = v[j];
+        out += 4LL * crs;
+      }
+      for (; ow < Wo; ++ow) {
+        *out = inside && iw >= 0 && iw < W ? __ldg(in + iw) : T(0);
+        iw += sW;
+        out += crs;
+      }
     }
   }
 }
@@ -417,44 +421,59 @@ __global__ void __launch_bounds__(256) col2im_kernel(const T *__restrict__ col, 
   }
 }
 
-// The gradient of the pooling every config here uses (2x2 window, stride 2, no padding, W a multiple
-// of 4): windows do not overlap, so an input element receives at most one term, 0 + dy (the
-// reference adds into a zeroed array, which turns a -0.0 gradient into +0.0; so does this). One
-// thread handles two neighbouring windows: 8 bytes of gradient and 16 of mask in, two float4 rows
-// out. Rows and columns past the last whole window (odd H) are written as zeros.
+// The gradient of the pooling every config here uses (2x2 window, stride 2, no padding, W even):
+// windows do not overlap, so an input element receives at most one term, 0 + dy (the reference adds into
+// a zeroed array, which turns a -0.0 gradient into +0.0; so does this). One thread handles NW neighbouring
+// windows and writes 2 NW elements of two rows; nothing is summed over windows and nothing divided beyond
+// the 32-bit place of the thread. Two windows (16 bytes per row) where W is a multiple of 4, else one: a
+// 14-wide plane has 28 bytes of gradient per row, which only 8-byte accesses can follow.
+// Rows past the last whole window (odd H) are written as zeros.
+// 100 x 64 x 14 x 14 float32: 18.4 us through the general kernel -> 5 us.
+template <int NW>
 __global__ void __launch_bounds__(256) maxpool2x2_bwd_kernel(const float *__restrict__ dy,
                                                              const long long *__restrict__ mask,
                                                              float *__restrict__ dx, long long planes, int H, int W,
                                                              int Ho, int Wo) {
-  const int pairs = Wo >> 1;  // Wo = W/2 is even because W % 4 == 0
-  const int rows = (H + 1) >> 1;  // one extra, window-less row when H is odd
-  const long long total = planes * rows * pairs;
+  const uint32_t cols = (uint32_t)(Wo / NW), rows = (uint32_t)(H + 1) >> 1;  // one window-less row when H is odd
+  const long long total = planes * rows * cols;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const int j = (int)(t % pairs);
-    const int ph = (int)((t / pairs) % rows);
-    const long long plane = t / ((long long)pairs * rows);
-    float *out = dx + (plane * H + 2 * ph) * (long long)W + 4 * j;
+    const long long line = total <= 0xFFFFFFFFLL ? (long long)((uint32_t)t / cols) : t / cols;
+    const uint32_t j = (uint32_t)(t - line * cols);
+    const long long plane = total <= 0xFFFFFFFFLL ? (long long)((uint32_t)line / rows) : line / rows;
+    const int ph = (int)(line - plane * rows);
+    struct alignas(8 * NW) Row {
+      float v[2 * NW];
+    };
+    float *out = dx + (plane * H + 2 * ph) * (long long)W + 2 * NW * j;
+    Row r0, r1;
     if (ph >= Ho) {  // the last row of an odd-height plane belongs to no window
-      *reinterpret_cast<float4 *>(out) = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 2 * NW; ++k) r0.v[k] = 0.f;
+      *reinterpret_cast<Row *>(out) = r0;
       continue;
     }
-    const long long o = (plane * Ho + ph) * (long long)Wo + 2 * j;
-    const float2 g = *reinterpret_cast<const float2 *>(dy + o);
-    const longlong2 m = *reinterpret_cast<const longlong2 *>(mask + o);
-    const long long base = (long long)(2 * ph) * W + 4 * j;  // index of out[0] inside the plane
-    const float g0 = 0.f + g.x, g1 = 0.f + g.y;
-    float4 r0, r1;
-    r0.x = m.x == base ? g0 : 0.f;
-    r0.y = m.x == base + 1 ? g0 : 0.f;
-    r0.z = m.y == base + 2 ? g1 : 0.f;
-    r0.w = m.y == base + 3 ? g1 : 0.f;
-    r1.x = m.x == base + W ? g0 : 0.f;
-    r1.y = m.x == base + W + 1 ? g0 : 0.f;
-    r1.z = m.y == base + W + 2 ? g1 : 0.f;
-    r1.w = m.y == base + W + 3 ? g1 : 0.f;
-    *reinterpret_cast<float4 *>(out) = r0;
-    *reinterpret_cast<float4 *>(out + W) = r1;
+    const long long o = (plane * Ho + ph) * (long long)Wo + NW * j;
+    const long long base = (long long)(2 * ph) * W + 2 * NW * j;  // index of out[0] inside the plane
+    float g[NW];
+    long long m[NW];
+    if (NW == 2) {
+      const float2 gg = *reinterpret_cast<const float2 *>(dy + o);
+      const longlong2 mm = *reinterpret_cast<const longlong2 *>(mask + o);
+      g[0] = gg.x; g[NW - 1] = gg.y;
+      m[0] = mm.x; m[NW - 1] = mm.y;
+    } else {
+      g[0] = dy[o];
+      m[0] = mask[o];
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * NW; ++k) {
+      const float gk = 0.f + g[k / 2];
+      r0.v[k] = m[k / 2] == base + k ? gk : 0.f;
+      r1.v[k] = m[k / 2] == base + W + k ? gk : 0.f;
+    }
+    *reinterpret_cast<Row *>(out) = r0;
+    *reinterpret_cast<Row *>(out + W) = r1;
   }
 }
 
@@ -765,51 +784,40 @@ __global__ void __launch_bounds__(C2I_THREADS, 2) col2im_bulk_kernel(const float
 }
 
 // ---- BatchNormOp (op_nn.go:1346-1640) on (B, C, S) -------------------------------------------------
-// Three launches. (1) partial sums of x and x^2 per (channel, group of samples) in double; (2) one
-// thread per channel folds the groups in a fixed order and makes everything that is per channel:
+// Two launches in training. (1) Partial sums of x and x^2 per (channel, group of samples) in double; the
+// block that delivers a channel's last group folds the groups in a fixed order (one warp: lane l takes
+// groups l and l + 32, then a shuffle tree) and makes everything that is per channel:
 // saveMean = sum / n rounded to the tensor's type, saveVar = sum (x - saveMean)^2 (from the two sums:
 // sum x^2 - 2 m sum x + n m^2, in double), the running statistics, alpha = 1 / sqrt(var + eps) and
-// beta = -mean * alpha in the tensor's type as the reference computes them; (3) y = x * alpha + beta,
+// beta = -mean * alpha in the tensor's type as the reference computes them; (2) y = x * alpha + beta,
 // a product then a sum, plane by plane so that no element pays an index division. The reference sums
 // sequentially in the tensor's type; the double sums here are closer to the exact value.
-constexpr int BN_GROUPS = 64;
+// Folding in a launch of its own cost 10 us (a thread per channel reading 128 values one after the other);
+// 128 x 64 x 28 x 28 float32, partial sums and fold: 24 -> 14 us, and 40 -> 18 us backward.
+constexpr int BN_GROUPS = 64;  // at most; bn_groups() takes fewer where they would be short
 
-template <typename T>
-__global__ void __launch_bounds__(256) bn_partial_kernel(const T *__restrict__ x, long long B, int C, long long S,
-                                                         double *__restrict__ part) {
-  const int c = blockIdx.x, grp = blockIdx.y;
-  const long long per = (B + BN_GROUPS - 1) / BN_GROUPS;
-  const long long b0 = grp * per, b1 = min(B, b0 + per);
-  double s1 = 0.0, s2 = 0.0;
-  if (sizeof(T) == 4 && S % 4 == 0 && (uintptr_t)x % 16 == 0 && (b1 - b0) * (S >> 2) < (1LL << 31)) {
-    // float planes as float4; the threads spread over (sample, float4) pairs so that short planes
-    // keep the whole block busy
-    const uint32_t S4 = (uint32_t)(S >> 2), total4 = (uint32_t)(b1 > b0 ? (b1 - b0) * S4 : 0);
-    for (uint32_t i = threadIdx.x; i < total4; i += blockDim.x) {
-      const uint32_t bb = i / S4, d = i - bb * S4;
-      const float4 q = __ldg(reinterpret_cast<const float4 *>(x + ((b0 + bb) * C + c) * S) + d);
-      const double v0 = q.x, v1 = q.y, v2 = q.z, v3 = q.w;
-      s1 += (v0 + v1) + (v2 + v3);
-      s2 += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
-    }
-  } else if (S >= 32) {
-    for (long long b = b0; b < b1; ++b) {
-      const T *p = x + (b * C + c) * S;
-      for (long long d = threadIdx.x; d < S; d += blockDim.x) {
-        const double v = p[d];
-        s1 += v;
-        s2 += v * v;
-      }
-    }
-  } else {  // short planes (a matrix has S = 1): threads spread over (sample, position) pairs
-    for (long long i = b0 * S + threadIdx.x; i < b1 * S; i += blockDim.x) {
-      const long long b = i / S, d = i - b * S;
-      const double v = x[(b * C + c) * S + d];
-      s1 += v;
-      s2 += v * v;
-    }
+// Sums of both values over a channel's groups, to every lane of the calling warp.
+__device__ __forceinline__ void bn_fold_groups(const double *part, int c, int groups, double &s1, double &s2) {
+  const int lane = threadIdx.x & 31;
+  s1 = s2 = 0.0;
+  for (int gq = lane; gq < groups; gq += 32) {
+    s1 += __ldcg(part + ((long long)c * groups + gq) * 2);
+    s2 += __ldcg(part + ((long long)c * groups + gq) * 2 + 1);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+}
+
+// The end of a partial-sum block: leaves the block's two sums and, in the block that delivers the
+// channel's last group, hands warp 0 the channel's sums (returns true there, to whole warps only).
+__device__ __forceinline__ bool bn_deliver(int c, double s1, double s2, double *part, int *count, double &t1,
+                                           double &t2) {
   __shared__ double sh1[8], sh2[8];
+  __shared__ int s_last;
+  const int grp = blockIdx.y, groups = gridDim.y;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
@@ -826,41 +834,117 @@ __global__ void __launch_bounds__(256) bn_partial_kernel(const T *__restrict__ x
       a += sh1[w];
       b2 += sh2[w];
     }
-    part[((long long)c * BN_GROUPS + grp) * 2] = a;
-    part[((long long)c * BN_GROUPS + grp) * 2 + 1] = b2;
+    __stcg(part + ((long long)c * groups + grp) * 2, a);
+    __stcg(part + ((long long)c * groups + grp) * 2 + 1, b2);
+    __threadfence();
+    s_last = atomicAdd(count + blockIdx.x, 1) == groups - 1;
+    if (s_last) count[blockIdx.x] = 0;  // zero again for the next launch
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last || threadIdx.x >= 32) return false;
+  bn_fold_groups(part, c, groups, t1, t2);
+  return true;
+}
+
+// Walks the samples [b0, b1) of channel c and hands (x, dy) values to `take`: 16 bytes at a time where
+// planes allow it (float32, S a multiple of 4), the threads spread over (sample, piece) pairs so that
+// short planes keep the whole block busy, with 32-bit index arithmetic and two pieces in flight.
+template <typename T, bool TWO, typename F>
+__device__ __forceinline__ void bn_walk(const T *__restrict__ x, const T *__restrict__ g, long long b0, long long b1,
+                                        int C, int c, long long S, F take) {
+  if (b1 <= b0) return;
+  const bool vec = sizeof(T) == 4 && S % 4 == 0 && ((uintptr_t)x | (TWO ? (uintptr_t)g : 0)) % 16 == 0;
+  const long long per = vec ? S >> 2 : S, total = (b1 - b0) * per;
+  if (total >= (1LL << 31)) {  // planes this long fill the block by themselves
+    for (long long b = b0; b < b1; ++b)
+      for (long long d = threadIdx.x; d < S; d += 256) {
+        const long long at = (b * C + c) * S + d;
+        take((double)x[at], TWO ? (double)g[at] : 0.0);
+      }
+    return;
+  }
+  const uint32_t p32 = (uint32_t)per, n = (uint32_t)total;
+  auto at = [&](uint32_t i) {
+    const uint32_t bb = i / p32, d = i - bb * p32;
+    return ((b0 + bb) * C + c) * per + d;
+  };
+  if (vec) {
+    const float4 *x4 = reinterpret_cast<const float4 *>(x), *g4 = reinterpret_cast<const float4 *>(g);
+    auto take4 = [&](const float4 &a, const float4 &b) {
+      take((double)a.x, (double)b.x);
+      take((double)a.y, (double)b.y);
+      take((double)a.z, (double)b.z);
+      take((double)a.w, (double)b.w);
+    };
+    uint32_t i = threadIdx.x;
+    for (; i + 256 < n; i += 512) {
+      const long long o0 = at(i), o1 = at(i + 256);
+      const float4 a0 = __ldg(x4 + o0), a1 = __ldg(x4 + o1);
+      float4 b0v = make_float4(0.f, 0.f, 0.f, 0.f), b1v = b0v;
+      if (TWO) {
+        b0v = __ldg(g4 + o0);
+        b1v = __ldg(g4 + o1);
+      }
+      take4(a0, b0v);
+      take4(a1, b1v);
+    }
+    for (; i < n; i += 256) {
+      const long long o = at(i);
+      take4(__ldg(x4 + o), TWO ? __ldg(g4 + o) : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < n; i += 256) {
+      const long long o = at(i);
+      take((double)__ldg(x + o), TWO ? (double)__ldg(g + o) : 0.0);
+    }
   }
 }
 
+// What is per channel in training mode, from the sums of x and x^2 over all n values (one thread).
 template <typename T>
-__global__ void bn_finish_kernel(const double *__restrict__ part, int C, long long n, int training, T momentum, T eps,
-                                 T *__restrict__ running_mean, T *__restrict__ running_var, T *__restrict__ save_mean,
-                                 T *__restrict__ save_var, T *__restrict__ alpha_beta) {
+__device__ __forceinline__ void bn_channel(int c, double s1, double s2, long long n, T momentum, T eps,
+                                           T *running_mean, T *running_var, T *save_mean, T *save_var, T *alpha_beta) {
+  const T m = (T)(s1 / (double)n);
+  const double md = (double)m;
+  double vd = s2 - 2.0 * md * s1 + (double)n * md * md;
+  if (vd < 0.0) vd = 0.0;
+  const T v = (T)vd;
+  save_mean[c] = m;
+  save_var[c] = v;
+  running_mean[c] = momentum * m + (T(1) - momentum) * running_mean[c];
+  running_var[c] = momentum * (v / (T)(n - 1)) + (T(1) - momentum) * running_var[c];
+  const T inv = T(1) / sqrt(v / (T)n + eps);
+  alpha_beta[2 * c] = inv;
+  alpha_beta[2 * c + 1] = -m * inv;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) bn_sums_kernel(int c0, const T *__restrict__ x, long long B, int C, long long S,
+                                                      double *__restrict__ part, int *__restrict__ count, T momentum,
+                                                      T eps, T *__restrict__ running_mean, T *__restrict__ running_var,
+                                                      T *__restrict__ save_mean, T *__restrict__ save_var,
+                                                      T *__restrict__ alpha_beta) {
+  const int c = c0 + blockIdx.x;
+  const long long per = (B + gridDim.y - 1) / gridDim.y, b0 = blockIdx.y * per, b1 = min(B, b0 + per);
+  double s1 = 0.0, s2 = 0.0, t1, t2;
+  bn_walk<T, false>(x, x, b0, b1, C, c, S, [&](double v, double) {
+    s1 += v;
+    s2 += v * v;
+  });
+  if (bn_deliver(c, s1, s2, part, count, t1, t2) && threadIdx.x == 0)
+    bn_channel<T>(c, t1, t2, B * S, momentum, eps, running_mean, running_var, save_mean, save_var, alpha_beta);
+}
+
+// Inference: alpha and beta from the running statistics.
+template <typename T>
+__global__ void bn_inference_kernel(int C, T eps, const T *__restrict__ running_mean, const T *__restrict__ running_var,
+                                    T *__restrict__ alpha_beta) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
-  T mean, inv;
-  if (training) {
-    double s1 = 0.0, s2 = 0.0;
-    for (int gq = 0; gq < BN_GROUPS; ++gq) {
-      s1 += part[((long long)c * BN_GROUPS + gq) * 2];
-      s2 += part[((long long)c * BN_GROUPS + gq) * 2 + 1];
-    }
-    const T m = (T)(s1 / (double)n);
-    const double md = (double)m;
-    double vd = s2 - 2.0 * md * s1 + (double)n * md * md;
-    if (vd < 0.0) vd = 0.0;
-    const T v = (T)vd;
-    save_mean[c] = m;
-    save_var[c] = v;
-    running_mean[c] = momentum * m + (T(1) - momentum) * running_mean[c];
-    running_var[c] = momentum * (v / (T)(n - 1)) + (T(1) - momentum) * running_var[c];
-    mean = m;
-    inv = T(1) / sqrt(v / (T)n + eps);
-  } else {
-    mean = running_mean[c];
-    inv = T(1) / sqrt(running_var[c] + eps);
-  }
+  const T inv = T(1) / sqrt(running_var[c] + eps);
   alpha_beta[2 * c] = inv;
-  alpha_beta[2 * c + 1] = -mean * inv;
+  alpha_beta[2 * c + 1] = -running_mean[c] * inv;
 }
 
 __device__ __forceinline__ float bn_mul(float a, float b) { return __fmul_rn(a, b); }
@@ -900,67 +984,36 @@ __global__ void __launch_bounds__(256) bn_apply_kernel(const T *__restrict__ x, 
 }
 
 // ---- batchnormDiffOp (op_nn.go:1727-1940): the input gradient of BatchNormOp --------------------
-// Same three-launch shape as the forward op: partial sums of dy and x*dy per (channel, sample group)
-// in double; one thread per channel folds them into gradMean = sum dy / n, dotp = sum (x - mean) dy,
-// k = dotp * invstd^2 / n in the tensor's type; the output pass then evaluates the reference's
-// expression, including its order of subtractions, which differs between the matrix and the
+// Same shape as the forward op: partial sums of dy and x*dy per (channel, sample group) in double,
+// folded by the block that delivers a channel's last group into gradMean = sum dy / n, dotp = sum
+// (x - mean) dy, k = dotp * invstd^2 / n in the tensor's type; the output pass then evaluates the
+// reference's expression, including its order of subtractions, which differs between the matrix and the
 // spatial branch, and its choice of variance in inference mode.
 template <typename T>
-__global__ void __launch_bounds__(256) bn_bwd_partial_kernel(const T *__restrict__ x, const T *__restrict__ dy,
-                                                             long long B, int C, long long S,
-                                                             double *__restrict__ part) {
-  const int c = blockIdx.x, grp = blockIdx.y;
-  const long long per = (B + BN_GROUPS - 1) / BN_GROUPS;
-  const long long b0 = grp * per, b1 = min(B, b0 + per);
-  double s1 = 0.0, s2 = 0.0;
-  for (long long i = b0 * S + threadIdx.x; i < b1 * S; i += blockDim.x) {
-    const long long b = i / S, d = i - b * S;
-    const long long at = (b * C + c) * S + d;
-    const double g = dy[at];
+__global__ void __launch_bounds__(256) bn_bwd_sums_kernel(int c0, const T *__restrict__ x,
+                                                          const T *__restrict__ dy, long long B, int C, long long S, double *__restrict__ part,
+                                                          int *__restrict__ count, int training, T eps,
+                                                          const T *__restrict__ running_var,
+                                                          const T *__restrict__ save_mean,
+                                                          const T *__restrict__ save_var, T *__restrict__ coef) {
+  const int c = c0 + blockIdx.x;
+  const long long per = (B + gridDim.y - 1) / gridDim.y, b0 = blockIdx.y * per, b1 = min(B, b0 + per);
+  double s1 = 0.0, s2 = 0.0, t1, t2;
+  bn_walk<T, true>(x, dy, b0, b1, C, c, S, [&](double v, double g) {
     s1 += g;
-    s2 += (double)x[at] * g;
+    s2 += v * g;
+  });
+  if (bn_deliver(c, s1, s2, part, count, t1, t2) && threadIdx.x == 0) {
+    const long long n = B * S;
+    const T mean = save_mean[c];
+    const T sum = (T)t1, dotp = (T)(t2 - (double)mean * t1);
+    T invstd = T(1) / sqrt(save_var[c] / (T)n + eps);
+    if (!training && S == 1) invstd = T(1) / sqrt(running_var[c] + eps);
+    coef[4 * c] = mean;
+    coef[4 * c + 1] = (T)(dotp * invstd * invstd) / (T)n;  // k
+    coef[4 * c + 2] = sum / (T)n;                          // gradMean
+    coef[4 * c + 3] = invstd;
   }
-  __shared__ double sh1[8], sh2[8];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    sh1[threadIdx.x >> 5] = s1;
-    sh2[threadIdx.x >> 5] = s2;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, b2 = 0.0;
-    for (int w = 0; w < 8; ++w) {
-      a += sh1[w];
-      b2 += sh2[w];
-    }
-    part[((long long)c * BN_GROUPS + grp) * 2] = a;
-    part[((long long)c * BN_GROUPS + grp) * 2 + 1] = b2;
-  }
-}
-
-template <typename T>
-__global__ void bn_bwd_finish_kernel(const double *__restrict__ part, int C, long long n, long long S, int training,
-                                     T eps, const T *__restrict__ running_var, const T *__restrict__ save_mean,
-                                     const T *__restrict__ save_var, T *__restrict__ coef) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  double s1 = 0.0, s2 = 0.0;
-  for (int gq = 0; gq < BN_GROUPS; ++gq) {
-    s1 += part[((long long)c * BN_GROUPS + gq) * 2];
-    s2 += part[((long long)c * BN_GROUPS + gq) * 2 + 1];
-  }
-  const T mean = save_mean[c];
-  const T sum = (T)s1, dotp = (T)(s2 - (double)mean * s1);
-  T invstd = T(1) / sqrt(save_var[c] / (T)n + eps);
-  if (!training && S == 1) invstd = T(1) / sqrt(running_var[c] + eps);
-  coef[4 * c] = mean;
-  coef[4 * c + 1] = (T)(dotp * invstd * invstd) / (T)n;  // k
-  coef[4 * c + 2] = sum / (T)n;                          // gradMean
-  coef[4 * c + 3] = invstd;
 }
 
 __device__ __forceinline__ float bn_sub(float a, float b) { return __fsub_rn(a, b); }
@@ -969,7 +1022,7 @@ __device__ __forceinline__ double bn_sub(double a, double b) { return __dsub_rn(
 template <typename T>
 __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const T *__restrict__ x, const T *__restrict__ dy,
                                                            T *__restrict__ dx, long long planes, int C, long long S,
-                                                           int training, const T *__restrict__ coef) {
+                                                           int training, const T *__restrict__ coef, bool vec4) {
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -978,6 +1031,18 @@ __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const T *__restrict__
     const T mean = coef[4 * c], k = coef[4 * c + 1], gm = coef[4 * c + 2], inv = coef[4 * c + 3];
     const T *xp = x + pl * S, *gp = dy + pl * S;
     T *op = dx + pl * S;
+    if (sizeof(T) == 4 && vec4) {  // S % 4 == 0 and all tensors 16-byte aligned; S > 1: the spatial order
+      const float fm = (float)mean, fk = (float)k, fg = (float)gm, fi = (float)inv;
+      auto one = [&](float xv, float gv) {
+        return training ? __fmul_rn(__fsub_rn(__fsub_rn(gv, fg), __fmul_rn(__fsub_rn(xv, fm), fk)), fi)
+                        : __fmul_rn(gv, fi);
+      };
+      for (long long d = lane; d < (S >> 2); d += 32) {
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(xp) + d), g = __ldg(reinterpret_cast<const float4 *>(gp) + d);
+        reinterpret_cast<float4 *>(op)[d] = make_float4(one(a.x, g.x), one(a.y, g.y), one(a.z, g.z), one(a.w, g.w));
+      }
+      continue;
+    }
     for (long long d = lane; d < S; d += 32) {
       if (!training) {
         op[d] = bn_mul(gp[d], inv);
@@ -992,6 +1057,11 @@ __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const T *__restrict__
 
 static int grid_for(b200_engine *e, long long work) {
   return (int)std::max<long long>(1, std::min<long long>((work + 255) / 256, (long long)e->sm_count * 16));
+}
+
+// Groups of samples a channel's sums are cut into: about eight blocks per SM over all channels.
+static int bn_groups(const b200_engine *e, long long B, int channels) {
+  return (int)std::max<long long>(1, std::min<long long>({(8LL * e->sm_count + channels - 1) / channels, B, BN_GROUPS}));
 }
 
 template <typename T>
@@ -1009,18 +1079,23 @@ static int batchnorm_fwd_t(b200_engine *e, const T *x, T *y, long long B, int C,
     b200_put(e, ab, 0);
     return r;
   };
+  cudaError_t le = cudaSuccess;
   if (training) {
-    bn_partial_kernel<T><<<dim3(C, BN_GROUPS), 256, 0, e->stream>>>(x, B, C, S, (double *)part);
-    cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_partial_kernel: %s", cudaGetErrorString(le)));
+    for (int c0 = 0; c0 < C && le == cudaSuccess; c0 += b200_engine::kSkCounters) {
+      const int nc = std::min(C - c0, (int)b200_engine::kSkCounters);
+      bn_sums_kernel<T><<<dim3(nc, bn_groups(e, B, nc)), 256, 0, e->stream>>>(
+          c0, x, B, C, S, (double *)part, e->sk_counters, (T)momentum, (T)eps, running_mean, running_var, save_mean,
+          save_var, (T *)ab);
+      le = cudaGetLastError();
+      e->launches++;
+    }
+    if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_sums_kernel: %s", cudaGetErrorString(le)));
+  } else {
+    bn_inference_kernel<T><<<(C + 127) / 128, 128, 0, e->stream>>>(C, (T)eps, running_mean, running_var, (T *)ab);
+    le = cudaGetLastError();
+    if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_inference_kernel: %s", cudaGetErrorString(le)));
     e->launches++;
   }
-  bn_finish_kernel<T><<<(C + 127) / 128, 128, 0, e->stream>>>((const double *)part, C, B * S, training, (T)momentum,
-                                                              (T)eps, running_mean, running_var, save_mean, save_var,
-                                                              (T *)ab);
-  cudaError_t le = cudaGetLastError();
-  if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_finish_kernel: %s", cudaGetErrorString(le)));
-  e->launches++;
   const long long planes = B * C;
   const bool vec4 = S % 4 == 0 && ((uintptr_t)x | (uintptr_t)y) % 16 == 0;
   if (S >= 2048) {
@@ -1051,18 +1126,19 @@ static int batchnorm_bwd_t(b200_engine *e, const T *x, const T *dy, T *dx, long 
     b200_put(e, coef, 0);
     return r;
   };
-  bn_bwd_partial_kernel<T><<<dim3(C, BN_GROUPS), 256, 0, e->stream>>>(x, dy, B, C, S, (double *)part);
-  cudaError_t le = cudaGetLastError();
-  if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_bwd_partial_kernel: %s", cudaGetErrorString(le)));
-  e->launches++;
-  bn_bwd_finish_kernel<T><<<(C + 127) / 128, 128, 0, e->stream>>>((const double *)part, C, B * S, S, training, (T)eps,
-                                                                  running_var, save_mean, save_var, (T *)coef);
-  le = cudaGetLastError();
-  if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_bwd_finish_kernel: %s", cudaGetErrorString(le)));
-  e->launches++;
+  cudaError_t le = cudaSuccess;
+  for (int c0 = 0; c0 < C && le == cudaSuccess; c0 += b200_engine::kSkCounters) {
+    const int nc = std::min(C - c0, (int)b200_engine::kSkCounters);
+    bn_bwd_sums_kernel<T><<<dim3(nc, bn_groups(e, B, nc)), 256, 0, e->stream>>>(
+        c0, x, dy, B, C, S, (double *)part, e->sk_counters, training, (T)eps, running_var, save_mean, save_var, (T *)coef);
+    le = cudaGetLastError();
+    e->launches++;
+  }
+  if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_bwd_sums_kernel: %s", cudaGetErrorString(le)));
   const long long planes = B * C;
   const int blocks = (int)std::max<long long>(1, std::min<long long>((planes + 7) / 8, (long long)e->sm_count * 16));
-  bn_bwd_apply_kernel<T><<<blocks, 256, 0, e->stream>>>(x, dy, dx, planes, C, S, training, (const T *)coef);
+  const bool vec4 = S % 4 == 0 && ((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) % 16 == 0;
+  bn_bwd_apply_kernel<T><<<blocks, 256, 0, e->stream>>>(x, dy, dx, planes, C, S, training, (const T *)coef, vec4);
   le = cudaGetLastError();
   if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_bwd_apply_kernel: %s", cudaGetErrorString(le)));
   e->launches++;
@@ -1227,12 +1303,14 @@ int b200_maxpool2d_bwd(b200_engine *e, int dtype, const void *dy, const int64_t 
   const int ow0 = explicit_padding ? pad_east : pad_west;
   const long long total = B * C * H * W;
   if (dtype == B200_F32 && kh == 2 && kw == 2 && stride_h == 2 && stride_w == 2 && pad_north == 0 && pad_south == 0 &&
-      pad_west == 0 && pad_east == 0 && W % 4 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)dy % 8 == 0 &&
-      (uintptr_t)mask % 16 == 0) {
-    const long long work = B * C * ((H + 1) / 2) * (Wo / 2);
-    maxpool2x2_bwd_kernel<<<grid_for(e, work), 256, 0, e->stream>>>((const float *)dy, (const long long *)mask,
-                                                                   (float *)dx, B * C, (int)H, (int)W, (int)Ho,
-                                                                   (int)Wo);
+      pad_west == 0 && pad_east == 0 && W % 2 == 0 && (uintptr_t)dx % 8 == 0) {
+    const long long lines = B * C * ((H + 1) / 2);
+    if (W % 4 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)dy % 8 == 0 && (uintptr_t)mask % 16 == 0)
+      maxpool2x2_bwd_kernel<2><<<grid_for(e, lines * (Wo / 2)), 256, 0, e->stream>>>(
+          (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo);
+    else
+      maxpool2x2_bwd_kernel<1><<<grid_for(e, lines * Wo), 256, 0, e->stream>>>(
+          (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo);
     B200_CHECK_LAUNCH(e, "maxpool2x2_bwd_kernel");
     return B200_OK;
   }
@@ -1377,15 +1455,17 @@ int b200_im2col(b200_engine *e, int dtype, const void *x, void *col, int64_t B, 
   int rc = flush_pending(e);
   if (rc != B200_OK) return rc;
   const int crs = (int)(C * kh * kw);
-  const long long total = B * Ho * Wo * crs;
+  // image rows per block: enough (row, 32 entries) pieces to keep its eight warps evenly busy
+  const int rows = std::max(1, 32 / ((crs + 31) / 32));
+  const int blocks = (int)std::min<long long>((B * Ho + rows - 1) / rows, 1LL << 30);
   if (dtype == B200_F32)
-    im2col_kernel<float, false><<<grid_for(e, total), 256, 0, e->stream>>>(
-        (const float *)x, (float *)col, nullptr, B, (int)C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w,
-        stride_h, stride_w, dil_h, dil_w, crs);
+    im2col_kernel<float><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)col, B * Ho, (int)C, (int)H, (int)W,
+                                                       (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h, stride_w,
+                                                       dil_h, dil_w, rows);
   else
-    im2col_kernel<double, false><<<grid_for(e, total), 256, 0, e->stream>>>(
-        (const double *)x, (double *)col, nullptr, B, (int)C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w,
-        stride_h, stride_w, dil_h, dil_w, crs);
+    im2col_kernel<double><<<blocks, 256, 0, e->stream>>>((const double *)x, (double *)col, B * Ho, (int)C, (int)H,
+                                                        (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h,
+                                                        stride_w, dil_h, dil_w, rows);
   B200_CHECK_LAUNCH(e, "im2col_kernel");
   return B200_OK;
 }
