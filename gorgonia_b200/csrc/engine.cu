@@ -164,6 +164,7 @@ int b200_engine_create(int device, size_t arena_bytes, unsigned flags, b200_engi
     if (e->slab) cudaFree(e->slab);
     if (e->d_flags) cudaFree(e->d_flags);
     if (e->sk_counters) cudaFree(e->sk_counters);
+    if (e->f16_recs) cudaFree(e->f16_recs);
     if (e->h_flags) cudaFreeHost(e->h_flags);
     if (e->upload_done) cudaEventDestroy(e->upload_done);
     if (e->compute_mark) cudaEventDestroy(e->compute_mark);
@@ -206,6 +207,8 @@ int b200_engine_create(int device, size_t arena_bytes, unsigned flags, b200_engi
     return fail("cudaMalloc(counters)", err);
   if ((err = cudaMemset(e->sk_counters, 0, b200_engine::kSkCounters * sizeof(int))) != cudaSuccess)
     return fail("cudaMemset", err);
+  if ((err = cudaMalloc((void **)&e->f16_recs, 256)) != cudaSuccess) return fail("cudaMalloc(records)", err);
+  if ((err = cudaMemset(e->f16_recs, 0, 256)) != cudaSuccess) return fail("cudaMemset", err);
   if ((err = cudaHostAlloc((void **)&e->h_flags, 16 * sizeof(int), cudaHostAllocDefault)) != cudaSuccess)
     return fail("cudaHostAlloc", err);
   memset(e->h_flags, 0, 16 * sizeof(int));
@@ -225,6 +228,7 @@ int b200_engine_destroy(b200_engine *e) {
     if (e->slab) cudaFree(e->slab);
     if (e->d_flags) cudaFree(e->d_flags);
     if (e->sk_counters) cudaFree(e->sk_counters);
+    if (e->f16_recs) cudaFree(e->f16_recs);
     if (e->reduce_scratch) cudaFree(e->reduce_scratch);
     if (e->h_flags) cudaFreeHost(e->h_flags);
     cudaStreamSynchronize(e->copy_stream);

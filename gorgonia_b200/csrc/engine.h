@@ -15,8 +15,10 @@
 #include "bfc.h"
 
 namespace b200 {
+struct F16Rec;
 // A derived form of a constant buffer (weights) kept for reuse: the TF32 head/tail split of a
-// matrix (kind 0) or of convolution filters permuted to (tap, channel) order (kind 1).
+// matrix (kind 0) or of convolution filters permuted to (tap, channel) order (kind 1), or a matrix as pairs
+// of fp16 behind a 256-byte block that begins with its F16Rec (kind 2).
 struct CachedSplit {
   int kind;
   long long d0, d1, d2, ld_in;  // the shape it was made for
@@ -61,6 +63,9 @@ struct b200_engine {
   // tile). Zero between launches: the CTA that completes a tile puts its counter back to zero.
   int *sk_counters = nullptr;
   static constexpr int kSkCounters = 1 << 16;
+  // Records of the operands that a float32 product splits into pairs of fp16 (split.h): two for the
+  // operands, zero between products, and a word that says whether the product has to be made over.
+  b200::F16Rec *f16_recs = nullptr;
 
   // lazily created resources of other translation units (gemm.cu etc.)
   void *gemm_state = nullptr;

@@ -19,10 +19,15 @@
 // transposed storages swap that. All four combinations run without a transposing pass: only the
 // TMA box shape and two fields of the shared-memory descriptor differ.
 //
-// float32 runs as 3xTF32: each operand is split once into a TF32 head and a TF32 tail
-// (x = hi + lo up to 2^-22 relative), and three products hi*lo, lo*hi, hi*hi are accumulated in
-// fp32 into the same accumulator, smallest terms first. The split is one streaming pass into
-// arena scratch; the main loop then loads four tiles per stage and issues three MMAs per slice.
+// float32 runs on pairs of narrower values (split.cu): each operand is split once into heads and tails
+// (x = hi + lo up to 2^-22 relative), and the products hi*hi, hi*lo and lo*hi are accumulated in fp32. The
+// split is a streaming pass into arena scratch; the main loop then loads four tiles per stage. Two kinds:
+//   TF32 (TERMS 3): any float32 values; 32 k per 128-byte row.
+//   fp16 (TERMS 2): 64 k per 128-byte row and twice the tensor rate, so half the shared-memory traffic and
+//     half the tensor time for a product, with the same 11 + 11 significant bits, for operands whose values
+//     lie within 2^-29 of their largest (nearly all of them: F16Rec). Operands that do not are found on the
+//     device; the kernel then returns at once and the TF32 launch behind it makes the product.
+//     4096^3: 591 -> 317 us alone, 642 -> 400 with all passes; 8192^3 5106 -> 2870 with all passes.
 //
 // CTA pairs (PAIR, bf16 only): large problems run as clusters of two CTAs on neighbouring SMs that
 // share one 256-row tile: each CTA loads its own 128 rows of A and only half of the tile's B rows,
@@ -51,6 +56,7 @@
 #include "engine.h"
 #include "epilogue.cuh"
 #include "ptx.cuh"
+#include "split.h"
 #include "tc_common.cuh"
 #include "tc_operand.h"
 
@@ -87,12 +93,19 @@ struct GemmTcParams {
   int *tile_count;              // parts delivered per tile; zero between launches
   int workers;                  // CTAs, or CTA pairs, that share the tiles out
   int sk_first, sk_workers;     // k ranges are shared from this tile on, among this many CTAs (TilePieces)
+  // fp16 pairs: what is known about the operands; the launch does nothing if either is unusable
+  const F16Rec *rec_a, *rec_b;
+  unsigned limit_a, limit_b;
+  // TF32 pairs behind a launch of fp16 pairs: nothing is done unless *redo; clears the records of the
+  // operands that were split for this product alone
+  const int *redo;
+  F16Rec *clear_a, *clear_b;
   Epilogue ep;
   int *err_flag;
 };
 
-// TERMS = 1: bf16 operands (kind::f16). TERMS = 3: fp32 as 3xTF32 (kind::tf32), tensor maps
-// 0/1 = head/tail of A, 2/3 = head/tail of B.
+// TERMS = 1: bf16 operands (kind::f16). TERMS = 3: fp32 as pairs of TF32 (kind::tf32), TERMS = 2: as pairs of
+// fp16 (kind::f16); tensor maps 0/1 = head/tail of A, 2/3 = head/tail of B.
 // PAIR: two CTAs per 256-row tile (see the file comment); then B's map has a box of BN / 2 rows.
 template <int TERMS, int BN, bool A_MN, bool B_MN, bool PAIR>
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -100,8 +113,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                    const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
                    const __grid_constant__ GemmTcParams p) {
   static_assert(!PAIR || TERMS == 1, "only bf16 tiles are shared by a pair of CTAs");
-  constexpr int ES = TERMS == 1 ? 2 : 4;           // operand element size
-  constexpr int BK = TC_ROW_BYTES / ES;            // k elements per stage: 64 bf16 / 32 fp32
+  constexpr int ES = TERMS == 3 ? 4 : 2;           // operand element size
+  constexpr int BK = TC_ROW_BYTES / ES;            // k elements per stage: 64 (16-bit values) / 32 (TF32)
   constexpr int UK = 32 / ES;                      // k elements per MMA: 16 / 8
   constexpr int NSPLIT = TERMS == 1 ? 1 : 2;       // copies of each operand per stage (head, tail)
   constexpr int A_BYTES = TC_BM * TC_ROW_BYTES;    // 16 KB
@@ -111,14 +124,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   constexpr int STAGE_BYTES = !PAIR ? NSPLIT * (A_BYTES + B_BYTES) : A_BYTES + BH_BYTES;
   constexpr int MN_PER_BOX = TC_ROW_BYTES / ES;    // m/n elements covered by one MN-major box
   constexpr int MMA_M = PAIR ? 2 * TC_BM : TC_BM;
-  constexpr uint32_t IDESC = make_idesc(TERMS == 1 ? 1 : 2, A_MN, B_MN, MMA_M, BN);
-  // 3xTF32: B's head and tail slabs are adjacent in shared memory, and so are the main and the
+  constexpr int FMT = TERMS == 1 ? 1 : (TERMS == 2 ? 0 : 2);  // bf16, fp16, TF32
+  constexpr uint32_t IDESC = make_idesc(FMT, A_MN, B_MN, MMA_M, BN);
+  // pairs: B's head and tail slabs are adjacent in shared memory, and so are the main and the
   // cross-term accumulator in tensor memory, so A_head x [B_head | B_tail] is ONE instruction of
   // width 2*BN. An instruction costs a fixed ~65 cycles on top of its arithmetic: two per k step
   // beat three.
-  constexpr uint32_t IDESC_WIDE = make_idesc(2, A_MN, B_MN, MMA_M, TERMS == 1 ? BN : 2 * BN);
+  constexpr uint32_t IDESC_WIDE = make_idesc(FMT, A_MN, B_MN, MMA_M, TERMS == 1 ? BN : 2 * BN);
   constexpr int MAX_STAGES = 8;
-  // TMEM columns of one accumulator buffer: 3xTF32 keeps the cross terms in a second accumulator
+  // TMEM columns of one accumulator buffer: pairs keep the cross terms in a second accumulator
   constexpr int ACC_COLS = TERMS == 1 ? BN : 2 * BN;
   constexpr int TMEM_COLS = 2 * ACC_COLS;  // double-buffered; a power of two >= 32 for every BN used
 
@@ -128,6 +142,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_fail, s_last;
 
+  // which of the two float32 launches makes the product (the same answer in every thread of the grid)
+  if (TERMS == 2 && (f16_unusable(p.rec_a, p.limit_a) || f16_unusable(p.rec_b, p.limit_b))) return;
+  if (TERMS == 3 && p.redo) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (p.clear_a) *p.clear_a = F16Rec{0, 0, 0, 0};
+      if (p.clear_b) *p.clear_b = F16Rec{0, 0, 0, 0};
+    }
+    if (*(volatile const int *)p.redo == 0) return;
+  }
   // the ring must start on a 1024-byte boundary for the 128-byte swizzle
   unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -163,7 +186,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (warp == 0 && lane == 0) {
     ptx::prefetch_tmap(&tmA0);
     ptx::prefetch_tmap(&tmB0);
-    if (TERMS == 3) {
+    if (TERMS != 1) {
       ptx::prefetch_tmap(&tmA1);
       ptx::prefetch_tmap(&tmB1);
     }
@@ -301,7 +324,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           }
           ptx::tc_fence_after_sync();
           const uint32_t d_main = tmem_base + (uint32_t)(buf * ACC_COLS);
-          const uint32_t d_tail = d_main + BN;  // 3xTF32 only: the small cross terms
+          const uint32_t d_tail = d_main + BN;  // pairs only: the small cross terms
           const int kend = kc + p.chunk_k < kb1 ? kc + p.chunk_k : kb1;
           for (int kb = kc; kb < kend; ++kb) {
             if (!ready && !ptx::mbar_wait(&full_bar[stage], phase)) {
@@ -319,9 +342,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
               ready = ptx::kblock_f16<PAIR, A_STEP, B_STEP>(d_main, a_desc0[0] + soff, b_desc0[0] + soff, IDESC, first, eb,
                                                             ebp, nf, nphase);
             else  // hi * [hi | lo] into d_main (width 2 BN), lo * hi into d_tail
-              ready = ptx::kblock_tf32x3<false, A_STEP, B_STEP>(d_main, d_tail, a_desc0[0] + soff, a_desc0[NSPLIT - 1] + soff,
-                                                                b_desc0[0] + soff, b_desc0[0] + soff, IDESC_WIDE, IDESC, first,
-                                                                eb, ebp, nf, nphase);
+              ready = ptx::kblock_x3<TERMS == 2, A_STEP, B_STEP>(d_main, d_tail, a_desc0[0] + soff,
+                                                                 a_desc0[NSPLIT - 1] + soff, b_desc0[0] + soff,
+                                                                 b_desc0[0] + soff, IDESC_WIDE, IDESC, first, eb, nf,
+                                                                 nphase);
             stage = ns;
             phase = nphase;
           }
@@ -343,6 +367,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const int quarter = warp & 3;        // the TMEM lanes this warp may read: 32*quarter .. +31
     const int half = (warp - 2) >> 2;    // which half of the tile's columns it takes
     const int ch0 = half * HALF;
+    float unscale1 = 1.f, unscale2 = 1.f;  // fp16 pairs: the operands were scaled by powers of two
+    if (TERMS == 2) f16_unscale(p.rec_a->scale_exp, p.rec_b->scale_exp, unscale1, unscale2);
     int use = 0;
     uint32_t epi_phase = 0;
     bool ok = true;
@@ -447,13 +473,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           else ptx::mbar_arrive(&acc_empty[buf]);
         }
       } else {
-        // 3xTF32: the tensor core adds into its accumulator with truncation, a bias that grows
+        // pairs: the tensor core adds into its accumulator with truncation, a bias that grows
         // with the length of the accumulation chain. Chains are therefore cut into k-chunks; each
         // chunk's two accumulators (main and cross terms) are folded here into fp32 registers
         // with round-to-nearest adds while the next chunk is being multiplied.
-        float acc[TERMS == 3 ? HALF : 1];
+        float acc[TERMS != 1 ? HALF : 1];
 #pragma unroll
-        for (int j = 0; j < (TERMS == 3 ? HALF : 1); ++j) acc[j] = 0.f;
+        for (int j = 0; j < (TERMS != 1 ? HALF : 1); ++j) acc[j] = 0.f;
         for (int kc = kb0; kc < kb1 && ok; kc += p.chunk_k) {
           const int buf = use & 1;
           const uint32_t acc_phase = (uint32_t)((use >> 1) & 1);
@@ -464,14 +490,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           }
           ptx::tc_fence_after_sync();
 #pragma unroll
-          for (int c = 0; c < (TERMS == 3 ? HALF : 0); c += 16) {
+          for (int c = 0; c < (TERMS != 1 ? HALF : 0); c += 16) {
             uint32_t rm[16], rt[16];
             ptx::tmem_ld_32x16(lane_addr + (uint32_t)(buf * ACC_COLS + ch0 + c), rm);
             ptx::tmem_ld_32x16(lane_addr + (uint32_t)(buf * ACC_COLS + BN + ch0 + c), rt);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j)
-              acc[c + j] = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(rm[j]), __uint_as_float(rt[j])));
+              // the tails of fp16 pairs carry a factor of 2^11
+              acc[c + j] = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(rm[j]),
+                                                           TERMS == 2 ? __fmul_rn(__uint_as_float(rt[j]), 4.8828125e-4f)
+                                                                      : __uint_as_float(rt[j])));
           }
           ptx::tc_fence_before_sync();
           __syncwarp();
@@ -482,7 +511,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
         if (kb0 != 0 || kb1 != p.num_k) {
           // part of a tile: leave it in the workspace; the CTA that delivers the last part finishes the tile
-          constexpr int NACC = TERMS == 3 ? HALF : 1;
+          constexpr int NACC = TERMS != 1 ? HALF : 1;
           const int tile_u0 = (tile - p.sk_first) * p.num_k;  // among the units that are shared out
           const size_t slot_floats = (size_t)TC_BM * BN;
           const size_t within = ((size_t)(warp - 2) * HALF) * 32 + lane;
@@ -518,10 +547,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
         if (ok) {
 #pragma unroll
-          for (int c = 0; c < (TERMS == 3 ? HALF : 0); c += 32) {
+          for (int c = 0; c < (TERMS != 1 ? HALF : 0); c += 32) {
             float v[32];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = acc[c + j];
+            for (int j = 0; j < 32; ++j) v[j] = TERMS == 2 ? __fmul_rn(__fmul_rn(acc[c + j], unscale1), unscale2) : acc[c + j];
             store32(v, c);
           }
         }
@@ -598,59 +627,6 @@ __global__ void __launch_bounds__(128, 1) tf32_peak_kernel(int batches, int *err
   if (warp == 0) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, 512);
-  }
-}
-
-// ------------------------------------------------------------------------------------------
-// TF32 split: x -> (head, tail), both TF32 values in fp32 containers, written densely with the
-// row length padded to a multiple of 4 elements (so that TMA row pitches stay 16-byte multiples)
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ float to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
-}
-
-__global__ void __launch_bounds__(256) split_tf32_kernel(const float *__restrict__ src, long long ld_in,
-                                                         long long stride_in, float *__restrict__ hi,
-                                                         float *__restrict__ lo, long long rows, long long cols,
-                                                         long long ld_out, long long batch) {
-  const long long per = rows * ld_out;
-  const long long total = per * batch;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const long long b = t / per, rem = t % per;
-    const long long r = rem / ld_out, c = rem % ld_out;
-    float x = 0.f;
-    if (c < cols) x = src[b * stride_in + r * ld_in + c];
-    const float h = to_tf32(x);
-    hi[t] = h;
-    lo[t] = to_tf32(__fsub_rn(x, h));
-  }
-}
-
-// The same for rows that can be read 16 bytes at a time (pitch and width multiples of 4, aligned
-// base): a block walks whole rows, a thread takes four elements per step, and nothing is divided
-// per element.
-__global__ void __launch_bounds__(256) split_tf32_rows4_kernel(const float *__restrict__ src, long long ld_in,
-                                                               long long stride_in, float *__restrict__ hi,
-                                                               float *__restrict__ lo, long long rows, int cols4,
-                                                               long long batch) {
-  const long long total_rows = rows * batch;
-  for (long long row = blockIdx.x; row < total_rows; row += gridDim.x) {
-    const long long b = row / rows, r = row - b * rows;
-    const float4 *in = reinterpret_cast<const float4 *>(src + b * stride_in + r * ld_in);
-    float4 *oh = reinterpret_cast<float4 *>(hi) + row * cols4;
-    float4 *ol = reinterpret_cast<float4 *>(lo) + row * cols4;
-    for (int c = threadIdx.x; c < cols4; c += blockDim.x) {
-      const float4 v = __ldg(in + c);
-      float4 h, l;
-      h.x = to_tf32(v.x); h.y = to_tf32(v.y); h.z = to_tf32(v.z); h.w = to_tf32(v.w);
-      l.x = to_tf32(__fsub_rn(v.x, h.x)); l.y = to_tf32(__fsub_rn(v.y, h.y));
-      l.z = to_tf32(__fsub_rn(v.z, h.z)); l.w = to_tf32(__fsub_rn(v.w, h.w));
-      oh[c] = h;
-      ol[c] = l;
-    }
   }
 }
 
@@ -784,16 +760,25 @@ static int launch_tc_layout(b200_engine *e, bool a_mn, bool b_mn, const CUtensor
 }
 
 
-// terms = 1 (bf16) or 3 (fp32 split into head/tail). a_mn / b_mn: the operand is stored with its
-// m / n index contiguous (see the file comment).
+// Which of a float32 product's two launches this is, and what decides on the device whether it runs.
+struct F16Gate {
+  const F16Rec *rec_a = nullptr, *rec_b = nullptr;
+  unsigned limit_a = 0, limit_b = 0;
+  const int *redo = nullptr;
+  F16Rec *clear_a = nullptr, *clear_b = nullptr;
+};
+
+// terms = 1 (bf16), 2 or 3 (fp32 split into head/tail, fp16 or TF32). a_mn / b_mn: the operand is stored
+// with its m / n index contiguous (see the file comment).
 int gemm_tc_core(b200_engine *e, int terms, bool a_mn, bool b_mn, long long M, long long N, long long K,
                  const TcOperand &a, const TcOperand &b, void *C, long long ldc, long long batch, long long strideC,
-                 const Epilogue &ep, float *C_hi = nullptr, float *C_lo = nullptr, long long ld_split = 0) {
-  const int es = terms == 1 ? 2 : 4;
+                 const Epilogue &ep, float *C_hi = nullptr, float *C_lo = nullptr, long long ld_split = 0,
+                 const F16Gate &gate = F16Gate()) {
+  const int es = terms == 3 ? 4 : 2;
   const int bk = TC_ROW_BYTES / es;
   // tile width: the widest that still gives every SM a tile, to keep small problems spread out
   const int tiles_m = (int)((M + TC_BM - 1) / TC_BM);
-  const bool may_share_k = terms == 3 && !(e->flags & B200_ENGINE_NO_STREAMK);
+  const bool may_share_k = terms != 1 && !(e->flags & B200_ENGINE_NO_STREAMK);
   int bn = terms == 1 ? 256 : 128;
   // tile width: the widest that still gives every SM a tile. A problem too small for that gets the
   // narrow tiles whether or not its k range is shared out as well: one SM pulls operands from L2 at a
@@ -846,9 +831,18 @@ int gemm_tc_core(b200_engine *e, int terms, bool a_mn, bool b_mn, long long M, l
   p.tiles_m = tiles_m;
   p.tiles_n = tiles_n;
   p.num_k = (int)((K + bk - 1) / bk);
-  // bf16: one chain per tile. 3xTF32: 8 k-blocks = 256 k = 32 accumulation steps per chain, which
-  // keeps the truncation bias of the tensor core's adder near 5e-7 relative.
-  p.chunk_k = terms == 1 ? p.num_k : 8;
+  // bf16: one chain per tile. TF32 pairs: 8 k-blocks = 256 k = 32 accumulation steps per chain, which keeps
+  // the truncation bias of the tensor core's adder near 5e-7 relative (4096^3: 6.4e-7 of the result's norm in
+  // all). fp16 pairs: 6 k-blocks = 384 k = 24 steps: 5.0e-7 at 401 us; 8 blocks 6.5e-7 at 396, 4 blocks
+  // 3.6e-7 at 413.
+  p.chunk_k = terms == 1 ? p.num_k : (terms == 2 ? 6 : 8);
+  p.rec_a = gate.rec_a;
+  p.rec_b = gate.rec_b;
+  p.limit_a = gate.limit_a;
+  p.limit_b = gate.limit_b;
+  p.redo = gate.redo;
+  p.clear_a = gate.clear_a;
+  p.clear_b = gate.clear_b;
   p.group_m = std::min(tiles_m, 8);
   p.c_vec = (C && ldc % 4 == 0 && (uintptr_t)C % 16 == 0 && (batch == 1 || strideC % 4 == 0)) ? 1 : 0;
   p.a_zmul = a.shared ? 0 : 1;
@@ -907,30 +901,37 @@ int gemm_tc_core(b200_engine *e, int terms, bool a_mn, bool b_mn, long long M, l
       p.ws = (float *)ws;
     }
   }
-  const int rc = bn == 128 ? launch_tc_layout<3, 128>(e, a_mn, b_mn, tm, p, grid)
-                           : launch_tc_layout<3, 64>(e, a_mn, b_mn, tm, p, grid);
+  int rc;
+  if (terms == 2)
+    rc = bn == 128 ? launch_tc_layout<2, 128>(e, a_mn, b_mn, tm, p, grid)
+                   : launch_tc_layout<2, 64>(e, a_mn, b_mn, tm, p, grid);
+  else
+    rc = bn == 128 ? launch_tc_layout<3, 128>(e, a_mn, b_mn, tm, p, grid)
+                   : launch_tc_layout<3, 64>(e, a_mn, b_mn, tm, p, grid);
   if (ws) b200_put(e, ws, 0);  // stream order: whoever gets the block next runs after this kernel
   return rc;
 }
 
-// Splits a row-major fp32 matrix (rows x cols, pitch ld, `batch` of them) into TF32 head and tail
-// in arena scratch with a pitch that is a multiple of 4 elements. The caller hands the two
-// blocks back with b200_put once the consuming kernel has been launched.
-int split_operand_tf32(b200_engine *e, const float *src, long long rows, long long cols, long long ld,
-                       long long batch, long long batch_stride, TcOperand *out, void **blk_hi, void **blk_lo) {
+// Finds or makes room for the TF32 head and tail of a row-major fp32 matrix (rows x cols, pitch ld,
+// `batch` of them), with a pitch that is a multiple of 4 elements. What is left to do is put into *job
+// (job->src stays null if a constant's split was there already); blk_hi / blk_lo are the blocks that the
+// caller hands back with b200_put once the consuming kernel has been launched.
+static int plan_split_tf32(b200_engine *e, const float *src, long long rows, long long cols, long long ld,
+                           long long batch, long long batch_stride, TcOperand *out, SplitJob *job, void **blk_hi,
+                           void **blk_lo) {
   const long long ldo = (cols + 3) / 4 * 4;
   const long long elems = rows * ldo * batch;
   *blk_hi = *blk_lo = nullptr;
+  out->ld = ldo;
+  out->batch_stride = rows * ldo;
+  out->shared = false;
   // a buffer declared constant (weights) is split once; the split is kept until the buffer is
   // released or un-declared, and the caller gets no blocks to hand back
-  const bool constant = is_constant(e, src);
-  if (constant) {
+  if (is_constant(e, src)) {
     if (CachedSplit *c = find_cached(e, src, 0, rows, cols, batch, ld)) {
       out->p0 = c->hi;
       out->p1 = c->lo;
       out->ld = c->ld_out;
-      out->batch_stride = rows * c->ld_out;
-      out->shared = false;
       return B200_OK;
     }
   }
@@ -942,33 +943,192 @@ int split_operand_tf32(b200_engine *e, const float *src, long long rows, long lo
     *blk_hi = nullptr;
     return rc;
   }
-  if (cols % 4 == 0 && ld % 4 == 0 && batch_stride % 4 == 0 && (uintptr_t)src % 16 == 0 && cols >= 256) {
-    const int blocks = (int)std::max<long long>(1, std::min<long long>(rows * batch, e->sm_count * 16LL));
-    split_tf32_rows4_kernel<<<blocks, 256, 0, e->stream>>>(src, ld, batch_stride, (float *)*blk_hi, (float *)*blk_lo,
-                                                           rows, (int)(cols / 4), batch);
-  } else {
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((elems + 255) / 256, e->sm_count * 16LL));
-    split_tf32_kernel<<<blocks, 256, 0, e->stream>>>(src, ld, batch_stride, (float *)*blk_hi, (float *)*blk_lo, rows,
-                                                     cols, ldo, batch);
-  }
-  cudaError_t le = cudaGetLastError();
-  if (le != cudaSuccess) {
-    b200_put(e, *blk_hi, 0);
-    b200_put(e, *blk_lo, 0);
-    *blk_hi = *blk_lo = nullptr;
-    return set_error(e, B200_ERR_CUDA, "launch of split_tf32_kernel failed: %s", cudaGetErrorString(le));
-  }
-  e->launches++;
   out->p0 = *blk_hi;
   out->p1 = *blk_lo;
-  out->ld = ldo;
-  out->batch_stride = rows * ldo;
-  out->shared = false;
-  if (constant) {
-    add_cached(e, src, CachedSplit{0, rows, cols, batch, ld, *blk_hi, *blk_lo, ldo});
-    *blk_hi = *blk_lo = nullptr;  // kept: nothing for the caller to release
-  }
+  job->src = src;
+  job->ld = ld;
+  job->stride = batch_stride;
+  job->rows = rows;
+  job->cols = cols;
+  job->batch = batch;
+  job->hi = *blk_hi;
+  job->lo = *blk_lo;
+  job->ldo = ldo;
   return B200_OK;
+}
+// Once the split has been launched: a constant's is kept, and the blocks are no longer the caller's.
+static void keep_split_tf32(b200_engine *e, const SplitJob &job, void **blk_hi, void **blk_lo) {
+  if (!job.src || !is_constant(e, job.src)) return;
+  add_cached(e, job.src, CachedSplit{0, job.rows, job.cols, job.batch, job.ld, *blk_hi, *blk_lo, job.ldo});
+  *blk_hi = *blk_lo = nullptr;
+}
+
+// The TF32 split of one operand (conv_tc.cu).
+int split_operand_tf32(b200_engine *e, const float *src, long long rows, long long cols, long long ld,
+                       long long batch, long long batch_stride, TcOperand *out, void **blk_hi, void **blk_lo) {
+  SplitJob job;
+  int rc = plan_split_tf32(e, src, rows, cols, ld, batch, batch_stride, out, &job, blk_hi, blk_lo);
+  if (rc == B200_OK && job.src) rc = launch_split_tf32(e, job, SplitJob());
+  if (rc == B200_OK) {
+    keep_split_tf32(e, job, blk_hi, blk_lo);
+    return B200_OK;
+  }
+  for (void **b : {blk_hi, blk_lo})
+    if (*b) {
+      b200_put(e, *b, 0);
+      *b = nullptr;
+    }
+  return rc;
+}
+
+// One float32 operand of a product: A or B as it is stored.
+struct F32Operand {
+  const float *src;
+  long long rows, cols, ld, batch, stride;
+};
+
+// The product from TF32 pairs. a_given: A is already split (TcOperand filled in).
+static int gemm_f32_tf32(b200_engine *e, bool a_mn, bool b_mn, long long M, long long N, long long K,
+                         const F32Operand *A, const TcOperand *a_given, const F32Operand &B, void *C, long long ldc,
+                         long long batch, long long strideC, const Epilogue &ep, float *C_hi = nullptr,
+                         float *C_lo = nullptr, long long ld_split = 0) {
+  TcOperand a, b;
+  SplitJob ja, jb;
+  void *blk[4] = {nullptr, nullptr, nullptr, nullptr};
+  int rc = B200_OK;
+  if (a_given) a = *a_given;
+  else rc = plan_split_tf32(e, A->src, A->rows, A->cols, A->ld, A->batch, A->stride, &a, &ja, &blk[0], &blk[1]);
+  if (rc == B200_OK) rc = plan_split_tf32(e, B.src, B.rows, B.cols, B.ld, B.batch, B.stride, &b, &jb, &blk[2], &blk[3]);
+  // one launch for both, but a constant's split, which is made once, is a launch of its own
+  if (rc == B200_OK && B.src && is_constant(e, B.src)) {
+    rc = launch_split_tf32(e, ja, SplitJob());
+    if (rc == B200_OK) rc = launch_split_tf32(e, jb, SplitJob());
+  } else if (rc == B200_OK) {
+    rc = launch_split_tf32(e, ja, jb);
+  }
+  if (rc == B200_OK) {
+    keep_split_tf32(e, ja, &blk[0], &blk[1]);
+    // one matrix as both operands: only one of two equal entries is kept
+    if (!(jb.src && is_constant(e, jb.src) && find_cached(e, jb.src, 0, jb.rows, jb.cols, jb.batch, jb.ld)))
+      keep_split_tf32(e, jb, &blk[2], &blk[3]);
+    rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, a, b, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split);
+  }
+  // stream order makes handing the scratch back safe: later users run after this kernel
+  for (void *s2 : blk)
+    if (s2) b200_put(e, s2, 0);
+  return rc;
+}
+
+// Room for an operand's fp16 pairs (pitch a multiple of 8 values), or a constant's that are there already.
+// The blocks are as large as the TF32 pairs need, which take their place if the fp16 pairs turn out unusable.
+static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_rec, TcOperand *out, SplitJob *job,
+                          F16Rec **rec, void **blk) {
+  const long long ldo = (x.cols + 7) / 8 * 8, elems = x.rows * ldo * x.batch;
+  out->ld = ldo;
+  out->batch_stride = x.rows * ldo;
+  out->shared = false;
+  int rc = B200_OK;
+  const bool constant = is_constant(e, x.src);
+  if (constant) {
+    if (CachedSplit *c = find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld)) {
+      *rec = (F16Rec *)c->hi;
+      out->p0 = (char *)c->hi + 256;
+      out->p1 = c->lo;
+    } else {  // a record and the heads, the tails
+      void *hi = nullptr, *lo = nullptr;
+      rc = b200_get(e, 256 + elems * 2, &hi);
+      if (rc == B200_OK && (rc = b200_get(e, elems * 2, &lo)) != B200_OK) b200_put(e, hi, 0);
+      if (rc != B200_OK) return rc;
+      if (cudaMemsetAsync(hi, 0, sizeof(F16Rec), e->stream) != cudaSuccess) {
+        b200_put(e, hi, 0);
+        b200_put(e, lo, 0);
+        return set_error(e, B200_ERR_CUDA, "b200_gemm: clearing a record failed");
+      }
+      add_cached(e, x.src, CachedSplit{2, x.rows, x.cols, x.batch, x.ld, hi, lo, ldo});
+      *rec = (F16Rec *)hi;
+      out->p0 = (char *)hi + 256;
+      out->p1 = lo;
+      job->src = x.src;
+    }
+  } else {
+    *rec = scratch_rec;
+    job->src = x.src;
+  }
+  // the TF32 pairs' place; a temporary operand's fp16 pairs lie in the same blocks
+  for (int h = 0; h < 2 && rc == B200_OK; ++h) rc = b200_get(e, elems * 4, &blk[h]);
+  if (rc != B200_OK) return rc;
+  if (!constant) {
+    out->p0 = blk[0];
+    out->p1 = blk[1];
+  }
+  job->ld = x.ld;
+  job->stride = x.stride;
+  job->rows = x.rows;
+  job->cols = x.cols;
+  job->batch = x.batch;
+  job->hi = const_cast<void *>(out->p0);
+  job->lo = const_cast<void *>(out->p1);
+  job->ldo = ldo;
+  job->rec = *rec;
+  return B200_OK;
+}
+
+// Whether a product is worth fp16 pairs. They save about half of the 2 M N K / 200 TFLOP/s that TF32 pairs
+// take; finding the largest magnitudes reads both operands once more (5 TB/s), and the launches that find
+// nothing to do cost 8 us.
+static bool f16_pays(b200_engine *e, long long M, long long N, long long K, long long batch, const F32Operand &A,
+                     const F32Operand &B) {
+  const double saves = (double)M * N * K * batch / 200e12;
+  const double reads = ((is_constant(e, A.src) ? 0.0 : (double)M * K) + (is_constant(e, B.src) ? 0.0 : (double)N * K)) * 4.0 * batch / 5e12;
+  return saves > 1.3 * (reads + 8e-6);
+}
+
+// The product from fp16 pairs, with the TF32 launches behind it that run only if the pairs are unusable.
+static int gemm_f32_f16(b200_engine *e, bool a_mn, bool b_mn, long long M, long long N, long long K,
+                        const F32Operand &A, const F32Operand &B, void *C, long long ldc, long long batch,
+                        long long strideC, const Epilogue &ep, float *C_hi = nullptr, float *C_lo = nullptr,
+                        long long ld_split = 0) {
+  TcOperand a, b;
+  SplitJob ja, jb;
+  F16Rec *ra = nullptr, *rb = nullptr;
+  void *blk[4] = {nullptr, nullptr, nullptr, nullptr};
+  int rc = plan_split_f16(e, A, e->f16_recs, &a, &ja, &ra, &blk[0]);
+  if (rc == B200_OK) rc = plan_split_f16(e, B, e->f16_recs + 1, &b, &jb, &rb, &blk[2]);
+  const unsigned la = f16_small_limit(A.rows * A.cols * A.batch), lb = f16_small_limit(B.rows * B.cols * B.batch);
+  if (rc == B200_OK && ja.src) rc = launch_split_f16(e, ja, jb);
+  else if (rc == B200_OK && jb.src) rc = launch_split_f16(e, jb, SplitJob());
+  F16Gate gate;
+  gate.rec_a = ra;
+  gate.rec_b = rb;
+  gate.limit_a = la;
+  gate.limit_b = lb;
+  if (rc == B200_OK) rc = gemm_tc_core(e, 2, a_mn, b_mn, M, N, K, a, b, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split, gate);
+  if (rc == B200_OK) {
+    TcOperand ta, tb;
+    SplitJob *jobs[2] = {&ja, &jb};
+    TcOperand *ops[2] = {&ta, &tb};
+    const F32Operand *xs[2] = {&A, &B};
+    for (int i = 0; i < 2; ++i) {
+      jobs[i]->src = xs[i]->src;
+      jobs[i]->hi = blk[2 * i];
+      jobs[i]->lo = blk[2 * i + 1];
+      jobs[i]->ldo = (xs[i]->cols + 3) / 4 * 4;
+      ops[i]->p0 = blk[2 * i];
+      ops[i]->p1 = blk[2 * i + 1];
+      ops[i]->ld = jobs[i]->ldo;
+      ops[i]->batch_stride = xs[i]->rows * jobs[i]->ldo;
+    }
+    F16Gate redo;
+    redo.redo = (int *)(e->f16_recs + 2);
+    redo.clear_a = ra == e->f16_recs ? ra : nullptr;
+    redo.clear_b = rb == e->f16_recs + 1 ? rb : nullptr;
+    rc = launch_split_tf32_redo(e, ja, jb, ra, la, rb, lb, (int *)(e->f16_recs + 2));
+    if (rc == B200_OK) rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, ta, tb, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split,
+                                       redo);
+  }
+  for (void *s2 : blk)
+    if (s2) b200_put(e, s2, 0);
+  return rc;
 }
 
 static int gemm_tc(b200_engine *e, int dtype, int transA, int transB, long long M, long long N, long long K,
@@ -987,16 +1147,13 @@ static int gemm_tc(b200_engine *e, int dtype, int transA, int transB, long long 
     return gemm_tc_core(e, 1, a_mn, b_mn, M, N, K, a, b, C, ldc, batch, strideC, ep);
   }
   // stored shapes (rows x contiguous)
-  const long long a_rows = transA ? K : M, a_cols = transA ? M : K;
-  const long long b_rows = transB ? N : K, b_cols = transB ? K : N;
-  void *blk[4] = {nullptr, nullptr, nullptr, nullptr};
-  int rc = split_operand_tf32(e, (const float *)A, a_rows, a_cols, lda, batch, strideA, &a, &blk[0], &blk[1]);
-  if (rc == B200_OK) rc = split_operand_tf32(e, (const float *)B, b_rows, b_cols, ldb, batch, strideB, &b, &blk[2], &blk[3]);
-  if (rc == B200_OK) rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, a, b, C, ldc, batch, strideC, ep);
-  // stream order makes handing the scratch back safe: later users run after this kernel
-  for (void *s2 : blk)
-    if (s2) b200_put(e, s2, 0);
-  return rc;
+  const F32Operand fa{(const float *)A, transA ? K : M, transA ? M : K, lda, batch, strideA};
+  const F32Operand fb{(const float *)B, transB ? N : K, transB ? K : N, ldb, batch, strideB};
+  if (f16_pays(e, M, N, K, batch, fa, fb)) {
+    const int rc = gemm_f32_f16(e, a_mn, b_mn, M, N, K, fa, fb, C, ldc, batch, strideC, ep);
+    if (rc != B200_ERR_OOM) return rc;  // else: the TF32 pairs of constants may be there already
+  }
+  return gemm_f32_tf32(e, a_mn, b_mn, M, N, K, &fa, nullptr, fb, C, ldc, batch, strideC, ep);
 }
 
 }  // namespace b200
@@ -1034,24 +1191,20 @@ int b200_gemm_chain(b200_engine *e, int transB, int64_t M, int64_t N, int64_t K,
   const Epilogue ep = make_epilogue(epi);
   const void *probe = A ? A : A_hi;
   if (tc_eligible(B200_F32, M, N, K, lda, ldb, ldc, 1, 0, 0, probe, B, C ? C : C_hi)) {
-    TcOperand a, b;
-    void *blk[4] = {nullptr, nullptr, nullptr, nullptr};
-    if (A_hi) {
-      a.p0 = A_hi;
-      a.p1 = A_lo;
-      a.ld = lda;
-      a.batch_stride = M * lda;
-    } else {
-      rc = split_operand_tf32(e, (const float *)A, M, K, lda, 1, 0, &a, &blk[0], &blk[1]);
-    }
-    const long long b_rows = transB ? N : K, b_cols = transB ? K : N;
-    if (rc == B200_OK) rc = split_operand_tf32(e, (const float *)B, b_rows, b_cols, ldb, 1, 0, &b, &blk[2], &blk[3]);
-    if (rc == B200_OK)
-      rc = gemm_tc_core(e, 3, false, transB == 0, M, N, K, a, b, C, ldc, 1, M * ldc, ep, (float *)C_hi, (float *)C_lo,
+    const F32Operand fa{(const float *)A, M, K, lda, 1, 0};
+    const F32Operand fb{(const float *)B, transB ? N : K, transB ? K : N, ldb, 1, 0};
+    TcOperand given;
+    given.p0 = A_hi;
+    given.p1 = A_lo;
+    given.ld = lda;
+    given.batch_stride = M * lda;
+    if (!A_hi && f16_pays(e, M, N, K, 1, fa, fb)) {
+      rc = gemm_f32_f16(e, false, transB == 0, M, N, K, fa, fb, C, ldc, 1, M * ldc, ep, (float *)C_hi, (float *)C_lo,
                         ld_split);
-    for (void *s2 : blk)
-      if (s2) b200_put(e, s2, 0);
-    return rc;
+      if (rc != B200_ERR_OOM) return rc;
+    }
+    return gemm_f32_tf32(e, false, transB == 0, M, N, K, &fa, A_hi ? &given : nullptr, fb, C, ldc, 1, M * ldc, ep,
+                         (float *)C_hi, (float *)C_lo, ld_split);
   }
   // small or oddly shaped: the plain product, then the rewrite pass; both need the tensors unsplit
   if (!A)
@@ -1068,12 +1221,16 @@ int b200_gemm_chain(b200_engine *e, int transB, int64_t M, int64_t N, int64_t K,
   }
   rc = gemm_simt(e, B200_F32, 0, transB, M, N, K, A, lda, B, ldb, cf, ldc_eff, 1, 0, 0, 0, ep);
   if (rc == B200_OK && C_hi) {
-    const long long elems = M * ld_split;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((elems + 255) / 256, e->sm_count * 16LL));
-    split_tf32_kernel<<<blocks, 256, 0, e->stream>>>(cf, ldc_eff, 0, (float *)C_hi, (float *)C_lo, M, N, ld_split, 1);
-    cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) rc = set_error(e, B200_ERR_CUDA, "launch of split_tf32_kernel failed: %s", cudaGetErrorString(le));
-    else e->launches++;
+    SplitJob job;
+    job.src = cf;
+    job.ld = ldc_eff;
+    job.rows = M;
+    job.cols = N;
+    job.batch = 1;
+    job.hi = C_hi;
+    job.lo = C_lo;
+    job.ldo = ld_split;
+    rc = launch_split_tf32(e, job, SplitJob());
   }
   if (tmp) b200_put(e, tmp, 0);
   return rc;

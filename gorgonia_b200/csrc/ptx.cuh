@@ -354,48 +354,48 @@ __device__ __forceinline__ uint32_t kblock_f16(uint32_t d, uint64_t a, uint64_t 
   return ready;
 }
 
-// 3xTF32: per k-slice a_head x b_wide (width 2 BN, into d_main) and a_tail x b_narrow (width BN,
-// into d_tail, always accumulating).
-template <bool PAIR, int SA, int SB>
-__device__ __forceinline__ uint32_t kblock_tf32x3(uint32_t d_main, uint32_t d_tail, uint64_t a_head, uint64_t a_tail,
+// Pairs of TF32 (F16: of fp16) values: per k-slice a_head x b_wide (width 2 BN, into d_main) and
+// a_tail x b_narrow (width BN, into d_tail, always accumulating).
+template <bool F16, int SA, int SB>
+__device__ __forceinline__ uint32_t kblock_x3(uint32_t d_main, uint32_t d_tail, uint64_t a_head, uint64_t a_tail,
                                                   uint64_t b_wide, uint64_t b_narrow, uint32_t idesc_wide,
                                                   uint32_t idesc, uint32_t acc_first, uint32_t empty_bar,
-                                                  uint32_t empty_peer, uint32_t next_full, uint32_t next_parity) {
+                                                  uint32_t next_full, uint32_t next_parity) {
   uint32_t ready;
-#define B200_KB_STEP(CG)                                                       \
-  "add.s64 ah, ah, %14;\n\t"                                                   \
-  "add.s64 al, al, %14;\n\t"                                                   \
-  "add.s64 bw, bw, %15;\n\t"                                                   \
-  "add.s64 bn, bn, %15;\n\t"                                                   \
-  "tcgen05.mma.cta_group::" CG ".kind::tf32 [%1], ah, bw, %7, p1;\n\t"         \
-  "tcgen05.mma.cta_group::" CG ".kind::tf32 [%2], al, bn, %8, p1;\n\t"
-#define B200_KB_TF32(CG, SECOND_COMMIT)                                                                  \
+#define B200_KB_STEP(KIND)                                                     \
+  "add.s64 ah, ah, %13;\n\t"                                                   \
+  "add.s64 al, al, %13;\n\t"                                                   \
+  "add.s64 bw, bw, %14;\n\t"                                                   \
+  "add.s64 bn, bn, %14;\n\t"                                                   \
+  "tcgen05.mma.cta_group::1.kind::" KIND " [%1], ah, bw, %7, p1;\n\t"         \
+  "tcgen05.mma.cta_group::1.kind::" KIND " [%2], al, bn, %8, p1;\n\t"
+#define B200_KB_X3(KIND)                                                                  \
   asm volatile(                                                                                        \
       "{\n\t"                                                                                          \
       ".reg .pred pn, pa, p1;\n\t"                                                                     \
       ".reg .b64 ah, al, bw, bn;\n\t"                                                                  \
       "setp.ne.b32 pa, %9, 0;\n\t"                                                                     \
       "setp.eq.b32 p1, %9, %9;\n\t"                                                                    \
-      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%12], %13;\n\t"                                  \
-      "tcgen05.mma.cta_group::" CG ".kind::tf32 [%1], %3, %5, %7, pa;\n\t"                             \
-      "tcgen05.mma.cta_group::" CG ".kind::tf32 [%2], %4, %6, %8, p1;\n\t"                             \
+      "mbarrier.test_wait.parity.shared::cta.b64 pn, [%11], %12;\n\t"                                  \
+      "tcgen05.mma.cta_group::1.kind::" KIND " [%1], %3, %5, %7, pa;\n\t"                             \
+      "tcgen05.mma.cta_group::1.kind::" KIND " [%2], %4, %6, %8, p1;\n\t"                             \
       "mov.b64 ah, %3;\n\t"                                                                            \
       "mov.b64 al, %4;\n\t"                                                                            \
       "mov.b64 bw, %5;\n\t"                                                                            \
-      "mov.b64 bn, %6;\n\t" B200_KB_STEP(CG) B200_KB_STEP(CG) B200_KB_STEP(CG)                         \
-      "tcgen05.commit.cta_group::" CG ".mbarrier::arrive::one.shared::cluster.b64 [%10];\n\t" SECOND_COMMIT \
+      "mov.b64 bn, %6;\n\t" B200_KB_STEP(KIND) B200_KB_STEP(KIND) B200_KB_STEP(KIND)                         \
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%10];\n\t" \
       "selp.u32 %0, 1, 0, pn;\n\t"                                                                     \
       "}"                                                                                              \
       : "=r"(ready)                                                                                    \
       : "r"(d_main), "r"(d_tail), "l"(a_head), "l"(a_tail), "l"(b_wide), "l"(b_narrow), "r"(idesc_wide),      \
-        "r"(idesc), "r"(acc_first), "r"(empty_bar), "r"(empty_peer), "r"(next_full), "r"(next_parity),       \
+        "r"(idesc), "r"(acc_first), "r"(empty_bar), "r"(next_full), "r"(next_parity),       \
         "n"(SA), "n"(SB)                                                                               \
       : "memory")
-  if (PAIR)
-    B200_KB_TF32("2", "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t");
+  if (F16)
+    B200_KB_X3("f16");
   else
-    B200_KB_TF32("1", "");
-#undef B200_KB_TF32
+    B200_KB_X3("tf32");
+#undef B200_KB_X3
 #undef B200_KB_STEP
   return ready;
 }

@@ -1,0 +1,173 @@
+// float32 operands as pairs of narrower values whose products the tensor cores add up in float32.
+//
+// TF32 pairs: x = head + tail, both TF32 (11 significant bits) in float32 containers, 8 bytes per value.
+//
+// fp16 pairs: the whole operand is scaled by the power of two that brings its largest magnitude into
+// [2^14, 2^15); then x * 2^e = head + tail * 2^-11 with head = fp16(x * 2^e) and tail = fp16 of the (exact)
+// remainder times 2^11. fp16 has the 11 significant bits of TF32, so the pair carries x as closely as the
+// TF32 pair does, in half the bytes and at twice the tensor-core rate. What fp16 lacks is range: a value
+// below 2^-14 after scaling (2^-29 of the largest) keeps an absolute error of 2^-36 instead of a relative
+// one. Such values are counted, and infinities and NaNs are noted, in the operand's F16Rec. A product whose
+// operands hold more than n / 65536 of them, or any infinity or NaN, is made from TF32 pairs instead: the
+// kernels of both ways are launched, and one of them returns at once (the host never waits to find out).
+// N(0, 1) draws hold about one such value in 10^8.
+//
+// All of these passes are bound by HBM: 4 bytes read and 4 (fp16) or 8 (TF32) written per value. A thread
+// takes eight (four) neighbouring columns, 16 bytes per store; both operands of a product share a launch.
+// The row-wise and element-wise kernels this replaces took a launch per operand, and 7 to 10 us for 2.5 MB
+// with a pitch that is no multiple of four, most of it 64-bit divisions.
+#include "split.h"
+
+#include <algorithm>
+
+#include "engine.h"
+
+namespace b200 {
+
+enum { SPLIT_AMAX, SPLIT_F16, SPLIT_TF32, SPLIT_TF32_REDO };
+
+struct SplitRedo {
+  const F16Rec *ra, *rb;
+  unsigned limit_a, limit_b;
+  int *redo;
+};
+
+__device__ __forceinline__ float split_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ SplitJob ja, const __grid_constant__ SplitJob jb,
+                                                    int blocks_a, SplitRedo redo) {
+  constexpr int V = MODE == SPLIT_TF32 || MODE == SPLIT_TF32_REDO ? 4 : 8;
+  __shared__ unsigned s_red[8], s_bad[8];
+  if (MODE == SPLIT_TF32_REDO) {
+    // one thread asks for its block: a million threads reading the same words took 41 us
+    if (threadIdx.x == 0) {
+      s_bad[0] = f16_unusable(redo.ra, redo.limit_a) || f16_unusable(redo.rb, redo.limit_b) ? 1u : 0u;
+      if (blockIdx.x == 0) *redo.redo = (int)s_bad[0];
+    }
+    __syncthreads();
+    if (s_bad[0] == 0) return;
+  }
+  const bool second = (int)blockIdx.x >= blocks_a;
+  const SplitJob &j = second ? jb : ja;
+  const float *src = j.src;
+  const long long ld = j.ld, stride = j.stride, rows = j.rows, cols = j.cols;
+  const long long per_row = (MODE == SPLIT_AMAX ? (cols + V - 1) / V : j.ldo / V);
+  const long long total = rows * j.batch * per_row;
+  const bool vec = ((ld | stride) & 3) == 0 && ((uintptr_t)src & 15) == 0;
+  const int nblk = second ? (int)gridDim.x - blocks_a : blocks_a, blk = second ? (int)blockIdx.x - blocks_a : (int)blockIdx.x;
+  const bool narrow = total <= 0xFFFFFFFFLL;  // 32-bit divisions
+  float scale = 0.f;
+  if (MODE == SPLIT_F16) {
+    const int ex = f16_scale_exp(*(volatile const unsigned *)&j.rec->amax);
+    scale = pow2(ex);
+    if (blk == 0 && threadIdx.x == 0) j.rec->scale_exp = ex;
+  }
+  unsigned amax = 0, bad = 0;  // SPLIT_F16: `bad` counts the small values
+  for (long long t = (long long)blk * 256 + threadIdx.x; t < total; t += (long long)nblk * 256) {
+    long long row, g, b, r;
+    if (narrow) {
+      const uint32_t rr = (uint32_t)t / (uint32_t)per_row, bb = rr / (uint32_t)rows;
+      row = rr;
+      g = (uint32_t)t - rr * (uint32_t)per_row;
+      b = bb;
+      r = rr - bb * (uint32_t)rows;
+    } else {
+      row = t / per_row;
+      g = t - row * per_row;
+      b = row / rows;
+      r = row - b * rows;
+    }
+    const long long c0 = g * V;
+    const float *p = src + b * stride + r * ld + c0;
+    float x[V];
+    if (vec && c0 + V <= cols) {
+#pragma unroll
+      for (int q = 0; q < V / 4; ++q) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(p) + q);
+        x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < V; ++q) x[q] = c0 + q < cols ? __ldg(p + q) : 0.f;
+    }
+    if (MODE == SPLIT_AMAX) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        const unsigned m = __float_as_uint(x[q]) & 0x7FFFFFFFu;
+        if (m >= 0x7F800000u) bad = 1;
+        else amax = amax > m ? amax : m;
+      }
+    } else if (MODE == SPLIT_F16) {
+      __align__(16) __half h[V], l[V];
+#pragma unroll
+      for (int q = 0; q < V; ++q) bad += f16_pair(x[q], scale, h[q], l[q]) ? 1u : 0u;
+      reinterpret_cast<uint4 *>(j.hi)[t] = *reinterpret_cast<const uint4 *>(h);
+      reinterpret_cast<uint4 *>(j.lo)[t] = *reinterpret_cast<const uint4 *>(l);
+    } else {
+      float h[4], l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        h[q] = split_tf32(x[q]);
+        l[q] = split_tf32(__fsub_rn(x[q], h[q]));
+      }
+      reinterpret_cast<float4 *>(j.hi)[t] = make_float4(h[0], h[1], h[2], h[3]);
+      reinterpret_cast<float4 *>(j.lo)[t] = make_float4(l[0], l[1], l[2], l[3]);
+    }
+  }
+  if (MODE == SPLIT_F16) {
+    if (bad) atomicAdd(&j.rec->small, bad);  // rare
+  }
+  if (MODE == SPLIT_AMAX) {
+    amax = __reduce_max_sync(0xffffffffu, amax);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+      s_red[threadIdx.x >> 5] = amax;
+      s_bad[threadIdx.x >> 5] = bad;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) {
+        amax = amax > s_red[w] ? amax : s_red[w];
+        bad |= s_bad[w];
+      }
+      atomicMax(&j.rec->amax, amax);
+      if (bad) atomicOr(&j.rec->bad, 1u);
+    }
+  }
+}
+
+template <int MODE>
+static int launch_split(b200_engine *e, const SplitJob &a, const SplitJob &b, const SplitRedo &redo) {
+  constexpr int V = MODE == SPLIT_TF32 || MODE == SPLIT_TF32_REDO ? 4 : 8;
+  auto blocks_of = [&](const SplitJob &j) -> long long {
+    if (!j.src) return 0;
+    const long long groups = j.rows * j.batch * ((j.cols + V - 1) / V);
+    // the launch that usually finds nothing to do has no more blocks than start at once
+    const long long most = MODE == SPLIT_TF32_REDO ? e->sm_count * 4LL : e->sm_count * 16LL;
+    return std::max<long long>(1, std::min<long long>((groups + 255) / 256, most));
+  };
+  const long long ba = blocks_of(a), bb = blocks_of(b);
+  if (ba + bb == 0) return B200_OK;
+  split_kernel<MODE><<<(int)(ba + bb), 256, 0, e->stream>>>(a, b, (int)ba, redo);
+  B200_CHECK_LAUNCH(e, "split_kernel");
+  return B200_OK;
+}
+
+int launch_split_tf32(b200_engine *e, const SplitJob &a, const SplitJob &b) {
+  return launch_split<SPLIT_TF32>(e, a, b, SplitRedo());
+}
+int launch_split_f16(b200_engine *e, const SplitJob &a, const SplitJob &b) {
+  const int rc = launch_split<SPLIT_AMAX>(e, a, b, SplitRedo());
+  return rc != B200_OK ? rc : launch_split<SPLIT_F16>(e, a, b, SplitRedo());
+}
+int launch_split_tf32_redo(b200_engine *e, const SplitJob &a, const SplitJob &b, const F16Rec *ra, unsigned limit_a,
+                           const F16Rec *rb, unsigned limit_b, int *redo) {
+  return launch_split<SPLIT_TF32_REDO>(e, a, b, SplitRedo{ra, rb, limit_a, limit_b, redo});
+}
+
+}  // namespace b200

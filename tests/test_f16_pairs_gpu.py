@@ -1,0 +1,130 @@
+"""float32 products made from pairs of fp16 (large ones) and their way back to pairs of TF32 where fp16's
+range is not enough (GPU tests against float64)."""
+import numpy as np
+import pytest
+
+from tests import util
+from tests.util import assert_gemm_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _product(e, a, b, transA=False, transB=False, constant=False, **kw):
+    ta, tb = e.tensor(a), e.tensor(b)
+    if constant:
+        e.constant(tb)
+    M = a.shape[-1] if transA else a.shape[-2]
+    N = b.shape[-2] if transB else b.shape[-1]
+    tc = e.empty(a.shape[:-2] + (M, N))
+    out = []
+    for _ in range(2):      # twice: the operands' records must be clear again, a constant's must stay
+        e.MatMul(ta, tb, tc, transA, transB, **kw)
+        out.append(tc.numpy())
+    for t in (ta, tb, tc):
+        t.free()
+    assert np.array_equal(out[0], out[1], equal_nan=True)
+    return out[1]
+
+
+def _want(a, b, transA=False, transB=False):
+    a, b = a.astype(np.float64), b.astype(np.float64)
+    return (np.swapaxes(a, -1, -2) if transA else a) @ (np.swapaxes(b, -1, -2) if transB else b)
+
+
+@pytest.mark.parametrize("transA,transB", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("shape", [(2048, 2048, 2048), (2051, 1999, 2309), (1030, 3001, 1000), (3000, 130, 9000)])
+def test_large_products(fresh, shape, transA, transB):
+    M, N, K = shape
+    a = util.normal(1, (K, M) if transA else (M, K))
+    b = util.normal(2, (N, K) if transB else (K, N), scale=0.02)
+    want = _want(a, b, transA, transB)
+    got = _product(fresh, a, b, transA, transB)
+    assert_gemm_close(got, want, 1e-5)
+    # sums of exact products of pairs: no worse than the TF32 pairs' 7e-7 of the result's norm
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
+def test_large_batched_and_constant(fresh):
+    a, b = util.normal(3, (6, 1024, 1100)), util.normal(4, (6, 1100, 1024), scale=0.02)
+    assert_gemm_close(_product(fresh, a, b), _want(a, b), 1e-5)
+    a, b = util.normal(5, (4000, 1152)), util.normal(6, (1152, 2000), scale=0.02)
+    assert_gemm_close(_product(fresh, a, b, constant=True), _want(a, b), 1e-5)
+
+
+@pytest.mark.parametrize("scale_a,scale_b", [(1e-30, 1.0), (1e30, 1e-30), (3e37, 1e-20), (1e-32, 1e30), (1e20, 1e15)])
+def test_any_magnitude(fresh, scale_a, scale_b):
+    # the whole operand far from 1: taken up by its power of two, or, near the ends of float32, by TF32 pairs,
+    # which need their tails, 2^-11 of the values, above float32's smallest normal number, 1.2e-38
+    a = (util.normal(7, (2048, 2048)).astype(np.float64) * scale_a).astype(np.float32)
+    b = (util.normal(8, (2048, 2048)).astype(np.float64) * scale_b).astype(np.float32)
+    want = _want(a, b)
+    got = _product(fresh, a, b)
+    assert_gemm_close(got, want, 1e-5)
+
+
+@pytest.mark.parametrize("constant", [False, True])
+def test_wide_range_rows_keep_their_precision(fresh, constant):
+    # rows of A from 1e-18 to 1e18: each row of the result is as exact as its neighbours
+    a = util.normal(9, (2048, 2048)) * (10.0 ** np.linspace(-18, 18, 2048)).astype(np.float32)[:, None]
+    b = util.normal(10, (2048, 2048))
+    want = _want(a, b)
+    got = _product(fresh, a, b, constant=constant)
+    row = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert row.max() < 2e-6
+    # and the same in the other operand's columns
+    want = _want(b, a.T)
+    got = _product(fresh, b, np.ascontiguousarray(a.T), constant=constant)
+    assert (np.linalg.norm(got - want, axis=0) / np.linalg.norm(want, axis=0)).max() < 2e-6
+
+
+def test_lowest_value_masks(fresh):
+    # a column of A near the type's lowest value meets a row of zeros: the others must not notice (the lowest
+    # value itself rounds to an infinite TF32 head)
+    low = np.float32(-3.0e38)
+    a, b = util.normal(11, (2048, 2048)), util.normal(12, (2048, 2048))
+    a[:, 7] = low
+    b[7] = 0.0
+    assert_gemm_close(_product(fresh, a, b), _want(a, b), 1e-5)
+    a[:, 7] = util.normal(13, 2048)
+    b[7] = 1.0
+    a[5, 7] = low          # one element only: its row is that element's, the others as ever
+    want = _want(a, b)
+    got = _product(fresh, a, b)
+    assert_gemm_close(np.delete(got, 5, 0), np.delete(want, 5, 0), 1e-5)
+    assert_gemm_close(got[5], want[5], 1e-5)
+
+
+def test_infinities_and_nans(fresh):
+    a, b = util.normal(14, (2048, 2048)), util.normal(15, (2048, 2048))
+    a[3, 9], a[4, 10], b[11, 6] = np.inf, np.nan, -np.inf
+    got = _product(fresh, a, b)
+    clean = np.ones((2048, 2048), bool)
+    clean[3], clean[4], clean[:, 6] = False, False, False
+    az, bz = np.nan_to_num(a, nan=0, posinf=0, neginf=0), np.nan_to_num(b, nan=0, posinf=0, neginf=0)
+    want = _want(az, bz)
+    assert np.isfinite(got[clean]).all() and not np.isfinite(got[~clean]).any()
+    assert np.abs(got - want)[clean].max() <= 1e-5 * np.abs(want).max()
+
+
+def test_all_zero_and_recorded(fresh):
+    e = fresh
+    z = np.zeros((2048, 2048), np.float32)
+    assert not _product(e, z, util.normal(16, (2048, 2048))).any()
+    # a recorded product replays on new operands, some within fp16's range and some not
+    ta, tb, tc = e.tensor(z), e.tensor(z), e.empty((2048, 2048))
+    e.MatMul(ta, tb, tc)
+    e.Signal()
+    e.tape_begin()
+    e.MatMul(ta, tb, tc)
+    tape = e.tape_end()
+    b = util.normal(17, (2048, 2048))
+    for k, spread in enumerate((0, 30, 0)):
+        a = util.normal(18 + k, (2048, 2048)) * (10.0 ** np.linspace(0, spread, 2048)).astype(np.float32)[:, None]
+        ta.set(a)
+        tb.set(b)
+        e.tape_launch(tape)
+        e.Signal()
+        want = _want(a, b)
+        row = np.linalg.norm(tc.numpy() - want, axis=1) / np.linalg.norm(want, axis=1)
+        assert row.max() < 2e-6
+    e.tape_destroy(tape)
