@@ -173,6 +173,12 @@ _SIGS = {
                                      _i, _P(Epilogue), _i, _i, _i, _i]),
     "b200_conv2d_chain_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i, _i, _i, _i,
                                    _i, _i, _i, _i, _P(Epilogue), _i]),
+    "b200_conv2d_pairs_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _i, _i, _i, _i,
+                                   _P(Epilogue), _i]),
+    "b200_maxpool2d_pairs_fwd": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _i, _i, _i, _i, _i]),
+    "b200_pairs_magnitude": (_i, [_vp, _vp, _i64, _vp]),
+    "b200_pairs_check": (_i, [_vp, _vp, _P(_i64), _i, _vp]),
+    "b200_only_if": (_i, [_vp, _vp]),
     "b200_conv2d_path": (_i, [_vp, _i, _i64, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _i, _i, _i, _i]),
     "b200_im2col": (_i, [_vp, _i, _vp, _vp, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _i, _i, _i, _i]),
     "b200_batchnorm_fwd": (_i, [_vp, _i, _vp, _vp, _i64, _i64, _i64, _i, C.c_double, C.c_double, _vp, _vp, _vp, _vp]),

@@ -13,6 +13,7 @@
 
 #include "engine.h"
 #include "epilogue.cuh"
+#include "pairs.cuh"
 
 namespace b200 {
 
@@ -25,6 +26,13 @@ int conv2d_tma(b200_engine *e, const float *x, const float *w, float *y, long lo
 int conv2d_win(b200_engine *e, const float *x, const float *w, float *y, long long B, int C, int H, int W, int K,
                int kh, int kw, int padH, int padW, int dH, int dW, int Ho, int Wo, const Epilogue &ep, bool pool2,
                const float *x_hi, const float *x_lo, float *y_hi, float *y_lo);
+int conv2d_tma_pairs(b200_engine *e, const __half *x_pairs, const TcOperand &wf, float *y, long long B, int C, int H,
+                     int W, int K, int kh, int kw, int padH, int padW, int sH, int sW, int dH, int dW, int Ho, int Wo,
+                     const Epilogue &ep, const PairsIn &in, const PairsOut &out);
+int conv2d_win_pairs(b200_engine *e, const __half *x_pairs, const TcOperand &wf, float *y, long long B, int C, int H,
+                     int W, int K, int kh, int kw, int padH, int padW, int dH, int dW, int Ho, int Wo,
+                     const Epilogue &ep, bool pool2, const PairsIn &in, const PairsOut &out);
+int conv_nhwc_pairs(b200_engine *e, const float *x, long long B, int C, int HW, __half *pairs, F16Rec *rec);
 int conv_nhwc_split_into(b200_engine *e, const float *x, long long B, int C, int HW, float *hi, float *lo);
 bool conv_win_eligible(const b200_engine *e, long long B, int C, int H, int W, int K, int kh, int kw, int padH,
                        int padW, int sH, int sW, int dH, int dW, int Ho, int Wo);
@@ -251,14 +259,19 @@ static int launch_conv3x3_first(b200_engine *e, const float *x, const float *w, 
 // thread computes a 2 x 4 block of outputs for 8 filters at a time from a 4 x 6 patch of inputs
 // per channel and stores the two pooled values of each filter as one float2. The convolution output
 // itself (four times the pooled bytes, and the largest tensor of the network) is never written.
-template <int C, int ACT, bool BIAS>
+// F16: the output goes out as pairs of fp16 (pairs.cuh; K a multiple of 8). x_rec->amax is the largest
+// magnitude of x, or of a sample of it: a result beyond the bound that follows from it is marked.
+template <int C, int ACT, bool BIAS, bool F16>
 __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float *__restrict__ x,
                                                                     const float *__restrict__ w,
                                                                     float *__restrict__ y,
                                                                     const float *__restrict__ bias, float alpha,
                                                                     long long groups, int H, int W, int K,
                                                                     float *__restrict__ y_hi,
-                                                                    float *__restrict__ y_lo) {
+                                                                    float *__restrict__ y_lo,
+                                                                    const int *__restrict__ only_if,
+                                                                    const F16Rec *__restrict__ x_rec, PairsOut out16) {
+  if (!F16 && skip_launch(only_if)) return;
   constexpr int Q = C * 9;
   __shared__ __align__(16) float ws[Q * 32];  // [q][k], zero for k >= K
   __shared__ float bs[32];
@@ -268,6 +281,20 @@ __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float 
   }
   if (threadIdx.x < 32) bs[threadIdx.x] = (BIAS && threadIdx.x < K) ? bias[threadIdx.x] : 0.f;
   __syncthreads();
+  PairStats stats;
+  float out_scale = 1.f;
+  if (F16) {
+    float l1 = 0.f;  // of this lane's filter
+    for (int q = 0; q < Q; ++q) l1 += fabsf(ws[(q << 5) + (threadIdx.x & 31)]);
+    // a NaN among the filters ends up as a magnitude above every number, i.e. the smallest scale
+    l1 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(l1) & 0x7FFFFFFFu));
+    const int ex = pairs_out_exp(__uint_as_float(x_rec->amax), l1, BIAS ? bias : nullptr, K, ACT, alpha);
+    out_scale = pow2(ex);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      out16.rec->scale_exp = ex;
+      if (x_rec->bad) out16.rec->bad = 1;
+    }
+  }
   const int Wg = W >> 2, Hq = H >> 1, Wq = W >> 1;
   const long long per_image = (long long)Hq * Wg;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -343,10 +370,18 @@ __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float 
             }
           pooled[half][k] = best;
         }
-        if (y && k0 + k < K)
+        if (!F16 && y && k0 + k < K)
           *reinterpret_cast<float2 *>(yb + (long long)(k0 + k) * Hq * Wq) = make_float2(pooled[0][k], pooled[1][k]);
       }
-      if (y_hi) {  // the same values as NHWC TF32 head / tail for the next convolution (K a multiple of 4)
+      if (F16) {
+        const long long pos = (b * Hq + ph) * (long long)Wq + (ow >> 1);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) stats.see(pooled[half][k]);
+          store_pairs<8>(pooled[half], 8, out_scale, out16.h + (pos + half) * K + k0, out16.l + (pos + half) * K + k0, stats);
+        }
+      } else if (y_hi) {  // the same values as NHWC TF32 head / tail for the next convolution (K a multiple of 4)
         const long long pos = (b * Hq + ph) * (long long)Wq + (ow >> 1);
 #pragma unroll
         for (int half = 0; half < 2; ++half)
@@ -366,18 +401,20 @@ __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float 
       }
     }
   }
+  if (F16) stats.deliver(out16.rec);
 }
 
-template <int C>
+template <int C, bool F16>
 static int launch_conv3x3_first_pool(b200_engine *e, const float *x, const float *w, float *y, long long B, int H,
-                                     int W, int K, const Epilogue &ep, float *y_hi = nullptr, float *y_lo = nullptr) {
+                                     int W, int K, const Epilogue &ep, float *y_hi = nullptr, float *y_lo = nullptr,
+                                     const F16Rec *x_rec = nullptr, const PairsOut &out16 = PairsOut()) {
   const long long groups = B * (H / 2) * (W / 4);
   const int blocks = (int)std::max<long long>(1, std::min<long long>((groups + 255) / 256, (long long)e->sm_count * 16));
   const float *bias = (const float *)ep.bias;
   const float alpha = (float)ep.alpha;
-#define B200_FIRSTP(ACT, BIAS) \
-  conv3x3_first_pool_kernel<C, ACT, BIAS><<<blocks, 256, 0, e->stream>>>(x, w, y, bias, alpha, groups, H, W, K, y_hi, \
-                                                                         y_lo)
+#define B200_FIRSTP(ACT, BIAS)                                                                                        \
+  conv3x3_first_pool_kernel<C, ACT, BIAS, F16><<<blocks, 256, 0, e->stream>>>(x, w, y, bias, alpha, groups, H, W, K, y_hi, \
+                                                                              y_lo, e->only_if, x_rec, out16)
   const bool hb = ep.bias_kind != B200_BIAS_NONE;
   if (ep.act == B200_ACT_NONE) { if (hb) B200_FIRSTP(B200_ACT_NONE, true); else B200_FIRSTP(B200_ACT_NONE, false); }
   else if (ep.act == B200_ACT_RECTIFY) { if (hb) B200_FIRSTP(B200_ACT_RECTIFY, true); else B200_FIRSTP(B200_ACT_RECTIFY, false); }
@@ -415,6 +452,143 @@ static int conv_direct_small(b200_engine *e, const float *x, const float *w, flo
 #undef B200_DIRECT
   B200_CHECK_LAUNCH(e, "conv_direct_small_kernel");
   return B200_OK;
+}
+
+// ---- pairs of fp16 --------------------------------------------------------------------------------
+// Filters (K, C, taps) as pairs of fp16 in (tap, channel) order. A block takes one filter: it sums the
+// magnitudes, and writes the pairs scaled by what the largest magnitude of all filters asks for. Made once
+// for a constant; otherwise a few kilobytes to a few megabytes, bound by the launch.
+__global__ void __launch_bounds__(256) filter_pairs_kernel(const float *__restrict__ w, __half *__restrict__ hi,
+                                                           __half *__restrict__ lo, int C, int taps, F16Filters *f) {
+  __shared__ float red[8];
+  const int crs = C * taps;
+  const float *in = w + (long long)blockIdx.x * crs;
+  const int ex = f16_scale_exp(*(volatile const unsigned *)&f->rec.amax);
+  const float scale = pow2(ex);
+  unsigned small = 0;
+  float sum = 0.f;
+  for (int i = threadIdx.x; i < crs; i += 256) {  // consecutive threads: consecutive channels of a tap
+    const int tap = i / C, c = i - tap * C;
+    const float v = __ldg(in + c * taps + tap);
+    sum += fabsf(v);
+    __half h, l;
+    small += f16_pair(v, scale, h, l) ? 1u : 0u;
+    hi[(long long)blockIdx.x * crs + i] = h;
+    lo[(long long)blockIdx.x * crs + i] = l;
+  }
+  if (small) atomicAdd(&f->rec.small, small);
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) sum += red[k];
+    atomicMax(&f->l1, __float_as_uint(sum));  // a NaN: above every number
+    if (blockIdx.x == 0) f->rec.scale_exp = ex;
+  }
+}
+
+// blk[] receives the arena blocks the caller must release, or nulls when the result came from (or went
+// into) the cache of a buffer declared constant.
+static int conv_filters_pairs(b200_engine *e, const float *w, int K, int C, int taps, TcOperand *wf, F16Filters **f,
+                              void **blk) {
+  const int crs = C * taps;
+  blk[0] = blk[1] = nullptr;
+  wf->ld = crs;
+  if (CachedSplit *c = find_cached(e, w, 3, K, C, taps, crs)) {
+    *f = (F16Filters *)c->hi;
+    wf->p0 = (char *)c->hi + 256;
+    wf->p1 = c->lo;
+    return B200_OK;
+  }
+  const long long n = (long long)K * crs;
+  int rc = b200_get(e, 256 + n * 2, &blk[0]);
+  if (rc == B200_OK) rc = b200_get(e, n * 2, &blk[1]);
+  if (rc == B200_OK && cudaMemsetAsync(blk[0], 0, sizeof(F16Filters), e->stream) != cudaSuccess)
+    rc = set_error(e, B200_ERR_CUDA, "convolution: clearing a record failed");
+  *f = (F16Filters *)blk[0];
+  wf->p0 = (char *)blk[0] + 256;
+  wf->p1 = blk[1];
+  if (rc == B200_OK) rc = launch_magnitude(e, w, n, 1, &(*f)->rec);
+  if (rc == B200_OK) {
+    filter_pairs_kernel<<<K, 256, 0, e->stream>>>(w, (__half *)const_cast<void *>(wf->p0),
+                                                  (__half *)const_cast<void *>(wf->p1), C, taps, *f);
+    if (cudaGetLastError() != cudaSuccess) rc = set_error(e, B200_ERR_CUDA, "launch of filter_pairs_kernel failed");
+    else e->launches++;
+  }
+  if (rc == B200_OK && is_constant(e, w)) {
+    add_cached(e, w, CachedSplit{3, K, C, taps, crs, blk[0], blk[1], crs});
+    blk[0] = blk[1] = nullptr;
+  }
+  if (rc != B200_OK)
+    for (int i = 0; i < 2; ++i)
+      if (blk[i]) {
+        b200_put(e, blk[i], 0);
+        blk[i] = nullptr;
+      }
+  return rc;
+}
+
+// One convolution of a chain on pairs of fp16 (path: a tensor-core kernel). x16: the input in pairs form.
+static int conv2d_pairs(b200_engine *e, int path, const __half *x16, const F16Rec *x_rec, const float *w, float *y,
+                        const PairsOut &out, long long B, int C, int H, int W, int K, int kh, int kw, int padH,
+                        int padW, int sH, int sW, int dH, int dW, int Ho, int Wo, const Epilogue &ep, bool pool2) {
+  TcOperand wf;
+  F16Filters *f = nullptr;
+  void *blk[2];
+  int rc = conv_filters_pairs(e, w, K, C, kh * kw, &wf, &f, blk);
+  if (rc != B200_OK) return rc;
+  PairsIn in;
+  in.x = x_rec;
+  in.w = f;
+  in.limit_x = f16_small_limit(B * C * H * W);
+  in.limit_w = f16_small_limit((long long)K * C * kh * kw);
+  if (path == B200_CONV_TC_WINDOW)
+    rc = conv2d_win_pairs(e, x16, wf, y, B, C, H, W, K, kh, kw, padH, padW, dH, dW, Ho, Wo, ep, pool2, in, out);
+  else
+    rc = conv2d_tma_pairs(e, x16, wf, y, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho, Wo, ep, in, out);
+  for (void *b : blk)
+    if (b) b200_put(e, b, 0);
+  return rc;
+}
+
+// Whether a single convolution is worth pairs of fp16. They save about 0.35 of what TF32 pairs take (160
+// TFLOP/s); finding the input's largest magnitude reads it once more, and the four more launches cost 20 us
+// (16 x 128 x 26 x 26 to 256 channels, 6.4 GFLOP: 45 us with TF32 pairs, 55 with fp16), two more with filters
+// that are not constant.
+static bool conv_pairs_pay(b200_engine *e, const float *w, long long B, int C, int H, int W, int K, int taps, int Ho, int Wo) {
+  const double saves = 0.35 * 2.0 * B * Ho * Wo * K * (double)C * taps / 160e12;
+  const double costs = 4.0 * B * C * H * (double)W / 5e12 + (is_constant(e, w) ? 20e-6 : 27e-6);
+  return C % 16 == 0 && saves > 1.2 * costs;
+}
+
+// x (NCHW) through pairs of fp16, with the TF32 launches behind it that run only if the pairs are unusable.
+static int conv2d_eager_pairs(b200_engine *e, int path, const float *x, const float *w, float *y, long long B, int C,
+                              int H, int W, int K, int kh, int kw, int padH, int padW, int sH, int sW, int dH, int dW,
+                              int Ho, int Wo, const Epilogue &ep, bool pool2) {
+  const long long n = B * C * H * W;
+  F16Rec *rx = e->f16_recs, *ry = e->f16_recs + 1;  // the output's only takes the filters' mark
+  int *redo = (int *)(e->f16_recs + 2);
+  void *x16 = nullptr;
+  int rc = b200_get(e, n * 4, &x16);
+  if (rc != B200_OK) return rc;
+  rc = launch_magnitude(e, x, n, 1, rx);
+  if (rc == B200_OK) rc = conv_nhwc_pairs(e, x, B, C, H * W, (__half *)x16, rx);
+  PairsOut out;
+  out.rec = ry;
+  if (rc == B200_OK)
+    rc = conv2d_pairs(e, path, (const __half *)x16, rx, w, y, out, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho,
+                      Wo, ep, pool2);
+  b200_put(e, x16, 0);  // stream order; the TF32 pairs may take its place
+  const unsigned limits[2] = {f16_small_limit(n), 0xFFFFFFFFu};
+  if (rc == B200_OK) rc = launch_pairs_check(e, rx, limits, 2, redo);
+  if (rc == B200_OK) {
+    e->only_if = redo;
+    rc = path == B200_CONV_TC_WINDOW
+             ? conv2d_win(e, x, w, y, B, C, H, W, K, kh, kw, padH, padW, dH, dW, Ho, Wo, ep, pool2, nullptr, nullptr, nullptr, nullptr)
+             : conv2d_tma(e, x, w, y, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho, Wo, ep, nullptr, nullptr, nullptr, nullptr);
+    e->only_if = nullptr;
+  }
+  return rc;
 }
 
 // scratch budget for the col data of one chunk (head + tail together)
@@ -481,7 +655,14 @@ int b200_conv2d_fwd(b200_engine *e, int dtype, const void *x, const void *w, voi
   const long long img_bytes = hw * crs * (long long)es;
   long long chunk = std::max<long long>(1, std::min<long long>(B, kColChunkBytes / std::max<long long>(1, img_bytes)));
 
-  switch (conv_path(e, dtype, B, C, H, W, K, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, Ho, Wo)) {
+  const int path = conv_path(e, dtype, B, C, H, W, K, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, Ho, Wo);
+  if ((path == B200_CONV_TC_TMA || path == B200_CONV_TC_WINDOW) &&
+      conv_pairs_pay(e, (const float *)w, B, (int)C, (int)H, (int)W, (int)K, kh * kw, (int)Ho, (int)Wo)) {
+    rc = conv2d_eager_pairs(e, path, (const float *)x, (const float *)w, (float *)y, B, (int)C, (int)H, (int)W, (int)K,
+                            kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, (int)Ho, (int)Wo, ep, false);
+    if (rc != B200_ERR_OOM) return rc;  // else: the TF32 pairs alone, as far as the arena goes
+  }
+  switch (path) {
     case B200_CONV_DIRECT:
       return conv_direct_small(e, (const float *)x, (const float *)w, (float *)y, B, (int)C, (int)H, (int)W, (int)K,
                                kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, (int)Ho, (int)Wo, ep);
@@ -550,12 +731,17 @@ int b200_conv2d_maxpool_fwd(b200_engine *e, int dtype, const void *x, const void
       int rc = flush_pending(e);
       if (rc != B200_OK) return rc;
       const Epilogue ep = make_epilogue(epi);
+      if (path == B200_CONV_TC_WINDOW && conv_pairs_pay(e, (const float *)w, B, (int)C, (int)H, (int)W, (int)K, kh * kw, (int)Ho, (int)Wo)) {
+        rc = conv2d_eager_pairs(e, path, (const float *)x, (const float *)w, (float *)y, B, (int)C, (int)H, (int)W, (int)K,
+                                kh, kw, pad_h, pad_w, 1, 1, dil_h, dil_w, (int)Ho, (int)Wo, ep, true);
+        if (rc != B200_ERR_OOM) return rc;
+      }
       if (path == B200_CONV_TC_WINDOW)
         return conv2d_win(e, (const float *)x, (const float *)w, (float *)y, B, (int)C, (int)H, (int)W, (int)K, kh, kw,
                           pad_h, pad_w, dil_h, dil_w, (int)Ho, (int)Wo, ep, true, nullptr, nullptr, nullptr, nullptr);
-      if (C == 1) return launch_conv3x3_first_pool<1>(e, (const float *)x, (const float *)w, (float *)y, B, (int)H, (int)W, (int)K, ep);
-      if (C == 2) return launch_conv3x3_first_pool<2>(e, (const float *)x, (const float *)w, (float *)y, B, (int)H, (int)W, (int)K, ep);
-      return launch_conv3x3_first_pool<3>(e, (const float *)x, (const float *)w, (float *)y, B, (int)H, (int)W, (int)K, ep);
+      if (C == 1) return launch_conv3x3_first_pool<1, false>(e, (const float *)x, (const float *)w, (float *)y, B, (int)H, (int)W, (int)K, ep);
+      if (C == 2) return launch_conv3x3_first_pool<2, false>(e, (const float *)x, (const float *)w, (float *)y, B, (int)H, (int)W, (int)K, ep);
+      return launch_conv3x3_first_pool<3, false>(e, (const float *)x, (const float *)w, (float *)y, B, (int)H, (int)W, (int)K, ep);
     }
   }
   // any other shape: the two operations one after the other, the convolution output in arena scratch
@@ -605,6 +791,7 @@ int b200_conv2d_chain_fwd(b200_engine *e, const void *x, const void *x_hi, const
       (path == B200_CONV_DIRECT && pool2 && even && x &&
        conv3x3_first_ok(x, y, C, W, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w))) {
     DeviceGuard g(e);
+    OnlyIfAllowed allowed(e);
     int rc = flush_pending(e);
     if (rc != B200_OK) return rc;
     const Epilogue ep = make_epilogue(epi);
@@ -616,9 +803,9 @@ int b200_conv2d_chain_fwd(b200_engine *e, const void *x, const void *x_hi, const
       return conv2d_tma(e, xf, wf, yf, B, (int)C, (int)H, (int)W, (int)K, kh, kw, pad_h, pad_w, stride_h, stride_w,
                         dil_h, dil_w, (int)Ho, (int)Wo, ep, (const float *)x_hi, (const float *)x_lo, (float *)y_hi,
                         (float *)y_lo);
-    if (C == 1) return launch_conv3x3_first_pool<1>(e, xf, wf, yf, B, (int)H, (int)W, (int)K, ep, (float *)y_hi, (float *)y_lo);
-    if (C == 2) return launch_conv3x3_first_pool<2>(e, xf, wf, yf, B, (int)H, (int)W, (int)K, ep, (float *)y_hi, (float *)y_lo);
-    return launch_conv3x3_first_pool<3>(e, xf, wf, yf, B, (int)H, (int)W, (int)K, ep, (float *)y_hi, (float *)y_lo);
+    if (C == 1) return launch_conv3x3_first_pool<1, false>(e, xf, wf, yf, B, (int)H, (int)W, (int)K, ep, (float *)y_hi, (float *)y_lo);
+    if (C == 2) return launch_conv3x3_first_pool<2, false>(e, xf, wf, yf, B, (int)H, (int)W, (int)K, ep, (float *)y_hi, (float *)y_lo);
+    return launch_conv3x3_first_pool<3, false>(e, xf, wf, yf, B, (int)H, (int)W, (int)K, ep, (float *)y_hi, (float *)y_lo);
   }
   // any other shape: the plain calls, then the rewrite pass; both need the tensors in NCHW
   if (!x)
@@ -642,6 +829,88 @@ int b200_conv2d_chain_fwd(b200_engine *e, const void *x, const void *x_hi, const
   }
   if (tmp) b200_put(e, tmp, 0);
   return rc;
+}
+
+int b200_conv2d_pairs_fwd(b200_engine *e, const void *x, const void *x_pairs, const void *x_rec, const void *w, void *y,
+                          void *y_pairs, void *y_rec, int64_t B, int64_t C, int64_t H, int64_t W, int64_t K, int kh,
+                          int kw, int pad_h, int pad_w, const b200_epilogue *epi, int pool2) {
+  if (!e) return B200_ERR_INVALID;
+  std::lock_guard<std::recursive_mutex> lk(e->mu);
+  B200_REQUIRE(e, B >= 0 && C > 0 && H > 0 && W > 0 && K > 0 && kh > 0 && kw > 0 && pad_h >= 0 && pad_w >= 0,
+               "b200_conv2d_pairs_fwd: bad convolution shape");
+  B200_REQUIRE(e, (x || x_pairs) && (y || y_pairs) && x_rec && y_rec && w, "b200_conv2d_pairs_fwd: null pointer");
+  B200_REQUIRE(e, ((uintptr_t)x_pairs | (uintptr_t)y_pairs) % 16 == 0, "b200_conv2d_pairs_fwd: unaligned pairs");
+  const long long Ho = H + 2 * pad_h - (kh - 1), Wo = W + 2 * pad_w - (kw - 1);
+  B200_REQUIRE(e, Ho > 0 && Wo > 0, "b200_conv2d_pairs_fwd: kernel larger than the padded image");
+  if (epi) {
+    B200_REQUIRE(e, epi->bias_kind == B200_BIAS_NONE || epi->bias_kind == B200_BIAS_ROW,
+                 "b200_conv2d_pairs_fwd: the bias is one value per output channel (B200_BIAS_ROW)");
+    B200_REQUIRE(e, epi->act >= 0 && epi->act <= 2, "b200_conv2d_pairs_fwd: bad activation");
+    B200_REQUIRE(e, epi->bias_kind == 0 || epi->bias != nullptr, "b200_conv2d_pairs_fwd: bias is null");
+    B200_REQUIRE(e, epi->accumulate == 0, "b200_conv2d_pairs_fwd: accumulate is a matrix-product option");
+  }
+  if (B == 0) return B200_OK;
+  const int path = conv_path(e, B200_F32, B, C, H, W, K, kh, kw, pad_h, pad_w, 1, 1, 1, 1, Ho, Wo);
+  const bool even = Ho % 2 == 0 && Wo % 2 == 0;
+  const bool first = path == B200_CONV_DIRECT && pool2 && even && x && y_pairs && !y && K % 8 == 0 &&
+                     conv3x3_first_ok(x, y_pairs, C, W, kh, kw, pad_h, pad_w, 1, 1, 1, 1);
+  const bool window = path == B200_CONV_TC_WINDOW && (!pool2 || even), tma = path == B200_CONV_TC_TMA && !pool2;
+  if (!first && !((window || tma) && x_pairs && C % 16 == 0 && (!y_pairs || K % 8 == 0)))
+    return set_error(e, B200_ERR_UNSUPPORTED, "b200_conv2d_pairs_fwd: no kernel takes this shape as pairs of fp16");
+  DeviceGuard g(e);
+  int rc = flush_pending(e);
+  if (rc != B200_OK) return rc;
+  const Epilogue ep = make_epilogue(epi);
+  const long long ny = B * K * (pool2 ? (Ho / 2) * (Wo / 2) : Ho * Wo);
+  PairsOut out;
+  out.h = (__half *)y_pairs;
+  out.l = y_pairs ? (__half *)y_pairs + ny : nullptr;
+  out.rec = (F16Rec *)y_rec;
+  const F16Rec *rx = (const F16Rec *)x_rec;
+  const float *xf = (const float *)x, *wf = (const float *)w;
+  if (first) {
+    if (C == 1) return launch_conv3x3_first_pool<1, true>(e, xf, wf, nullptr, B, (int)H, (int)W, (int)K, ep, nullptr, nullptr, rx, out);
+    if (C == 2) return launch_conv3x3_first_pool<2, true>(e, xf, wf, nullptr, B, (int)H, (int)W, (int)K, ep, nullptr, nullptr, rx, out);
+    return launch_conv3x3_first_pool<3, true>(e, xf, wf, nullptr, B, (int)H, (int)W, (int)K, ep, nullptr, nullptr, rx, out);
+  }
+  return conv2d_pairs(e, path, (const __half *)x_pairs, rx, wf, (float *)y, out, B, (int)C, (int)H, (int)W, (int)K, kh,
+                      kw, pad_h, pad_w, 1, 1, 1, 1, (int)Ho, (int)Wo, ep, pool2 != 0);
+}
+
+int b200_pairs_magnitude(b200_engine *e, const void *x, int64_t n, void *rec) {
+  if (!e) return B200_ERR_INVALID;
+  std::lock_guard<std::recursive_mutex> lk(e->mu);
+  B200_REQUIRE(e, n >= 0 && rec && (x || n == 0), "b200_pairs_magnitude: null pointer or negative count");
+  if (n == 0) return B200_OK;
+  DeviceGuard g(e);
+  int rc = flush_pending(e);
+  if (rc != B200_OK) return rc;
+  return launch_magnitude(e, (const float *)x, n, 16, (F16Rec *)rec);
+}
+
+int b200_pairs_check(b200_engine *e, void *recs, const int64_t *counts, int k, int *verdict) {
+  if (!e) return B200_ERR_INVALID;
+  std::lock_guard<std::recursive_mutex> lk(e->mu);
+  B200_REQUIRE(e, recs && counts && verdict && k >= 0 && k <= kMaxPairsRecs, "b200_pairs_check: null pointer or bad count");
+  DeviceGuard g(e);
+  int rc = flush_pending(e);
+  if (rc != B200_OK) return rc;
+  unsigned limits[kMaxPairsRecs];
+  for (int i = 0; i < k; ++i) limits[i] = f16_small_limit(counts[i]);
+  return launch_pairs_check(e, (F16Rec *)recs, limits, k, verdict);
+}
+
+int b200_only_if(b200_engine *e, const int *flag) {
+  if (!e) return B200_ERR_INVALID;
+  std::lock_guard<std::recursive_mutex> lk(e->mu);
+  if (flag) {
+    B200_REQUIRE(e, !e->only_if, "b200_only_if: already in effect");
+    DeviceGuard g(e);
+    int rc = flush_pending(e);
+    if (rc != B200_OK) return rc;
+  }
+  e->only_if = flag;
+  return B200_OK;
 }
 
 int b200_conv2d_path(b200_engine *e, int dtype, int64_t B, int64_t C, int64_t H, int64_t W, int64_t K, int kh, int kw,

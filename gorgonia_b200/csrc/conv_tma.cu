@@ -11,7 +11,12 @@
 // the slab in the swizzled K-major layout the tensor core reads. The rewrite costs 12 bytes per
 // input element; the 9 (kh*kw) re-reads of the activations come from L2.
 //
-// CK = 32 channels per k-block (128-byte rows, 128-byte swizzle), so C must be a multiple of 32.
+// Pairs of fp16 (F16, split.cu and pairs.cuh) take the place of the TF32 pairs where their range allows it:
+// 64 channels per 128-byte row (32 per 64-byte row where C is no multiple of 64) and twice the tensor rate.
+// What bounds this kernel, bytes into and out of shared memory per k-block, is then halved per channel:
+// 512 -> 1024 channels, 3x3 on 13 x 13 planes of 64 images 802 -> 464 us.
+//
+// CK = 32 channels per k-block (128-byte rows, 128-byte swizzle) of TF32, so C must be a multiple of 32.
 // (The kernel is also correct with CK = 16, 64-byte rows and swizzle, but at C = 16 the col slabs
 // are re-read from L2 nine times at 8 bytes per element and the gather kernel, which reads 4, wins.)
 // A 1x1 convolution has no re-reads to save, but it runs here as well: in a chain its input arrives
@@ -29,6 +34,7 @@
 
 #include "engine.h"
 #include "epilogue.cuh"
+#include "pairs.cuh"
 #include "ptx.cuh"
 #include "tc_common.cuh"
 #include "tc_operand.h"
@@ -58,6 +64,9 @@ struct ConvTmaParams {
   int sk_first, sk_workers;  // k ranges are shared from this tile on, among this many CTAs (TilePieces)
   float *ws;        // partial tiles: slot 2c (a part that begins CTA c's share) and 2c + 1 (one that ends it)
   int *tile_count;  // parts delivered per tile; zero between launches
+  PairsIn in16;       // F16: the operands, and
+  PairsOut out16;     // the output in pairs form (h may be null) and what is recorded of it
+  const int *only_if; // TF32: run only if this word says so (skip_launch)
   Epilogue ep;     // bias_kind ROW = per output channel
   int *err_flag;
 };
@@ -77,22 +86,24 @@ __device__ __forceinline__ void ct_tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) 
       : "memory");
 }
 
-template <int BN, int CK>
+// ROW_BYTES: one pixel's (or one filter's) channels of a k-block, 128 or 64 bytes
+template <int BN, int ROW_BYTES, bool F16>
 __global__ void __launch_bounds__(CT_THREADS, 1)
     conv_tma_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                     const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                     const __grid_constant__ ConvTmaParams p) {
-  constexpr int ROW_BYTES = CK * 4;               // one pixel's (or one filter's) channels of a k-block
+  constexpr int CK = ROW_BYTES / (F16 ? 2 : 4);
   constexpr int A_BYTES = CT_BM * ROW_BYTES;      // one copy (head or tail) of the col slab
   constexpr int B_BYTES = BN * ROW_BYTES;
   constexpr int STAGE_BYTES = 2 * (A_BYTES + B_BYTES);
   constexpr uint32_t SBO = 8 * ROW_BYTES;         // 8-row groups of the swizzle pattern
-  constexpr uint32_t LAYOUT = CK == 32 ? 2 : 4;   // 128-byte / 64-byte swizzle
-  constexpr int KK = CK / 8;                      // MMAs (k = 8) per k-block
-  constexpr uint32_t IDESC = make_idesc(2, 0, 0, CT_BM, BN);
+  constexpr uint32_t LAYOUT = ROW_BYTES == 128 ? 2 : 4;  // 128-byte / 64-byte swizzle
+  constexpr int KK = ROW_BYTES / 32;              // MMAs (k = 8 or 16) per k-block
+  constexpr uint32_t FMT = F16 ? 0 : 2;
+  constexpr uint32_t IDESC = make_idesc(FMT, 0, 0, CT_BM, BN);
   // head x [filter head | filter tail] as ONE instruction of width 2*BN: the tail slab follows the
   // head slab in shared memory, the cross-term accumulator follows the main one in tensor memory
-  constexpr uint32_t IDESC_WIDE = make_idesc(2, 0, 0, CT_BM, 2 * BN);
+  constexpr uint32_t IDESC_WIDE = make_idesc(FMT, 0, 0, CT_BM, 2 * BN);
   constexpr int ACC_COLS = 2 * BN;
   constexpr int TMEM_COLS = 2 * ACC_COLS;
   constexpr int HALF = BN / 2;
@@ -105,6 +116,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
   __shared__ int s_fail, s_last;
   __shared__ float bias_s[8][BN / 2];
 
+  // the same answer in every thread of the grid
+  if (F16 ? !pairs_usable(p.in16, p.out16.rec) : skip_launch(p.only_if)) return;
   unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)ct_smem_raw + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int stages = p.stages;
@@ -219,8 +232,13 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
               const uint64_t a_lo = make_smem_desc(st + A_BYTES + kk * 32, 16, SBO, LAYOUT);
               const uint64_t b_hi = make_smem_desc(st + 2 * A_BYTES + kk * 32, 16, SBO, LAYOUT);
               const uint32_t accumulate = (kb > kc || kk > 0) ? 1u : 0u;
-              ptx::mma_tf32(d_main, a_hi, b_hi, IDESC_WIDE, accumulate);
-              ptx::mma_tf32(d_tail, a_lo, b_hi, IDESC, 1u);
+              if (F16) {
+                ptx::mma_f16(d_main, a_hi, b_hi, IDESC_WIDE, accumulate);
+                ptx::mma_f16(d_tail, a_lo, b_hi, IDESC, 1u);
+              } else {
+                ptx::mma_tf32(d_main, a_hi, b_hi, IDESC_WIDE, accumulate);
+                ptx::mma_tf32(d_tail, a_lo, b_hi, IDESC, 1u);
+              }
             }
             ptx::mma_commit(&empty_bar[stage]);
             if (++stage == stages) {
@@ -240,6 +258,17 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const bool has_bias = p.ep.bias_kind != B200_BIAS_NONE;
     const float *bias_g = reinterpret_cast<const float *>(p.ep.bias);
+    float unscale1 = 1.f, unscale2 = 1.f, out_scale = 1.f;
+    PairStats stats;
+    if (F16) {
+      f16_unscale(p.in16.x->scale_exp, p.in16.w->rec.scale_exp, unscale1, unscale2);
+      if (p.out16.h) {
+        const int ex = pairs_out_exp(__uint_as_float(p.in16.x->amax), __uint_as_float(p.in16.w->l1),
+                                     has_bias ? bias_g : nullptr, p.K, p.ep.act, (float)p.ep.alpha);
+        out_scale = pow2(ex);
+        if (blockIdx.x == 0 && warp == 2 && lane == 0) p.out16.rec->scale_exp = ex;
+      }
+    }
     int use = 0;
     uint32_t epi_phase = 0;
     bool ok = true;
@@ -275,7 +304,9 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
           ptx::tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            acc[c + j] = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(rm[j]), __uint_as_float(rt[j])));
+            acc[c + j] = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(rm[j]),
+                                                         F16 ? __fmul_rn(__uint_as_float(rt[j]), 4.8828125e-4f)
+                                                             : __uint_as_float(rt[j])));
         }
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -340,7 +371,25 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
         for (int j = lane; j < HALF; j += 32) bias_s[warp - 2][j] = n0 + j < p.K ? bias_g[n0 + j] : 0.f;
         __syncwarp();
       }
-      if (p.y_hi)  // position m of the flattened (b, oh, ow) index is row m of the NHWC tensor
+      if (F16) {
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) acc[j] = __fmul_rn(__fmul_rn(acc[j], unscale1), unscale2);
+        finish_channels<HALF>(acc, has_bias ? bias_s[warp - 2] : nullptr, p.ep.act, (float)p.ep.alpha);
+        const int valid = p.K - n0;
+        if (m < p.Mtot) {
+          if (p.out16.rec) {
+#pragma unroll
+            for (int j = 0; j < HALF; ++j)
+              if (j < valid) stats.see(acc[j]);
+          }
+          if (p.out16.h) store_pairs<HALF>(acc, valid, out_scale, p.out16.h + m * p.K + n0, p.out16.l + m * p.K + n0, stats);
+          if (yb) {
+#pragma unroll
+            for (int j = 0; j < HALF; ++j)
+              if (j < valid) yb[(long long)j * p.hw] = acc[j];
+          }
+        }
+      } else if (p.y_hi)  // position m of the flattened (b, oh, ow) index is row m of the NHWC tensor
         store_channels_split<HALF, false>(acc, yb, p.hw, p.K - n0, has_bias ? bias_s[warp - 2] : nullptr, p.ep.act,
                                           (float)p.ep.alpha, m < p.Mtot, p.y_hi + (m < p.Mtot ? m : 0) * p.K + n0,
                                           p.y_lo + (m < p.Mtot ? m : 0) * p.K + n0);
@@ -348,6 +397,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
         store_channels<HALF>(acc, yb, p.hw, p.K - n0, has_bias ? bias_s[warp - 2] : nullptr, p.ep.act,
                              (float)p.ep.alpha);
     }
+    if (F16 && p.out16.rec) stats.deliver(p.out16.rec);
     if (!ok) s_fail = 1;
   }
 
@@ -360,11 +410,62 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
   }
 }
 
-// x (B, C, HW) -> head/tail (B, HW, C): channels innermost, each value split into its TF32 head
-// and the TF32 rounding of the remainder. One 32 x 32 tile per step through shared memory, so both
+// Where a rewrite puts its pairs: TF32 (float tensors) or fp16 (half tensors, scaled by what *rec says).
+struct NhwcOut {
+  void *hi, *lo;
+  F16Rec *rec;         // F16: in: the largest magnitude; out: the exponent used, and the small values
+  const int *only_if;  // TF32: skip_launch
+};
+template <bool F16>
+__device__ __forceinline__ float nhwc_begin(const NhwcOut &out) {
+  if (!F16) return 1.f;
+  const int ex = f16_scale_exp(*(volatile const unsigned *)&out.rec->amax);
+  if (blockIdx.x == 0 && threadIdx.x == 0) out.rec->scale_exp = ex;
+  return pow2(ex);
+}
+// N (4 or 1) neighbouring channels at element `at`
+template <bool F16, int N>
+__device__ __forceinline__ void nhwc_store(const NhwcOut &out, long long at, const float (&v)[N], float scale,
+                                           unsigned &small) {
+  if (F16) {
+    __align__(8) __half h[4], l[4];
+#pragma unroll
+    for (int k = 0; k < N; ++k) small += f16_pair(v[k], scale, h[k], l[k]) ? 1u : 0u;
+    __half *hp = (__half *)out.hi + at, *lp = (__half *)out.lo + at;
+    if (N == 4) {
+      *reinterpret_cast<uint2 *>(hp) = *reinterpret_cast<const uint2 *>(h);
+      *reinterpret_cast<uint2 *>(lp) = *reinterpret_cast<const uint2 *>(l);
+    } else {
+      *hp = h[0];
+      *lp = l[0];
+    }
+  } else {
+    float h[4], l[4];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      h[k] = ct_tf32(v[k]);
+      l[k] = ct_tf32(__fsub_rn(v[k], h[k]));
+    }
+    float *hp = (float *)out.hi + at, *lp = (float *)out.lo + at;
+    if (N == 4) {
+      *reinterpret_cast<float4 *>(hp) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4 *>(lp) = make_float4(l[0], l[1], l[2], l[3]);
+    } else {
+      *hp = h[0];
+      *lp = l[0];
+    }
+  }
+}
+
+// x (B, C, HW) -> head/tail (B, HW, C): channels innermost, each value split into its head and the
+// rounding of the remainder. One 32 x 32 tile per step through shared memory, so both
 // the reads (along HW) and the writes (along C) are contiguous.
-__global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict__ x, float *__restrict__ hi,
-                                                         float *__restrict__ lo, long long B, int C, int HW) {
+template <bool F16>
+__global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict__ x, NhwcOut out, long long B, int C,
+                                                         int HW) {
+  if (!F16 && skip_launch(out.only_if)) return;
+  const float scale = nhwc_begin<F16>(out);
+  unsigned small = 0;
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int ptiles = (HW + 31) / 32, ctiles = (C + 31) / 32;
@@ -386,15 +487,13 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
     for (int j = ty; j < 32; j += 8) {
       const int pp = p0 + j, c = c0 + tx;
       if (pp < HW && c < C) {
-        const float v = tile[tx][j];
-        const float h = ct_tf32(v);
-        const long long o = ob + (long long)pp * C + c;
-        hi[o] = h;
-        lo[o] = ct_tf32(__fsub_rn(v, h));
+        const float v[1] = {tile[tx][j]};
+        nhwc_store<F16, 1>(out, ob + (long long)pp * C + c, v, scale, small);
       }
     }
     __syncthreads();
   }
+  if (F16 && small) atomicAdd(&out.rec->small, small);  // rare
 }
 
 // The same rewrite for planes whose size is a multiple of 4 (so every channel row starts on a
@@ -402,9 +501,12 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
 // (512 contiguous bytes per warp and channel), turned in shared memory (row pitch 129 words: the
 // four channels a thread gathers for one position fall into distinct banks), and written as float4
 // along the channels, CT * 4 contiguous bytes per position.
-template <int CT>
-__global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restrict__ x, float *__restrict__ hi,
-                                                          float *__restrict__ lo, long long B, int C, int HW) {
+template <int CT, bool F16>
+__global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restrict__ x, NhwcOut out, long long B, int C,
+                                                          int HW) {
+  if (!F16 && skip_launch(out.only_if)) return;
+  const float scale = nhwc_begin<F16>(out);
+  unsigned small = 0;
   constexpr int PT = 128, PITCH = PT + 1;
   __shared__ float tile[CT * PITCH];
   const int ptiles = (HW + PT - 1) / PT, ctiles = C / CT;
@@ -426,34 +528,32 @@ __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restric
     }
     __syncthreads();
     // store: thread -> (position, group of 4 channels), channel groups fastest
-    float *ho = hi + (b * HW + p0) * (long long)C + c0;
-    float *lo_o = lo + (b * HW + p0) * (long long)C + c0;
+    const long long o0 = (b * HW + p0) * (long long)C + c0;
 #pragma unroll
     for (int i = threadIdx.x; i < PT * (CT / 4); i += 256) {
       const int pp = i / (CT / 4), cg = i - pp * (CT / 4);
       if (p0 + pp < HW) {
-        float v[4], h[4], l[4];
+        float v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          v[k] = tile[(4 * cg + k) * PITCH + pp];
-          h[k] = ct_tf32(v[k]);
-          l[k] = ct_tf32(__fsub_rn(v[k], h[k]));
-        }
-        *reinterpret_cast<float4 *>(ho + (long long)pp * C + 4 * cg) = make_float4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<float4 *>(lo_o + (long long)pp * C + 4 * cg) = make_float4(l[0], l[1], l[2], l[3]);
+        for (int k = 0; k < 4; ++k) v[k] = tile[(4 * cg + k) * PITCH + pp];
+        nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, small);
       }
     }
     __syncthreads();
   }
+  if (F16 && small) atomicAdd(&out.rec->small, small);
 }
 
 // The same rewrite for small planes of any size (7x7, 13x13): a block takes 32 channels of one
 // image, which are 32 * HW contiguous floats starting on a 16-byte boundary whatever HW is, loads
 // them as float4, and writes every position's 32 channels as float4. The shared-memory pitch is
 // HW rounded up to 1 (mod 8), which spreads the (position, channel group) reads over all banks.
-__global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__restrict__ x, float *__restrict__ hi,
-                                                             float *__restrict__ lo, long long B, int C, int HW,
-                                                             int pitch) {
+template <bool F16>
+__global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__restrict__ x, NhwcOut out, long long B,
+                                                             int C, int HW, int pitch) {
+  if (!F16 && skip_launch(out.only_if)) return;
+  const float scale = nhwc_begin<F16>(out);
+  unsigned small = 0;
   extern __shared__ __align__(16) float img[];
   const int chunks = C >> 5;
   const long long total = B * chunks;
@@ -473,44 +573,31 @@ __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__rest
       }
     }
     __syncthreads();
-    float *ho = hi + (b * HW) * (long long)C + c0;
-    float *lo_o = lo + (b * HW) * (long long)C + c0;
+    const long long o0 = (b * HW) * (long long)C + c0;
     for (int i = threadIdx.x; i < HW * 8; i += 256) {
       const int pp = i >> 3, cg = i & 7;
-      float h[4], l[4];
+      float v[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float v = img[(4 * cg + k) * pitch + pp];
-        h[k] = ct_tf32(v);
-        l[k] = ct_tf32(__fsub_rn(v, h[k]));
-      }
-      *reinterpret_cast<float4 *>(ho + (long long)pp * C + 4 * cg) = make_float4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<float4 *>(lo_o + (long long)pp * C + 4 * cg) = make_float4(l[0], l[1], l[2], l[3]);
+      for (int k = 0; k < 4; ++k) v[k] = img[(4 * cg + k) * pitch + pp];
+      nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, small);
     }
     __syncthreads();
   }
+  if (F16 && small) atomicAdd(&out.rec->small, small);
 }
 
 // Rewrites x (B, C, HW) as NHWC TF32 head/tail into two fresh arena blocks xs[0], xs[1], which the
 // caller releases.
-static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, void **xs);
-int conv_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, void **xs) {
-  const long long xbytes = B * C * HW * 4;
-  xs[0] = xs[1] = nullptr;
-  int rc = b200_get(e, xbytes, &xs[0]);
-  if (rc == B200_OK) rc = b200_get(e, xbytes, &xs[1]);
-  if (rc != B200_OK) return rc;
-  return launch_nhwc_split(e, x, B, C, HW, xs);
-}
-static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, void **xs) {
+template <bool F16>
+static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, const NhwcOut &out) {
   if (HW % 4 == 0 && C % 16 == 0 && (uintptr_t)x % 16 == 0) {
     const int ct = C % 32 == 0 ? 32 : 16;
     const long long tiles = B * ((HW + 127) / 128) * (C / ct);
     const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, e->sm_count * 32LL));
     if (ct == 32)
-      nhwc_split4_kernel<32><<<blocks, 256, 0, e->stream>>>(x, (float *)xs[0], (float *)xs[1], B, C, HW);
+      nhwc_split4_kernel<32, F16><<<blocks, 256, 0, e->stream>>>(x, out, B, C, HW);
     else
-      nhwc_split4_kernel<16><<<blocks, 256, 0, e->stream>>>(x, (float *)xs[0], (float *)xs[1], B, C, HW);
+      nhwc_split4_kernel<16, F16><<<blocks, 256, 0, e->stream>>>(x, out, B, C, HW);
     B200_CHECK_LAUNCH(e, "nhwc_split4_kernel");
     return B200_OK;
   }
@@ -519,22 +606,33 @@ static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C,
     while (pitch % 8 != 1) ++pitch;
     const long long work = B * (C / 32);
     const int blocks = (int)std::max<long long>(1, std::min<long long>(work, e->sm_count * 16LL));
-    nhwc_split_img_kernel<<<blocks, 256, (size_t)32 * pitch * 4, e->stream>>>(x, (float *)xs[0], (float *)xs[1], B, C,
-                                                                             HW, pitch);
+    nhwc_split_img_kernel<F16><<<blocks, 256, (size_t)32 * pitch * 4, e->stream>>>(x, out, B, C, HW, pitch);
     B200_CHECK_LAUNCH(e, "nhwc_split_img_kernel");
     return B200_OK;
   }
   const long long tiles = B * ((HW + 31) / 32) * ((C + 31) / 32);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, e->sm_count * 16LL));
-  nhwc_split_kernel<<<blocks, 256, 0, e->stream>>>(x, (float *)xs[0], (float *)xs[1], B, C, HW);
+  nhwc_split_kernel<F16><<<blocks, 256, 0, e->stream>>>(x, out, B, C, HW);
   B200_CHECK_LAUNCH(e, "nhwc_split_kernel");
   return B200_OK;
+}
+int conv_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, void **xs) {
+  const long long xbytes = B * C * HW * 4;
+  xs[0] = xs[1] = nullptr;
+  int rc = b200_get(e, xbytes, &xs[0]);
+  if (rc == B200_OK) rc = b200_get(e, xbytes, &xs[1]);
+  if (rc != B200_OK) return rc;
+  return launch_nhwc_split<false>(e, x, B, C, HW, NhwcOut{xs[0], xs[1], nullptr, e->only_if});
 }
 
 // The same rewrite into buffers the caller owns (B * C * HW floats each).
 int conv_nhwc_split_into(b200_engine *e, const float *x, long long B, int C, int HW, float *hi, float *lo) {
-  void *xs[2] = {hi, lo};
-  return launch_nhwc_split(e, x, B, C, HW, xs);
+  return launch_nhwc_split<false>(e, x, B, C, HW, NhwcOut{hi, lo, nullptr, nullptr});
+}
+
+// As pairs of fp16: heads, then tails, from `pairs` on. rec holds the largest magnitude of x.
+int conv_nhwc_pairs(b200_engine *e, const float *x, long long B, int C, int HW, __half *pairs, F16Rec *rec) {
+  return launch_nhwc_split<true>(e, x, B, C, HW, NhwcOut{pairs, pairs + B * C * HW, rec, nullptr});
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -553,10 +651,10 @@ static void *driver_entry(const char *name) {
   return nullptr;
 }
 
-template <int BN, int CK>
+template <int BN, int ROW_BYTES, bool F16>
 static int launch_conv_tma(b200_engine *e, const CUtensorMap *tm, ConvTmaParams &p) {
-  constexpr int STAGE_BYTES = 2 * (CT_BM + BN) * CK * 4;
-  auto kern = conv_tma_kernel<BN, CK>;
+  constexpr int STAGE_BYTES = 2 * (CT_BM + BN) * ROW_BYTES;
+  auto kern = conv_tma_kernel<BN, ROW_BYTES, F16>;
   static std::atomic<int> attr_dev_mask{0};  // devices on which the attribute is set; engines on other threads share it
   const size_t optin = std::min<size_t>(e->smem_optin, 227 * 1024);
   if (!(attr_dev_mask & (1 << (e->device & 31)))) {
@@ -627,23 +725,81 @@ bool conv_tma_eligible(long long B, int C, int H, int W, int kh, int kw, int pad
   return true;
 }
 
-// x (B,C,H,W) * w (K,C,kh,kw) -> y (B,K,Ho,Wo), float32. ep.bias_kind ROW = one value per channel.
-int conv2d_tma(b200_engine *e, const float *x, const float *w, float *y, long long B, int C, int H, int W, int K,
-               int kh, int kw, int padH, int padW, int sH, int sW, int dH, int dW, int Ho, int Wo,
-               const Epilogue &ep, const float *x_hi, const float *x_lo, float *y_hi, float *y_lo) {
+// The tensor maps of a convolution and its launch. xin / win: heads and tails, `es` bytes per value.
+static int conv_tma_run(b200_engine *e, int es, int ck, const void *const *xin, const void *const *win, long long wld,
+                        long long B, int C, int H, int W, int K, int kh, int kw, int padH, int padW, int sH, int sW,
+                        int dH, int dW, int Ho, int Wo, ConvTmaParams &p) {
   static EncodeTiledFn enc_tiled = (EncodeTiledFn)driver_entry("cuTensorMapEncodeTiled");
   static EncodeIm2colFn enc_im2col = (EncodeIm2colFn)driver_entry("cuTensorMapEncodeIm2col");
   if (!enc_tiled || !enc_im2col)
     return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled / cuTensorMapEncodeIm2col are not available");
   const int taps = kh * kw, crs = C * taps;
-  const int ck = 32;
-  const CUtensorMapSwizzle swz = CU_TENSOR_MAP_SWIZZLE_128B;
+  const CUtensorMapSwizzle swz = ck * es == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  const CUtensorMapDataType type = es == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
 
+  int bn = 128;
+  while (bn > 32 && bn / 2 >= K) bn /= 2;
+  p.Mtot = B * Ho * Wo;
+  p.K = K; p.Wo = Wo; p.hw = Ho * Wo;
+  p.kw = kw; p.padH = padH; p.padW = padW; p.sH = sH; p.sW = sW; p.dH = dH; p.dW = dW;
+  p.cblocks = C / ck;
+  p.num_k = taps * p.cblocks;
+  // accumulation chains of 32 steps of TF32, 24 of fp16 (as in gemm_tc.cu)
+  p.chunk_k = es == 2 ? 24 / (ck / 16) : 256 / ck;
+  p.tiles_m = (int)((p.Mtot + CT_BM - 1) / CT_BM);
+  p.tiles_n = (K + bn - 1) / bn;
+  p.err_flag = e->d_flags + 2;
+
+  CUtensorMap tm[4];
+  memset((void *)tm, 0, sizeof tm);
+  // activations as (C, W, H, N); the bounding box of window origins runs from -pad to the last
+  // origin whose window still touches the padded image
+  cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)C * es, (cuuint64_t)W * C * es, (cuuint64_t)H * W * C * es};
+  int lower[2] = {-padW, -padH};
+  int upper[2] = {padW - (kw - 1) * dW, padH - (kh - 1) * dH};
+  cuuint32_t estr[4] = {1, (cuuint32_t)sW, (cuuint32_t)sH, 1};
+  for (int h = 0; h < 2; ++h) {
+    CUresult r = enc_im2col(&tm[h], type, 4, const_cast<void *>(xin[h]), dims, strides, lower, upper, (cuuint32_t)ck,
+                            CT_BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+      return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeIm2col failed (%d): C %d W %d H %d N %lld", (int)r, C, W, H, B);
+  }
+  // filters as (crs, K, 1), box ck x bn
+  cuuint64_t wdims[3] = {(cuuint64_t)crs, (cuuint64_t)K, 1};
+  cuuint64_t wstrides[2] = {(cuuint64_t)wld * es, (cuuint64_t)K * wld * es};
+  cuuint32_t wbox[3] = {(cuuint32_t)ck, (cuuint32_t)bn, 1};
+  cuuint32_t westr[3] = {1, 1, 1};
+  for (int h = 0; h < 2; ++h) {
+    CUresult r = enc_tiled(&tm[2 + h], type, 3, const_cast<void *>(win[h]), wdims, wstrides, wbox, westr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for filters", (int)r);
+  }
+  if (es == 4) {
+    if (bn == 128) return launch_conv_tma<128, 128, false>(e, tm, p);
+    if (bn == 64) return launch_conv_tma<64, 128, false>(e, tm, p);
+    return launch_conv_tma<32, 128, false>(e, tm, p);
+  }
+  if (ck == 64) {
+    if (bn == 128) return launch_conv_tma<128, 128, true>(e, tm, p);
+    if (bn == 64) return launch_conv_tma<64, 128, true>(e, tm, p);
+    return launch_conv_tma<32, 128, true>(e, tm, p);
+  }
+  if (bn == 128) return launch_conv_tma<128, 64, true>(e, tm, p);
+  if (bn == 64) return launch_conv_tma<64, 64, true>(e, tm, p);
+  return launch_conv_tma<32, 64, true>(e, tm, p);
+}
+
+// x (B,C,H,W) * w (K,C,kh,kw) -> y (B,K,Ho,Wo), float32. ep.bias_kind ROW = one value per channel.
+int conv2d_tma(b200_engine *e, const float *x, const float *w, float *y, long long B, int C, int H, int W, int K,
+               int kh, int kw, int padH, int padW, int sH, int sW, int dH, int dW, int Ho, int Wo,
+               const Epilogue &ep, const float *x_hi, const float *x_lo, float *y_hi, float *y_lo) {
   TcOperand wf;
   void *wblk[2] = {nullptr, nullptr};
-  int rc = conv_filters_tap_major(e, w, K, C, taps, &wf, wblk);
+  int rc = conv_filters_tap_major(e, w, K, C, kh * kw, &wf, wblk);
   if (rc != B200_OK) return rc;
-
   // activations: NHWC, TF32 head and tail
   void *xs[2] = {nullptr, nullptr};
   const void *xin[2] = {x_hi, x_lo};  // the caller's pre-split input, or this call's own rewrite
@@ -652,65 +808,35 @@ int conv2d_tma(b200_engine *e, const float *x, const float *w, float *y, long lo
     xin[0] = xs[0];
     xin[1] = xs[1];
   }
-
-  int bn = 128;
-  while (bn > 32 && bn / 2 >= K) bn /= 2;
   ConvTmaParams p = ConvTmaParams();
   p.y = y;
   p.y_hi = y_hi;
   p.y_lo = y_lo;
-  p.Mtot = B * Ho * Wo;
-  p.K = K; p.Wo = Wo; p.hw = Ho * Wo;
-  p.kw = kw; p.padH = padH; p.padW = padW; p.sH = sH; p.sW = sW; p.dH = dH; p.dW = dW;
-  p.cblocks = C / ck;
-  p.num_k = taps * p.cblocks;
-  p.chunk_k = 256 / ck;
-  p.tiles_m = (int)((p.Mtot + CT_BM - 1) / CT_BM);
-  p.tiles_n = (K + bn - 1) / bn;
   p.ep = ep;
-  p.err_flag = e->d_flags + 2;
-
-  CUtensorMap tm[4];
-  memset((void *)tm, 0, sizeof tm);
-  if (rc == B200_OK) {
-    // activations as (C, W, H, N); the bounding box of window origins runs from -pad to the last
-    // origin whose window still touches the padded image
-    cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    cuuint64_t strides[3] = {(cuuint64_t)C * 4, (cuuint64_t)W * C * 4, (cuuint64_t)H * W * C * 4};
-    int lower[2] = {-padW, -padH};
-    int upper[2] = {padW - (kw - 1) * dW, padH - (kh - 1) * dH};
-    cuuint32_t estr[4] = {1, (cuuint32_t)sW, (cuuint32_t)sH, 1};
-    for (int h = 0; h < 2 && rc == B200_OK; ++h) {
-      CUresult r = enc_im2col(&tm[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void *>(xin[h]), dims, strides,
-                              lower, upper,
-                              (cuuint32_t)ck, CT_BM, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS)
-        rc = set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeIm2col failed (%d): C %d W %d H %d N %lld", (int)r, C, W,
-                       H, B);
-    }
-    // filters as (crs, K, 1), box ck x bn
-    cuuint64_t wdims[3] = {(cuuint64_t)crs, (cuuint64_t)K, 1};
-    cuuint64_t wstrides[2] = {(cuuint64_t)wf.ld * 4, (cuuint64_t)K * wf.ld * 4};
-    cuuint32_t wbox[3] = {(cuuint32_t)ck, (cuuint32_t)bn, 1};
-    cuuint32_t westr[3] = {1, 1, 1};
-    for (int h = 0; h < 2 && rc == B200_OK; ++h) {
-      CUresult r = enc_tiled(&tm[2 + h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(h ? wf.p1 : wf.p0),
-                             wdims, wstrides, wbox, westr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) rc = set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for filters", (int)r);
-    }
-  }
-  if (rc == B200_OK) {
-    if (bn == 128) rc = launch_conv_tma<128, 32>(e, tm, p);
-    else if (bn == 64) rc = launch_conv_tma<64, 32>(e, tm, p);
-    else rc = launch_conv_tma<32, 32>(e, tm, p);
-  }
+  p.only_if = e->only_if;
+  const void *win[2] = {wf.p0, wf.p1};
+  if (rc == B200_OK)
+    rc = conv_tma_run(e, 4, 32, xin, win, wf.ld, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho, Wo, p);
   for (int h = 0; h < 2; ++h) {
     if (xs[h]) b200_put(e, xs[h], 0);
     if (wblk[h]) b200_put(e, wblk[h], 0);
   }
   return rc;
+}
+
+// The same from pairs of fp16: x_pairs / wf as pairs.cuh says, their records in `in`. y (NCHW) and out.h may
+// be null, not both.
+int conv2d_tma_pairs(b200_engine *e, const __half *x_pairs, const TcOperand &wf, float *y, long long B, int C, int H,
+                     int W, int K, int kh, int kw, int padH, int padW, int sH, int sW, int dH, int dW, int Ho, int Wo,
+                     const Epilogue &ep, const PairsIn &in, const PairsOut &out) {
+  ConvTmaParams p = ConvTmaParams();
+  p.y = y;
+  p.ep = ep;
+  p.in16 = in;
+  p.out16 = out;
+  const void *xin[2] = {x_pairs, x_pairs + B * C * H * W}, *win[2] = {wf.p0, wf.p1};
+  return conv_tma_run(e, 2, C % 64 == 0 ? 64 : 32, xin, win, wf.ld, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW,
+                      Ho, Wo, p);
 }
 
 }  // namespace b200

@@ -21,12 +21,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstring>
-
 #include <atomic>
+#include <cstring>
+#include <type_traits>
 
 #include "engine.h"
 #include "epilogue.cuh"
+#include "pairs.cuh"
 #include "ptx.cuh"
 #include "tc_common.cuh"
 #include "tc_operand.h"
@@ -55,6 +56,9 @@ struct ConvWinParams {
   int tiles_h, tiles_w, tiles_n;
   long long total_tiles;  // B * tiles_h * tiles_w * tiles_n
   int b_stages;
+  PairsIn in16;       // F16: the operands, and
+  PairsOut out16;     // the (pooled) output in pairs form (h may be null) and what is recorded of it
+  const int *only_if; // TF32: run only if this word says so (skip_launch)
   Epilogue ep;       // bias_kind ROW = per output channel
   int pool2;         // fold a 2x2 / stride-2 max-pool into the store: y is (B, K, Ho/2, Wo/2)
   int *err_flag;
@@ -78,19 +82,24 @@ __device__ __forceinline__ void cw_tma_load_4d(void *smem_dst, const void *tmap,
       : "memory");
 }
 
-template <int BN, int CK>
+// F16: pairs of fp16 (pairs.cuh) instead of TF32 pairs: half the bytes per channel, and half the instructions,
+// which is what bounds this kernel: an instruction reads 128 rows of 32 bytes, 16 channels of fp16 against 8.
+// 16 -> 32 channels with pool on 208 x 208 planes of 64 images: 337 -> 315 us; 32 -> 64 on 104 x 104:
+// 147 -> 130.
+template <int BN, int CK, bool F16>
 __global__ void __launch_bounds__(CW_THREADS, 1)
     conv_win_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                     const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                     const __grid_constant__ ConvWinParams p) {
-  constexpr int ROW_BYTES = CK * 4;
+  constexpr int ROW_BYTES = CK * (F16 ? 2 : 4);
   constexpr int B_BYTES = BN * ROW_BYTES;
   constexpr int B_STAGE_BYTES = 2 * B_BYTES;      // head + tail
   constexpr uint32_t B_SBO = 8 * ROW_BYTES;
-  constexpr uint32_t LAYOUT = CK == 32 ? 2 : 4;   // 128-byte / 64-byte swizzle
-  constexpr int KK = CK / 8;                      // MMAs (k = 8) per k-block
-  constexpr uint32_t IDESC = make_idesc(2, 0, 0, 128, BN);
-  constexpr uint32_t IDESC2 = make_idesc(2, 0, 0, 128, 2 * BN);  // [head | tail] filter slabs as one operand
+  constexpr uint32_t LAYOUT = ROW_BYTES == 128 ? 2 : (ROW_BYTES == 64 ? 4 : 6);  // 128 / 64 / 32-byte swizzle
+  constexpr int KK = ROW_BYTES / 32;              // MMAs (k = 8 or 16) per k-block
+  constexpr uint32_t FMT = F16 ? 0 : 2;
+  constexpr uint32_t IDESC = make_idesc(FMT, 0, 0, 128, BN);
+  constexpr uint32_t IDESC2 = make_idesc(FMT, 0, 0, 128, 2 * BN);  // [head | tail] filter slabs as one operand
   constexpr int ACC_COLS = 4 * BN;                // two tile halves x (main + cross-term)
   constexpr int TMEM_COLS = 2 * ACC_COLS;         // double-buffered: 256 (BN 32) or 512 (BN 64)
 
@@ -101,6 +110,8 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
   __shared__ int s_fail;
   __shared__ float bias_s[8][BN];
 
+  // the same answer in every thread of the grid
+  if (F16 ? !pairs_usable(p.in16, p.out16.rec) : skip_launch(p.only_if)) return;
   unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)cw_smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char *smem_b = smem + (size_t)CW_WIN_STAGES * 2 * p.win_bytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -237,7 +248,7 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
             ptx::tc_fence_after_sync();
             const uint32_t sb = smem_b_u + (uint32_t)bs * B_STAGE_BYTES;
             const uint32_t row0 = (uint32_t)((r * p.dH) * p.win_w + sx * p.dW);
-            // low descriptor words: (address >> 4) | LBO field; a k step of 8 floats adds 32 bytes = 2
+            // low descriptor words: (address >> 4) | LBO field; a k step adds 32 bytes = 2
             const uint32_t a_lo32 = desc_lo(win + row0 * ROW_BYTES);
             const uint32_t a_lo32_tail = desc_lo(win + (uint32_t)p.win_bytes + row0 * ROW_BYTES);
             const uint32_t b_lo32 = desc_lo(sb);
@@ -254,8 +265,13 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
                 // head x [head | tail] of the filters is ONE instruction of width 2*BN: the filter
                 // tail slab follows the head slab in shared memory, the cross-term accumulator
                 // follows the main one in tensor memory.
-                ptx::mma_tf32(d, a_hi, b_hi, IDESC2, accumulate);
-                ptx::mma_tf32(d + BN, a_lo, b_hi, IDESC, 1u);
+                if (F16) {
+                  ptx::mma_f16(d, a_hi, b_hi, IDESC2, accumulate);
+                  ptx::mma_f16(d + BN, a_lo, b_hi, IDESC, 1u);
+                } else {
+                  ptx::mma_tf32(d, a_hi, b_hi, IDESC2, accumulate);
+                  ptx::mma_tf32(d + BN, a_lo, b_hi, IDESC, 1u);
+                }
               }
               ptx::mma_commit(&b_empty[bs]);
             }
@@ -289,6 +305,17 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
     const int num_k = taps * p.cblocks;
     const bool has_bias = p.ep.bias_kind != B200_BIAS_NONE;
     const float *bias_g = reinterpret_cast<const float *>(p.ep.bias);
+    float unscale1 = 1.f, unscale2 = 1.f, out_scale = 1.f;
+    PairStats stats;
+    if (F16) {
+      f16_unscale(p.in16.x->scale_exp, p.in16.w->rec.scale_exp, unscale1, unscale2);
+      if (p.out16.h) {
+        const int ex = pairs_out_exp(__uint_as_float(p.in16.x->amax), __uint_as_float(p.in16.w->l1),
+                                     has_bias ? bias_g : nullptr, p.K, p.ep.act, (float)p.ep.alpha);
+        out_scale = pow2(ex);
+        if (blockIdx.x == 0 && warp == 2 && lane == 0) p.out16.rec->scale_exp = ex;
+      }
+    }
     int use = 0;
     bool ok = true;
     for (long long tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
@@ -312,7 +339,9 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
           ptx::tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            acc[c + j] = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(rm[j]), __uint_as_float(rt[j])));
+            acc[c + j] = __fadd_rn(acc[c + j], __fadd_rn(__uint_as_float(rm[j]),
+                                                         F16 ? __fmul_rn(__uint_as_float(rt[j]), 4.8828125e-4f)
+                                                             : __uint_as_float(rt[j])));
         }
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -334,7 +363,46 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
         __syncwarp();
       }
       const float *bias_w = has_bias ? bias_s[warp - 2] : nullptr;
-      if (p.pool2) {
+      if (F16) {
+#pragma unroll
+        for (int j = 0; j < BN; ++j) acc[j] = __fmul_rn(__fmul_rn(acc[j], unscale1), unscale2);
+        const bool inside = oh < p.Ho && ow < p.Wo;
+        const int Hq = p.pool2 ? p.Ho >> 1 : p.Ho, Wq = p.pool2 ? p.Wo >> 1 : p.Wo;
+        const int qh = p.pool2 ? oh >> 1 : oh, qw = p.pool2 ? ow >> 1 : ow;
+        const long long plane = (long long)Hq * Wq;
+        const long long pos = inside ? ((long long)b * Hq + qh) * Wq + qw : 0;
+        auto store = [&](float *v, int c0, auto size) {  // channels from column c0 of this tile on
+          constexpr int N = decltype(size)::value;
+          const int valid = p.K - n0 - c0;
+#pragma unroll
+          for (int j = 0; j < N; ++j)
+            if (j < valid) stats.see(v[j]);
+          if (p.out16.h)
+            store_pairs<N>(v, valid, out_scale, p.out16.h + pos * p.K + n0 + c0, p.out16.l + pos * p.K + n0 + c0, stats);
+          if (p.y) {
+            float *yb = p.y + ((long long)b * p.K + n0 + c0) * plane + (long long)qh * Wq + qw;
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+              if (j < valid) yb[(long long)j * plane] = v[j];
+          }
+        };
+        if (p.pool2) {
+          // the window's four lanes share the channels out (store_channels_pool4); the order of the four
+          // sums is that of their activated values unless a slope is negative, and numbers that are not
+          // finite are marked for the way behind this one
+          float q[BN / 4];
+          const bool b0 = (lane & 1) != 0, b1 = (lane & 8) != 0;
+          if (p.ep.act == B200_ACT_LEAKY && !((float)p.ep.alpha >= 0.f)) finish_channels<BN>(acc, bias_w, p.ep.act, (float)p.ep.alpha);
+          pool4_exchange<BN>(acc, q);
+          const int c0 = (b0 ? BN / 2 : 0) + (b1 ? BN / 4 : 0);
+          if (!(p.ep.act == B200_ACT_LEAKY && !((float)p.ep.alpha >= 0.f)))
+            finish_channels<BN / 4>(q, bias_w ? bias_w + c0 : nullptr, p.ep.act, (float)p.ep.alpha);
+          if (inside) store(q, c0, std::integral_constant<int, BN / 4>());
+        } else {
+          finish_channels<BN>(acc, bias_w, p.ep.act, (float)p.ep.alpha);
+          if (inside) store(acc, 0, std::integral_constant<int, BN>());
+        }
+      } else if (p.pool2) {
         // Ho and Wo are even, so a pooling window lies wholly inside the image or wholly outside
         const int Hq = p.Ho >> 1, Wq = p.Wo >> 1;
         const long long plane = (long long)Hq * Wq;
@@ -364,6 +432,7 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
         store_channels<BN>(acc, yb, plane, p.K - n0, bias_w, p.ep.act, (float)p.ep.alpha);
       }
     }
+    if (F16 && p.out16.rec) stats.deliver(p.out16.rec);
     if (!ok) s_fail = 1;
   }
 
@@ -391,13 +460,14 @@ static CwEncodeTiledFn cw_encode_fn() {
 
 static size_t cw_smem_budget(const b200_engine *e) { return std::min<size_t>(e->smem_optin, 227 * 1024) - 4096; }
 
-static void cw_geometry(int C, int K, int kh, int kw, int dH, int dW, int *ck, int *bn, int *win_w, int *win_h,
+// es: bytes per value, 4 (TF32; 32 or 16 channels per row) or 2 (fp16; all of 16, 32 or 64 channels)
+static void cw_geometry(int es, int C, int K, int kh, int kw, int dH, int dW, int *ck, int *bn, int *win_w, int *win_h,
                         int *win_bytes) {
-  *ck = C % 32 == 0 ? 32 : 16;
+  *ck = es == 2 ? C : (C % 32 == 0 ? 32 : 16);
   *bn = K <= 32 ? 32 : 64;
   *win_w = CW_TILE + (kw - 1) * dW;
   *win_h = CW_TILE + (kh - 1) * dH;
-  *win_bytes = ((*win_w) * (*win_h) * (*ck) * 4 + 1023) / 1024 * 1024;
+  *win_bytes = ((*win_w) * (*win_h) * (*ck) * es + 1023) / 1024 * 1024;
 }
 
 // Whether the window kernel takes a convolution: stride 1, channels 16 or a multiple of 32 (and
@@ -411,7 +481,7 @@ bool conv_win_eligible(const b200_engine *e, long long B, int C, int H, int W, i
   if (kh * kw == 1) return false;
   if (B >= (1LL << 31) || B * C * H * W * 4 < 131072) return false;
   int ck, bn, win_w, win_h, win_bytes;
-  cw_geometry(C, K, kh, kw, dH, dW, &ck, &bn, &win_w, &win_h, &win_bytes);
+  cw_geometry(4, C, K, kh, kw, dH, dW, &ck, &bn, &win_w, &win_h, &win_bytes);
   if (win_w > 256 || win_h > 256) return false;
   const size_t need = (size_t)CW_WIN_STAGES * 2 * win_bytes + 3 * (size_t)(2 * bn * ck * 4) + 1024;
   if (need > cw_smem_budget(e)) return false;
@@ -422,10 +492,10 @@ bool conv_win_eligible(const b200_engine *e, long long B, int C, int H, int W, i
   return true;
 }
 
-template <int BN, int CK>
+template <int BN, int CK, bool F16>
 static int launch_conv_win(b200_engine *e, const CUtensorMap *tm, ConvWinParams &p) {
-  constexpr int B_STAGE_BYTES = 2 * BN * CK * 4;
-  auto kern = conv_win_kernel<BN, CK>;
+  constexpr int B_STAGE_BYTES = 2 * BN * CK * (F16 ? 2 : 4);
+  auto kern = conv_win_kernel<BN, CK, F16>;
   static std::atomic<int> attr_dev_mask{0};  // devices on which the attribute is set; engines on other threads share it
   const size_t optin = std::min<size_t>(e->smem_optin, 227 * 1024);
   if (!(attr_dev_mask & (1 << (e->device & 31)))) {
@@ -446,6 +516,67 @@ static int launch_conv_win(b200_engine *e, const CUtensorMap *tm, ConvWinParams 
   return B200_OK;
 }
 
+// The tensor maps of a convolution and its launch. xin / win: heads and tails, `es` bytes per value.
+static int conv_win_run(b200_engine *e, int es, const void *const *xin, const void *const *win, long long wld,
+                        long long B, int C, int H, int W, int K, int kh, int kw, int padH, int padW, int dH, int dW,
+                        int Ho, int Wo, bool pool2, ConvWinParams &p) {
+  static CwEncodeTiledFn enc = cw_encode_fn();
+  if (!enc) return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const int taps = kh * kw, crs = C * taps;
+  int ck, bn, win_w, win_h, win_bytes;
+  cw_geometry(es, C, K, kh, kw, dH, dW, &ck, &bn, &win_w, &win_h, &win_bytes);
+  const int row = ck * es;
+  const CUtensorMapSwizzle swz = row == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                            : (row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+  const CUtensorMapDataType type = es == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  p.K = K; p.Ho = Ho; p.Wo = Wo;
+  p.kh = kh; p.kw = kw; p.dH = dH; p.dW = dW; p.padH = padH; p.padW = padW;
+  p.win_w = win_w;
+  p.win_bytes = win_bytes;
+  p.cblocks = C / ck;
+  p.C = C;
+  // accumulation chains of 32 steps of TF32, 24 of fp16 (as in gemm_tc.cu)
+  p.chunk_k = es == 2 ? 24 / (ck / 16) : 256 / ck;
+  p.tiles_h = (Ho + CW_TILE - 1) / CW_TILE;
+  p.tiles_w = (Wo + CW_TILE - 1) / CW_TILE;
+  p.tiles_n = (K + bn - 1) / bn;
+  p.total_tiles = B * p.tiles_h * p.tiles_w * p.tiles_n;
+  p.pool2 = pool2 ? 1 : 0;
+  p.err_flag = e->d_flags + 2;
+
+  CUtensorMap tm[4];
+  memset((void *)tm, 0, sizeof tm);
+  // activations as (C, W, H, N), box = CK channels x window; positions outside the image read as zero
+  cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+  cuuint64_t strides[3] = {(cuuint64_t)C * es, (cuuint64_t)W * C * es, (cuuint64_t)H * W * C * es};
+  cuuint32_t box[4] = {(cuuint32_t)ck, (cuuint32_t)win_w, (cuuint32_t)win_h, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  for (int h = 0; h < 2; ++h) {
+    CUresult r = enc(&tm[h], type, 4, const_cast<void *>(xin[h]), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+      return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a %d x %d window", (int)r, win_w, win_h);
+  }
+  cuuint64_t wdims[3] = {(cuuint64_t)crs, (cuuint64_t)K, 1};
+  cuuint64_t wstrides[2] = {(cuuint64_t)wld * es, (cuuint64_t)K * wld * es};
+  cuuint32_t wbox[3] = {(cuuint32_t)ck, (cuuint32_t)bn, 1};
+  cuuint32_t westr[3] = {1, 1, 1};
+  for (int h = 0; h < 2; ++h) {
+    CUresult r = enc(&tm[2 + h], type, 3, const_cast<void *>(win[h]), wdims, wstrides, wbox, westr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for filters", (int)r);
+  }
+  if (es == 4) {
+    if (ck == 32) return bn == 64 ? launch_conv_win<64, 32, false>(e, tm, p) : launch_conv_win<32, 32, false>(e, tm, p);
+    return bn == 64 ? launch_conv_win<64, 16, false>(e, tm, p) : launch_conv_win<32, 16, false>(e, tm, p);
+  }
+  if (ck == 64) return bn == 64 ? launch_conv_win<64, 64, true>(e, tm, p) : launch_conv_win<32, 64, true>(e, tm, p);
+  if (ck == 32) return bn == 64 ? launch_conv_win<64, 32, true>(e, tm, p) : launch_conv_win<32, 32, true>(e, tm, p);
+  return bn == 64 ? launch_conv_win<64, 16, true>(e, tm, p) : launch_conv_win<32, 16, true>(e, tm, p);
+}
+
 // x (B,C,H,W) * w (K,C,kh,kw) -> y (B,K,Ho,Wo), float32, stride 1. ep.bias_kind ROW = per channel.
 // pool2 (Ho, Wo even): y is (B,K,Ho/2,Wo/2), the 2x2 / stride-2 max-pool of the activated output.
 // x_hi / x_lo: the input already in NHWC TF32 head / tail form (x is then unused). y_hi / y_lo: the
@@ -453,16 +584,9 @@ static int launch_conv_win(b200_engine *e, const CUtensorMap *tm, ConvWinParams 
 int conv2d_win(b200_engine *e, const float *x, const float *w, float *y, long long B, int C, int H, int W, int K,
                int kh, int kw, int padH, int padW, int dH, int dW, int Ho, int Wo, const Epilogue &ep, bool pool2,
                const float *x_hi, const float *x_lo, float *y_hi, float *y_lo) {
-  static CwEncodeTiledFn enc = cw_encode_fn();
-  if (!enc) return set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  const int taps = kh * kw, crs = C * taps;
-  int ck, bn, win_w, win_h, win_bytes;
-  cw_geometry(C, K, kh, kw, dH, dW, &ck, &bn, &win_w, &win_h, &win_bytes);
-  const CUtensorMapSwizzle swz = ck == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-
   TcOperand wf;
   void *wblk[2] = {nullptr, nullptr};
-  int rc = conv_filters_tap_major(e, w, K, C, taps, &wf, wblk);
+  int rc = conv_filters_tap_major(e, w, K, C, kh * kw, &wf, wblk);
   if (rc != B200_OK) return rc;
   void *xs[2] = {nullptr, nullptr};
   const void *xin[2] = {x_hi, x_lo};  // the caller's pre-split input, or this call's own rewrite
@@ -471,67 +595,33 @@ int conv2d_win(b200_engine *e, const float *x, const float *w, float *y, long lo
     xin[0] = xs[0];
     xin[1] = xs[1];
   }
-
   ConvWinParams p = ConvWinParams();
   p.y = y;
   p.y_hi = y_hi;
   p.y_lo = y_lo;
-  p.K = K; p.Ho = Ho; p.Wo = Wo;
-  p.kh = kh; p.kw = kw; p.dH = dH; p.dW = dW; p.padH = padH; p.padW = padW;
-  p.win_w = win_w;
-  p.win_bytes = win_bytes;
-  p.cblocks = C / ck;
-  p.C = C;
-  p.chunk_k = 256 / ck;
-  p.tiles_h = (Ho + CW_TILE - 1) / CW_TILE;
-  p.tiles_w = (Wo + CW_TILE - 1) / CW_TILE;
-  p.tiles_n = (K + bn - 1) / bn;
-  p.total_tiles = B * p.tiles_h * p.tiles_w * p.tiles_n;
   p.ep = ep;
-  p.pool2 = pool2 ? 1 : 0;
-  p.err_flag = e->d_flags + 2;
-
-  CUtensorMap tm[4];
-  memset((void *)tm, 0, sizeof tm);
-  if (rc == B200_OK) {
-    // activations as (C, W, H, N), box = CK channels x window; positions outside the image read as zero
-    cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
-    cuuint64_t strides[3] = {(cuuint64_t)C * 4, (cuuint64_t)W * C * 4, (cuuint64_t)H * W * C * 4};
-    cuuint32_t box[4] = {(cuuint32_t)ck, (cuuint32_t)win_w, (cuuint32_t)win_h, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    for (int h = 0; h < 2 && rc == B200_OK; ++h) {
-      CUresult r = enc(&tm[h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void *>(xin[h]), dims, strides, box, estr,
-                       CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS)
-        rc = set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a %d x %d window", (int)r, win_w,
-                       win_h);
-    }
-    cuuint64_t wdims[3] = {(cuuint64_t)crs, (cuuint64_t)K, 1};
-    cuuint64_t wstrides[2] = {(cuuint64_t)wf.ld * 4, (cuuint64_t)K * wf.ld * 4};
-    cuuint32_t wbox[3] = {(cuuint32_t)ck, (cuuint32_t)bn, 1};
-    cuuint32_t westr[3] = {1, 1, 1};
-    for (int h = 0; h < 2 && rc == B200_OK; ++h) {
-      CUresult r = enc(&tm[2 + h], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(h ? wf.p1 : wf.p0), wdims,
-                       wstrides, wbox, westr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) rc = set_error(e, B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for filters", (int)r);
-    }
-  }
-  if (rc == B200_OK) {
-    if (ck == 32) {
-      if (bn == 64) rc = launch_conv_win<64, 32>(e, tm, p);
-      else rc = launch_conv_win<32, 32>(e, tm, p);
-    } else {
-      if (bn == 64) rc = launch_conv_win<64, 16>(e, tm, p);
-      else rc = launch_conv_win<32, 16>(e, tm, p);
-    }
-  }
+  p.only_if = e->only_if;
+  const void *win[2] = {wf.p0, wf.p1};
+  if (rc == B200_OK)
+    rc = conv_win_run(e, 4, xin, win, wf.ld, B, C, H, W, K, kh, kw, padH, padW, dH, dW, Ho, Wo, pool2, p);
   for (int h = 0; h < 2; ++h) {
     if (xs[h]) b200_put(e, xs[h], 0);
     if (wblk[h]) b200_put(e, wblk[h], 0);
   }
   return rc;
+}
+
+// The same from pairs of fp16 (conv2d_tma_pairs).
+int conv2d_win_pairs(b200_engine *e, const __half *x_pairs, const TcOperand &wf, float *y, long long B, int C, int H,
+                     int W, int K, int kh, int kw, int padH, int padW, int dH, int dW, int Ho, int Wo,
+                     const Epilogue &ep, bool pool2, const PairsIn &in, const PairsOut &out) {
+  ConvWinParams p = ConvWinParams();
+  p.y = y;
+  p.ep = ep;
+  p.in16 = in;
+  p.out16 = out;
+  const void *xin[2] = {x_pairs, x_pairs + B * C * H * W}, *win[2] = {wf.p0, wf.p1};
+  return conv_win_run(e, 2, xin, win, wf.ld, B, C, H, W, K, kh, kw, padH, padW, dH, dW, Ho, Wo, pool2, p);
 }
 
 }  // namespace b200

@@ -103,6 +103,7 @@ int sync_stream_checked(b200_engine *e) {
       cudaMemsetAsync(e->d_flags + 2, 0, sizeof(int), e->stream);
       // a kernel that gave up may have left tiles half delivered: re-arm the arrival counters
       cudaMemsetAsync(e->sk_counters, 0, b200_engine::kSkCounters * sizeof(int), e->stream);
+      cudaMemsetAsync(e->f16_recs, 0, 256, e->stream);
       return set_error(e, B200_ERR_TIMEOUT, "a device-side wait ran out of time; results of the last "
                        "kernels are incomplete");
     }

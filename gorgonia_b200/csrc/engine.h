@@ -18,7 +18,7 @@ namespace b200 {
 struct F16Rec;
 // A derived form of a constant buffer (weights) kept for reuse: the TF32 head/tail split of a
 // matrix (kind 0) or of convolution filters permuted to (tap, channel) order (kind 1), or a matrix as pairs
-// of fp16 behind a 256-byte block that begins with its F16Rec (kind 2).
+// of fp16 behind a 256-byte block that begins with its F16Rec (kind 2), or filters both (kind 3).
 struct CachedSplit {
   int kind;
   long long d0, d1, d2, ld_in;  // the shape it was made for
@@ -66,6 +66,10 @@ struct b200_engine {
   // Records of the operands that a float32 product splits into pairs of fp16 (split.h): two for the
   // operands, zero between products, and a word that says whether the product has to be made over.
   b200::F16Rec *f16_recs = nullptr;
+  // While set, launches run only if the device word it names is not zero (b200_only_if): the way that stands
+  // behind one of fp16 pairs. Only entry points that say so can be called then (allow_only_if, flush_pending).
+  const int *only_if = nullptr;
+  bool allow_only_if = false;
 
   // lazily created resources of other translation units (gemm.cu etc.)
   void *gemm_state = nullptr;
@@ -159,6 +163,13 @@ void drop_constant(b200_engine *e, const void *ptr);
 void arena_release(b200_engine *e, int64_t off);
 // Called with a derived form that a launch is about to read: a recording keeps it alive.
 void pin_cached(b200_engine *e, const CachedSplit &c);
+
+// In the entry points whose launches honour b200_only_if.
+struct OnlyIfAllowed {
+  b200_engine *e;
+  explicit OnlyIfAllowed(b200_engine *e_) : e(e_) { e->allow_only_if = true; }
+  ~OnlyIfAllowed() { e->allow_only_if = false; }
+};
 
 // Waits for the engine's stream; B200_ERR_TIMEOUT if a kernel launched since the last check gave
 // up a bounded wait. Every entry point that synchronises goes through it.

@@ -164,11 +164,10 @@ __device__ __forceinline__ float epi_tf32(float v) {
 // x*(x>=0) forms and then never wins a window): if any result of the warp is not finite the function
 // stores nothing and returns false, and the caller takes the long way, which follows the reference
 // step by step. `inside`: this lane's pooling window lies in the image. The result is warp-uniform.
-template <int N, int ACT, bool BIAS>
-__device__ __forceinline__ bool store_channels_pool4_variant(const float (&acc)[N], float *y, long long plane,
-                                                             int valid, const float *bias, float alpha, bool inside,
-                                                             float *nh, float *nl) {
-  static_assert(N % 16 == 0, "a lane keeps N / 4 channels, stored four at a time");
+// Exchanges raw sums between the four lanes of a window: q[j] = the maximum over the window of channel
+// (lane bit 0 ? N/2 : 0) + (lane bit 3 ? N/4 : 0) + j.
+template <int N>
+__device__ __forceinline__ void pool4_exchange(const float (&acc)[N], float (&q)[N / 4]) {
   const int lane = threadIdx.x & 31;
   const bool b0 = (lane & 1) != 0, b1 = (lane & 8) != 0;
   float h[N / 2];
@@ -178,13 +177,22 @@ __device__ __forceinline__ bool store_channels_pool4_variant(const float (&acc)[
     const float send = b0 ? acc[j] : acc[j + N / 2];
     h[j] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, 1));
   }
-  float q[N / 4];
 #pragma unroll
   for (int j = 0; j < N / 4; ++j) {
     const float keep = b1 ? h[j + N / 4] : h[j];
     const float send = b1 ? h[j] : h[j + N / 4];
     q[j] = fmaxf(keep, __shfl_xor_sync(0xffffffffu, send, 8));
   }
+}
+template <int N, int ACT, bool BIAS>
+__device__ __forceinline__ bool store_channels_pool4_variant(const float (&acc)[N], float *y, long long plane,
+                                                             int valid, const float *bias, float alpha, bool inside,
+                                                             float *nh, float *nl) {
+  static_assert(N % 16 == 0, "a lane keeps N / 4 channels, stored four at a time");
+  const int lane = threadIdx.x & 31;
+  const bool b0 = (lane & 1) != 0, b1 = (lane & 8) != 0;
+  float q[N / 4];
+  pool4_exchange<N>(acc, q);
   const int cb = (b0 ? N / 2 : 0) + (b1 ? N / 4 : 0);  // first channel this lane keeps
   bool bad = false;
 #pragma unroll

@@ -11,6 +11,7 @@
 #include <atomic>
 
 #include "engine.h"
+#include "pairs.cuh"
 #include "ptx.cuh"
 
 namespace b200 {
@@ -69,11 +70,25 @@ __device__ __forceinline__ float pool_tf32(float v) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
   return __uint_as_float(r);
 }
-template <bool K2>  // K2: a 2 x 2 window, whose four loads are issued together
+// F16: as pairs of fp16 instead (pairs.cuh), scaled by the largest magnitude x_rec has of x.
+template <bool K2, bool F16>  // K2: a 2 x 2 window, whose four loads are issued together
 __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restrict__ x, float *__restrict__ y,
                                                             float *__restrict__ hi, float *__restrict__ lo,
+                                                            const int *__restrict__ only_if,
+                                                            const F16Rec *__restrict__ x_rec, PairsOut out16,
                                                             long long B, int C, int H, int W, int Ho, int Wo, int kh,
                                                             int kw, int sH, int sW, int oh0, int ow0) {
+  if (!F16 && skip_launch(only_if)) return;
+  PairStats stats;
+  float scale = 1.f;
+  if (F16) {
+    const int ex = f16_scale_exp(x_rec->amax);
+    scale = pow2(ex);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      out16.rec->scale_exp = ex;
+      if (x_rec->bad) out16.rec->bad = 1;
+    }
+  }
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int HWo = Ho * Wo;
@@ -143,14 +158,24 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
       const int q = p0 + j, c = c0 + tx;
       if (q < HWo && c < C) {
         const float v = tile[tx][j];
-        const float h = pool_tf32(v);
         const long long o = ob + (long long)q * C + c;
-        hi[o] = h;
-        lo[o] = pool_tf32(__fsub_rn(v, h));
+        if (F16) {
+          __half hh, ll;
+          stats.see(v);
+          stats.small += f16_pair(v, scale, hh, ll) ? 1u : 0u;
+          if (!(fabsf(v * scale) <= 65504.f)) stats.bad = 1;
+          out16.h[o] = hh;
+          out16.l[o] = ll;
+        } else {
+          const float h = pool_tf32(v);
+          hi[o] = h;
+          lo[o] = pool_tf32(__fsub_rn(v, h));
+        }
       }
     }
     __syncthreads();
   }
+  if (F16) stats.deliver(out16.rec);
 }
 
 // The pooling every config here uses: 2x2 window, stride 2, no padding, W a multiple of 4, no mask.
@@ -158,7 +183,9 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
 // them with one 8-byte store. Same comparison order as the general kernel: row-major inside the
 // window, strict '>', starting from -FLT_MAX.
 __global__ void __launch_bounds__(256) maxpool2x2_kernel(const float *__restrict__ x, float *__restrict__ y,
-                                                         long long planes, int H, int W, int Ho, int Wo) {
+                                                         long long planes, int H, int W, int Ho, int Wo,
+                                                              const int *__restrict__ only_if) {
+  if (skip_launch(only_if)) return;
   const int pairs = Wo >> 1;  // Wo = W/2 is even because W % 4 == 0
   const long long total = planes * Ho * pairs;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -185,7 +212,9 @@ __global__ void __launch_bounds__(256) maxpool2x2_kernel(const float *__restrict
 // The same for any even W and any H: one output per thread from two 8-byte loads. A trailing
 // odd input row (H odd) is simply never read, as the output size formula drops it.
 __global__ void __launch_bounds__(256) maxpool2x2_even_kernel(const float *__restrict__ x, float *__restrict__ y,
-                                                              long long planes, int H, int W, int Ho, int Wo) {
+                                                              long long planes, int H, int W, int Ho, int Wo,
+                                                              const int *__restrict__ only_if) {
+  if (skip_launch(only_if)) return;
   const long long total = planes * Ho * Wo;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -210,7 +239,9 @@ __global__ void __launch_bounds__(256) maxpool2x2_even_kernel(const float *__res
 // kernel: row-major inside the clipped window, strict '>', starting from -FLT_MAX.
 __global__ void __launch_bounds__(256) maxpool2x2_any_kernel(const float *__restrict__ x, float *__restrict__ y,
                                                              uint32_t planes, int H, int W, int Ho, int Wo, int sH,
-                                                             int sW, int oh0, int ow0) {
+                                                             int sW, int oh0, int ow0,
+                                                             const int *__restrict__ only_if) {
+  if (skip_launch(only_if)) return;
   const uint32_t per = (uint32_t)Ho * Wo, total = planes * per, hw = (uint32_t)H * W;
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -1167,19 +1198,57 @@ int b200_maxpool2d_split_fwd(b200_engine *e, const void *x, void *y, void *y_hi,
   if (B * C == 0) return B200_OK;
   B200_REQUIRE(e, x && y_hi && y_lo, "b200_maxpool2d_split_fwd: null pointer");
   DeviceGuard g(e);
+  OnlyIfAllowed allowed(e);
   int rc = flush_pending(e);
   if (rc != B200_OK) return rc;
   const long long tiles = B * ((Ho * Wo + 31) / 32) * ((C + 31) / 32);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)e->sm_count * 32));
   const int oh0 = explicit_padding ? pad_south : pad_north, ow0 = explicit_padding ? pad_east : pad_west;
   if (kh == 2 && kw == 2)
-    maxpool_split_kernel<true><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)y, (float *)y_hi,
-                                                              (float *)y_lo, B, (int)C, (int)H, (int)W, (int)Ho,
+    maxpool_split_kernel<true, false><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)y, (float *)y_hi,
+                                                              (float *)y_lo, e->only_if, nullptr, PairsOut(), B, (int)C, (int)H, (int)W, (int)Ho,
                                                               (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   else
-    maxpool_split_kernel<false><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)y, (float *)y_hi,
-                                                               (float *)y_lo, B, (int)C, (int)H, (int)W, (int)Ho,
+    maxpool_split_kernel<false, false><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)y, (float *)y_hi,
+                                                               (float *)y_lo, e->only_if, nullptr, PairsOut(), B, (int)C, (int)H, (int)W, (int)Ho,
                                                                (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
+  B200_CHECK_LAUNCH(e, "maxpool_split_kernel");
+  return B200_OK;
+}
+
+int b200_maxpool2d_pairs_fwd(b200_engine *e, const void *x, const void *x_rec, void *y_pairs, void *y_rec, int64_t B,
+                             int64_t C, int64_t H, int64_t W, int kh, int kw, int pad_north, int pad_south, int pad_west,
+                             int pad_east, int explicit_padding, int stride_h, int stride_w) {
+  if (!e) return B200_ERR_INVALID;
+  std::lock_guard<std::recursive_mutex> lk(e->mu);
+  B200_REQUIRE(e, B >= 0 && C >= 0 && H > 0 && W > 0, "b200_maxpool2d_pairs_fwd: bad input shape");
+  B200_REQUIRE(e, kh > 0 && kw > 0 && stride_h > 0 && stride_w > 0, "b200_maxpool2d_pairs_fwd: bad kernel or stride");
+  B200_REQUIRE(e, pad_north >= 0 && pad_south >= 0 && pad_west >= 0 && pad_east >= 0,
+               "b200_maxpool2d_pairs_fwd: bad pad");
+  B200_REQUIRE(e, H < 32768 && W < 32768 && C < (1LL << 30), "b200_maxpool2d_pairs_fwd: image too large");
+  const long long Ho = (H + pad_south + pad_north - (kh - 1) - 1) / stride_h + 1;
+  const long long Wo = (W + pad_east + pad_west - (kw - 1) - 1) / stride_w + 1;
+  B200_REQUIRE(e, Ho > 0 && Wo > 0, "b200_maxpool2d_pairs_fwd: window larger than the padded image");
+  if (B * C == 0) return B200_OK;
+  B200_REQUIRE(e, x && x_rec && y_pairs && y_rec, "b200_maxpool2d_pairs_fwd: null pointer");
+  DeviceGuard g(e);
+  int rc = flush_pending(e);
+  if (rc != B200_OK) return rc;
+  const long long tiles = B * ((Ho * Wo + 31) / 32) * ((C + 31) / 32);
+  const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)e->sm_count * 32));
+  const int oh0 = explicit_padding ? pad_south : pad_north, ow0 = explicit_padding ? pad_east : pad_west;
+  PairsOut out;
+  out.h = (__half *)y_pairs;
+  out.l = out.h + B * C * Ho * Wo;
+  out.rec = (F16Rec *)y_rec;
+  if (kh == 2 && kw == 2)
+    maxpool_split_kernel<true, true><<<blocks, 256, 0, e->stream>>>(
+        (const float *)x, nullptr, nullptr, nullptr, nullptr, (const F16Rec *)x_rec, out, B, (int)C, (int)H, (int)W,
+        (int)Ho, (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
+  else
+    maxpool_split_kernel<false, true><<<blocks, 256, 0, e->stream>>>(
+        (const float *)x, nullptr, nullptr, nullptr, nullptr, (const F16Rec *)x_rec, out, B, (int)C, (int)H, (int)W,
+        (int)Ho, (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   B200_CHECK_LAUNCH(e, "maxpool_split_kernel");
   return B200_OK;
 }
@@ -1200,6 +1269,7 @@ int b200_maxpool2d_fwd(b200_engine *e, int dtype, const void *x, void *y, int64_
   if (B * C == 0) return B200_OK;
   B200_REQUIRE(e, x && y, "b200_maxpool2d_fwd: null pointer");
   DeviceGuard g(e);
+  OnlyIfAllowed allowed(e);
   int rc = flush_pending(e);
   if (rc != B200_OK) return rc;
   const int oh0 = explicit_padding ? pad_south : pad_north;
@@ -1209,24 +1279,25 @@ int b200_maxpool2d_fwd(b200_engine *e, int dtype, const void *x, void *y, int64_
       pad_south == 0 && pad_west == 0 && pad_east == 0 && W % 4 == 0 && (uintptr_t)x % 16 == 0 &&
       (uintptr_t)y % 8 == 0) {
     maxpool2x2_kernel<<<grid_for(e, total / 2), 256, 0, e->stream>>>((const float *)x, (float *)y, B * C, (int)H,
-                                                                    (int)W, (int)Ho, (int)Wo);
+                                                                    (int)W, (int)Ho, (int)Wo, e->only_if);
     B200_CHECK_LAUNCH(e, "maxpool2x2_kernel");
     return B200_OK;
   }
   if (dtype == B200_F32 && !mask && kh == 2 && kw == 2 && stride_h == 2 && stride_w == 2 && pad_north == 0 &&
       pad_south == 0 && pad_west == 0 && pad_east == 0 && W % 2 == 0 && (uintptr_t)x % 8 == 0) {
     maxpool2x2_even_kernel<<<grid_for(e, total), 256, 0, e->stream>>>((const float *)x, (float *)y, B * C, (int)H,
-                                                                     (int)W, (int)Ho, (int)Wo);
+                                                                     (int)W, (int)Ho, (int)Wo, e->only_if);
     B200_CHECK_LAUNCH(e, "maxpool2x2_even_kernel");
     return B200_OK;
   }
   if (dtype == B200_F32 && !mask && kh == 2 && kw == 2 && total < (1LL << 31) && B * C * H * W < (1LL << 32)) {
     maxpool2x2_any_kernel<<<grid_for(e, total), 256, 0, e->stream>>>((const float *)x, (float *)y, (uint32_t)(B * C),
                                                                     (int)H, (int)W, (int)Ho, (int)Wo, stride_h,
-                                                                    stride_w, oh0, ow0);
+                                                                    stride_w, oh0, ow0, e->only_if);
     B200_CHECK_LAUNCH(e, "maxpool2x2_any_kernel");
     return B200_OK;
   }
+  if (e->only_if) return set_error(e, B200_ERR_STATE, "this pooling cannot be made while b200_only_if is in effect");
   if (dtype == B200_F32)
     maxpool_kernel<float><<<grid_for(e, total), 256, 0, e->stream>>>((const float *)x, (float *)y, (long long *)mask,
                                                                     B * C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw,

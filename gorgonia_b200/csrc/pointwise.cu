@@ -1238,6 +1238,8 @@ int plan_pending(b200_engine *e, int *n_kernels) {
 }
 
 int flush_pending(b200_engine *e) {
+  if (e->only_if && !e->allow_only_if)
+    return set_error(e, B200_ERR_STATE, "this call cannot be made while b200_only_if is in effect");
   if (e->pending.empty()) {
     e->dead.clear();
     return B200_OK;

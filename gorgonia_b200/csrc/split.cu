@@ -170,4 +170,68 @@ int launch_split_tf32_redo(b200_engine *e, const SplitJob &a, const SplitJob &b,
   return launch_split<SPLIT_TF32_REDO>(e, a, b, SplitRedo{ra, rb, limit_a, limit_b, redo});
 }
 
+// The largest magnitude of n values into rec->amax, and rec->bad for infinities and NaNs; with step > 1, of
+// every step-th 4 KB only where there are more than 4 MB.
+__global__ void __launch_bounds__(256) magnitude_kernel(const float *__restrict__ x, long long n, int step, F16Rec *rec) {
+  __shared__ unsigned s_max[8], s_bad[8];
+  unsigned amax = 0, bad = 0;
+  auto see = [&](float v) {
+    const unsigned m = __float_as_uint(v) & 0x7FFFFFFFu;
+    if (m >= 0x7F800000u) bad = 1;
+    else amax = amax > m ? amax : m;
+  };
+  const long long groups = (n + 1023) / 1024;
+  if (n <= (1 << 20)) step = 1;
+  const bool vec = ((uintptr_t)x & 15) == 0;
+  for (long long g = (long long)blockIdx.x * step; g < groups; g += (long long)gridDim.x * step) {
+    const long long i = g * 1024 + threadIdx.x * 4;
+    if (vec && i + 4 <= n) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(x + i));
+      see(v.x); see(v.y); see(v.z); see(v.w);
+    } else {
+      for (long long k = i; k < i + 4 && k < n; ++k) see(__ldg(x + k));
+    }
+  }
+  amax = __reduce_max_sync(0xffffffffu, amax);
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    s_max[threadIdx.x >> 5] = amax;
+    s_bad[threadIdx.x >> 5] = bad;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      amax = amax > s_max[w] ? amax : s_max[w];
+      bad |= s_bad[w];
+    }
+    if (amax) atomicMax(&rec->amax, amax);
+    if (bad) atomicOr(&rec->bad, 1u);
+  }
+}
+int launch_magnitude(b200_engine *e, const float *x, long long n, int step, F16Rec *rec) {
+  const long long groups = ((n + 1023) / 1024 + (n > (1 << 20) ? step : 1) - 1) / (n > (1 << 20) ? step : 1);
+  magnitude_kernel<<<(int)std::max<long long>(1, std::min<long long>(groups, e->sm_count * 8LL)), 256, 0, e->stream>>>(x, n, step, rec);
+  B200_CHECK_LAUNCH(e, "magnitude_kernel");
+  return B200_OK;
+}
+
+// Whether any of k records says that its tensor is unusable; clears them for the next round.
+struct PairsLimits {
+  unsigned limit[kMaxPairsRecs];
+};
+__global__ void pairs_check_kernel(F16Rec *recs, PairsLimits l, int k, int *verdict) {
+  const int i = threadIdx.x;
+  const bool bad = i < k && f16_unusable(recs + i, l.limit[i]);
+  const bool any = __any_sync(0xffffffffu, bad);
+  if (i < k) recs[i] = F16Rec{0, 0, 0, 0};
+  if (i == 0) *verdict = any ? 1 : 0;
+}
+int launch_pairs_check(b200_engine *e, F16Rec *recs, const unsigned *limits, int k, int *verdict) {
+  PairsLimits l;
+  for (int i = 0; i < kMaxPairsRecs; ++i) l.limit[i] = i < k ? limits[i] : 0xFFFFFFFFu;
+  pairs_check_kernel<<<1, 32, 0, e->stream>>>(recs, l, k, verdict);
+  B200_CHECK_LAUNCH(e, "pairs_check_kernel");
+  return B200_OK;
+}
+
 }  // namespace b200

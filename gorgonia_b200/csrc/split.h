@@ -40,6 +40,13 @@ int launch_split_f16(b200_engine *e, const SplitJob &a, const SplitJob &b);
 int launch_split_tf32_redo(b200_engine *e, const SplitJob &a, const SplitJob &b, const F16Rec *ra, unsigned limit_a,
                            const F16Rec *rb, unsigned limit_b, int *redo);
 
+// The largest magnitude of n values, or of a sample of them (step > 1), into rec.
+int launch_magnitude(b200_engine *e, const float *x, long long n, int step, F16Rec *rec);
+// Whether any of k <= kMaxPairsRecs records, one after the other in memory, says that its tensor is unusable
+// goes to *verdict; the records are cleared.
+constexpr int kMaxPairsRecs = 32;
+int launch_pairs_check(b200_engine *e, F16Rec *recs, const unsigned *limits, int k, int *verdict);
+
 #ifdef __CUDACC__
 // Scale that brings a largest magnitude (bits of a finite float >= 0) into [2^14, 2^15): at least 2^-113.
 // Kept below 2^110 so that it and its inverse are normal numbers; values that this leaves small are counted.

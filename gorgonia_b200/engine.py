@@ -10,6 +10,7 @@ class exists so the parity tests read like gorgonia's own tests.
 
 Nothing here computes on the host: every method forwards to libgorgonia_b200.so.
 """
+import contextlib
 import ctypes as C
 
 import numpy as np
@@ -467,6 +468,34 @@ class Engine:
                                         B, Cc, H, W, K, kh, kw, pad[0], pad[1], stride[0], stride[1], dil[0], dil[1],
                                         C.byref(ep) if ep else None, int(pool2)), self.h)
 
+    def Conv2dPairs(self, x, w, y, in_shape, x_rec, y_rec, pad=(0, 0), bias=None, act=None, alpha=0.0, pool2=False,
+                    x_pairs=None, y_pairs=None):
+        """One link of a chain on pairs of fp16. x_pairs / y_pairs: tensors that hold heads and tails; x_rec /
+        y_rec: device addresses of the tensors' records (see b200_conv2d_pairs_fwd)."""
+        B, Cc, H, W = in_shape
+        K, _, kh, kw = w.shape
+        ep = _epilogue(bias, "row", act, alpha)
+        check(lib.b200_conv2d_pairs_fwd(self.h, x.ptr if x is not None else None,
+                                        x_pairs.ptr if x_pairs is not None else None, x_rec, w.ptr,
+                                        y.ptr if y is not None else None,
+                                        y_pairs.ptr if y_pairs is not None else None, y_rec, B, Cc, H, W, K, kh, kw,
+                                        pad[0], pad[1], C.byref(ep) if ep else None, int(pool2)), self.h)
+
+    def pairs_magnitude(self, x, rec):
+        check(lib.b200_pairs_magnitude(self.h, x.ptr, x.size, rec), self.h)
+
+    def pairs_check(self, recs, counts, verdict):
+        check(lib.b200_pairs_check(self.h, recs, (C.c_int64 * len(counts))(*counts), len(counts), verdict), self.h)
+
+    @contextlib.contextmanager
+    def only_if(self, flag):
+        """Launches made inside run only if the device word at `flag` is not zero (see b200_only_if)."""
+        check(lib.b200_only_if(self.h, flag), self.h)
+        try:
+            yield
+        finally:
+            check(lib.b200_only_if(self.h, None), self.h)
+
     def conv2d_path(self, x, w, pad=(0, 0), stride=(1, 1), dil=(1, 1)):
         """Which kernel Conv2d would run for these operands (one of the _lib.CONV_* values)."""
         B, Cc, H, W = x.shape
@@ -506,6 +535,17 @@ class Engine:
                                            split[0].ptr, split[1].ptr, B, Cc, H, W, kernel[0], kernel[1], pn, ps, pw,
                                            pe, explicit, stride[0], stride[1]), self.h)
         return split
+
+    def MaxPool2DPairs(self, x, x_rec, pairs, rec, kernel, pad, stride):
+        """MaxPool2D whose result goes to a chain on pairs of fp16 (see b200_maxpool2d_pairs_fwd)."""
+        B, Cc, H, W = x.shape
+        if len(pad) == 2:
+            pn, ps, pw, pe, explicit = pad[0], pad[0], pad[1], pad[1], 0
+        else:
+            pn, ps, pw, pe = pad
+            explicit = 1
+        check(lib.b200_maxpool2d_pairs_fwd(self.h, x.ptr, x_rec, pairs.ptr, rec, B, Cc, H, W, kernel[0], kernel[1], pn,
+                                           ps, pw, pe, explicit, stride[0], stride[1]), self.h)
 
     def BatchNorm(self, x, prealloc, running_mean, running_var, save_mean=None, save_var=None, training=True,
                   momentum=0.9, epsilon=1e-5):

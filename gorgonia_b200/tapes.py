@@ -65,6 +65,27 @@ class _Tape:
             self.tape = None
 
 
+class _Records:
+    """The records that go with the tensors of a chain on pairs of fp16, one after the other in one buffer,
+    and behind them the word that says whether the chain has to be made over."""
+    MOST = 32
+
+    def __init__(self, engine):
+        self.e, self.counts = engine, []
+        self.buf = engine.empty((self.MOST * 4 + 4,), np.int32).set(np.zeros(self.MOST * 4 + 4, np.int32))
+
+    def new(self, count):
+        self.counts.append(int(count))
+        return self.buf.ptr + 16 * (len(self.counts) - 1)
+
+    @property
+    def verdict(self):
+        return self.buf.ptr + 16 * self.MOST
+
+    def check(self):
+        self.e.pairs_check(self.buf.ptr, self.counts, self.verdict)
+
+
 class _ConvChain:
     """Plans a run of convolutions (each optionally followed by a 2x2/2 max-pool) as links of
     b200_conv2d_chain_fwd: which links fold their pool in, and which tensors between links exist in
@@ -118,6 +139,72 @@ class _ConvChain:
             if L["pool_split"] is not None:
                 a_split = e.MaxPool2DSplit(L["y"], None, L["pool_split"], (2, 2), (0, 0), (2, 2))
                 a = None
+            elif L["pooled"] is not None:
+                e.MaxPool2D(L["y"], L["pooled"], (2, 2), (0, 0), (2, 2))
+                a = L["pooled"]
+        return a
+
+    # Convolutions of this much work per pass are worth pairs of fp16: they save about 0.45 of what TF32 pairs
+    # take at 160 TFLOP/s, and the launches of the TF32 chain behind them, which find nothing to do, cost a
+    # microsecond or two each.
+    PAIRS_FLOPS = 12e9
+
+    @property
+    def flops(self):
+        f = 0
+        for L in self.layers:
+            B, K, Ho, Wo = L["conv_shape"]
+            _, Cc, kh, kw = L["w"].shape
+            f += 2 * B * K * Ho * Wo * Cc * kh * kw
+        return f
+
+    def can_pairs(self):
+        """Whether every link has a kernel that takes pairs of fp16 (and one that can stand behind it)."""
+        from . import _lib
+        for i, L in enumerate(self.layers):
+            K, Cc = L["w"].shape[:2]
+            tensor = L["path"] in (_lib.CONV_TC_WINDOW, _lib.CONV_TC_TMA) and Cc % 16 == 0
+            first = i == 0 and L["path"] == _lib.CONV_DIRECT and L["fuse_pool"]
+            last = i + 1 == len(self.layers)
+            if not (tensor or first) or (not last and K % 8) or (first and K % 8):
+                return False
+            if not last and L["split"] is None and L["pool_split"] is None:
+                return False
+            if first and L["y"] is not None:
+                return False
+            if L["pooled"] is not None and np.prod(L["conv_shape"], dtype=np.int64) >= 1 << 31:
+                return False
+        return True
+
+    def plan_pairs(self, records):
+        """Takes records for every tensor. A tensor's pairs lie where its TF32 head would: the TF32 chain runs
+        only if the pairs have turned out to be of no use, and then from its input on."""
+        self.records = records
+        n = 1
+        for d in self.layers[0]["in_shape"]:
+            n *= d
+        self.x_rec = records.new(n)
+        for L in self.layers:
+            L["rec"] = records.new(int(np.prod(L["out_shape"] if L["fuse_pool"] else L["conv_shape"], dtype=np.int64)))
+            if L["pool_split"] is not None:
+                L["pool_rec"] = records.new(int(np.prod(L["out_shape"], dtype=np.int64)))
+
+    def forward_pairs(self, x, x_pairs=None, x_rec=None):
+        """forward() on pairs of fp16; the records have to be checked afterwards, and forward() made under
+        that condition."""
+        e, a, a_pairs = self.e, x, x_pairs
+        if x_rec is None:
+            x_rec = self.x_rec
+            e.pairs_magnitude(x, x_rec)
+        for L in self.layers:
+            y_pairs = L["split"][0] if L["split"] else None
+            e.Conv2dPairs(a if a_pairs is None else None, L["w"], L["y"], L["in_shape"], x_rec, L["rec"], pad=L["pad"],
+                          bias=L["bias"], act=L["act"], alpha=L["alpha"], pool2=L["fuse_pool"], x_pairs=a_pairs,
+                          y_pairs=y_pairs)
+            a, a_pairs, x_rec = L["y"], y_pairs, L["rec"]
+            if L["pool_split"] is not None:
+                e.MaxPool2DPairs(L["y"], L["rec"], L["pool_split"][0], L["pool_rec"], (2, 2), (0, 0), (2, 2))
+                a, a_pairs, x_rec = None, L["pool_split"][0], L["pool_rec"]
             elif L["pooled"] is not None:
                 e.MaxPool2D(L["y"], L["pooled"], (2, 2), (0, 0), (2, 2))
                 a = L["pooled"]
@@ -226,6 +313,10 @@ class LeNet(_Tape):
         self.chain = _ConvChain(e, batch, (1, 28, 28), [
             {"w": self.wc[i], "pad": (1, 1), "bias": None, "act": "rectify", "alpha": 0.0, "pool": "2x2/2"}
             for i in range(3)]) if fused else None
+        self.records = None
+        if fused and self.chain.can_pairs() and self.chain.flops >= self.chain.PAIRS_FLOPS:
+            self.records = _Records(e)
+            self.chain.plan_pairs(self.records)
         self.dense = _DenseChain(e, batch, [{"w": self.wd[0], "bias": None, "act": "rectify"},
                                             {"w": self.wd[1], "bias": None, "act": None}]) if fused else None
         self.fc = e.empty((batch, 625))
@@ -235,7 +326,12 @@ class LeNet(_Tape):
 
     def forward(self):
         e, a = self.e, self.x
-        if self.fused:
+        if self.fused and self.records is not None:
+            self.chain.forward_pairs(a)
+            self.records.check()
+            with e.only_if(self.records.verdict):
+                a = self.chain.forward(a)
+        elif self.fused:
             a = self.chain.forward(a)
         else:
             for i in range(3):
@@ -296,6 +392,12 @@ class TinyYolo(_Tape):
             if self.chain_b.reads_split:
                 self.pool5_split = (e.empty((batch, s, s, ch[6])), e.empty((batch, s, s, ch[6])))
             self.out = self.chain_b.layers[-1]["y"]
+            a, b = self.chain_a, self.chain_b
+            self.records = None
+            if self.pool5_split is not None and a.can_pairs() and b.can_pairs() and a.flops + b.flops >= a.PAIRS_FLOPS:
+                self.records = _Records(e)
+                a.plan_pairs(self.records)
+                b.plan_pairs(self.records)
         else:
             self.out = self.conv[8]
 
@@ -320,7 +422,23 @@ class TinyYolo(_Tape):
             self.record()
         return self
 
+    def _forward_pairs(self):
+        e, a, b = self.e, self.chain_a, self.chain_b
+        a.forward_pairs(self.x)
+        last = a.layers[-1]
+        # chain_b's record of its input is written by the pool in front of it
+        e.MaxPool2DPairs(last["y"], last["rec"], self.pool5_split[0], b.x_rec, (2, 2), (1, 0, 1, 0), (1, 1))
+        b.forward_pairs(None, self.pool5_split[0], b.x_rec)
+        self.records.check()
+        with e.only_if(self.records.verdict):
+            return self._forward_tf32()
+
     def forward(self):
+        if self.fused and self.records is not None:
+            return self._forward_pairs()
+        return self._forward_tf32()
+
+    def _forward_tf32(self):
         e, a = self.e, self.x
         if self.fused:
             a = self.chain_a.forward(a)

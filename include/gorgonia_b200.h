@@ -353,7 +353,8 @@ int b200_tf32_peak(b200_engine *e, int batches, double *tflops);
  * multiple of 4; C may be NULL) and the next link reads it as its A (A_hi, A_lo with lda = that pitch; A may be
  * NULL), which spares the split pass over every activation. Columns N .. ld_split-1 are zero-filled.
  * Shapes that run on the CUDA-core kernel need A and answer B200_ERR_UNSUPPORTED without it.
- * Results are bit-identical to b200_gemm. */
+ * Results are bit-identical to b200_gemm, except that large products of an unsplit A may be made from
+ * pairs of fp16 instead of TF32 (same tolerance; b200_gemm does so too). */
 int b200_gemm_chain(b200_engine *e, int transB, int64_t M, int64_t N, int64_t K, const void *A,
                     const void *A_hi, const void *A_lo, int64_t lda, const void *B, int64_t ldb,
                     void *C, void *C_hi, void *C_lo, int64_t ldc, int64_t ld_split,
@@ -464,12 +465,43 @@ int b200_conv2d_maxpool_fwd(b200_engine *e, int dtype, const void *x, const void
  * its epilogue, and a next link that reads it (x_hi, x_lo; x may be NULL), together skip the
  * rewrite pass each tensor-core convolution otherwise starts with. Shapes whose kernel reads NCHW
  * need x and answer B200_ERR_UNSUPPORTED without it; shapes whose kernel cannot write the split
- * form get it from a rewrite pass. Results are bit-identical to the unchained calls. */
+ * form get it from a rewrite pass. Results are bit-identical to those of the unchained calls where these
+ * use TF32 pairs too, and within the same tolerance where they are large enough for pairs of fp16. */
 int b200_conv2d_chain_fwd(b200_engine *e, const void *x, const void *x_hi, const void *x_lo,
                           const void *w, void *y, void *y_hi, void *y_lo, int64_t B, int64_t C,
                           int64_t H, int64_t W, int64_t K, int kh, int kw, int pad_h, int pad_w,
                           int stride_h, int stride_w, int dil_h, int dil_w, const b200_epilogue *ep,
                           int pool2);
+/* The same chain on pairs of fp16: half the bytes and twice the tensor-core rate of TF32 pairs, with the
+ * same 11 + 11 significant bits per value, for tensors whose values lie within 2^-29 of the largest (of a
+ * bound on it, in a chain). Whether they do is found out on the device; a chain is therefore followed by
+ * b200_pairs_check and, under b200_only_if, by the same chain of b200_conv2d_chain_fwd calls, which then
+ * runs only if it has to.
+ *   A tensor in pairs form is B*H*W*C fp16 heads (channels innermost) followed by as many tails, 16-byte
+ *   aligned; with it goes a 16-byte record on the device, zero before the chain runs.
+ *   b200_conv2d_pairs_fwd: one link (unit stride, no dilation). The first link of an image network reads x
+ *     (NCHW, with pool2, C <= 3, 3x3, K a multiple of 8); every other reads x_pairs (C a multiple of 16) and
+ *     writes y (NCHW), y_pairs (K a multiple of 8) or both. x_rec / y_rec: the tensors' records. Shapes
+ *     without such a kernel answer B200_ERR_UNSUPPORTED.
+ *   b200_maxpool2d_pairs_fwd: b200_maxpool2d_split_fwd for this form; x_rec is the record that the link that
+ *     made x wrote.
+ *   b200_pairs_magnitude: the record of a network's input: its largest magnitude (a sample's for large n).
+ *   b200_pairs_check: *verdict (on the device) = 1 if any of k <= 32 adjacent records says that its tensor
+ *     (of counts[i] values) was unusable, else 0; clears the records.
+ *   b200_only_if: until it is called with NULL, launches are made that run only if *flag is not zero.
+ *     b200_conv2d_chain_fwd (shapes of the tensor-core and first-layer kernels), b200_maxpool2d_split_fwd and
+ *     b200_maxpool2d_fwd (2x2, no mask) can be called then; everything else answers B200_ERR_STATE. */
+int b200_conv2d_pairs_fwd(b200_engine *e, const void *x, const void *x_pairs, const void *x_rec,
+                          const void *w, void *y, void *y_pairs, void *y_rec, int64_t B, int64_t C, int64_t H,
+                          int64_t W, int64_t K, int kh, int kw, int pad_h, int pad_w, const b200_epilogue *ep,
+                          int pool2);
+int b200_maxpool2d_pairs_fwd(b200_engine *e, const void *x, const void *x_rec, void *y_pairs, void *y_rec,
+                             int64_t B, int64_t C, int64_t H, int64_t W, int kh, int kw, int pad_north,
+                             int pad_south, int pad_west, int pad_east, int explicit_padding, int stride_h,
+                             int stride_w);
+int b200_pairs_magnitude(b200_engine *e, const void *x, int64_t n, void *rec);
+int b200_pairs_check(b200_engine *e, void *recs, const int64_t *counts, int k, int *verdict);
+int b200_only_if(b200_engine *e, const int *flag);
 /* Which kernel b200_conv2d_fwd would pick for a problem (no device work; -1 for a bad shape):
  * CUDA cores over an im2col scratch; the direct kernel for a first layer (C*kh*kw <= 32, K <= 32);
  * tensor cores with the col operand gathered by warps; tensor cores with the col operand built

@@ -1,0 +1,214 @@
+"""Convolutions on pairs of fp16: each kernel at the sizes where its tiles and rows meet, and whole chains whose
+tensors do not fit fp16's range and have to come out as the TF32 chain makes them (GPU tests)."""
+import numpy as np
+import pytest
+
+from gorgonia_b200 import B200Error, tapes
+from oracle import oracle
+from tests import util
+from tests.util import assert_bits_equal, assert_gemm_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(e, x):
+    """x (B, C, H, W) in pairs form, made on the host, and its record."""
+    amax = np.abs(x).max()
+    exp = 14 - int(np.floor(np.log2(amax)))
+    v = np.ascontiguousarray(x.transpose(0, 2, 3, 1)).astype(np.float64) * 2.0 ** exp
+    h = v.astype(np.float16)
+    l = ((v - h) * 2048).astype(np.float16)
+    rec = np.array([np.float32(amax).view(np.int32), 0, 0, exp], np.int32)
+    both = np.concatenate([h.ravel(), l.ravel()]).view(np.float32)
+    return e.tensor(both), e.tensor(rec)
+
+
+def _unpair(t, rec, shape):
+    B, C, H, W = shape
+    r = rec.numpy()
+    v = t.numpy().view(np.float16).astype(np.float64).reshape(2, B, H, W, C)
+    return ((v[0] + v[1] / 2048) * 2.0 ** -int(r[3])).transpose(0, 3, 1, 2), r
+
+
+def _oracle(x, w, pad, bias, act, alpha, pool):
+    y = oracle.conv2d(x, w, pad=pad)
+    if bias is not None:
+        y = (y + bias[None, :, None, None]).astype(np.float32)
+    y = {"rectify": oracle.rectify, "leaky": lambda t: oracle.leaky_relu(t, alpha), None: lambda t: t}[act](y)
+    return oracle.maxpool2d(y, (2, 2), (0, 0), (2, 2))[0] if pool else y
+
+
+LINKS = [
+    # B, C, H, W, K, kernel, pad, act, alpha, pool: the window kernel (32, 64 and 128-byte rows)
+    (3, 16, 32, 32, 32, 3, 1, "leaky", 0.1, True), (2, 16, 48, 46, 24, 3, 1, None, 0.0, False),
+    (4, 32, 28, 28, 64, 3, 1, "rectify", 0.0, True), (2, 32, 30, 32, 40, 5, 2, "leaky", 1.5, False),
+    (2, 64, 16, 31, 72, 3, 1, "leaky", -0.5, False), (2, 64, 32, 32, 64, 3, 1, "leaky", -0.5, True),
+    (9, 32, 14, 14, 64, 3, 1, "rectify", 0.0, True),
+    # the im2col kernel (128 and 64-byte rows), k shared between blocks and not
+    (5, 128, 13, 13, 256, 3, 1, "leaky", 0.1, False), (7, 96, 9, 11, 48, 3, 1, None, 0.0, False),
+    (3, 128, 26, 26, 125, 1, 0, "leaky", 1.0, False), (40, 64, 7, 7, 128, 3, 1, "rectify", 0.0, False),
+    (2, 512, 13, 13, 136, 3, 1, "leaky", 0.1, False), (30, 128, 26, 26, 512, 3, 0, "rectify", 0.0, False),
+]
+
+
+@pytest.mark.parametrize("case", LINKS)
+@pytest.mark.parametrize("scale", [1.0, 3e-20])
+def test_link(fresh, case, scale):
+    e = fresh
+    B, C, H, W, K, k, pad, act, alpha, pool = case
+    if scale != 1.0 and B * C * K > 40000:
+        pytest.skip("magnitudes are tried on the small links")
+    x = (util.normal(41, (B, C, H, W)) * np.float32(scale)).astype(np.float32)
+    w = util.normal(42, (K, C, k, k), scale=0.05)
+    bias = (util.normal(43, K) * np.float32(scale)).astype(np.float32)
+    want = _oracle(x, w, (pad, pad), bias, act, alpha, pool)
+    tx, rx = _pairs(e, x)
+    y, yp = e.empty(want.shape), e.empty((want.size,)) if K % 8 == 0 else None
+    for _ in range(2):
+        ry = e.tensor(np.zeros(4, np.int32))
+        e.Conv2dPairs(None, e.tensor(w), y, x.shape, rx.ptr, ry.ptr, pad=(pad, pad), bias=e.tensor(bias), act=act,
+                      alpha=alpha, pool2=pool, x_pairs=tx, y_pairs=yp)
+    got = y.numpy()
+    assert_gemm_close(got, want, 1e-5)
+    if yp is not None:
+        back, r = _unpair(yp, ry, want.shape)
+        assert r[2] == 0 and np.int32(r[0]).view(np.float32) == np.abs(got).max()
+        # heads and tails: 2^-22 of a value, or 2^-36 of the scaled range for the small ones
+        assert (np.abs(back - got) <= 2.0 ** -22 * np.abs(got) + 2.0 ** (-36 - int(r[3]))).all()
+        assert np.abs(back).max() * 2.0 ** int(r[3]) <= 65504
+
+
+@pytest.mark.parametrize("C", [1, 2, 3])
+def test_first_link_and_pool(fresh, C):
+    e = fresh
+    x, w, bias = util.uniform(51, (3, C, 28, 36)), util.normal(52, (16, C, 3, 3), scale=0.3), util.normal(53, 16)
+    want = _oracle(x, w, (1, 1), bias, "leaky", 0.1, True)
+    tx, recs = e.tensor(x), e.tensor(np.zeros(12, np.int32))
+    e.pairs_magnitude(tx, recs.ptr)
+    yp = e.empty((want.size,))
+    e.Conv2dPairs(tx, e.tensor(w), None, x.shape, recs.ptr, recs.ptr + 16, pad=(1, 1), bias=e.tensor(bias), act="leaky",
+                  alpha=0.1, pool2=True, y_pairs=yp)
+    r1 = e.empty((4,), np.int32)
+    r1.set(recs.numpy()[4:8])
+    back, r = _unpair(yp, r1, want.shape)
+    assert_gemm_close(back, want, 1e-6)
+    # a pool in front of the next link, with gorgonia's explicit padding, and an odd number of channels
+    z = util.normal(54, (2, 40, 13, 11))
+    tz = e.tensor(z)
+    rz = e.tensor(np.array([np.abs(z).max().view(np.int32), 0, 0, 0], np.int32))
+    for kernel, pad, stride in (((2, 2), (1, 0, 1, 0), (1, 1)), ((2, 2), (0, 0), (2, 2)), ((3, 3), (1, 1), (2, 2))):
+        p4 = pad if len(pad) == 4 else (pad[0], pad[0], pad[1], pad[1])
+        Ho, Wo = (13 + p4[0] + p4[1] - kernel[0]) // stride[0] + 1, (11 + p4[2] + p4[3] - kernel[1]) // stride[1] + 1
+        ref, got, rec = e.empty((2, 40, Ho, Wo)), e.empty((2 * 40 * Ho * Wo,)), e.tensor(np.zeros(4, np.int32))
+        e.MaxPool2D(tz, ref, kernel, pad, stride)
+        e.MaxPool2DPairs(tz, rz.ptr, got, rec.ptr, kernel, pad, stride)
+        back, r = _unpair(got, rec, ref.shape)
+        assert np.abs(back - ref.numpy()).max() <= 2.0 ** -22 * np.abs(z).max() and r[2] == 0
+
+
+@pytest.mark.parametrize("constant", [False, True])
+@pytest.mark.parametrize("case", [(32, 128, 26, 26, 256, 3, 1, 1), (128, 64, 32, 32, 64, 3, 1, 1), (32, 96, 40, 41, 250, 3, 2, 1),
+                                  (48, 256, 13, 13, 256, 3, 1, 1)])
+def test_single_convolutions(fresh, case, constant):
+    # large enough for pairs; then with values that are not: the TF32 launches behind them answer
+    e = fresh
+    B, C, H, W, K, k, stride, pad = case
+    x, w, bias = util.normal(61, (B, C, H, W)), util.normal(62, (K, C, k, k), scale=0.05), util.normal(63, K)
+    tx, tw, tb = e.tensor(x), e.tensor(w), e.tensor(bias)
+    if constant:
+        e.constant(tw)
+    Ho, Wo = (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1
+    y = e.empty((B, K, Ho, Wo))
+
+    def run():
+        e.Conv2d(tx, tw, y, pad=(pad, pad), stride=(stride, stride), bias=tb, act="leaky", alpha=0.1)
+        return y.numpy()
+
+    def want(x):
+        c = oracle.conv2d(x, w, pad=(pad, pad), stride=(stride, stride))
+        return oracle.leaky_relu((c + bias[None, :, None, None]).astype(np.float32), 0.1)
+
+    ref = want(x)
+    assert_gemm_close(run(), ref, 1e-5)
+    assert_gemm_close(run(), ref, 1e-5)
+    wide = x.copy()
+    wide[1] *= np.float32(1e-25)          # one image far below the others: exact in itself all the same
+    wide[2, :, 3, 3] = np.float32(1e20)
+    tx.set(wide)
+    got, ref = run(), want(wide)
+    for b in range(3):
+        assert_gemm_close(got[b], ref[b], 1e-5)
+    bad = x.copy()
+    bad[0, 0, 0, 0], bad[3, 1, 5, 5] = np.inf, np.nan
+    tx.set(bad)
+    got, ref = run(), want(bad)
+    assert np.isfinite(got).sum() == np.isfinite(ref).sum() and not np.isfinite(got[0]).all() and np.isfinite(got[1]).all()
+    assert_gemm_close(got[1], ref[1], 1e-5)
+    tx.set(x)                             # and back again
+    assert_gemm_close(run(), want(x), 1e-5)
+
+
+def _lenet(e, monkeypatch, flops, batch=40):
+    monkeypatch.setattr(tapes._ConvChain, "PAIRS_FLOPS", flops)
+    return tapes.LeNet(e, batch, seed=11)
+
+
+def _yolo(e, monkeypatch, flops, batch=4):
+    monkeypatch.setattr(tapes._ConvChain, "PAIRS_FLOPS", flops)
+    m = tapes.TinyYolo(e, batch, seed=12, channels=(3, 16, 32, 64, 64, 128, 128, 256, 128, 24))
+    for b in m.b:       # a bias would lift an image of 1e-25 into the others' range
+        b.set(np.zeros(b.shape, np.float32))
+    return m
+
+
+@pytest.mark.parametrize("make", [_lenet, _yolo])
+@pytest.mark.parametrize("kind", ["plain", "small", "large", "wide", "inf", "nan", "zero"])
+def test_chains_against_tf32(fresh, monkeypatch, make, kind):
+    e = fresh
+    m16, m32 = make(e, monkeypatch, 0), make(e, monkeypatch, 1e30)
+    assert m16.records is not None and m32.records is None
+    x = util.uniform(71, m16.x.shape)
+    x = {"small": lambda: x * np.float32(1e-12), "large": lambda: x * np.float32(1e12), "zero": lambda: x * 0,
+         "wide": lambda: x * np.where(np.arange(len(x)) % 2, 1e-25, 1.0).astype(np.float32)[:, None, None, None]
+         }.get(kind, lambda: x)()
+    if kind in ("inf", "nan"):
+        x[1, 0, 3, 3] = np.inf if kind == "inf" else np.nan
+    out = []
+    for m in (m16, m32):
+        m.x.set(x)
+        m.record()
+        for _ in range(2):
+            m.replay()
+        out.append(m.out.numpy())
+        redo = m.records.buf.numpy()[-4] if m.records is not None else None
+        if m is m16:
+            # what fp16's range is not enough for comes out as the TF32 chain makes it, to the bit
+            assert redo == (1 if kind in ("wide", "inf", "nan") else 0)
+    if kind in ("wide", "inf", "nan"):
+        assert_bits_equal(out[0], out[1])
+    else:
+        rms = np.sqrt(np.mean(out[1].astype(np.float64) ** 2))
+        assert np.abs(out[0] - out[1]).max() <= 4e-5 * max(rms, np.abs(out[1]).max())
+    # a replay on ordinary values after one that was made over
+    m16.x.set(util.uniform(72, m16.x.shape))
+    m16.replay()
+    first = m16.out.numpy()
+    m32.x.set(util.uniform(72, m16.x.shape))
+    m32.replay()
+    second = m32.out.numpy()
+    assert m16.records.buf.numpy()[-4] == 0
+    assert np.abs(first - second).max() <= 4e-5 * np.abs(second).max()
+    m16.close()
+    m32.close()
+
+
+def test_only_if_refuses_other_calls(fresh):
+    e = fresh
+    flag, a = e.tensor(np.zeros(4, np.int32)), e.tensor(util.normal(81, (64, 64)))
+    with e.only_if(flag.ptr):
+        with pytest.raises(B200Error):
+            e.MatMul(a, a, e.empty((64, 64)))
+        with pytest.raises(B200Error):
+            e.DoWork()
+    e.MatMul(a, a, e.empty((64, 64)))
+    e.Signal()
