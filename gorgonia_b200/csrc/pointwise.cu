@@ -9,10 +9,10 @@
 //   - each thread owns 16-byte chunks (4 floats / 2 doubles), grid-stride, 64-bit indices;
 //   - all sources of a chunk are loaded first (independent 128-bit loads in flight), then the
 //     program runs on registers, then the outputs are stored with 128-bit stores;
-//   - the program is interpreted with warp-uniform branches: the instruction loop is unrolled,
-//     instruction k writes register slot k (a compile-time index) and its operands are picked
-//     by a switch whose selector is the same for every thread, so nothing diverges and no
-//     value leaves the register file;
+//   - short programs on small tensors are interpreted in registers with warp-uniform branches: the
+//     instruction loop is unrolled, instruction k writes register slot k (a compile-time index) and
+//     its operands are picked by a switch whose selector is the same for every thread. Everything
+//     else addresses its operands in shared memory (pw_tile);
 //   - multiplies and adds are never contracted into FMAs (the reference builds its kernels
 //     with -fmad=false and the Go CPU engine does not fuse either).
 #include <cuda_runtime.h>
@@ -47,13 +47,14 @@ struct PwDev {
   long long src_div[B200_PW_MAX_SRC];
   long long src_mod[B200_PW_MAX_SRC];
   double imm[B200_PW_MAX_IMM];
+  float immf[B200_PW_MAX_IMM];  // the same, rounded
   uint8_t n_instr, n_src, n_out, pad0;
   uint8_t src_mode[B200_PW_MAX_SRC];
   uint8_t op[B200_PW_MAX_INSTR];
   uint8_t ra[B200_PW_MAX_INSTR];  // operand selectors: [0,NS) sources, [16,24) immediates, [32,48) results
   uint8_t rb[B200_PW_MAX_INSTR];
   uint8_t out_ins[B200_PW_MAX_OUT];
-  // ---- streaming kernel only: operands addressed in shared memory
+  // ---- pw_tile only: operands addressed in shared memory
   uint8_t n_full;                      // number of SRC_FULL sources (they travel through the ring)
   uint8_t n_file;                      // number of per-thread slots outside the ring
   uint8_t src_slot[B200_PW_MAX_SRC];   // SRC_FULL: index inside a ring stage; otherwise: file slot
@@ -61,6 +62,7 @@ struct PwDev {
   uint8_t kb[B200_PW_MAX_INSTR], xb[B200_PW_MAX_INSTR];
   uint8_t keep_slot[B200_PW_MAX_INSTR];  // file slot that keeps the result for later, or 0xFF
   uint8_t out_of[B200_PW_MAX_INSTR];     // output index this instruction's result is stored to, or 0xFF
+  uint2 code[B200_PW_MAX_INSTR];         // the six above in one load: op, ka | kb << 4, xa, xb; keep, out
 };
 
 enum OperandKind : uint8_t {
@@ -69,6 +71,13 @@ enum OperandKind : uint8_t {
   K_RING = 2,  // full-size source: slot xa of the current ring stage
   K_FILE = 3   // file slot xa: a broadcast source or a kept result
 };
+
+template <typename T>
+__device__ __forceinline__ T immediate(const PwDev &p, int i);
+template <>
+__device__ __forceinline__ float immediate<float>(const PwDev &p, int i) { return p.immf[i]; }
+template <>
+__device__ __forceinline__ double immediate<double>(const PwDev &p, int i) { return p.imm[i]; }
 
 #define SEL_IMM 16
 #define SEL_INS 32
@@ -277,7 +286,7 @@ __device__ __forceinline__ void fetch(T (&d)[V], int sel, const T (&S)[NS][V], c
       for (int j = 0; j < V; ++j) d[j] = T(0);
     }
   } else if (sel >= SEL_IMM) {
-    const T v = (T)p.imm[sel - SEL_IMM];
+    const T v = immediate<T>(p, sel - SEL_IMM);
 #pragma unroll
     for (int j = 0; j < V; ++j) d[j] = v;
   } else {
@@ -419,19 +428,20 @@ __device__ __forceinline__ void sts128(uint32_t addr, const uint4 &v) {
 // of complete 16-byte chunks, which is every tile but possibly the last one: no bounds logic.
 // ring_s / file_s: shared-memory addresses of this stage's ring slots and of the file slots,
 // already offset by this thread's lane (tid * 16).
-template <typename T, int V, int U, bool INSIDE>
+// ALIGNED: every tensor starts on a 16-byte boundary (else its elements are moved one at a time).
+template <typename T, int V, int U, int THREADS, bool INSIDE, bool ALIGNED>
 __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_t file_s, long long c_tile,
                                         int tid) {
   constexpr int W = U * V;
-  constexpr uint32_t SLOT_BYTES = PW_STREAM_THREADS * U * 16;
-  constexpr uint32_t USTRIDE = PW_STREAM_THREADS * 16;  // bytes between a thread's consecutive chunks
+  constexpr uint32_t SLOT_BYTES = THREADS * U * 16;
+  constexpr uint32_t USTRIDE = THREADS * 16;  // bytes between a thread's consecutive chunks
   int valid[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     if (INSIDE) {
       valid[u] = V;
     } else {
-      const long long left = p.n - (c_tile + u * PW_STREAM_THREADS + tid) * V;
+      const long long left = p.n - (c_tile + u * THREADS + tid) * V;
       valid[u] = left >= V ? V : (left > 0 ? (int)left : 0);
     }
   }
@@ -448,7 +458,7 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
         const uint32_t base = (uint32_t)((c_tile * V) % p.src_mod[s]);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const uint32_t off = (base + (uint32_t)(u * PW_STREAM_THREADS + tid) * V) % mod;
+          const uint32_t off = (base + (uint32_t)(u * THREADS + tid) * V) % mod;
           uint4 raw = make_uint4(0, 0, 0, 0);
           if (valid[u] > 0) raw = *reinterpret_cast<const uint4 *>(sp + off);
           sts128(slot + u * USTRIDE, raw);
@@ -456,7 +466,7 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
       } else {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const long long i = (c_tile + u * PW_STREAM_THREADS + tid) * V;
+          const long long i = (c_tile + u * THREADS + tid) * V;
           T v[V];
           if (mode == SRC_SCALAR) {
             const T x = sp[0];
@@ -478,30 +488,12 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
       }
     }
   }
-  if (!INSIDE) {
-    // the ragged last chunk of the tensor is not part of the bulk copy: its owner patches it in
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (valid[u] > 0 && valid[u] < V) {
-        for (int s = 0; s < p.n_src; ++s)
-          if (p.src_mode[s] == SRC_FULL) {
-            const T *sp = reinterpret_cast<const T *>(p.src[s]);
-            T v[V];
-#pragma unroll
-            for (int j = 0; j < V; ++j)
-              v[j] = j < valid[u] ? sp[(c_tile + u * PW_STREAM_THREADS + tid) * V + j] : T(0);
-            uint4 raw;
-            memcpy(&raw, v, sizeof raw);
-            sts128(ring_s + p.src_slot[s] * SLOT_BYTES + u * USTRIDE, raw);
-          }
-      }
-    }
-  }
-
   T acc[W];
 #pragma unroll
   for (int j = 0; j < W; ++j) acc[j] = T(0);
   const int n_instr = p.n_instr;
+  // One 8-byte load decodes an instruction; the one after it is fetched while this one runs.
+  uint2 code = p.code[0];
 #pragma unroll 1
   for (int q = 0; q < n_instr; ++q) {
     T a[W], b[W];
@@ -517,21 +509,23 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
 #pragma unroll
         for (int j = 0; j < W; ++j) d[j] = acc[j];
       } else {
-        const T x = (T)p.imm[idx];
+        const T x = immediate<T>(p, idx);
 #pragma unroll
         for (int j = 0; j < W; ++j) d[j] = x;
       }
     };
-    const int op = p.op[q];
-    fetch_op(a, p.ka[q], p.xa[q]);
+    const uint2 now = code;
+    code = p.code[q + 1 < n_instr ? q + 1 : q];
+    const int op = now.x & 0xFF;
+    fetch_op(a, (now.x >> 8) & 15, (now.x >> 16) & 0xFF);
     if (op < B200_OP_ABS) {
-      fetch_op(b, p.kb[q], p.xb[q]);
+      fetch_op(b, (now.x >> 12) & 15, now.x >> 24);
     } else {
 #pragma unroll
       for (int j = 0; j < W; ++j) b[j] = a[j];
     }
     pw_apply<T, W>(op, a, b, acc);
-    const int keep = p.keep_slot[q];
+    const int keep = now.y & 0xFF;
     if (keep != 0xFF) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -540,7 +534,7 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
         sts128(file_s + (uint32_t)keep * SLOT_BYTES + u * USTRIDE, raw);
       }
     }
-    const int o = p.out_of[q];
+    const int o = (now.y >> 8) & 0xFF;
     if (o != 0xFF) {
       unsigned char *op_ = reinterpret_cast<unsigned char *>(p.out[o]) + (c_tile + tid) * 16;
 #pragma unroll
@@ -550,11 +544,62 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
           memcpy(&raw, &acc[u * V], sizeof raw);
           *reinterpret_cast<uint4 *>(op_ + (size_t)u * USTRIDE) = raw;
         } else {
-          store_chunk<T, V>(reinterpret_cast<T *>(p.out[o]), (c_tile + u * PW_STREAM_THREADS + tid) * V,
-                            &acc[u * V], valid[u]);
+          T *dst = reinterpret_cast<T *>(p.out[o]);
+          const long long i = (c_tile + u * THREADS + tid) * V;
+          if (ALIGNED) {
+            store_chunk<T, V>(dst, i, &acc[u * V], valid[u]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+              if (j < valid[u]) dst[i + j] = acc[u * V + j];
+          }
         }
       }
     }
+  }
+}
+
+// This thread's elements of the full-size sources into their slots with plain loads: what the ring's bulk
+// copies do not bring (RAGGED_ONLY: just the ragged last chunk of the tensor).
+template <typename T, int V, int U, int THREADS, bool RAGGED_ONLY, bool ALIGNED>
+__device__ __forceinline__ void pw_fill(const PwDev &p, uint32_t ring_s, long long c_tile, int tid) {
+  constexpr uint32_t SLOT_BYTES = THREADS * U * 16, USTRIDE = THREADS * 16;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long i = (c_tile + u * THREADS + tid) * V;
+    const long long left = p.n - i;
+    const int valid = left >= V ? V : (left > 0 ? (int)left : 0);
+    if (valid == 0 || (RAGGED_ONLY && valid == V)) continue;
+    for (int s = 0; s < p.n_src; ++s) {
+      if (p.src_mode[s] != SRC_FULL) continue;
+      const T *sp = reinterpret_cast<const T *>(p.src[s]);
+      T v[V];
+      if (ALIGNED) {
+        load_chunk<T, V>(v, sp, i, valid);
+      } else {
+#pragma unroll
+        for (int j = 0; j < V; ++j) v[j] = j < valid ? sp[i + j] : T(0);
+      }
+      uint4 raw;
+      memcpy(&raw, v, sizeof raw);
+      sts128(ring_s + p.src_slot[s] * SLOT_BYTES + u * USTRIDE, raw);
+    }
+  }
+}
+
+// Programs too long for the register kernel, on tensors too small (or not aligned) for the ring: the
+// same interpreter over shared-memory slots that every thread fills for itself, so nothing is waited for.
+constexpr int PW_LOOP_THREADS = 128;
+template <typename T, int V, bool ALIGNED>
+__global__ void __launch_bounds__(PW_LOOP_THREADS) pw_loop_kernel(const __grid_constant__ PwDev p) {
+  extern __shared__ __align__(128) unsigned char pw_loop_smem[];
+  const int tid = threadIdx.x;
+  const uint32_t ring_s = ptx::smem_addr(pw_loop_smem) + (uint32_t)tid * 16;
+  const uint32_t file_s = ring_s + (uint32_t)p.n_full * PW_LOOP_THREADS * 16;
+  const long long ntiles = ((p.n + V - 1) / V + PW_LOOP_THREADS - 1) / PW_LOOP_THREADS;
+  for (long long k = blockIdx.x; k < ntiles; k += gridDim.x) {
+    pw_fill<T, V, 1, PW_LOOP_THREADS, false, ALIGNED>(p, ring_s, k * PW_LOOP_THREADS, tid);
+    pw_tile<T, V, 1, PW_LOOP_THREADS, false, ALIGNED>(p, ring_s, file_s, k * PW_LOOP_THREADS, tid);
   }
 }
 
@@ -603,8 +648,8 @@ __device__ __forceinline__ void pw_tile_single(int op, bool a_imm, bool b_imm, b
 // full tiles take the lean path above. A separate instantiation, so that the general kernel's code
 // and register allocation are not touched by it (measured: sharing one kernel cost the fused
 // chains 5 %).
-template <typename T, int V, int U, bool SINGLE>
-__global__ void __launch_bounds__(PW_STREAM_THREADS, 2)
+template <typename T, int V, int U, bool SINGLE, int CTAS>
+__global__ void __launch_bounds__(PW_STREAM_THREADS, CTAS)
     pw_stream_kernel(const __grid_constant__ PwDev p, int stages, int *err_flag) {
   constexpr int TILE_CHUNKS = PW_STREAM_THREADS * U;
   constexpr int SLOT_BYTES = TILE_CHUNKS * 16;
@@ -653,8 +698,8 @@ __global__ void __launch_bounds__(PW_STREAM_THREADS, 2)
   const int s_op = p.op[0];
   const bool s_unary = s_op >= B200_OP_ABS;
   const bool s_a_imm = p.ka[0] == K_IMM, s_b_imm = p.kb[0] == K_IMM;
-  const T s_imm_a = (SINGLE && s_a_imm) ? (T)p.imm[p.xa[0]] : T(0);
-  const T s_imm_b = (SINGLE && !s_unary && s_b_imm) ? (T)p.imm[p.xb[0]] : T(0);
+  const T s_imm_a = (SINGLE && s_a_imm) ? immediate<T>(p, p.xa[0]) : T(0);
+  const T s_imm_b = (SINGLE && !s_unary && s_b_imm) ? immediate<T>(p, p.xb[0]) : T(0);
   const uint32_t s_a_off = (uint32_t)p.xa[0] * SLOT_BYTES, s_b_off = (uint32_t)p.xb[0] * SLOT_BYTES;
   unsigned char *const s_out = reinterpret_cast<unsigned char *>(p.out[0]) + (size_t)tid * 16;
 
@@ -668,10 +713,12 @@ __global__ void __launch_bounds__(PW_STREAM_THREADS, 2)
     if (SINGLE && c_tile + TILE_CHUNKS <= nchunks_full)
       pw_tile_single<T, V, U>(s_op, s_a_imm, s_b_imm, s_unary, s_imm_a, s_imm_b, ring_s + s_a_off, ring_s + s_b_off,
                               s_out + c_tile * 16);
-    else if (c_tile + TILE_CHUNKS <= nchunks_full)
-      pw_tile<T, V, U, true>(p, ring_s, file_s, c_tile, tid);
-    else
-      pw_tile<T, V, U, false>(p, ring_s, file_s, c_tile, tid);
+    else if (c_tile + TILE_CHUNKS <= nchunks_full) {
+      pw_tile<T, V, U, PW_STREAM_THREADS, true, true>(p, ring_s, file_s, c_tile, tid);
+    } else {
+      pw_fill<T, V, U, PW_STREAM_THREADS, true, true>(p, ring_s, c_tile, tid);  // the ragged last chunk
+      pw_tile<T, V, U, PW_STREAM_THREADS, false, true>(p, ring_s, file_s, c_tile, tid);
+    }
     __syncthreads();    // every thread is done reading this ring stage
     if (s_fail) break;  // uniform: s_fail was written before the barrier
     if (tid == 0 && k + stages < my_count) issue(k + stages, stage);
@@ -736,7 +783,7 @@ static int launch_stream_wide(b200_engine *e, const PwDev &d, size_t budget, int
   const size_t smem = (size_t)stages * TILE_CHUNKS * 16;
   const int blocks = (int)std::min<long long>(ntiles, 2LL * e->sm_count);
   static std::atomic<int> attr_dev_mask{0};
-  auto kern = pw_stream_kernel<T, V, U, true>;
+  auto kern = pw_stream_kernel<T, V, U, true, 2>;
   if (!(attr_dev_mask & (1 << (e->device & 31)))) {
     B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     attr_dev_mask |= 1 << (e->device & 31);
@@ -747,25 +794,25 @@ static int launch_stream_wide(b200_engine *e, const PwDev &d, size_t budget, int
   return B200_OK;
 }
 
-template <typename T, int V, int U>
+template <typename T, int V, int U, int CTAS>
 static int launch_stream_u(b200_engine *e, const PwDev &d, size_t budget, int stages) {
   constexpr int TILE_CHUNKS = PW_STREAM_THREADS * U;
   constexpr int SLOT_BYTES = TILE_CHUNKS * 16;
   const long long nchunks = (d.n + V - 1) / V;
   const long long ntiles = (nchunks + TILE_CHUNKS - 1) / TILE_CHUNKS;
   const size_t smem = ((size_t)stages * d.n_full + d.n_file) * SLOT_BYTES;
-  const bool single = pw_is_single(d);
-  const int blocks = (int)std::min<long long>(ntiles, 2LL * e->sm_count);  // two resident CTAs per SM
+  const bool single = CTAS == 2 && pw_is_single(d);
+  const int blocks = (int)std::min<long long>(ntiles, (long long)CTAS * e->sm_count);
   static std::atomic<int> attr_dev_mask[2];  // per instantiation: devices on which the attribute is set
   if (single) {
-    auto kern = pw_stream_kernel<T, V, U, true>;
+    auto kern = pw_stream_kernel<T, V, U, true, 2>;
     if (!(attr_dev_mask[1] & (1 << (e->device & 31)))) {
       B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
       attr_dev_mask[1] |= 1 << (e->device & 31);
     }
     kern<<<blocks, PW_STREAM_THREADS, smem, e->stream>>>(d, stages, e->d_flags + 2);
   } else {
-    auto kern = pw_stream_kernel<T, V, U, false>;
+    auto kern = pw_stream_kernel<T, V, U, false, CTAS>;
     if (!(attr_dev_mask[0] & (1 << (e->device & 31)))) {
       B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
       attr_dev_mask[0] |= 1 << (e->device & 31);
@@ -789,15 +836,33 @@ static int launch_stream(b200_engine *e, const PwDev &d) {
     if (budget / slot >= 3 && nchunks >= 8LL * 2 * e->sm_count * PW_STREAM_THREADS * 4)
       return launch_stream_wide<T, V>(e, d, budget, (int)std::min<size_t>(budget / slot, PW_MAX_STAGES));
   }
-  for (int u = 2; u >= 1; --u) {
-    const size_t slot = (size_t)PW_STREAM_THREADS * u * 16;
-    if (budget < d.n_file * slot) continue;
-    int stages = (int)((budget - d.n_file * slot) / ((size_t)d.n_full * slot));
-    stages = std::min(stages, PW_MAX_STAGES);
-    if (stages >= (u == 2 ? 3 : 2))
-      return u == 2 ? launch_stream_u<T, V, 2>(e, d, budget, stages) : launch_stream_u<T, V, 1>(e, d, budget, stages);
-  }
+  // tiles of u chunks per thread in a ring of `stages`, with `ctas` CTAs per SM; 0 stages: does not fit
+  auto stages_of = [&](int u, int ctas) -> int {
+    const size_t slot = (size_t)PW_STREAM_THREADS * u * 16, room = budget * 2 / ctas;
+    if (room < d.n_file * slot) return 0;
+    return std::min((int)((room - d.n_file * slot) / ((size_t)d.n_full * slot)), PW_MAX_STAGES);
+  };
+  if (const int st = stages_of(2, 2); st >= 3) return launch_stream_u<T, V, 2, 2>(e, d, budget, st);
+  // Programs of many tensors: one CTA per SM with two chunks per thread ahead of two CTAs with one. What an
+  // instruction costs besides its arithmetic (decoding, operand addresses, the branch to its code) is per
+  // thread and tile, and these programs are bound by instruction issue: a gated unit on 2^24 float32 takes
+  // 146 us this way and 177 the other.
+  if (const int st = stages_of(2, 1); st >= 2) return launch_stream_u<T, V, 2, 1>(e, d, budget * 2, st);
+  if (const int st = stages_of(1, 2); st >= 2) return launch_stream_u<T, V, 1, 2>(e, d, budget, st);
+  if (const int st = stages_of(1, 1); st >= 2) return launch_stream_u<T, V, 1, 1>(e, d, budget * 2, st);
   return -1;
+}
+
+// V == 1: some tensor is not aligned; the loop kernel still takes 16 bytes per thread and step.
+template <typename T, int V>
+static int launch_loop(b200_engine *e, const PwDev &d) {
+  constexpr int VV = Vec<T>::N;
+  const size_t smem = (size_t)(d.n_full + d.n_file) * PW_LOOP_THREADS * 16;  // at most 6 + 7 slots of 2 KB
+  const long long tiles = ((d.n + VV - 1) / VV + PW_LOOP_THREADS - 1) / PW_LOOP_THREADS;
+  const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)e->sm_count * 16));
+  pw_loop_kernel<T, VV, (V > 1)><<<blocks, PW_LOOP_THREADS, smem, e->stream>>>(d);
+  B200_CHECK_LAUNCH(e, "pw_loop_kernel");
+  return B200_OK;
 }
 
 template <typename T, int V>
@@ -820,7 +885,7 @@ static int launch_sized(b200_engine *e, const PwDev &d, int ns, int ni) {
   else if (ns <= 3 && ni <= 4)
     pw_kernel<T, V, 3, 4><<<blocks, threads, 0, e->stream>>>(d);
   else
-    pw_kernel<T, V, B200_PW_MAX_SRC, B200_PW_MAX_INSTR><<<blocks, threads, 0, e->stream>>>(d);
+    return launch_loop<T, V>(e, d);
   B200_CHECK_LAUNCH(e, "pw_kernel");
   return B200_OK;
 }
@@ -831,8 +896,7 @@ static int run_program(b200_engine *e, int dtype, const b200_pw_prog *prog, void
   B200_REQUIRE(e, prog && outs && (srcs || prog->n_src == 0), "pointwise: null argument");
   B200_REQUIRE(e, dtype == B200_F32 || dtype == B200_F64, "pointwise: dtype %d not supported", dtype);
   B200_REQUIRE(e, n >= 0, "pointwise: negative element count");
-  B200_REQUIRE(e, prog->n_instr >= 1 && prog->n_instr <= B200_PW_MAX_INSTR, "pointwise: %u instructions",
-               prog->n_instr);
+  B200_REQUIRE(e, prog->n_instr >= 1 && prog->n_instr <= B200_PW_MAX_INSTR, "pointwise: %u instructions", prog->n_instr);
   B200_REQUIRE(e, prog->n_src <= B200_PW_MAX_SRC, "pointwise: %u sources", prog->n_src);
   B200_REQUIRE(e, prog->n_imm <= B200_PW_MAX_IMM, "pointwise: %u immediates", prog->n_imm);
   B200_REQUIRE(e, prog->n_out >= 1 && prog->n_out <= B200_PW_MAX_OUT, "pointwise: %u outputs", prog->n_out);
@@ -841,7 +905,7 @@ static int run_program(b200_engine *e, int dtype, const b200_pw_prog *prog, void
   const size_t es = dtype_size(dtype);
   const int V = (int)(16 / es);
   PwDev d;
-  memset(&d, 0, sizeof d);
+  memset((void *)&d, 0, sizeof d);
   d.n = n;
   d.n_instr = (uint8_t)prog->n_instr;
   d.n_src = (uint8_t)prog->n_src;
@@ -870,7 +934,10 @@ static int run_program(b200_engine *e, int dtype, const b200_pw_prog *prog, void
         d.src_mode[s] = SRC_GENERAL;
     }
   }
-  for (uint32_t k = 0; k < prog->n_imm; ++k) d.imm[k] = prog->imm[k];
+  for (uint32_t k = 0; k < prog->n_imm; ++k) {
+    d.imm[k] = prog->imm[k];
+    d.immf[k] = (float)prog->imm[k];
+  }
   for (uint32_t k = 0; k < prog->n_instr; ++k) {
     const b200_pw_instr &in = prog->instr[k];
     B200_REQUIRE(e, is_binary(in.op) || is_unary(in.op), "pointwise: unknown op %d in instr %u", in.op, k);
@@ -928,6 +995,10 @@ static int run_program(b200_engine *e, int dtype, const b200_pw_prog *prog, void
       d.out_of[d.out_ins[o]] = (uint8_t)o;
     }
   }
+  for (uint32_t k = 0; k < prog->n_instr; ++k)
+    d.code[k] = make_uint2((uint32_t)d.op[k] | (uint32_t)d.ka[k] << 8 | (uint32_t)d.kb[k] << 12 |
+                               (uint32_t)d.xa[k] << 16 | (uint32_t)d.xb[k] << 24,
+                           (uint32_t)d.keep_slot[k] | (uint32_t)d.out_of[k] << 8);
   // a ROWVEC source needs the chunk grid itself aligned, which `aligned` guarantees
   if (!aligned)
     for (uint32_t s = 0; s < prog->n_src; ++s)
@@ -997,12 +1068,16 @@ struct Builder {
       if (l.ptr == ptr) return &l;
     return nullptr;
   }
-  int count_outputs() const {
+  // buffers that a kernel closed in front of call `end` has to store
+  int count_outputs(const b200_pw_call *calls, int n_calls, int end, const int *released_at) const {
     int k = 0;
     for (auto &l : locs)
-      if (l.writer >= 0) ++k;
+      if (l.writer >= 0 && !dead(calls, n_calls, l, end, released_at)) ++k;
     return k;
   }
+  // Whether the result that `l` holds needs no store if the kernel ends in front of call `end`: it was
+  // released, and no call queued between `end` and its release reads it.
+  bool dead(const b200_pw_call *calls, int n_calls, const Loc &l, int end, const int *released_at) const;
 };
 
 // Number of new source slots / immediates / output buffers a call would add, and whether it
@@ -1073,11 +1148,6 @@ bool can_join(const Builder &b, const b200_pw_call &c, size_t es, int max_instr)
   if (c.bcast == 1 && overlaps(d, Range{c.b, c.b + (uint64_t)c.bmod * es})) return false;
   if (c.bcast == 2 && overlaps(d, Range{c.a, c.a + (uint64_t)c.bmod * es})) return false;
   if (c.scalar_ptr && overlaps(d, Range{c.scalar_ptr, c.scalar_ptr + es})) return false;
-  int outs = b.count_outputs();
-  bool dst_written = false;
-  for (auto &l : b.locs)
-    if (l.ptr == c.dst && l.writer >= 0) dst_written = true;
-  if (!dst_written && outs + 1 > B200_PW_MAX_OUT) return false;
   return true;
 }
 
@@ -1138,9 +1208,24 @@ void join(Builder &b, const b200_pw_call &c, int idx, size_t es) {
   b.write_ranges.push_back({c.dst, c.dst + bytes});
 }
 
-// Closes the kernel: every buffer written becomes an output unless it was released before
-// any call outside this kernel could have read it.
-void finish(Builder &b, int end, const int *released_at, FusedKernel *fk) {
+bool Builder::dead(const b200_pw_call *calls, int n_calls, const Loc &l, int end, const int *released_at) const {
+  const int rel = released_at ? released_at[l.writer] : -1;
+  if (rel < 0 || rel <= l.writer) return false;
+  const size_t es = dtype_size(dtype);
+  const Range mine{l.ptr, l.ptr + (uint64_t)n * es};
+  for (int k = end; k < rel && k < n_calls; ++k) {
+    const b200_pw_call &c = calls[k];
+    const size_t ces = dtype_size(c.dtype);
+    const uint64_t full = (uint64_t)c.n * ces, small = (uint64_t)c.bmod * ces;
+    if (c.a && overlaps(mine, Range{c.a, c.a + (c.bcast == 2 ? small : full)})) return false;
+    if (c.b && overlaps(mine, Range{c.b, c.b + (c.bcast == 1 ? small : full)})) return false;
+    if (c.scalar_ptr && overlaps(mine, Range{c.scalar_ptr, c.scalar_ptr + ces})) return false;
+  }
+  return true;
+}
+
+// Closes the kernel: every buffer written becomes an output unless nothing can read it any more.
+void finish(Builder &b, const b200_pw_call *calls, int n_calls, int end, const int *released_at, FusedKernel *fk) {
   fk->dtype = b.dtype;
   fk->n = b.n;
   fk->first = b.first;
@@ -1155,9 +1240,7 @@ void finish(Builder &b, int end, const int *released_at, FusedKernel *fk) {
     auto &l = b.locs[i];
     if (l.writer < 0) continue;
     last_out_candidate = (int)i;
-    const int rel = released_at ? released_at[l.writer] : -1;
-    const bool dead = rel >= 0 && rel > l.writer && rel <= end;
-    if (dead) continue;
+    if (b.dead(calls, n_calls, l, end, released_at)) continue;
     fk->outs[nout] = (void *)l.ptr;
     b.prog.out_instr[nout] = (uint8_t)(l.ref & 0x3F);
     ++nout;
@@ -1178,28 +1261,72 @@ void finish(Builder &b, int end, const int *released_at, FusedKernel *fk) {
 
 }  // namespace
 
-// The fused kernels never exceed the program capacity of the largest kernel instantiation.
+// The fused kernels never exceed the program capacity.
 static const int kMaxFusedInstr = B200_PW_MAX_INSTR;
+
+// Joins calls from `i` on, as many as fit but no further than `limit`. Returns the last point at which the
+// buffers that live on are few enough to be stored (temporaries that nobody reads after it need no output);
+// *full: it was the program's length that ended the run. streams[j - i - 1], if wanted: the tensors a kernel
+// of the calls [i, j) reads and writes, or -1 where it cannot end.
+static int extend(Builder &b, const b200_pw_call *calls, int n_calls, const int *released_at, int i, int limit,
+                  bool *full, int *streams) {
+  const size_t es = dtype_size(calls[i].dtype);
+  b.start(calls[i], i);
+  join(b, calls[i], i, es);
+  int j = i + 1, best = j;
+  auto note = [&](int outs) {
+    if (!streams) return;
+    int loads = 0;
+    for (uint32_t s = 0; s < b.prog.n_src; ++s)
+      if (b.prog.src_div[s] == 0) ++loads;
+    streams[j - i - 1] = outs <= B200_PW_MAX_OUT ? loads + std::max(outs, 1) : -1;
+  };
+  note(b.count_outputs(calls, n_calls, j, released_at));
+  while (j < limit && can_join(b, calls[j], es, kMaxFusedInstr)) {
+    join(b, calls[j], j, es);
+    ++j;
+    const int outs = b.count_outputs(calls, n_calls, j, released_at);
+    if (outs <= B200_PW_MAX_OUT) best = j;
+    note(outs);
+  }
+  if (full) *full = j < limit && (int)b.prog.n_instr == kMaxFusedInstr;
+  return best;
+}
 
 static void plan(const b200_pw_call *calls, int n_calls, const int *released_at,
                  std::vector<FusedKernel> *out) {
   out->clear();
-  Builder b;
+  static thread_local Builder b, next;  // scratch: their vectors keep their capacity
   int i = 0;
   while (i < n_calls) {
-    const size_t es = dtype_size(calls[i].dtype);
-    b.start(calls[i], i);
-    join(b, calls[i], i, es);
-    int j = i + 1;
-    while (j < n_calls && can_join(b, calls[j], es, kMaxFusedInstr)) {
-      join(b, calls[j], j, es);
-      ++j;
+    bool full = false;
+    int streams[B200_PW_MAX_INSTR];
+    int best = extend(b, calls, n_calls, released_at, i, n_calls, &full, streams);
+    if (full) {
+      // A run longer than one program: cut it where this kernel and the next one move the fewest tensors per
+      // call (the longer one where that is the same), not simply where the program is full. Only shorter
+      // kernels that move fewer tensors themselves can gain.
+      const int mine = streams[best - i - 1];
+      double least = 0;
+      int cut = 0;
+      for (int j = best; j > i + (best - i) / 2; --j) {
+        if (streams[j - i - 1] < 0 || (j < best && streams[j - i - 1] >= mine)) continue;
+        int after[B200_PW_MAX_INSTR];
+        const int end = extend(next, calls, n_calls, released_at, j, n_calls, nullptr, after);
+        const double cost = (double)(streams[j - i - 1] + after[end - j - 1]) / (end - i);
+        if (cut == 0 || cost < least - 1e-9) {
+          least = cost;
+          cut = j;
+        }
+      }
+      best = cut;
     }
+    if (best - i != (int)b.prog.n_instr) extend(b, calls, n_calls, released_at, i, best, nullptr, nullptr);
     FusedKernel fk;
     memset(&fk, 0, sizeof fk);
-    finish(b, j, released_at, &fk);
+    finish(b, calls, n_calls, best, released_at, &fk);
     out->push_back(fk);
-    i = j;
+    i = best;
   }
 }
 

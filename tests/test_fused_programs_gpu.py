@@ -1,0 +1,108 @@
+"""Fused runs of calls that do not fit one program, that release their temporaries, or that take the shared-memory
+interpreter on small and unaligned tensors (GPU tests against the CPU oracle)."""
+import numpy as np
+import pytest
+
+from gorgonia_b200.engine import Tensor
+from oracle import oracle
+from tests import util
+from tests.util import assert_bits_equal, assert_pointwise_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _at(e, a, start):
+    """The array on the device, `start` elements into a larger buffer."""
+    whole = np.concatenate([np.zeros(start, a.dtype), a])
+    return Tensor(e, e.tensor(whole).ptr + start * a.itemsize, a.shape, a.dtype, owned=False)
+
+
+SIZES = [1, 3, 127, 128 * 4, 128 * 4 + 1, 5000, 1 << 20, 3_000_001]
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("start", [0, 1])
+def test_gated_unit(fresh, n, dt, start):
+    e = fresh
+    v = {k: util.normal(100 + i, n, dt) for i, k in enumerate("ifgoc")}
+    d = {k: _at(e, a, start) for k, a in v.items()}
+    c, h = (_at(e, np.zeros(n, dt), start) for _ in range(2))
+    e.Signal()
+    i, f, g, q = (e.empty((n,), dt) for _ in range(4))
+    e.Unary("sigmoid", d["i"], reuse=i)
+    e.Unary("sigmoid", d["f"], reuse=f)
+    e.Unary("tanh", d["g"], reuse=g)
+    e.Mul(f, d["c"], reuse=c)
+    e.Mul(i, g, unsafe=True)
+    e.Add(c, i, unsafe=True)
+    e.Unary("sigmoid", d["o"], reuse=q)
+    e.Unary("tanh", c, reuse=h)
+    e.Mul(h, q, unsafe=True)
+    for t in (i, f, g, q):
+        t.free()
+    assert e.pending() == (9, 2)
+    e.DoWork()
+    un = oracle.unary
+    wc = oracle.binary("add", oracle.binary("mul", un("sigmoid", v["f"]), v["c"]),
+                       oracle.binary("mul", un("sigmoid", v["i"]), un("tanh", v["g"])))
+    got = c.numpy()
+    # each factor within 1e-6 (1e-13) of its own, and the sum may cancel
+    rel = 4e-6 if dt == np.float32 else 4e-13
+    assert (np.abs(got - wc) <= rel * (np.abs(v["c"]) + 1)).all()
+    assert_pointwise_close(h.numpy(), oracle.binary("mul", un("tanh", got), un("sigmoid", v["o"])), rel)
+
+
+@pytest.mark.parametrize("n", [777, 1 << 20])
+@pytest.mark.parametrize("length", [7, 8, 9, 17, 30])
+def test_runs_of_any_length(fresh, n, length):
+    # a run in place; one that keeps every result; one whose temporaries are released at its end
+    e = fresh
+    x, y = util.normal(5, n), util.normal(6, n)
+    want = [x]
+    for k in range(length):
+        want.append(oracle.binary("add" if k % 2 else "mul", want[-1], y))
+    tx, ty = e.tensor(x), e.tensor(y)
+    for k in range(length):
+        (e.Add if k % 2 else e.Mul)(tx, ty, unsafe=True)
+    e.DoWork()
+    assert_bits_equal(tx.numpy(), want[-1])
+    tx.set(x)
+    kept = [e.empty(n) for _ in range(length)]
+    e.Signal()
+    a = tx
+    for k in range(length):
+        a = (e.Add if k % 2 else e.Mul)(a, ty, reuse=kept[k])
+    e.DoWork()
+    for k in range(length):
+        assert_bits_equal(kept[k].numpy(), want[k + 1])
+    out = e.empty(n)
+    a = tx
+    for k in range(length):
+        a = (e.Add if k % 2 else e.Mul)(a, ty, reuse=kept[k] if k + 1 < length else out)
+    for t in kept[:-1]:
+        t.free()
+    e.DoWork()
+    assert_bits_equal(out.numpy(), want[-1])
+
+
+def test_released_temporary_that_is_read_later_is_stored(fresh):
+    # more results than one kernel stores, read again after the point where it has to end
+    e = fresh
+    n = 1 << 18
+    xs = [util.normal(20 + k, n) for k in range(6)]
+    ts = [e.tensor(a) for a in xs]
+    tmp, out = [e.empty(n) for _ in range(6)], [e.empty(n) for _ in range(6)]
+    e.Signal()
+    for k in range(6):
+        e.Unary("square", ts[k], reuse=tmp[k])
+    for k in range(6):
+        e.Add(tmp[k], ts[(k + 1) % 6], reuse=out[k])
+    for t in tmp:
+        t.free()
+    again = e.empty(n)      # may well be one of the released buffers
+    e.Unary("neg", out[0], reuse=again)
+    e.DoWork()
+    for k in range(6):
+        assert_bits_equal(out[k].numpy(), oracle.binary("add", oracle.unary("square", xs[k]), xs[(k + 1) % 6]))
+    assert_bits_equal(again.numpy(), oracle.unary("neg", out[0].numpy()))
