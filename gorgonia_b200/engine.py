@@ -45,11 +45,19 @@ def _epilogue(bias=None, bias_kind=None, act=None, alpha=0.0, accumulate=False):
     return ep
 
 
+def _count(shape):
+    """Elements of a shape. (np.prod takes 2.5 us, which is half of what a small call costs in all.)"""
+    n = 1
+    for s in shape:
+        n *= int(s)
+    return n
+
+
 def dtype_code(dt):
-    dt = np.dtype(dt)
-    if dt not in _DT:
+    code = _DT.get(np.dtype(dt))
+    if code is None:
         raise B200Error(_lib.ERR_UNSUPPORTED, f"dtype {dt} not supported")
-    return _DT[dt]
+    return code
 
 
 class Tensor:
@@ -62,13 +70,7 @@ class Tensor:
         self.shape = tuple(int(s) for s in shape)
         self.dtype = np.dtype(dtype)
         self.owned = owned
-
-    @property
-    def size(self):
-        n = 1
-        for s in self.shape:
-            n *= s
-        return n
+        self.size = _count(self.shape)
 
     @property
     def nbytes(self):
@@ -215,8 +217,7 @@ class Engine:
         if isinstance(shape, int):
             shape = (shape,)
         dtype = np.dtype(dtype)
-        n = int(np.prod(shape, dtype=np.int64)) if len(shape) else 1
-        ptr = self.Get(max(n, 1) * dtype.itemsize)
+        ptr = self.Get(max(_count(shape), 1) * dtype.itemsize)
         return Tensor(self, ptr, shape, dtype)
 
     def tensor(self, arr, dtype=None):
@@ -400,9 +401,7 @@ class Engine:
     @staticmethod
     def _oli(shape, axis):
         axis %= len(shape)
-        o = int(np.prod(shape[:axis], dtype=np.int64))
-        i = int(np.prod(shape[axis + 1:], dtype=np.int64))
-        return o, shape[axis], i, axis
+        return _count(shape[:axis]), shape[axis], _count(shape[axis + 1:]), axis
 
     def SoftMax(self, x, prealloc, axis=-1, log=False):
         o, l, i, _ = self._oli(x.shape, axis)
