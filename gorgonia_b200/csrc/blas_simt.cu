@@ -13,6 +13,7 @@
 
 #include "engine.h"
 #include "epilogue.cuh"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -23,6 +24,7 @@ __device__ __forceinline__ double fma_(double a, double b, double c) { return fm
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) gemv_n_kernel(const T *__restrict__ A, long long lda, const T *__restrict__ x,
                                                      T *__restrict__ y, long long M, long long N) {
+  ptx::grid_begin();
   constexpr int V = 16 / sizeof(T);
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -82,6 +84,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gemv_n_smemx_kernel(const T *__restrict__ A, long long lda,
                                                            const T *__restrict__ x, T *__restrict__ y, long long M,
                                                            long long N) {
+  ptx::grid_begin();
   constexpr int V = 16 / sizeof(T);
   constexpr int CH = 2048;  // 16-byte pieces of x per chunk
   __shared__ uint4 xs[CH];
@@ -143,6 +146,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gemv_t_partial_kernel(const T *__restrict__ A, long long lda,
                                                              const T *__restrict__ x, T *__restrict__ part,
                                                              long long M, long long N, long long rows_per_chunk) {
+  ptx::grid_begin();
   const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long r0 = (long long)blockIdx.y * rows_per_chunk;
   const long long r1 = r0 + rows_per_chunk < M ? r0 + rows_per_chunk : M;
@@ -164,6 +168,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gemv_t_partial_vec_kernel(const T *__restrict__ A, long long lda,
                                                                  const T *__restrict__ x, T *__restrict__ part,
                                                                  long long M, long long N, long long rows_per_chunk) {
+  ptx::grid_begin();
   constexpr int V = 16 / sizeof(T);
   const long long cv = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // column group
   const long long r0 = (long long)blockIdx.y * rows_per_chunk;
@@ -207,6 +212,7 @@ __global__ void __launch_bounds__(256) gemv_t_partial_vec_kernel(const T *__rest
 template <typename T>
 __global__ void __launch_bounds__(256) fold_rows_kernel(const T *__restrict__ part, T *__restrict__ y, long long N,
                                                         int chunks) {
+  ptx::grid_begin();
   const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= N) return;
   T s = 0;
@@ -218,6 +224,7 @@ __global__ void __launch_bounds__(256) fold_rows_kernel(const T *__restrict__ pa
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) ger_kernel(const T *__restrict__ x, const T *__restrict__ y, T *__restrict__ A,
                                                   long long M, long long N) {
+  ptx::grid_begin();
   constexpr int V = 16 / sizeof(T);
   if (VEC) {
     // A block takes groups of four consecutive rows (group blockIdx.x, blockIdx.x + gridDim.x, ...; the
@@ -269,6 +276,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(int transA, int transB, 
                                                         const T *__restrict__ B, long long ldb, T *__restrict__ C,
                                                         long long ldc, long long strideA, long long strideB,
                                                         long long strideC, Epilogue ep) {
+  ptx::grid_begin();
   constexpr int BM = 64, BN = 64, BK = 16;
   __shared__ T As[BK][BM + 1];
   __shared__ T Bs[BK][BN + 1];
@@ -352,6 +360,7 @@ __global__ void __launch_bounds__(256) gemm_skinny_kernel(int transB, long long 
                                                           const T *__restrict__ B, long long ldb, T *__restrict__ C,
                                                           long long ldc, long long strideA, long long strideB,
                                                           long long strideC, Epilogue ep) {
+  ptx::grid_begin();
   constexpr int NMAX = 16;
   A += (long long)blockIdx.y * strideA;
   B += (long long)blockIdx.y * strideB;
@@ -396,11 +405,11 @@ int gemm_simt(b200_engine *e, int dtype, int transA, int transB, long long M, lo
     const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((M + 7) / 8, (long long)e->sm_count * 8));
     dim3 sgrid(blocks, (unsigned)batch);
     if (dtype == B200_F32)
-      gemm_skinny_kernel<float><<<sgrid, 256, 0, e->stream>>>(transB, M, (int)N, K, (const float *)A, lda,
+      launch_kernel(e, gemm_skinny_kernel<float>, sgrid, 256, 0, transB, M, (int)N, K, (const float *)A, lda,
                                                              (const float *)B, ldb, (float *)C, ldc, strideA, strideB,
                                                              strideC, ep);
     else
-      gemm_skinny_kernel<double><<<sgrid, 256, 0, e->stream>>>(transB, M, (int)N, K, (const double *)A, lda,
+      launch_kernel(e, gemm_skinny_kernel<double>, sgrid, 256, 0, transB, M, (int)N, K, (const double *)A, lda,
                                                               (const double *)B, ldb, (double *)C, ldc, strideA,
                                                               strideB, strideC, ep);
     B200_CHECK_LAUNCH(e, "gemm_skinny_kernel");
@@ -410,7 +419,7 @@ int gemm_simt(b200_engine *e, int dtype, int transA, int transB, long long M, lo
     return gemm_f64(e, transA, transB, M, N, K, (const double *)A, lda, (const double *)B, ldb, (double *)C, ldc,
                     batch, strideA, strideB, strideC, ep);
   dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64), (unsigned)batch);
-  gemm_simt_kernel<float><<<grid, 256, 0, e->stream>>>(transA, transB, M, N, K, (const float *)A, lda,
+  launch_kernel(e, gemm_simt_kernel<float>, grid, 256, 0, transA, transB, M, N, K, (const float *)A, lda,
                                                       (const float *)B, ldb, (float *)C, ldc, strideA, strideB,
                                                       strideC, ep);
   B200_CHECK_LAUNCH(e, "gemm_simt_kernel");
@@ -432,11 +441,11 @@ static int gemv_typed(b200_engine *e, int transA, long long M, long long N, cons
     // measured 5.6 against 4.8 TB/s at 8192 x 32768; with more blocks than fit, the plain kernel is ahead
     // (5.6 against 5.5 at 16384 x 16384, 5.3 against 5.2 at 40000 x 6000). The two give the same bits.
     if (vec && N >= 4096 && (M + 7) / 8 <= cap)
-      gemv_n_smemx_kernel<T><<<blocks, 256, 0, e->stream>>>(A, lda, x, y, M, N);
+      launch_kernel(e, gemv_n_smemx_kernel<T>, blocks, 256, 0, A, lda, x, y, M, N);
     else if (vec)
-      gemv_n_kernel<T, true><<<blocks, 256, 0, e->stream>>>(A, lda, x, y, M, N);
+      launch_kernel(e, gemv_n_kernel<T, true>, blocks, 256, 0, A, lda, x, y, M, N);
     else
-      gemv_n_kernel<T, false><<<blocks, 256, 0, e->stream>>>(A, lda, x, y, M, N);
+      launch_kernel(e, gemv_n_kernel<T, false>, blocks, 256, 0, A, lda, x, y, M, N);
     B200_CHECK_LAUNCH(e, "gemv_n_kernel");
     return B200_OK;
   }
@@ -453,13 +462,13 @@ static int gemv_typed(b200_engine *e, int transA, long long M, long long N, cons
   if (rc != B200_OK) return rc;
   dim3 grid((unsigned)col_blocks, (unsigned)chunks);
   if (tvec)
-    gemv_t_partial_vec_kernel<T><<<grid, 256, 0, e->stream>>>(A, lda, x, (T *)part, M, N, rows_per_chunk);
+    launch_kernel(e, gemv_t_partial_vec_kernel<T>, grid, 256, 0, A, lda, x, (T *)part, M, N, rows_per_chunk);
   else
-    gemv_t_partial_kernel<T><<<grid, 256, 0, e->stream>>>(A, lda, x, (T *)part, M, N, rows_per_chunk);
+    launch_kernel(e, gemv_t_partial_kernel<T>, grid, 256, 0, A, lda, x, (T *)part, M, N, rows_per_chunk);
   cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) {
     e->launches++;
-    fold_rows_kernel<T><<<(unsigned)((N + 255) / 256), 256, 0, e->stream>>>((const T *)part, y, N, (int)chunks);
+    launch_kernel(e, fold_rows_kernel<T>, (unsigned)((N + 255) / 256), 256, 0, (const T *)part, y, N, (int)chunks);
     le = cudaGetLastError();
     if (le == cudaSuccess) e->launches++;
   }
@@ -514,14 +523,14 @@ int b200_ger(b200_engine *e, int dtype, int64_t M, int64_t N, const void *x, con
   if (vec) blocks = (int)std::max<long long>(1, std::min<long long>((M + 3) / 4, (long long)e->sm_count * 64));  // groups of four rows
   if (dtype == B200_F32) {
     if (vec)
-      ger_kernel<float, true><<<blocks, 256, 0, e->stream>>>((const float *)x, (const float *)y, (float *)A, M, N);
+      launch_kernel(e, ger_kernel<float, true>, blocks, 256, 0, (const float *)x, (const float *)y, (float *)A, M, N);
     else
-      ger_kernel<float, false><<<blocks, 256, 0, e->stream>>>((const float *)x, (const float *)y, (float *)A, M, N);
+      launch_kernel(e, ger_kernel<float, false>, blocks, 256, 0, (const float *)x, (const float *)y, (float *)A, M, N);
   } else {
     if (vec)
-      ger_kernel<double, true><<<blocks, 256, 0, e->stream>>>((const double *)x, (const double *)y, (double *)A, M, N);
+      launch_kernel(e, ger_kernel<double, true>, blocks, 256, 0, (const double *)x, (const double *)y, (double *)A, M, N);
     else
-      ger_kernel<double, false><<<blocks, 256, 0, e->stream>>>((const double *)x, (const double *)y, (double *)A, M,
+      launch_kernel(e, ger_kernel<double, false>, blocks, 256, 0, (const double *)x, (const double *)y, (double *)A, M,
                                                               N);
   }
   B200_CHECK_LAUNCH(e, "ger_kernel");

@@ -14,6 +14,7 @@
 #include "engine.h"
 #include "epilogue.cuh"
 #include "pairs.cuh"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(256) conv_direct_small_kernel(const float *__r
                                                                 int Wo, int kh, int kw, int padH, int padW, int sH,
                                                                 int sW, int dH, int dW, Epilogue ep,
                                                                 const float *__restrict__ zero) {
+  ptx::grid_begin();
   __shared__ __align__(16) float ws[32 * KP];
   __shared__ int q_off[32];  // offset of tap q relative to the pixel's window origin, inside one image
   __shared__ int q_tap[32];  // r*kw + s of tap q, or 32 for q past the end of the filter
@@ -159,6 +161,7 @@ template <int C, int ACT, bool BIAS>
 __global__ void __launch_bounds__(256, 2) conv3x3_first_kernel(const float *__restrict__ x, const float *__restrict__ w,
                                                             float *__restrict__ y, const float *__restrict__ bias,
                                                             float alpha, long long groups, int H, int W, int K) {
+  ptx::grid_begin();
   constexpr int Q = C * 9;
   __shared__ __align__(16) float ws[Q * 32];  // [q][k], zero for k >= K
   __shared__ float bs[32];
@@ -245,7 +248,7 @@ static int launch_conv3x3_first(b200_engine *e, const float *x, const float *w, 
   const float *bias = (const float *)ep.bias;
   const float alpha = (float)ep.alpha;
 #define B200_FIRST(ACT, BIAS) \
-  conv3x3_first_kernel<C, ACT, BIAS><<<blocks, 256, 0, e->stream>>>(x, w, y, bias, alpha, groups, H, W, K)
+  launch_kernel(e, conv3x3_first_kernel<C, ACT, BIAS>, blocks, 256, 0, x, w, y, bias, alpha, groups, H, W, K)
   const bool hb = ep.bias_kind != B200_BIAS_NONE;
   if (ep.act == B200_ACT_NONE) { if (hb) B200_FIRST(B200_ACT_NONE, true); else B200_FIRST(B200_ACT_NONE, false); }
   else if (ep.act == B200_ACT_RECTIFY) { if (hb) B200_FIRST(B200_ACT_RECTIFY, true); else B200_FIRST(B200_ACT_RECTIFY, false); }
@@ -271,6 +274,7 @@ __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float 
                                                                     float *__restrict__ y_lo,
                                                                     const int *__restrict__ only_if,
                                                                     const F16Rec *__restrict__ x_rec, PairsOut out16) {
+  ptx::grid_begin();
   if (!F16 && skip_launch(only_if)) return;
   constexpr int Q = C * 9;
   __shared__ __align__(16) float ws[Q * 32];  // [q][k], zero for k >= K
@@ -413,7 +417,7 @@ static int launch_conv3x3_first_pool(b200_engine *e, const float *x, const float
   const float *bias = (const float *)ep.bias;
   const float alpha = (float)ep.alpha;
 #define B200_FIRSTP(ACT, BIAS)                                                                                        \
-  conv3x3_first_pool_kernel<C, ACT, BIAS, F16><<<blocks, 256, 0, e->stream>>>(x, w, y, bias, alpha, groups, H, W, K, y_hi, \
+  launch_kernel(e, conv3x3_first_pool_kernel<C, ACT, BIAS, F16>, blocks, 256, 0, x, w, y, bias, alpha, groups, H, W, K, y_hi, \
                                                                               y_lo, e->only_if, x_rec, out16)
   const bool hb = ep.bias_kind != B200_BIAS_NONE;
   if (ep.act == B200_ACT_NONE) { if (hb) B200_FIRSTP(B200_ACT_NONE, true); else B200_FIRSTP(B200_ACT_NONE, false); }
@@ -443,7 +447,7 @@ static int conv_direct_small(b200_engine *e, const float *x, const float *w, flo
   const float *zero = reinterpret_cast<const float *>(e->d_flags + 8);  // zeroed at engine creation, never written
   const int blocks = (int)std::max<long long>(1, std::min<long long>((Mtot + 255) / 256, (long long)e->sm_count * 16));
 #define B200_DIRECT(KP)                                                                                        \
-  conv_direct_small_kernel<KP><<<blocks, 256, 0, e->stream>>>(x, w, y, Mtot, C, H, W, K, Ho, Wo, kh, kw, padH, padW, \
+  launch_kernel(e, conv_direct_small_kernel<KP>, blocks, 256, 0, x, w, y, Mtot, C, H, W, K, Ho, Wo, kh, kw, padH, padW, \
                                                              sH, sW, dH, dW, ep, zero)
   if (K <= 8) B200_DIRECT(8);
   else if (K <= 16) B200_DIRECT(16);
@@ -460,6 +464,7 @@ static int conv_direct_small(b200_engine *e, const float *x, const float *w, flo
 // for a constant; otherwise a few kilobytes to a few megabytes, bound by the launch.
 __global__ void __launch_bounds__(256) filter_pairs_kernel(const float *__restrict__ w, __half *__restrict__ hi,
                                                            __half *__restrict__ lo, int C, int taps, F16Filters *f) {
+  ptx::grid_begin();
   __shared__ float red[8];
   const int crs = C * taps;
   const float *in = w + (long long)blockIdx.x * crs;
@@ -510,7 +515,7 @@ static int conv_filters_pairs(b200_engine *e, const float *w, int K, int C, int 
   wf->p1 = blk[1];
   if (rc == B200_OK) rc = launch_magnitude(e, w, n, 1, &(*f)->rec);
   if (rc == B200_OK) {
-    filter_pairs_kernel<<<K, 256, 0, e->stream>>>(w, (__half *)const_cast<void *>(wf->p0),
+    launch_kernel(e, filter_pairs_kernel, K, 256, 0, w, (__half *)const_cast<void *>(wf->p0),
                                                   (__half *)const_cast<void *>(wf->p1), C, taps, *f);
     if (cudaGetLastError() != cudaSuccess) rc = set_error(e, B200_ERR_CUDA, "launch of filter_pairs_kernel failed");
     else e->launches++;

@@ -97,6 +97,7 @@ template <int BN, int MODE>
 __global__ void __launch_bounds__(CV_THREADS, 1)
     conv_tc_kernel(const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                    const __grid_constant__ ConvTcParams p) {
+  ptx::grid_begin();
   constexpr int B_BYTES = BN * 128;
   constexpr int STAGE_BYTES = 2 * (CV_A_BYTES + B_BYTES);
   constexpr uint32_t IDESC = make_idesc(2, 0, 0, CV_BM, BN);
@@ -464,6 +465,7 @@ __global__ void __launch_bounds__(CV_THREADS, 1)
 // w (K, C, taps) -> head/tail (K, taps, C): out[k][tap*C + c] = split(w[k][c*taps + tap])
 __global__ void __launch_bounds__(256) split_permute_filters_kernel(const float *__restrict__ w, float *__restrict__ hi,
                                                                     float *__restrict__ lo, int K, int C, int taps) {
+  ptx::grid_begin();
   const long long total = (long long)K * C * taps;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -498,7 +500,7 @@ int conv_filters_tap_major(b200_engine *e, const float *w, int K, int C, int tap
   }
   const long long total = (long long)K * crs;
   const int blocks = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, e->sm_count * 16LL));
-  split_permute_filters_kernel<<<blocks, 256, 0, e->stream>>>(w, (float *)blk[0], (float *)blk[1], K, C, taps);
+  launch_kernel(e, split_permute_filters_kernel, blocks, 256, 0, w, (float *)blk[0], (float *)blk[1], K, C, taps);
   B200_CHECK_LAUNCH(e, "split_permute_filters_kernel");
   wf->p0 = blk[0];
   wf->p1 = blk[1];
@@ -526,7 +528,7 @@ static int launch_conv_tc(b200_engine *e, const CUtensorMap *tm, ConvTcParams &p
   const size_t smem = (size_t)p.stages * STAGE_BYTES + 1024;
   const long long tiles = (long long)p.tiles_m * p.tiles_n;
   const int grid = (int)std::min<long long>(tiles, e->sm_count);
-  kern<<<grid, CV_THREADS, smem, e->stream>>>(tm[0], tm[1], p);
+  launch_kernel(e, kern, grid, CV_THREADS, smem, tm[0], tm[1], p);
   B200_CHECK_LAUNCH(e, "conv_tc_kernel");
   e->flags_dirty = true;
   return B200_OK;

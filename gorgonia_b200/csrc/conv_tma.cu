@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
     conv_tma_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                     const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                     const __grid_constant__ ConvTmaParams p) {
+  ptx::grid_begin();
   constexpr int CK = ROW_BYTES / (F16 ? 2 : 4);
   constexpr int A_BYTES = CT_BM * ROW_BYTES;      // one copy (head or tail) of the col slab
   constexpr int B_BYTES = BN * ROW_BYTES;
@@ -463,6 +464,7 @@ __device__ __forceinline__ void nhwc_store(const NhwcOut &out, long long at, con
 template <bool F16>
 __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict__ x, NhwcOut out, long long B, int C,
                                                          int HW) {
+  ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
   unsigned small = 0;
@@ -504,6 +506,7 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
 template <int CT, bool F16>
 __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restrict__ x, NhwcOut out, long long B, int C,
                                                           int HW) {
+  ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
   unsigned small = 0;
@@ -551,6 +554,7 @@ __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restric
 template <bool F16>
 __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__restrict__ x, NhwcOut out, long long B,
                                                              int C, int HW, int pitch) {
+  ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
   unsigned small = 0;
@@ -595,9 +599,9 @@ static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C,
     const long long tiles = B * ((HW + 127) / 128) * (C / ct);
     const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, e->sm_count * 32LL));
     if (ct == 32)
-      nhwc_split4_kernel<32, F16><<<blocks, 256, 0, e->stream>>>(x, out, B, C, HW);
+      launch_kernel(e, nhwc_split4_kernel<32, F16>, blocks, 256, 0, x, out, B, C, HW);
     else
-      nhwc_split4_kernel<16, F16><<<blocks, 256, 0, e->stream>>>(x, out, B, C, HW);
+      launch_kernel(e, nhwc_split4_kernel<16, F16>, blocks, 256, 0, x, out, B, C, HW);
     B200_CHECK_LAUNCH(e, "nhwc_split4_kernel");
     return B200_OK;
   }
@@ -606,13 +610,13 @@ static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C,
     while (pitch % 8 != 1) ++pitch;
     const long long work = B * (C / 32);
     const int blocks = (int)std::max<long long>(1, std::min<long long>(work, e->sm_count * 16LL));
-    nhwc_split_img_kernel<F16><<<blocks, 256, (size_t)32 * pitch * 4, e->stream>>>(x, out, B, C, HW, pitch);
+    launch_kernel(e, nhwc_split_img_kernel<F16>, blocks, 256, (size_t)32 * pitch * 4, x, out, B, C, HW, pitch);
     B200_CHECK_LAUNCH(e, "nhwc_split_img_kernel");
     return B200_OK;
   }
   const long long tiles = B * ((HW + 31) / 32) * ((C + 31) / 32);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, e->sm_count * 16LL));
-  nhwc_split_kernel<F16><<<blocks, 256, 0, e->stream>>>(x, out, B, C, HW);
+  launch_kernel(e, nhwc_split_kernel<F16>, blocks, 256, 0, x, out, B, C, HW);
   B200_CHECK_LAUNCH(e, "nhwc_split_kernel");
   return B200_OK;
 }
@@ -700,7 +704,7 @@ static int launch_conv_tma(b200_engine *e, const CUtensorMap *tm, ConvTmaParams 
       p.ws = (float *)ws;
     }
   }
-  kern<<<grid, CT_THREADS, smem, e->stream>>>(tm[0], tm[1], tm[2], tm[3], p);
+  launch_kernel(e, kern, grid, CT_THREADS, smem, tm[0], tm[1], tm[2], tm[3], p);
   cudaError_t le = cudaGetLastError();
   if (ws) b200_put(e, ws, 0);  // stream order: whoever gets the block next runs after this kernel
   if (le != cudaSuccess)

@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
     conv_win_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                     const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1,
                     const __grid_constant__ ConvWinParams p) {
+  ptx::grid_begin();
   constexpr int ROW_BYTES = CK * (F16 ? 2 : 4);
   constexpr int B_BYTES = BN * ROW_BYTES;
   constexpr int B_STAGE_BYTES = 2 * B_BYTES;      // head + tail
@@ -510,7 +511,7 @@ static int launch_conv_win(b200_engine *e, const CUtensorMap *tm, ConvWinParams 
       2, std::min<size_t>(CW_MAX_BSTAGES, (cw_smem_budget(e) - 1024 - win_total) / B_STAGE_BYTES));
   const size_t smem = win_total + (size_t)p.b_stages * B_STAGE_BYTES + 1024;
   const int grid = (int)std::min<long long>(p.total_tiles, e->sm_count);
-  kern<<<grid, CW_THREADS, smem, e->stream>>>(tm[0], tm[1], tm[2], tm[3], p);
+  launch_kernel(e, kern, grid, CW_THREADS, smem, tm[0], tm[1], tm[2], tm[3], p);
   B200_CHECK_LAUNCH(e, "conv_win_kernel");
   e->flags_dirty = true;
   return B200_OK;

@@ -10,6 +10,7 @@
 // It tells kept elements from dropped ones by the forward output, not by a mask, and it divides by
 // the drop probability, not by the keep probability; both are reproduced.
 #include "engine.h"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -55,6 +56,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256) dropout_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, long long n,
                                                           T keep, const T *__restrict__ rnd, unsigned long long seed,
                                                           unsigned long long offset) {
+  ptx::grid_begin();
   struct alignas(V * sizeof(T)) Vec {
     T v[V];
   };
@@ -82,6 +84,7 @@ __global__ void __launch_bounds__(256) dropout_fwd_kernel(const T *__restrict__ 
 template <typename T, int V>
 __global__ void __launch_bounds__(256) dropout_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ out,
                                                           T *__restrict__ dx, long long n, T prob) {
+  ptx::grid_begin();
   struct alignas(V * sizeof(T)) Vec {
     T v[V];
   };
@@ -109,17 +112,17 @@ static void launch_dropout_fwd(b200_engine *e, const T *x, T *y, long long n, T 
                                uint64_t offset) {
   constexpr int V = 16 / sizeof(T);
   if (((uintptr_t)x | (uintptr_t)y | (uintptr_t)rnd) % 16 == 0)
-    dropout_fwd_kernel<T, V><<<grid_of(e, n / V), 256, 0, e->stream>>>(x, y, n, keep, rnd, seed, offset);
+    launch_kernel(e, dropout_fwd_kernel<T, V>, grid_of(e, n / V), 256, 0, x, y, n, keep, rnd, seed, offset);
   else
-    dropout_fwd_kernel<T, 1><<<grid_of(e, n), 256, 0, e->stream>>>(x, y, n, keep, rnd, seed, offset);
+    launch_kernel(e, dropout_fwd_kernel<T, 1>, grid_of(e, n), 256, 0, x, y, n, keep, rnd, seed, offset);
 }
 template <typename T>
 static void launch_dropout_bwd(b200_engine *e, const T *dy, const T *out, T *dx, long long n, T prob) {
   constexpr int V = 16 / sizeof(T);
   if (((uintptr_t)dy | (uintptr_t)out | (uintptr_t)dx) % 16 == 0)
-    dropout_bwd_kernel<T, V><<<grid_of(e, n / V), 256, 0, e->stream>>>(dy, out, dx, n, prob);
+    launch_kernel(e, dropout_bwd_kernel<T, V>, grid_of(e, n / V), 256, 0, dy, out, dx, n, prob);
   else
-    dropout_bwd_kernel<T, 1><<<grid_of(e, n), 256, 0, e->stream>>>(dy, out, dx, n, prob);
+    launch_kernel(e, dropout_bwd_kernel<T, 1>, grid_of(e, n), 256, 0, dy, out, dx, n, prob);
 }
 
 }  // namespace b200

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/gorgonia_b200.h"
@@ -135,6 +136,28 @@ struct DeviceGuard {
                              cudaGetErrorString(err__));                               \
     (e)->launches++;                                                                   \
   } while (0)
+
+// Every kernel of the library is launched through this, and begins with ptx::grid_begin(): the launch is
+// prepared while the kernel in front of it ends (programmatic dependent launch; in a recorded tape the edge
+// between the two is one of that kind), and its blocks wait there until that kernel has finished and its
+// writes are visible. What is saved is launch latency, about two microseconds per kernel: a 1000 x 1152 x 625
+// dense layer (seven launches) 108.6 -> 93.0 us, batch norm with dropout (eight) 119.9 -> 101.3 us. Letting
+// the next kernel's blocks in from the start of this one (griddepcontrol.launch_dependents) was measured too:
+// they pile up on the SMs that finish first, and LeNet at 8192 went from 799 to 816 us.
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(b200_engine *e, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = e->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 inline size_t dtype_size(int dtype) {
   switch (dtype) {

@@ -77,6 +77,7 @@ struct SlabF64 {
 
 template <int T, bool A_MN, bool B_MN, int V>
 __global__ void __launch_bounds__(F64_THREADS) gemm_f64_kernel(const __grid_constant__ GemmF64Params p) {
+  ptx::grid_begin();
   using SA = SlabF64<T, A_MN>;
   using SB = SlabF64<T, B_MN>;
   constexpr int F = T / 16;  // 8 x 8 fragments of a warp along either side: its quarter of the tile is T/2 x T/2
@@ -188,7 +189,7 @@ static int launch_f64(b200_engine *e, const GemmF64Params &p, dim3 grid) {
     B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_dev_mask |= 1 << (e->device & 31);
   }
-  kern<<<grid, F64_THREADS, smem, e->stream>>>(p);
+  launch_kernel(e, kern, grid, F64_THREADS, smem, p);
   B200_CHECK_LAUNCH(e, "gemm_f64_kernel");
   return B200_OK;
 }

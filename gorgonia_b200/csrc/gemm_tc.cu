@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                    const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
                    const __grid_constant__ GemmTcParams p) {
+  ptx::grid_begin();
   static_assert(!PAIR || TERMS == 1, "only bf16 tiles are shared by a pair of CTAs");
   constexpr int ES = TERMS == 3 ? 4 : 2;           // operand element size
   constexpr int BK = TC_ROW_BYTES / ES;            // k elements per stage: 64 (16-bit values) / 32 (TF32)
@@ -722,12 +723,14 @@ static int launch_tc(b200_engine *e, const CUtensorMap *tm, const GemmTcParams &
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = e->stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_kernel does
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
     cfg.numAttrs = 1;
     // Only clusters that are resident together may share the tiles out evenly: a GPU whose SMs do
     // not all pair up would otherwise run the left-over clusters as a second round.
@@ -741,9 +744,10 @@ static int launch_tc(b200_engine *e, const CUtensorMap *tm, const GemmTcParams &
     GemmTcParams pp = p;
     pp.workers = std::min(p.workers, mc);
     cfg.gridDim = dim3((unsigned)(2 * pp.workers));
+    cfg.numAttrs = 2;
     B200_CHECK_CUDA(e, cudaLaunchKernelEx(&cfg, kern, tm[0], tm[1], tm[2], tm[3], pp));
   } else {
-    kern<<<grid, TC_THREADS, smem, e->stream>>>(tm[0], tm[1], tm[2], tm[3], p);
+    launch_kernel(e, kern, grid, TC_THREADS, smem, tm[0], tm[1], tm[2], tm[3], p);
   }
   B200_CHECK_LAUNCH(e, "gemm_tc_kernel");
   e->flags_dirty = true;

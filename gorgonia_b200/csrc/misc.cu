@@ -10,6 +10,7 @@ namespace b200 {
 
 template <typename T, bool INF>
 __global__ void __launch_bounds__(256) has_special_kernel(const T *__restrict__ x, long long n, int *flag) {
+  ptx::grid_begin();
   const long long stride = (long long)gridDim.x * blockDim.x;
   bool hit = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -39,9 +40,9 @@ static int has_special(b200_engine *e, int dtype, const void *x, int64_t n, int 
   const long long want = (n + threads - 1) / threads;
   const int blocks = (int)std::max<long long>(1, std::min<long long>(want, (long long)e->sm_count * 8));
   if (dtype == B200_F32)
-    has_special_kernel<float, INF><<<blocks, threads, 0, e->stream>>>((const float *)x, n, flag);
+    launch_kernel(e, has_special_kernel<float, INF>, blocks, threads, 0, (const float *)x, n, flag);
   else
-    has_special_kernel<double, INF><<<blocks, threads, 0, e->stream>>>((const double *)x, n, flag);
+    launch_kernel(e, has_special_kernel<double, INF>, blocks, threads, 0, (const double *)x, n, flag);
   B200_CHECK_LAUNCH(e, "has_special_kernel");
   B200_CHECK_CUDA(e, cudaMemcpyAsync(e->h_flags, flag, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
   rc = sync_stream_checked(e);

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256) maxpool_kernel(const T *__restrict__ x, T
                                                       long long *__restrict__ mask, long long planes, int H, int W,
                                                       int Ho, int Wo, int kh, int kw, int sH, int sW, int oh0,
                                                       int ow0) {
+  ptx::grid_begin();
   const long long total = planes * Ho * Wo;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
                                                             const F16Rec *__restrict__ x_rec, PairsOut out16,
                                                             long long B, int C, int H, int W, int Ho, int Wo, int kh,
                                                             int kw, int sH, int sW, int oh0, int ow0) {
+  ptx::grid_begin();
   if (!F16 && skip_launch(only_if)) return;
   PairStats stats;
   float scale = 1.f;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
 __global__ void __launch_bounds__(256) maxpool2x2_kernel(const float *__restrict__ x, float *__restrict__ y,
                                                          long long planes, int H, int W, int Ho, int Wo,
                                                               const int *__restrict__ only_if) {
+  ptx::grid_begin();
   if (skip_launch(only_if)) return;
   const int pairs = Wo >> 1;  // Wo = W/2 is even because W % 4 == 0
   const long long total = planes * Ho * pairs;
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(256) maxpool2x2_kernel(const float *__restrict
 __global__ void __launch_bounds__(256) maxpool2x2_even_kernel(const float *__restrict__ x, float *__restrict__ y,
                                                               long long planes, int H, int W, int Ho, int Wo,
                                                               const int *__restrict__ only_if) {
+  ptx::grid_begin();
   if (skip_launch(only_if)) return;
   const long long total = planes * Ho * Wo;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -241,6 +245,7 @@ __global__ void __launch_bounds__(256) maxpool2x2_any_kernel(const float *__rest
                                                              uint32_t planes, int H, int W, int Ho, int Wo, int sH,
                                                              int sW, int oh0, int ow0,
                                                              const int *__restrict__ only_if) {
+  ptx::grid_begin();
   if (skip_launch(only_if)) return;
   const uint32_t per = (uint32_t)Ho * Wo, total = planes * per, hw = (uint32_t)H * W;
   const uint32_t stride = gridDim.x * blockDim.x;
@@ -277,6 +282,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T *__restrict__ col, long long out_rows,
                                                      int C, int H, int W, int Ho, int Wo, int kh, int kw, int padH,
                                                      int padW, int sH, int sW, int dH, int dW, int rows) {
+  ptx::grid_begin();
   const int crs = C * kh * kw, pieces = (crs + 31) / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (long long g0 = (long long)blockIdx.x * rows; g0 < out_rows; g0 += (long long)gridDim.x * rows) {
@@ -324,6 +330,7 @@ struct TransposeDesc {
 template <typename T>
 __global__ void __launch_bounds__(256) transpose_kernel(const T *__restrict__ x, T *__restrict__ y, long long n,
                                                         TransposeDesc d) {
+  ptx::grid_begin();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     long long rem = i, src = 0;
@@ -343,6 +350,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const T *__restrict__ x,
 template <typename T>
 __global__ void __launch_bounds__(256) transpose2d_kernel(const T *__restrict__ x, T *__restrict__ y, long long R,
                                                           long long Cc) {
+  ptx::grid_begin();
   __shared__ T tile[32][33];
   const long long b = blockIdx.z;
   const T *xb = x + b * R * Cc;
@@ -368,6 +376,7 @@ template <typename W>
 __global__ void __launch_bounds__(256) gather_rows_kernel(const W *__restrict__ x, const long long *__restrict__ idx,
                                                           W *__restrict__ y, long long outer, long long n_idx,
                                                           long long row_words, long long n_rows, int *bad) {
+  ptx::grid_begin();
   const long long total = outer * n_idx * row_words;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -393,6 +402,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const T *__restrict__ dy, const long long *__restrict__ mask,
                                                           T *__restrict__ dx, long long planes, int H, int W, int Ho,
                                                           int Wo, int kh, int kw, int sH, int sW, int oh0, int ow0) {
+  ptx::grid_begin();
   const long long total = planes * H * W;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -425,6 +435,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) col2im_kernel(const T *__restrict__ col, T *__restrict__ im, long long B, int C,
                                                      int H, int W, int Ho, int Wo, int kh, int kw, int padH, int padW,
                                                      int sH, int sW, int dH, int dW) {
+  ptx::grid_begin();
   const long long total = B * C * H * W;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int crs = C * kh * kw;
@@ -465,6 +476,7 @@ __global__ void __launch_bounds__(256) maxpool2x2_bwd_kernel(const float *__rest
                                                              const long long *__restrict__ mask,
                                                              float *__restrict__ dx, long long planes, int H, int W,
                                                              int Ho, int Wo) {
+  ptx::grid_begin();
   const uint32_t cols = (uint32_t)(Wo / NW), rows = (uint32_t)(H + 1) >> 1;  // one window-less row when H is odd
   const long long total = planes * rows * cols;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -518,6 +530,7 @@ template <typename T, bool UNIT_W>  // UNIT_W: stride 1 and no dilation along W 
 __global__ void __launch_bounds__(256) col2im_rows_kernel(const T *__restrict__ col, T *__restrict__ im, long long B,
                                                           int C, int H, int W, int Ho, int Wo, int kh, int kw,
                                                           int padH, int padW, int sW, int dW) {
+  ptx::grid_begin();
   extern __shared__ __align__(16) unsigned char c2i_smem[];
   T *ring = reinterpret_cast<T *>(c2i_smem);
   const int crs = C * kh * kw, khw = kh * kw;
@@ -581,6 +594,7 @@ template <bool UNIT_W>
 __global__ void __launch_bounds__(256) col2im_rows4_kernel(const float *__restrict__ col, float *__restrict__ im,
                                                            long long B, int C, int H, int W, int Ho, int Wo, int kh,
                                                            int kw, int padH, int padW, int sW, int dW) {
+  ptx::grid_begin();
   extern __shared__ __align__(16) unsigned char c2i4_smem[];
   float *ring = reinterpret_cast<float *>(c2i4_smem);
   const int crs = C * kh * kw, khw = kh * kw;
@@ -680,6 +694,7 @@ template <int KH, int KW>
 __global__ void __launch_bounds__(C2I_THREADS, 2) col2im_bulk_kernel(const float *__restrict__ col, float *__restrict__ im,
                                                           long long B, int C, int H, int W, int Ho, int Wo, int padH,
                                                           int padW, int R, int *err_flag) {
+  ptx::grid_begin();
   extern __shared__ __align__(128) unsigned char c2ib_smem[];
   __shared__ __align__(8) uint64_t full[C2I_MAX_RING];
   __shared__ int s_fail;
@@ -956,6 +971,7 @@ __global__ void __launch_bounds__(256) bn_sums_kernel(int c0, const T *__restric
                                                       T eps, T *__restrict__ running_mean, T *__restrict__ running_var,
                                                       T *__restrict__ save_mean, T *__restrict__ save_var,
                                                       T *__restrict__ alpha_beta) {
+  ptx::grid_begin();
   const int c = c0 + blockIdx.x;
   const long long per = (B + gridDim.y - 1) / gridDim.y, b0 = blockIdx.y * per, b1 = min(B, b0 + per);
   double s1 = 0.0, s2 = 0.0, t1, t2;
@@ -971,6 +987,7 @@ __global__ void __launch_bounds__(256) bn_sums_kernel(int c0, const T *__restric
 template <typename T>
 __global__ void bn_inference_kernel(int C, T eps, const T *__restrict__ running_mean, const T *__restrict__ running_var,
                                     T *__restrict__ alpha_beta) {
+  ptx::grid_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   const T inv = T(1) / sqrt(running_var[c] + eps);
@@ -988,6 +1005,7 @@ template <typename T, int GROUP>
 __global__ void __launch_bounds__(256) bn_apply_kernel(const T *__restrict__ x, T *__restrict__ y, long long planes,
                                                        int C, long long S, const T *__restrict__ alpha_beta,
                                                        bool vec4) {
+  ptx::grid_begin();
   const long long group0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / GROUP;
   const long long ngroups = ((long long)gridDim.x * blockDim.x) / GROUP;
   const int lane = threadIdx.x % GROUP;
@@ -1027,6 +1045,7 @@ __global__ void __launch_bounds__(256) bn_bwd_sums_kernel(int c0, const T *__res
                                                           const T *__restrict__ running_var,
                                                           const T *__restrict__ save_mean,
                                                           const T *__restrict__ save_var, T *__restrict__ coef) {
+  ptx::grid_begin();
   const int c = c0 + blockIdx.x;
   const long long per = (B + gridDim.y - 1) / gridDim.y, b0 = blockIdx.y * per, b1 = min(B, b0 + per);
   double s1 = 0.0, s2 = 0.0, t1, t2;
@@ -1054,6 +1073,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const T *__restrict__ x, const T *__restrict__ dy,
                                                            T *__restrict__ dx, long long planes, int C, long long S,
                                                            int training, const T *__restrict__ coef, bool vec4) {
+  ptx::grid_begin();
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -1114,7 +1134,7 @@ static int batchnorm_fwd_t(b200_engine *e, const T *x, T *y, long long B, int C,
   if (training) {
     for (int c0 = 0; c0 < C && le == cudaSuccess; c0 += b200_engine::kSkCounters) {
       const int nc = std::min(C - c0, (int)b200_engine::kSkCounters);
-      bn_sums_kernel<T><<<dim3(nc, bn_groups(e, B, nc)), 256, 0, e->stream>>>(
+      launch_kernel(e, bn_sums_kernel<T>, dim3(nc, bn_groups(e, B, nc)), 256, 0, 
           c0, x, B, C, S, (double *)part, e->sk_counters, (T)momentum, (T)eps, running_mean, running_var, save_mean,
           save_var, (T *)ab);
       le = cudaGetLastError();
@@ -1122,7 +1142,7 @@ static int batchnorm_fwd_t(b200_engine *e, const T *x, T *y, long long B, int C,
     }
     if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_sums_kernel: %s", cudaGetErrorString(le)));
   } else {
-    bn_inference_kernel<T><<<(C + 127) / 128, 128, 0, e->stream>>>(C, (T)eps, running_mean, running_var, (T *)ab);
+    launch_kernel(e, bn_inference_kernel<T>, (C + 127) / 128, 128, 0, C, (T)eps, running_mean, running_var, (T *)ab);
     le = cudaGetLastError();
     if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_inference_kernel: %s", cudaGetErrorString(le)));
     e->launches++;
@@ -1131,10 +1151,10 @@ static int batchnorm_fwd_t(b200_engine *e, const T *x, T *y, long long B, int C,
   const bool vec4 = S % 4 == 0 && ((uintptr_t)x | (uintptr_t)y) % 16 == 0;
   if (S >= 2048) {
     const int blocks = (int)std::max<long long>(1, std::min<long long>(planes, (long long)e->sm_count * 16));
-    bn_apply_kernel<T, 256><<<blocks, 256, 0, e->stream>>>(x, y, planes, C, S, (const T *)ab, vec4);
+    launch_kernel(e, bn_apply_kernel<T, 256>, blocks, 256, 0, x, y, planes, C, S, (const T *)ab, vec4);
   } else {
     const int blocks = (int)std::max<long long>(1, std::min<long long>((planes + 7) / 8, (long long)e->sm_count * 16));
-    bn_apply_kernel<T, 32><<<blocks, 256, 0, e->stream>>>(x, y, planes, C, S, (const T *)ab, vec4);
+    launch_kernel(e, bn_apply_kernel<T, 32>, blocks, 256, 0, x, y, planes, C, S, (const T *)ab, vec4);
   }
   le = cudaGetLastError();
   if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_apply_kernel: %s", cudaGetErrorString(le)));
@@ -1160,7 +1180,7 @@ static int batchnorm_bwd_t(b200_engine *e, const T *x, const T *dy, T *dx, long 
   cudaError_t le = cudaSuccess;
   for (int c0 = 0; c0 < C && le == cudaSuccess; c0 += b200_engine::kSkCounters) {
     const int nc = std::min(C - c0, (int)b200_engine::kSkCounters);
-    bn_bwd_sums_kernel<T><<<dim3(nc, bn_groups(e, B, nc)), 256, 0, e->stream>>>(
+    launch_kernel(e, bn_bwd_sums_kernel<T>, dim3(nc, bn_groups(e, B, nc)), 256, 0, 
         c0, x, dy, B, C, S, (double *)part, e->sk_counters, training, (T)eps, running_var, save_mean, save_var, (T *)coef);
     le = cudaGetLastError();
     e->launches++;
@@ -1169,7 +1189,7 @@ static int batchnorm_bwd_t(b200_engine *e, const T *x, const T *dy, T *dx, long 
   const long long planes = B * C;
   const int blocks = (int)std::max<long long>(1, std::min<long long>((planes + 7) / 8, (long long)e->sm_count * 16));
   const bool vec4 = S % 4 == 0 && ((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) % 16 == 0;
-  bn_bwd_apply_kernel<T><<<blocks, 256, 0, e->stream>>>(x, dy, dx, planes, C, S, training, (const T *)coef, vec4);
+  launch_kernel(e, bn_bwd_apply_kernel<T>, blocks, 256, 0, x, dy, dx, planes, C, S, training, (const T *)coef, vec4);
   le = cudaGetLastError();
   if (le != cudaSuccess) return done(set_error(e, B200_ERR_CUDA, "bn_bwd_apply_kernel: %s", cudaGetErrorString(le)));
   e->launches++;
@@ -1205,11 +1225,11 @@ int b200_maxpool2d_split_fwd(b200_engine *e, const void *x, void *y, void *y_hi,
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)e->sm_count * 32));
   const int oh0 = explicit_padding ? pad_south : pad_north, ow0 = explicit_padding ? pad_east : pad_west;
   if (kh == 2 && kw == 2)
-    maxpool_split_kernel<true, false><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)y, (float *)y_hi,
+    launch_kernel(e, maxpool_split_kernel<true, false>, blocks, 256, 0, (const float *)x, (float *)y, (float *)y_hi,
                                                               (float *)y_lo, e->only_if, nullptr, PairsOut(), B, (int)C, (int)H, (int)W, (int)Ho,
                                                               (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   else
-    maxpool_split_kernel<false, false><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)y, (float *)y_hi,
+    launch_kernel(e, maxpool_split_kernel<false, false>, blocks, 256, 0, (const float *)x, (float *)y, (float *)y_hi,
                                                                (float *)y_lo, e->only_if, nullptr, PairsOut(), B, (int)C, (int)H, (int)W, (int)Ho,
                                                                (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   B200_CHECK_LAUNCH(e, "maxpool_split_kernel");
@@ -1242,11 +1262,11 @@ int b200_maxpool2d_pairs_fwd(b200_engine *e, const void *x, const void *x_rec, v
   out.l = out.h + B * C * Ho * Wo;
   out.rec = (F16Rec *)y_rec;
   if (kh == 2 && kw == 2)
-    maxpool_split_kernel<true, true><<<blocks, 256, 0, e->stream>>>(
+    launch_kernel(e, maxpool_split_kernel<true, true>, blocks, 256, 0, 
         (const float *)x, nullptr, nullptr, nullptr, nullptr, (const F16Rec *)x_rec, out, B, (int)C, (int)H, (int)W,
         (int)Ho, (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   else
-    maxpool_split_kernel<false, true><<<blocks, 256, 0, e->stream>>>(
+    launch_kernel(e, maxpool_split_kernel<false, true>, blocks, 256, 0, 
         (const float *)x, nullptr, nullptr, nullptr, nullptr, (const F16Rec *)x_rec, out, B, (int)C, (int)H, (int)W,
         (int)Ho, (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   B200_CHECK_LAUNCH(e, "maxpool_split_kernel");
@@ -1278,20 +1298,20 @@ int b200_maxpool2d_fwd(b200_engine *e, int dtype, const void *x, void *y, int64_
   if (dtype == B200_F32 && !mask && kh == 2 && kw == 2 && stride_h == 2 && stride_w == 2 && pad_north == 0 &&
       pad_south == 0 && pad_west == 0 && pad_east == 0 && W % 4 == 0 && (uintptr_t)x % 16 == 0 &&
       (uintptr_t)y % 8 == 0) {
-    maxpool2x2_kernel<<<grid_for(e, total / 2), 256, 0, e->stream>>>((const float *)x, (float *)y, B * C, (int)H,
+    launch_kernel(e, maxpool2x2_kernel, grid_for(e, total / 2), 256, 0, (const float *)x, (float *)y, B * C, (int)H,
                                                                     (int)W, (int)Ho, (int)Wo, e->only_if);
     B200_CHECK_LAUNCH(e, "maxpool2x2_kernel");
     return B200_OK;
   }
   if (dtype == B200_F32 && !mask && kh == 2 && kw == 2 && stride_h == 2 && stride_w == 2 && pad_north == 0 &&
       pad_south == 0 && pad_west == 0 && pad_east == 0 && W % 2 == 0 && (uintptr_t)x % 8 == 0) {
-    maxpool2x2_even_kernel<<<grid_for(e, total), 256, 0, e->stream>>>((const float *)x, (float *)y, B * C, (int)H,
+    launch_kernel(e, maxpool2x2_even_kernel, grid_for(e, total), 256, 0, (const float *)x, (float *)y, B * C, (int)H,
                                                                      (int)W, (int)Ho, (int)Wo, e->only_if);
     B200_CHECK_LAUNCH(e, "maxpool2x2_even_kernel");
     return B200_OK;
   }
   if (dtype == B200_F32 && !mask && kh == 2 && kw == 2 && total < (1LL << 31) && B * C * H * W < (1LL << 32)) {
-    maxpool2x2_any_kernel<<<grid_for(e, total), 256, 0, e->stream>>>((const float *)x, (float *)y, (uint32_t)(B * C),
+    launch_kernel(e, maxpool2x2_any_kernel, grid_for(e, total), 256, 0, (const float *)x, (float *)y, (uint32_t)(B * C),
                                                                     (int)H, (int)W, (int)Ho, (int)Wo, stride_h,
                                                                     stride_w, oh0, ow0, e->only_if);
     B200_CHECK_LAUNCH(e, "maxpool2x2_any_kernel");
@@ -1299,11 +1319,11 @@ int b200_maxpool2d_fwd(b200_engine *e, int dtype, const void *x, void *y, int64_
   }
   if (e->only_if) return set_error(e, B200_ERR_STATE, "this pooling cannot be made while b200_only_if is in effect");
   if (dtype == B200_F32)
-    maxpool_kernel<float><<<grid_for(e, total), 256, 0, e->stream>>>((const float *)x, (float *)y, (long long *)mask,
+    launch_kernel(e, maxpool_kernel<float>, grid_for(e, total), 256, 0, (const float *)x, (float *)y, (long long *)mask,
                                                                     B * C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw,
                                                                     stride_h, stride_w, oh0, ow0);
   else
-    maxpool_kernel<double><<<grid_for(e, total), 256, 0, e->stream>>>((const double *)x, (double *)y,
+    launch_kernel(e, maxpool_kernel<double>, grid_for(e, total), 256, 0, (const double *)x, (double *)y,
                                                                      (long long *)mask, B * C, (int)H, (int)W,
                                                                      (int)Ho, (int)Wo, kh, kw, stride_h, stride_w,
                                                                      oh0, ow0);
@@ -1377,20 +1397,20 @@ int b200_maxpool2d_bwd(b200_engine *e, int dtype, const void *dy, const int64_t 
       pad_west == 0 && pad_east == 0 && W % 2 == 0 && (uintptr_t)dx % 8 == 0) {
     const long long lines = B * C * ((H + 1) / 2);
     if (W % 4 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)dy % 8 == 0 && (uintptr_t)mask % 16 == 0)
-      maxpool2x2_bwd_kernel<2><<<grid_for(e, lines * (Wo / 2)), 256, 0, e->stream>>>(
+      launch_kernel(e, maxpool2x2_bwd_kernel<2>, grid_for(e, lines * (Wo / 2)), 256, 0, 
           (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo);
     else
-      maxpool2x2_bwd_kernel<1><<<grid_for(e, lines * Wo), 256, 0, e->stream>>>(
+      launch_kernel(e, maxpool2x2_bwd_kernel<1>, grid_for(e, lines * Wo), 256, 0, 
           (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo);
     B200_CHECK_LAUNCH(e, "maxpool2x2_bwd_kernel");
     return B200_OK;
   }
   if (dtype == B200_F32)
-    maxpool_bwd_kernel<float><<<grid_for(e, total), 256, 0, e->stream>>>(
+    launch_kernel(e, maxpool_bwd_kernel<float>, grid_for(e, total), 256, 0, 
         (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw,
         stride_h, stride_w, oh0, ow0);
   else
-    maxpool_bwd_kernel<double><<<grid_for(e, total), 256, 0, e->stream>>>(
+    launch_kernel(e, maxpool_bwd_kernel<double>, grid_for(e, total), 256, 0, 
         (const double *)dy, (const long long *)mask, (double *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw,
         stride_h, stride_w, oh0, ow0);
   B200_CHECK_LAUNCH(e, "maxpool_bwd_kernel");
@@ -1453,7 +1473,7 @@ int b200_col2im(b200_engine *e, int dtype, const void *col, void *im, int64_t B,
         }
         const long long per_sm = std::max<long long>(1, (long long)(whole / (smem + 1024)));
         const int bblocks = (int)std::max<long long>(1, std::min<long long>(B, (long long)e->sm_count * per_sm));
-        col2im_bulk_kernel<3, 3><<<bblocks, C2I_THREADS, smem, e->stream>>>((const float *)col, (float *)im, B, (int)C, (int)H,
+        launch_kernel(e, col2im_bulk_kernel<3, 3>, bblocks, C2I_THREADS, smem, (const float *)col, (float *)im, B, (int)C, (int)H,
                                                                     (int)W, (int)Ho, (int)Wo, pad_h, pad_w, R,
                                                                     e->d_flags + 2);
         B200_CHECK_LAUNCH(e, "col2im_bulk_kernel");
@@ -1473,18 +1493,18 @@ int b200_col2im(b200_engine *e, int dtype, const void *col, void *im, int64_t B,
         attr4_dev_mask |= 1 << (e->device & 31);
       }
       if (unit_w)
-        col2im_rows4_kernel<true><<<blocks, 256, staged4, e->stream>>>((const float *)col, (float *)im, B, (int)C, (int)H,
+        launch_kernel(e, col2im_rows4_kernel<true>, blocks, 256, staged4, (const float *)col, (float *)im, B, (int)C, (int)H,
                                                                      (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w,
                                                                      stride_w, dil_w);
       else
-        col2im_rows4_kernel<false><<<blocks, 256, staged4, e->stream>>>((const float *)col, (float *)im, B, (int)C,
+        launch_kernel(e, col2im_rows4_kernel<false>, blocks, 256, staged4, (const float *)col, (float *)im, B, (int)C,
                                                                       (int)H, (int)W, (int)Ho, (int)Wo, kh, kw, pad_h,
                                                                       pad_w, stride_w, dil_w);
       B200_CHECK_LAUNCH(e, "col2im_rows4_kernel");
       return B200_OK;
     }
 #define B200_C2I(T, U)                                                                                          \
-  col2im_rows_kernel<T, U><<<blocks, 256, staged, e->stream>>>((const T *)col, (T *)im, B, (int)C, (int)H, (int)W, \
+  launch_kernel(e, col2im_rows_kernel<T, U>, blocks, 256, staged, (const T *)col, (T *)im, B, (int)C, (int)H, (int)W, \
                                                                (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_w, dil_w)
     if (dtype == B200_F32) {
       if (unit_w) B200_C2I(float, true); else B200_C2I(float, false);
@@ -1496,11 +1516,11 @@ int b200_col2im(b200_engine *e, int dtype, const void *col, void *im, int64_t B,
     return B200_OK;
   }
   if (dtype == B200_F32)
-    col2im_kernel<float><<<grid_for(e, total), 256, 0, e->stream>>>((const float *)col, (float *)im, B, (int)C, (int)H,
+    launch_kernel(e, col2im_kernel<float>, grid_for(e, total), 256, 0, (const float *)col, (float *)im, B, (int)C, (int)H,
                                                                    (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w,
                                                                    stride_h, stride_w, dil_h, dil_w);
   else
-    col2im_kernel<double><<<grid_for(e, total), 256, 0, e->stream>>>((const double *)col, (double *)im, B, (int)C,
+    launch_kernel(e, col2im_kernel<double>, grid_for(e, total), 256, 0, (const double *)col, (double *)im, B, (int)C,
                                                                     (int)H, (int)W, (int)Ho, (int)Wo, kh, kw, pad_h,
                                                                     pad_w, stride_h, stride_w, dil_h, dil_w);
   B200_CHECK_LAUNCH(e, "col2im_kernel");
@@ -1530,11 +1550,11 @@ int b200_im2col(b200_engine *e, int dtype, const void *x, void *col, int64_t B, 
   const int rows = std::max(1, 32 / ((crs + 31) / 32));
   const int blocks = (int)std::min<long long>((B * Ho + rows - 1) / rows, 1LL << 30);
   if (dtype == B200_F32)
-    im2col_kernel<float><<<blocks, 256, 0, e->stream>>>((const float *)x, (float *)col, B * Ho, (int)C, (int)H, (int)W,
+    launch_kernel(e, im2col_kernel<float>, blocks, 256, 0, (const float *)x, (float *)col, B * Ho, (int)C, (int)H, (int)W,
                                                        (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h, stride_w,
                                                        dil_h, dil_w, rows);
   else
-    im2col_kernel<double><<<blocks, 256, 0, e->stream>>>((const double *)x, (double *)col, B * Ho, (int)C, (int)H,
+    launch_kernel(e, im2col_kernel<double>, blocks, 256, 0, (const double *)x, (double *)col, B * Ho, (int)C, (int)H,
                                                         (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h,
                                                         stride_w, dil_h, dil_w, rows);
   B200_CHECK_LAUNCH(e, "im2col_kernel");
@@ -1599,11 +1619,11 @@ int b200_transpose(b200_engine *e, int elem_bytes, const void *x, void *y, int n
   if (is2d && Bt <= 65535 && (R + 31) / 32 <= 65535) {
     dim3 grid((unsigned)((Cc + 31) / 32), (unsigned)((R + 31) / 32), (unsigned)Bt);
     if (elem_bytes == 4)
-      transpose2d_kernel<uint32_t><<<grid, 256, 0, e->stream>>>((const uint32_t *)x, (uint32_t *)y, R, Cc);
+      launch_kernel(e, transpose2d_kernel<uint32_t>, grid, 256, 0, (const uint32_t *)x, (uint32_t *)y, R, Cc);
     else if (elem_bytes == 8)
-      transpose2d_kernel<uint64_t><<<grid, 256, 0, e->stream>>>((const uint64_t *)x, (uint64_t *)y, R, Cc);
+      launch_kernel(e, transpose2d_kernel<uint64_t>, grid, 256, 0, (const uint64_t *)x, (uint64_t *)y, R, Cc);
     else
-      transpose2d_kernel<uint16_t><<<grid, 256, 0, e->stream>>>((const uint16_t *)x, (uint16_t *)y, R, Cc);
+      launch_kernel(e, transpose2d_kernel<uint16_t>, grid, 256, 0, (const uint16_t *)x, (uint16_t *)y, R, Cc);
     B200_CHECK_LAUNCH(e, "transpose2d_kernel");
     return B200_OK;
   }
@@ -1614,11 +1634,11 @@ int b200_transpose(b200_engine *e, int elem_bytes, const void *x, void *y, int n
     d.in_stride_of_out_dim[k] = ostride[k];
   }
   if (elem_bytes == 4)
-    transpose_kernel<uint32_t><<<grid_for(e, n), 256, 0, e->stream>>>((const uint32_t *)x, (uint32_t *)y, n, d);
+    launch_kernel(e, transpose_kernel<uint32_t>, grid_for(e, n), 256, 0, (const uint32_t *)x, (uint32_t *)y, n, d);
   else if (elem_bytes == 8)
-    transpose_kernel<uint64_t><<<grid_for(e, n), 256, 0, e->stream>>>((const uint64_t *)x, (uint64_t *)y, n, d);
+    launch_kernel(e, transpose_kernel<uint64_t>, grid_for(e, n), 256, 0, (const uint64_t *)x, (uint64_t *)y, n, d);
   else
-    transpose_kernel<uint16_t><<<grid_for(e, n), 256, 0, e->stream>>>((const uint16_t *)x, (uint16_t *)y, n, d);
+    launch_kernel(e, transpose_kernel<uint16_t>, grid_for(e, n), 256, 0, (const uint16_t *)x, (uint16_t *)y, n, d);
   B200_CHECK_LAUNCH(e, "transpose_kernel");
   return B200_OK;
 }
@@ -1639,14 +1659,14 @@ int b200_gather_axis(b200_engine *e, const void *x, const int64_t *idx, void *y,
   const bool w4 = row_bytes % 4 == 0 && (uintptr_t)x % 4 == 0 && (uintptr_t)y % 4 == 0;
   if (w16) {
     const long long words = row_bytes / 16;
-    gather_rows_kernel<uint4><<<grid_for(e, outer * n_idx * words), 256, 0, e->stream>>>(
+    launch_kernel(e, gather_rows_kernel<uint4>, grid_for(e, outer * n_idx * words), 256, 0, 
         (const uint4 *)x, (const long long *)idx, (uint4 *)y, outer, n_idx, words, n_rows, bad);
   } else if (w4) {
     const long long words = row_bytes / 4;
-    gather_rows_kernel<uint32_t><<<grid_for(e, outer * n_idx * words), 256, 0, e->stream>>>(
+    launch_kernel(e, gather_rows_kernel<uint32_t>, grid_for(e, outer * n_idx * words), 256, 0, 
         (const uint32_t *)x, (const long long *)idx, (uint32_t *)y, outer, n_idx, words, n_rows, bad);
   } else {
-    gather_rows_kernel<unsigned char><<<grid_for(e, outer * n_idx * row_bytes), 256, 0, e->stream>>>(
+    launch_kernel(e, gather_rows_kernel<unsigned char>, grid_for(e, outer * n_idx * row_bytes), 256, 0, 
         (const unsigned char *)x, (const long long *)idx, (unsigned char *)y, outer, n_idx, row_bytes, n_rows, bad);
   }
   B200_CHECK_LAUNCH(e, "gather_rows_kernel");

@@ -349,6 +349,7 @@ __device__ __forceinline__ void store_chunk(T *p, long long i, const T *s, int v
 // NS / NI = compile-time capacity for sources and instructions.
 template <typename T, int V, int NS, int NI>
 __global__ void __launch_bounds__(256) pw_kernel(const __grid_constant__ PwDev p) {
+  ptx::grid_begin();
   const long long n = p.n;
   const long long nchunks = (n + V - 1) / V;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -592,6 +593,7 @@ __device__ __forceinline__ void pw_fill(const PwDev &p, uint32_t ring_s, long lo
 constexpr int PW_LOOP_THREADS = 128;
 template <typename T, int V, bool ALIGNED>
 __global__ void __launch_bounds__(PW_LOOP_THREADS) pw_loop_kernel(const __grid_constant__ PwDev p) {
+  ptx::grid_begin();
   extern __shared__ __align__(128) unsigned char pw_loop_smem[];
   const int tid = threadIdx.x;
   const uint32_t ring_s = ptx::smem_addr(pw_loop_smem) + (uint32_t)tid * 16;
@@ -651,6 +653,7 @@ __device__ __forceinline__ void pw_tile_single(int op, bool a_imm, bool b_imm, b
 template <typename T, int V, int U, bool SINGLE, int CTAS>
 __global__ void __launch_bounds__(PW_STREAM_THREADS, CTAS)
     pw_stream_kernel(const __grid_constant__ PwDev p, int stages, int *err_flag) {
+  ptx::grid_begin();
   constexpr int TILE_CHUNKS = PW_STREAM_THREADS * U;
   constexpr int SLOT_BYTES = TILE_CHUNKS * 16;
   extern __shared__ __align__(128) unsigned char pw_smem[];
@@ -788,7 +791,7 @@ static int launch_stream_wide(b200_engine *e, const PwDev &d, size_t budget, int
     B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     attr_dev_mask |= 1 << (e->device & 31);
   }
-  kern<<<blocks, PW_STREAM_THREADS, smem, e->stream>>>(d, stages, e->d_flags + 2);
+  launch_kernel(e, kern, blocks, PW_STREAM_THREADS, smem, d, stages, e->d_flags + 2);
   B200_CHECK_LAUNCH(e, "pw_stream_kernel");
   e->flags_dirty = true;
   return B200_OK;
@@ -810,14 +813,14 @@ static int launch_stream_u(b200_engine *e, const PwDev &d, size_t budget, int st
       B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
       attr_dev_mask[1] |= 1 << (e->device & 31);
     }
-    kern<<<blocks, PW_STREAM_THREADS, smem, e->stream>>>(d, stages, e->d_flags + 2);
+    launch_kernel(e, kern, blocks, PW_STREAM_THREADS, smem, d, stages, e->d_flags + 2);
   } else {
     auto kern = pw_stream_kernel<T, V, U, false, CTAS>;
     if (!(attr_dev_mask[0] & (1 << (e->device & 31)))) {
       B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
       attr_dev_mask[0] |= 1 << (e->device & 31);
     }
-    kern<<<blocks, PW_STREAM_THREADS, smem, e->stream>>>(d, stages, e->d_flags + 2);
+    launch_kernel(e, kern, blocks, PW_STREAM_THREADS, smem, d, stages, e->d_flags + 2);
   }
   B200_CHECK_LAUNCH(e, "pw_stream_kernel");
   e->flags_dirty = true;
@@ -860,7 +863,7 @@ static int launch_loop(b200_engine *e, const PwDev &d) {
   const size_t smem = (size_t)(d.n_full + d.n_file) * PW_LOOP_THREADS * 16;  // at most 6 + 7 slots of 2 KB
   const long long tiles = ((d.n + VV - 1) / VV + PW_LOOP_THREADS - 1) / PW_LOOP_THREADS;
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)e->sm_count * 16));
-  pw_loop_kernel<T, VV, (V > 1)><<<blocks, PW_LOOP_THREADS, smem, e->stream>>>(d);
+  launch_kernel(e, pw_loop_kernel<T, VV, (V > 1)>, blocks, PW_LOOP_THREADS, smem, d);
   B200_CHECK_LAUNCH(e, "pw_loop_kernel");
   return B200_OK;
 }
@@ -881,9 +884,9 @@ static int launch_sized(b200_engine *e, const PwDev &d, int ns, int ni) {
   long long cap = (long long)e->sm_count * 8;
   int blocks = (int)std::max<long long>(1, std::min(want, cap));
   if (ns <= 2 && ni <= 2)
-    pw_kernel<T, V, 2, 2><<<blocks, threads, 0, e->stream>>>(d);
+    launch_kernel(e, pw_kernel<T, V, 2, 2>, blocks, threads, 0, d);
   else if (ns <= 3 && ni <= 4)
-    pw_kernel<T, V, 3, 4><<<blocks, threads, 0, e->stream>>>(d);
+    launch_kernel(e, pw_kernel<T, V, 3, 4>, blocks, threads, 0, d);
   else
     return launch_loop<T, V>(e, d);
   B200_CHECK_LAUNCH(e, "pw_kernel");

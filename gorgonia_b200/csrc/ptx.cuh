@@ -26,6 +26,11 @@ __device__ __forceinline__ float ld_cg_ordered(const float *p) {
   return v;
 }
 
+// The first statement of every kernel (launch_kernel, engine.h): waits for the kernel in front of this one.
+__device__ __forceinline__ void grid_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---- mbarrier ------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include "engine.h"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -48,6 +49,7 @@ __device__ __forceinline__ T group_sum(T v, int width) {
 template <typename T, int PER, int MODE>
 __global__ void __launch_bounds__(256) row_kernel(const T *__restrict__ x, T *__restrict__ y, long long rows,
                                                   int len, int G) {
+  ptx::grid_begin();
   const int lane_in_group = threadIdx.x % G;
   const int group_in_warp = (threadIdx.x & 31) / G;
   const int groups_per_warp = 32 / G;
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(256) row_kernel(const T *__restrict__ x, T *__
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) col_kernel(const T *__restrict__ x, T *__restrict__ y, long long outer,
                                                   long long len, long long inner) {
+  ptx::grid_begin();
   const long long total = outer * inner;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += stride) {
@@ -167,6 +170,7 @@ template <typename T, int MODE, int CX>
 __global__ void __launch_bounds__(256) col_split_kernel(const T *__restrict__ x, T *__restrict__ y, long long len,
                                                         long long inner, int col_groups, long long rows_per_chunk,
                                                         T *__restrict__ ws, int *__restrict__ count) {
+  ptx::grid_begin();
   constexpr int ROWS = 256 / CX;
   __shared__ T part[256];
   __shared__ int s_last;
@@ -224,6 +228,7 @@ __global__ void __launch_bounds__(256) col_split_kernel(const T *__restrict__ x,
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) long_row_kernel(const T *__restrict__ x, T *__restrict__ y, long long rows,
                                                        long long len) {
+  ptx::grid_begin();
   __shared__ T red[256 / 32];
   __shared__ T bcast;
   auto block_reduce = [&](T v, bool is_max) -> T {
@@ -269,6 +274,7 @@ __global__ void __launch_bounds__(256) long_row_kernel(const T *__restrict__ x, 
 template <typename T>
 __global__ void __launch_bounds__(256) argmax_kernel(const T *__restrict__ x, long long *__restrict__ y,
                                                      long long outer, long long len, long long inner) {
+  ptx::grid_begin();
   const long long total = outer * inner;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < total; c += stride) {
@@ -298,6 +304,7 @@ constexpr size_t REDUCE_ALL_SCRATCH_BYTES = REDUCE_ALL_TICKET_OFFSET + 256;
 template <typename T, bool IS_MAX>
 __global__ void __launch_bounds__(256) reduce_all_kernel(const T *__restrict__ x, long long n,
                                                          unsigned char *__restrict__ scratch, T *__restrict__ y) {
+  ptx::grid_begin();
   T *partials = reinterpret_cast<T *>(scratch);
   unsigned int *ticket = reinterpret_cast<unsigned int *>(scratch + REDUCE_ALL_TICKET_OFFSET);
   __shared__ T red[256 / 32];
@@ -356,9 +363,9 @@ static int launch_reduce_all(b200_engine *e, int kind, const T *x, long long n, 
   want = std::min<long long>(want, REDUCE_ALL_MAX_BLOCKS);
   const int blocks = (int)std::max<long long>(1, want);
   if (kind == 0)
-    reduce_all_kernel<T, false><<<blocks, 256, 0, e->stream>>>(x, n, scratch, y);
+    launch_kernel(e, reduce_all_kernel<T, false>, blocks, 256, 0, x, n, scratch, y);
   else
-    reduce_all_kernel<T, true><<<blocks, 256, 0, e->stream>>>(x, n, scratch, y);
+    launch_kernel(e, reduce_all_kernel<T, true>, blocks, 256, 0, x, n, scratch, y);
   B200_CHECK_LAUNCH(e, "reduce_all_kernel");
   return B200_OK;
 }
@@ -400,7 +407,7 @@ static int launch_col_split(b200_engine *e, const T *x, T *y, long long outer, l
     chunks = 1;  // no room for the parts: whole columns
   const long long per = (len + chunks - 1) / chunks;
   chunks = (len + per - 1) / per;
-  col_split_kernel<T, MODE, CX><<<dim3((unsigned)blocks, (unsigned)chunks), 256, 0, e->stream>>>(
+  launch_kernel(e, col_split_kernel<T, MODE, CX>, dim3((unsigned)blocks, (unsigned)chunks), 256, 0, 
       x, y, len, inner, (int)groups, per, (T *)ws, e->sk_counters);
   if (ws) b200_put(e, ws, 0);  // stream order: whoever gets the block next runs after this kernel
   B200_CHECK_LAUNCH(e, "col_split_kernel");
@@ -418,7 +425,7 @@ static int launch_mode(b200_engine *e, const T *x, T *y, long long outer, long l
     const long long groups_per_block = threads / G;
     const int blocks = (int)std::max<long long>(1, std::min((outer + groups_per_block - 1) / groups_per_block, cap));
 #define B200_ROW(P)                                                                           \
-  row_kernel<T, P, MODE><<<blocks, threads, 0, e->stream>>>(x, y, outer, (int)len, G)
+  launch_kernel(e, row_kernel<T, P, MODE>, blocks, threads, 0, x, y, outer, (int)len, G)
     if (per <= 1) B200_ROW(1);
     else if (per <= 2) B200_ROW(2);
     else if (per <= 4) B200_ROW(4);
@@ -430,7 +437,7 @@ static int launch_mode(b200_engine *e, const T *x, T *y, long long outer, long l
     B200_CHECK_LAUNCH(e, "row_kernel");
   } else if (inner == 1) {
     const int blocks = (int)std::max<long long>(1, std::min(outer, cap));
-    long_row_kernel<T, MODE><<<blocks, threads, 0, e->stream>>>(x, y, outer, len);
+    launch_kernel(e, long_row_kernel<T, MODE>, blocks, threads, 0, x, y, outer, len);
     B200_CHECK_LAUNCH(e, "long_row_kernel");
   } else if ((MODE == 2 || MODE == 3) && len >= 32 && outer * inner < e->sm_count * 2048LL) {
     // Fewer columns than threads the GPU holds (2048 per SM): split the axis. With more columns the walk
@@ -443,7 +450,7 @@ static int launch_mode(b200_engine *e, const T *x, T *y, long long outer, long l
   } else {
     const long long total = outer * inner;
     const int blocks = (int)std::max<long long>(1, std::min((total + threads - 1) / threads, cap));
-    col_kernel<T, MODE><<<blocks, threads, 0, e->stream>>>(x, y, outer, len, inner);
+    launch_kernel(e, col_kernel<T, MODE>, blocks, threads, 0, x, y, outer, len, inner);
     B200_CHECK_LAUNCH(e, "col_kernel");
   }
   return B200_OK;
@@ -459,6 +466,7 @@ static int launch_mode(b200_engine *e, const T *x, T *y, long long outer, long l
 template <typename T, bool LOG>
 __global__ void __launch_bounds__(256) softmax_bwd_rows_kernel(const T *__restrict__ y, const T *__restrict__ g,
                                                                T *__restrict__ dx, long long rows, long long len) {
+  ptx::grid_begin();
   const int lane = threadIdx.x & 31;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -478,6 +486,7 @@ template <typename T, bool LOG>
 __global__ void __launch_bounds__(256) softmax_bwd_strided_kernel(const T *__restrict__ y, const T *__restrict__ g,
                                                                   T *__restrict__ dx, long long outer, long long len,
                                                                   long long inner) {
+  ptx::grid_begin();
   const long long total = outer * inner;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
@@ -500,6 +509,7 @@ __global__ void __launch_bounds__(256) softmax_bwd_strided_kernel(const T *__res
 template <typename T, bool LOG>
 __global__ void __launch_bounds__(128) softmax_bwd_short_kernel(const T *__restrict__ y, const T *__restrict__ g,
                                                                 T *__restrict__ dx, long long rows, int len) {
+  ptx::grid_begin();
   __shared__ __align__(16) T sy[4][32 * 16], sg[4][32 * 16];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -573,14 +583,14 @@ static int launch_softmax_bwd(b200_engine *e, const T *y, const T *g, T *dx, lon
     const long long groups = (outer + 31) / 32;
     // more blocks than are resident at once: groups of rows are then handed out as blocks retire
     const long long blocks = std::max<long long>(1, std::min<long long>((groups + 3) / 4, (long long)e->sm_count * 64));
-    softmax_bwd_short_kernel<T, LOG><<<(int)blocks, 128, 0, e->stream>>>(y, g, dx, outer, (int)len);
+    launch_kernel(e, softmax_bwd_short_kernel<T, LOG>, (int)blocks, 128, 0, y, g, dx, outer, (int)len);
   } else if (inner == 1) {
     const long long blocks = std::max<long long>(1, std::min<long long>((outer + 7) / 8, (long long)e->sm_count * 16));
-    softmax_bwd_rows_kernel<T, LOG><<<(int)blocks, 256, 0, e->stream>>>(y, g, dx, outer, len);
+    launch_kernel(e, softmax_bwd_rows_kernel<T, LOG>, (int)blocks, 256, 0, y, g, dx, outer, len);
   } else {
     const long long total = outer * inner;
     const long long blocks = std::max<long long>(1, std::min<long long>((total + 255) / 256, (long long)e->sm_count * 16));
-    softmax_bwd_strided_kernel<T, LOG><<<(int)blocks, 256, 0, e->stream>>>(y, g, dx, outer, len, inner);
+    launch_kernel(e, softmax_bwd_strided_kernel<T, LOG>, (int)blocks, 256, 0, y, g, dx, outer, len, inner);
   }
   B200_CHECK_LAUNCH(e, "softmax_bwd_kernel");
   return B200_OK;
@@ -701,14 +711,14 @@ int b200_reduce_all_static(b200_engine *e, int dtype, int kind, const void *x, i
   const int blocks = (int)std::max<long long>(1, want);
   if (dtype == B200_F32) {
     if (kind == 0)
-      reduce_all_kernel<float, false><<<blocks, 256, 0, e->stream>>>((const float *)x, n, scratch, (float *)y);
+      launch_kernel(e, reduce_all_kernel<float, false>, blocks, 256, 0, (const float *)x, n, scratch, (float *)y);
     else
-      reduce_all_kernel<float, true><<<blocks, 256, 0, e->stream>>>((const float *)x, n, scratch, (float *)y);
+      launch_kernel(e, reduce_all_kernel<float, true>, blocks, 256, 0, (const float *)x, n, scratch, (float *)y);
   } else {
     if (kind == 0)
-      reduce_all_kernel<double, false><<<blocks, 256, 0, e->stream>>>((const double *)x, n, scratch, (double *)y);
+      launch_kernel(e, reduce_all_kernel<double, false>, blocks, 256, 0, (const double *)x, n, scratch, (double *)y);
     else
-      reduce_all_kernel<double, true><<<blocks, 256, 0, e->stream>>>((const double *)x, n, scratch, (double *)y);
+      launch_kernel(e, reduce_all_kernel<double, true>, blocks, 256, 0, (const double *)x, n, scratch, (double *)y);
   }
   B200_CHECK_LAUNCH(e, "reduce_all_kernel");
   return B200_OK;
@@ -728,9 +738,9 @@ int b200_argmax(b200_engine *e, int dtype, const void *x, int64_t *y, int64_t ou
   const long long total = outer * inner;
   const int blocks = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, (long long)e->sm_count * 8));
   if (dtype == B200_F32)
-    argmax_kernel<float><<<blocks, 256, 0, e->stream>>>((const float *)x, (long long *)y, outer, len, inner);
+    launch_kernel(e, argmax_kernel<float>, blocks, 256, 0, (const float *)x, (long long *)y, outer, len, inner);
   else
-    argmax_kernel<double><<<blocks, 256, 0, e->stream>>>((const double *)x, (long long *)y, outer, len, inner);
+    launch_kernel(e, argmax_kernel<double>, blocks, 256, 0, (const double *)x, (long long *)y, outer, len, inner);
   B200_CHECK_LAUNCH(e, "argmax_kernel");
   return B200_OK;
 }

@@ -21,6 +21,7 @@
 #include <algorithm>
 
 #include "engine.h"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -41,6 +42,7 @@ __device__ __forceinline__ float split_tf32(float x) {
 template <int MODE>
 __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ SplitJob ja, const __grid_constant__ SplitJob jb,
                                                     int blocks_a, SplitRedo redo) {
+  ptx::grid_begin();
   constexpr int V = MODE == SPLIT_TF32 || MODE == SPLIT_TF32_REDO ? 4 : 8;
   __shared__ unsigned s_red[8], s_bad[8];
   if (MODE == SPLIT_TF32_REDO) {
@@ -153,7 +155,7 @@ static int launch_split(b200_engine *e, const SplitJob &a, const SplitJob &b, co
   };
   const long long ba = blocks_of(a), bb = blocks_of(b);
   if (ba + bb == 0) return B200_OK;
-  split_kernel<MODE><<<(int)(ba + bb), 256, 0, e->stream>>>(a, b, (int)ba, redo);
+  launch_kernel(e, split_kernel<MODE>, (int)(ba + bb), 256, 0, a, b, (int)ba, redo);
   B200_CHECK_LAUNCH(e, "split_kernel");
   return B200_OK;
 }
@@ -173,6 +175,7 @@ int launch_split_tf32_redo(b200_engine *e, const SplitJob &a, const SplitJob &b,
 // The largest magnitude of n values into rec->amax, and rec->bad for infinities and NaNs; with step > 1, of
 // every step-th 4 KB only where there are more than 4 MB.
 __global__ void __launch_bounds__(256) magnitude_kernel(const float *__restrict__ x, long long n, int step, F16Rec *rec) {
+  ptx::grid_begin();
   __shared__ unsigned s_max[8], s_bad[8];
   unsigned amax = 0, bad = 0;
   auto see = [&](float v) {
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(256) magnitude_kernel(const float *__restrict_
 }
 int launch_magnitude(b200_engine *e, const float *x, long long n, int step, F16Rec *rec) {
   const long long groups = ((n + 1023) / 1024 + (n > (1 << 20) ? step : 1) - 1) / (n > (1 << 20) ? step : 1);
-  magnitude_kernel<<<(int)std::max<long long>(1, std::min<long long>(groups, e->sm_count * 8LL)), 256, 0, e->stream>>>(x, n, step, rec);
+  launch_kernel(e, magnitude_kernel, (int)std::max<long long>(1, std::min<long long>(groups, e->sm_count * 8LL)), 256, 0, x, n, step, rec);
   B200_CHECK_LAUNCH(e, "magnitude_kernel");
   return B200_OK;
 }
@@ -220,6 +223,7 @@ struct PairsLimits {
   unsigned limit[kMaxPairsRecs];
 };
 __global__ void pairs_check_kernel(F16Rec *recs, PairsLimits l, int k, int *verdict) {
+  ptx::grid_begin();
   const int i = threadIdx.x;
   const bool bad = i < k && f16_unusable(recs + i, l.limit[i]);
   const bool any = __any_sync(0xffffffffu, bad);
@@ -229,7 +233,7 @@ __global__ void pairs_check_kernel(F16Rec *recs, PairsLimits l, int k, int *verd
 int launch_pairs_check(b200_engine *e, F16Rec *recs, const unsigned *limits, int k, int *verdict) {
   PairsLimits l;
   for (int i = 0; i < kMaxPairsRecs; ++i) l.limit[i] = i < k ? limits[i] : 0xFFFFFFFFu;
-  pairs_check_kernel<<<1, 32, 0, e->stream>>>(recs, l, k, verdict);
+  launch_kernel(e, pairs_check_kernel, 1, 32, 0, recs, l, k, verdict);
   B200_CHECK_LAUNCH(e, "pairs_check_kernel");
   return B200_OK;
 }
