@@ -56,6 +56,7 @@ struct ConvWinParams {
   int tiles_h, tiles_w, tiles_n;
   long long total_tiles;  // B * tiles_h * tiles_w * tiles_n
   int b_stages;
+  int resident;           // F16: one stage per k-block, loaded once per CTA and never handed back
   PairsIn in16;       // F16: the operands, and
   PairsOut out16;     // the (pooled) output in pairs form (h may be null) and what is recorded of it
   const int *only_if; // TF32: run only if this word says so (skip_launch)
@@ -189,7 +190,9 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
       int bs = 0;
       uint32_t bphase = 0;
       bool ok = true;
-      for (long long tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+      // resident filters: the one pass that fills the ring (its stages are free, so nothing is waited for)
+      const long long end = F16 && p.resident ? blockIdx.x + 1LL : p.total_tiles;
+      for (long long tile = blockIdx.x; tile < end && ok; tile += gridDim.x) {
         const int nt = (int)(tile % p.tiles_n);
         for (int cb = 0; cb < p.cblocks && ok; ++cb) {
           for (int tap = 0; tap < taps; ++tap) {
@@ -226,6 +229,58 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
     const int num_k = taps * p.cblocks;
     const uint32_t a_hi32 = desc_hi(a_sbo, LAYOUT), b_hi32 = desc_hi(B_SBO, LAYOUT);
     const uint32_t smem_u = ptx::smem_addr(smem), smem_b_u = ptx::smem_addr(smem_b);
+    if (F16 && p.resident) {
+      // A tile's instructions back to back: a window and an accumulator buffer are waited for once per tile,
+      // each filter slab once per launch, and nothing is committed but the tile's two ends. (With a ring of
+      // filter stages a k-block's wait and commit took longer than its instructions: with all but one tap's
+      // instructions left out, the 16 -> 32 channel layer below went from 302 to 267 us.) The issuing thread
+      // is the bound: 218 cycles per instruction where one lane alone ran this loop, because every descriptor
+      // then goes through vector registers. All lanes run it here, on values that are the same for the warp,
+      // and a 3 x 3 window's offsets are constants.
+      const bool lead = lane == 0;
+      for (int t = 0; t < taps && ok; ++t) ok = __all_sync(0xffffffffu, ptx::mbar_wait(&b_full[t], 0));
+      const uint32_t ah = mh * ((8u * ROW_BYTES) >> 4);  // right half: 8 window rows further
+      const uint32_t b_lo0 = desc_lo(smem_b_u);
+      for (long long tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x, ++use) {
+        const int buf = use & 1;
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&win_full[ws], wphase));
+        ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&acc_empty[buf], (uint32_t)((use >> 1) & 1) ^ 1u));
+        if (!ok) break;
+        ptx::tc_fence_after_sync();
+        const uint32_t a_lo0 = desc_lo(smem_u + (uint32_t)ws * 2u * (uint32_t)p.win_bytes) + ah;
+        const uint32_t a_lo0_tail = a_lo0 + ((uint32_t)p.win_bytes >> 4);
+        const uint32_t d = tmem_base + (uint32_t)(buf * ACC_COLS) + mh * (2 * BN);
+        auto run_tap = [&](uint32_t row0, uint32_t tap, uint32_t first) {
+#pragma unroll
+          for (int kk = 0; kk < KK; ++kk) {
+            const uint32_t ao = row0 * (ROW_BYTES >> 4) + 2u * kk;
+            const uint64_t b_hi = desc_pack(b_lo0 + tap * (B_STAGE_BYTES >> 4) + 2u * kk, b_hi32);
+            if (lead) {
+              ptx::mma_f16(d, desc_pack(a_lo0 + ao, a_hi32), b_hi, IDESC2, first && kk == 0 ? 0u : 1u);
+              ptx::mma_f16(d + BN, desc_pack(a_lo0_tail + ao, a_hi32), b_hi, IDESC, 1u);
+            }
+          }
+        };
+        if (p.kh == 3 && p.kw == 3 && p.win_w == CW_TILE + 2 && p.dH == 1) {
+#pragma unroll
+          for (int t = 0; t < 9; ++t) run_tap((uint32_t)((t / 3) * (CW_TILE + 2) + t % 3), (uint32_t)t, t == 0);
+        } else {
+          uint32_t tap = 0;
+          for (int r = 0; r < p.kh; ++r)
+            for (int sx = 0; sx < p.kw; ++sx, ++tap)
+              run_tap((uint32_t)((r * p.dH) * p.win_w + sx * p.dW), tap, tap == 0);
+        }
+        if (lead) {
+          ptx::mma_commit(&acc_full[buf]);
+          ptx::mma_commit(&win_empty[ws]);
+        }
+        __syncwarp();
+        if (++ws == CW_WIN_STAGES) {
+          ws = 0;
+          wphase ^= 1;
+        }
+      }
+    } else
     for (long long tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
       int kb = 0;       // k-block of this tile: (channel block, tap), taps fastest
       int in_chain = 0; // k-blocks issued into the open accumulation chain
@@ -509,6 +564,10 @@ static int launch_conv_win(b200_engine *e, const CUtensorMap *tm, ConvWinParams 
   const size_t win_total = (size_t)CW_WIN_STAGES * 2 * p.win_bytes;
   p.b_stages = (int)std::max<size_t>(
       2, std::min<size_t>(CW_MAX_BSTAGES, (cw_smem_budget(e) - 1024 - win_total) / B_STAGE_BYTES));
+  // all of a layer's filters stay in shared memory where they fit and make one accumulation chain
+  const int num_k = p.kh * p.kw * p.cblocks;
+  p.resident = F16 && p.tiles_n == 1 && p.cblocks == 1 && num_k <= p.b_stages && num_k <= p.chunk_k;
+  if (p.resident) p.b_stages = num_k;
   const size_t smem = win_total + (size_t)p.b_stages * B_STAGE_BYTES + 1024;
   const int grid = (int)std::min<long long>(p.total_tiles, e->sm_count);
   launch_kernel(e, kern, grid, CW_THREADS, smem, tm[0], tm[1], tm[2], tm[3], p);
