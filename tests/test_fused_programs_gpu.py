@@ -106,3 +106,17 @@ def test_released_temporary_that_is_read_later_is_stored(fresh):
     for k in range(6):
         assert_bits_equal(out[k].numpy(), oracle.binary("add", oracle.unary("square", xs[k]), xs[(k + 1) % 6]))
     assert_bits_equal(again.numpy(), oracle.unary("neg", out[0].numpy()))
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [4097, 3_000_001])
+@pytest.mark.parametrize("div,mod", [(1, 1), (1, 7), (3, 5), (4, 3), (49, 128), (784, 64), (1024, 1021), (1 << 20, 2), (999_999, 3)])
+def test_broadcast_index(fresh, n, dt, div, mod):
+    # two broadcast sources in one program; every element names its own
+    e = fresh
+    x, g, b = util.normal(31, n, dt), util.normal(32, mod, dt), util.normal(33, mod, dt)
+    y = e.empty((n,), dt)
+    e.BroadcastBinary("mul", e.tensor(x), e.tensor(g), div, mod, reuse=y)
+    e.BroadcastBinary("add", y, e.tensor(b), div, mod, unsafe=True)
+    at = np.arange(n) // div % mod
+    assert_bits_equal(y.numpy(), oracle.binary("add", oracle.binary("mul", x, g[at]), b[at]))
