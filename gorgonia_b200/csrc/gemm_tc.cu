@@ -49,9 +49,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <cstring>
-
 #include <atomic>
+#include <cstring>
+#include <type_traits>
 
 #include "engine.h"
 #include "epilogue.cuh"
@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   const int stages = p.stages;
   const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;  // 0: the CTA that issues the pair's MMAs
   const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const long long tiles_per_batch = (long long)p.tiles_m * p.tiles_n;
-  const long long total_tiles = tiles_per_batch * p.batch;
+  const int tiles_per_batch = p.tiles_m * p.tiles_n;  // the host refuses launches of 2^31 tiles
+  const int total_tiles = tiles_per_batch * (int)p.batch;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 
   // tile index -> (batch, m block, n block); m blocks are walked in groups so that the CTAs of
   // one wave share B columns and A rows in L2
-  auto decode = [&](long long tile, int &bz, int &mb, int &nb) {
-    bz = (int)(tile / tiles_per_batch);
-    const int t = (int)(tile % tiles_per_batch);
+  auto decode = [&](int tile, int &bz, int &mb, int &nb) {
+    bz = tile / tiles_per_batch;
+    const int t = tile - bz * tiles_per_batch;
     const int per_group = p.group_m * p.tiles_n;
     const int g = t / per_group;
     const int first_m = g * p.group_m;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      TilePieces pieces(p.streamk, p.units, p.num_k, (int)total_tiles, worker, p.workers, p.sk_first, p.sk_workers);
+      TilePieces pieces(p.streamk, p.units, p.num_k, total_tiles, worker, p.workers, p.sk_first, p.sk_workers);
       int tile, kb0, kb1;
       while (ok && pieces.next(tile, kb0, kb1)) {
         int bz, mb, nb;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       const uint32_t full0 = ptx::smem_addr(&full_bar[0]), empty0 = ptx::smem_addr(&empty_bar[0]);
       const uint32_t empty0_peer = PAIR ? ptx::map_to_rank(empty0, 1u) : 0u;
       uint32_t ready = 0;  // the poll behind the previous k-block saw this stage's barrier complete
-      TilePieces pieces(p.streamk, p.units, p.num_k, (int)total_tiles, worker, p.workers, p.sk_first, p.sk_workers);
+      TilePieces pieces(p.streamk, p.units, p.num_k, total_tiles, worker, p.workers, p.sk_first, p.sk_workers);
       int tile, kb0, kb1;
       while (ok && pieces.next(tile, kb0, kb1)) {
         for (int kc = kb0; kc < kb1 && ok; kc += p.chunk_k, ++use) {
@@ -381,69 +381,90 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
       epi_phase ^= 1;
       return done;
     };
-    TilePieces pieces(p.streamk, p.units, p.num_k, (int)total_tiles, worker, p.workers, p.sk_first, p.sk_workers);
+    TilePieces pieces(p.streamk, p.units, p.num_k, total_tiles, worker, p.workers, p.sk_first, p.sk_workers);
     int tile, kb0, kb1;
     while (ok && pieces.next(tile, kb0, kb1)) {
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
 
-      // where the tile lies is worked out when a store needs it, not before the k loop: the fold
-      // below wants every register it can get
-      auto store32 = [&](const float(&v)[32], int c) {
+      // Finishes and stores N columns of this thread's row, from column c of the warp's half on. A tile's
+      // epilogue runs once, so its code is as good as never in the instruction caches when it starts: what
+      // it costs is its length. Bias, activation and the kinds of store are therefore chosen outside the
+      // loops, and nothing is repeated per element. (Chosen per element it was some 4,000 instructions, and
+      // 19600 x 288 x 64, two k-blocks per tile, had ten warps waiting for code for each one that issued;
+      // the convolution's backward pass that this product belongs to went from 150 to 120 us.)
+      auto finish_store = [&](auto &v, auto size, int c) {
+        constexpr int NV = decltype(size)::value;
         int bz, mb, nb;
         decode(tile, bz, mb, nb);
         const long long m = (long long)(PAIR ? mb * 2 + (int)rank : mb) * TC_BM + quarter * 32 + lane;
-        float *crow = reinterpret_cast<float *>(p.C) + (long long)bz * p.strideC + m * p.ldc;
-        const long long n0 = (long long)nb * BN;
-        if (m >= p.M) return;
-        const long long nbase = n0 + ch0 + c;
+        const long long nbase = (long long)nb * BN + ch0 + c;
+        if (m >= p.M || nbase >= (p.C_hi ? p.ld_split : p.N)) return;
+        const int valid = p.N - nbase >= NV ? NV : (int)(p.N - nbase);  // may be <= 0 in front of a split's padding
+        const float *bias = reinterpret_cast<const float *>(p.ep.bias);
+        if (p.ep.bias_kind == B200_BIAS_COL) {
+          if (valid == NV) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) v[j] = __fadd_rn(v[j], __ldg(bias + nbase + j));
+          } else {
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+              if (j < valid) v[j] = __fadd_rn(v[j], __ldg(bias + nbase + j));
+          }
+        } else if (p.ep.bias_kind == B200_BIAS_ROW) {
+          const float bm = __ldg(bias + m);
+#pragma unroll
+          for (int j = 0; j < NV; ++j) v[j] = __fadd_rn(v[j], bm);
+        }
+        const float alpha = (float)p.ep.alpha;
+        if (p.ep.act == B200_ACT_RECTIFY) {
+#pragma unroll
+          for (int j = 0; j < NV; ++j) v[j] = apply_act<float>(v[j], B200_ACT_RECTIFY, alpha);
+        } else if (p.ep.act == B200_ACT_LEAKY) {
+#pragma unroll
+          for (int j = 0; j < NV; ++j) v[j] = apply_act<float>(v[j], B200_ACT_LEAKY, alpha);
+        }
+        if (p.C) {
+          float *crow = reinterpret_cast<float *>(p.C) + (long long)bz * p.strideC + m * p.ldc + nbase;
+          if (p.c_vec && valid == NV) {
+            if (p.ep.accumulate) {  // Incr mode: the rounded result is added to what C holds
+#pragma unroll
+              for (int j = 0; j < NV; j += 4) {
+                const float4 old = *reinterpret_cast<const float4 *>(crow + j);
+                *reinterpret_cast<float4 *>(crow + j) = make_float4(__fadd_rn(old.x, v[j]), __fadd_rn(old.y, v[j + 1]),
+                                                                    __fadd_rn(old.z, v[j + 2]), __fadd_rn(old.w, v[j + 3]));
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < NV; j += 4)
+                *reinterpret_cast<float4 *>(crow + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < NV; ++j)
+              if (j < valid) crow[j] = p.ep.accumulate ? __fadd_rn(crow[j], v[j]) : v[j];
+          }
+        }
         if (p.C_hi) {
           // the result as the next product's A operand: TF32 head and tail, 16 bytes at a time;
           // columns between N and the pitch hold zeros
-          float *hrow = p.C_hi + m * p.ld_split, *lrow = p.C_lo + m * p.ld_split;
+          float *hrow = p.C_hi + m * p.ld_split + nbase, *lrow = p.C_lo + m * p.ld_split + nbase;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            if (nbase + j >= p.ld_split) break;
-            float h[4], l[4];
+          for (int j = 0; j < NV; j += 4) {
+            if (nbase + j < p.ld_split) {
+              float h[4], l[4];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              float o = 0.f;
-              if (nbase + j + t < p.N) {
-                o = apply_epilogue<float>(v[j + t], p.ep, m, nbase + j + t);
-                if (p.C) crow[nbase + j + t] = o;
+              for (int t = 0; t < 4; ++t) {
+                const float o = j + t < valid ? v[j + t] : 0.f;
+                uint32_t hb;
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(o));
+                h[t] = __uint_as_float(hb);
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(__fsub_rn(o, h[t])));
+                l[t] = __uint_as_float(hb);
               }
-              uint32_t hb;
-              asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(o));
-              h[t] = __uint_as_float(hb);
-              asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(__fsub_rn(o, h[t])));
-              l[t] = __uint_as_float(hb);
+              *reinterpret_cast<float4 *>(hrow + j) = make_float4(h[0], h[1], h[2], h[3]);
+              *reinterpret_cast<float4 *>(lrow + j) = make_float4(l[0], l[1], l[2], l[3]);
             }
-            *reinterpret_cast<float4 *>(hrow + nbase + j) = make_float4(h[0], h[1], h[2], h[3]);
-            *reinterpret_cast<float4 *>(lrow + nbase + j) = make_float4(l[0], l[1], l[2], l[3]);
           }
-          return;
-        }
-        if (p.c_vec && nbase + 32 <= p.N) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            float4 o;
-            o.x = apply_epilogue<float>(v[j + 0], p.ep, m, nbase + j + 0);
-            o.y = apply_epilogue<float>(v[j + 1], p.ep, m, nbase + j + 1);
-            o.z = apply_epilogue<float>(v[j + 2], p.ep, m, nbase + j + 2);
-            o.w = apply_epilogue<float>(v[j + 3], p.ep, m, nbase + j + 3);
-            if (p.ep.accumulate) {  // Incr mode: the rounded result is added to what C holds
-              const float4 old = *reinterpret_cast<const float4 *>(crow + nbase + j);
-              o.x = __fadd_rn(old.x, o.x); o.y = __fadd_rn(old.y, o.y);
-              o.z = __fadd_rn(old.z, o.z); o.w = __fadd_rn(old.w, o.w);
-            }
-            *reinterpret_cast<float4 *>(crow + nbase + j) = o;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (nbase + j < p.N) {
-              const float o = apply_epilogue<float>(v[j], p.ep, m, nbase + j);
-              crow[nbase + j] = p.ep.accumulate ? __fadd_rn(crow[nbase + j], o) : o;
-            }
         }
       };
 
@@ -465,7 +486,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           float v[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-          store32(v, c);
+          finish_store(v, std::integral_constant<int, 32>(), c);
         }
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -540,20 +561,38 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           __threadfence();
 #pragma unroll
           for (int j = 0; j < NACC; ++j) acc[j] = 0.f;
-          for (int c = c_first; c <= c_last; ++c) {  // k order: CTA c's share precedes CTA c + 1's
-            const float *src = p.ws + (size_t)share_slot(c, tile_u0, p.units, p.sk_workers) * slot_floats + within;
+          // k order: CTA c's share precedes CTA c + 1's. On narrow tiles the loads of three parts are in
+          // flight together (a part is a latency of about a microsecond); on wide ones there are no registers
+          // for that, and one SM's share of the L2 rate is the bound.
+          constexpr int PF = NACC == 32 ? 3 : 1;
+          for (int c = c_first; c <= c_last; c += PF) {
+            float part[PF][NACC];
 #pragma unroll
-            for (int j = 0; j < NACC; ++j) acc[j] = __fadd_rn(acc[j], ptx::ld_cg_ordered(src + j * 32));
+            for (int q = 0; q < PF; ++q) {
+              if (c + q <= c_last) {
+                const float *src = p.ws + (size_t)share_slot(c + q, tile_u0, p.units, p.sk_workers) * slot_floats + within;
+#pragma unroll
+                for (int j = 0; j < NACC; ++j) part[q][j] = PF > 1 ? __ldcg(src + j * 32) : ptx::ld_cg_ordered(src + j * 32);
+              } else {
+#pragma unroll
+                for (int j = 0; j < NACC; ++j) part[q][j] = 0.f;
+              }
+            }
+#pragma unroll
+            for (int q = 0; q < PF; ++q) {
+              if (c + q <= c_last) {
+#pragma unroll
+                for (int j = 0; j < NACC; ++j) acc[j] = __fadd_rn(acc[j], part[q][j]);
+              }
+            }
           }
         }
         if (ok) {
+          if (TERMS == 2) {
 #pragma unroll
-          for (int c = 0; c < (TERMS != 1 ? HALF : 0); c += 32) {
-            float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = TERMS == 2 ? __fmul_rn(__fmul_rn(acc[c + j], unscale1), unscale2) : acc[c + j];
-            store32(v, c);
+            for (int j = 0; j < (TERMS != 1 ? HALF : 1); ++j) acc[j] = __fmul_rn(__fmul_rn(acc[j], unscale1), unscale2);
           }
+          finish_store(acc, std::integral_constant<int, TERMS != 1 ? HALF : 1>(), 0);
         }
       }
     }
