@@ -83,10 +83,10 @@ __device__ __forceinline__ void cw_tma_load_4d(void *smem_dst, const void *tmap,
       : "memory");
 }
 
-// F16: pairs of fp16 (pairs.cuh) instead of TF32 pairs: half the bytes per channel, and half the instructions,
-// which is what bounds this kernel: an instruction reads 128 rows of 32 bytes, 16 channels of fp16 against 8.
-// 16 -> 32 channels with pool on 208 x 208 planes of 64 images: 337 -> 315 us; 32 -> 64 on 104 x 104:
-// 147 -> 130.
+// F16: pairs of fp16 (pairs.cuh) instead of TF32 pairs: half the bytes per channel and half the instructions.
+// With the same issue loop that gained little (16 -> 32 channels with pool on 208 x 208 planes of 64 images
+// 337 -> 315 us; 32 -> 64 on 104 x 104 147 -> 130): the issuing threads were the bound. With the filters
+// resident and a lean issue (below) 132 and 73.
 template <int BN, int CK, bool F16>
 __global__ void __launch_bounds__(CW_THREADS, 1)
     conv_win_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
