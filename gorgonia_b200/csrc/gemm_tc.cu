@@ -1062,58 +1062,65 @@ static int gemm_f32_tf32(b200_engine *e, bool a_mn, bool b_mn, long long M, long
   return rc;
 }
 
-// Room for an operand's fp16 pairs (pitch a multiple of 8 values), or a constant's that are there already.
+// One operand on its way to fp16 pairs (pitch a multiple of 8 values).
+struct F16Operand {
+  TcOperand op;
+  SplitJob job;             // job.src stays null if a constant's pairs were there already
+  F16Rec *rec = nullptr;
+  void *blk[2] = {nullptr, nullptr};   // the TF32 pairs' place; a temporary operand's fp16 pairs lie in it too
+  void *kept[2] = {nullptr, nullptr};  // a constant's record and heads, and its tails, before they are kept
+};
+
+// Finds a constant's pairs or takes room for an operand's. Nothing is launched and nothing kept here: what was
+// taken is the caller's to hand back, also after an error.
 // The blocks are as large as the TF32 pairs need, which take their place if the fp16 pairs turn out unusable.
-static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_rec, TcOperand *out, SplitJob *job,
-                          F16Rec **rec, void **blk) {
+static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_rec, F16Operand *o) {
   const long long ldo = (x.cols + 7) / 8 * 8, elems = x.rows * ldo * x.batch;
-  out->ld = ldo;
-  out->batch_stride = x.rows * ldo;
-  out->shared = false;
+  o->op.ld = ldo;
+  o->op.batch_stride = x.rows * ldo;
+  o->op.shared = false;
   int rc = B200_OK;
   const bool constant = is_constant(e, x.src);
   if (constant) {
     if (CachedSplit *c = find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld)) {
-      *rec = (F16Rec *)c->hi;
-      out->p0 = (char *)c->hi + 256;
-      out->p1 = c->lo;
-    } else {  // a record and the heads, the tails
-      void *hi = nullptr, *lo = nullptr;
-      rc = b200_get(e, 256 + elems * 2, &hi);
-      if (rc == B200_OK && (rc = b200_get(e, elems * 2, &lo)) != B200_OK) b200_put(e, hi, 0);
-      if (rc != B200_OK) return rc;
-      if (cudaMemsetAsync(hi, 0, sizeof(F16Rec), e->stream) != cudaSuccess) {
-        b200_put(e, hi, 0);
-        b200_put(e, lo, 0);
-        return set_error(e, B200_ERR_CUDA, "b200_gemm: clearing a record failed");
-      }
-      add_cached(e, x.src, CachedSplit{2, x.rows, x.cols, x.batch, x.ld, hi, lo, ldo});
-      *rec = (F16Rec *)hi;
-      out->p0 = (char *)hi + 256;
-      out->p1 = lo;
-      job->src = x.src;
+      o->rec = (F16Rec *)c->hi;
+      o->op.p1 = c->lo;
+    } else {
+      rc = b200_get(e, 256 + elems * 2, &o->kept[0]);
+      if (rc == B200_OK) rc = b200_get(e, elems * 2, &o->kept[1]);
+      o->rec = (F16Rec *)o->kept[0];
+      o->op.p1 = o->kept[1];
+      o->job.src = x.src;
     }
+    o->op.p0 = (char *)o->rec + 256;
   } else {
-    *rec = scratch_rec;
-    job->src = x.src;
+    o->rec = scratch_rec;
+    o->job.src = x.src;
   }
-  // the TF32 pairs' place; a temporary operand's fp16 pairs lie in the same blocks
-  for (int h = 0; h < 2 && rc == B200_OK; ++h) rc = b200_get(e, elems * 4, &blk[h]);
+  for (int h = 0; h < 2 && rc == B200_OK; ++h) rc = b200_get(e, elems * 4, &o->blk[h]);
   if (rc != B200_OK) return rc;
   if (!constant) {
-    out->p0 = blk[0];
-    out->p1 = blk[1];
+    o->op.p0 = o->blk[0];
+    o->op.p1 = o->blk[1];
   }
-  job->ld = x.ld;
-  job->stride = x.stride;
-  job->rows = x.rows;
-  job->cols = x.cols;
-  job->batch = x.batch;
-  job->hi = const_cast<void *>(out->p0);
-  job->lo = const_cast<void *>(out->p1);
-  job->ldo = ldo;
-  job->rec = *rec;
+  o->job.ld = x.ld;
+  o->job.stride = x.stride;
+  o->job.rows = x.rows;
+  o->job.cols = x.cols;
+  o->job.batch = x.batch;
+  o->job.hi = const_cast<void *>(o->op.p0);
+  o->job.lo = const_cast<void *>(o->op.p1);
+  o->job.ldo = ldo;
+  o->job.rec = o->rec;
   return B200_OK;
+}
+
+// Once its split has been launched: a constant's pairs are kept, unless an equal entry (one matrix as both
+// operands) is there already.
+static void keep_split_f16(b200_engine *e, const F32Operand &x, F16Operand *o) {
+  if (!o->kept[0] || find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld)) return;
+  add_cached(e, x.src, CachedSplit{2, x.rows, x.cols, x.batch, x.ld, o->kept[0], o->kept[1], o->op.ld});
+  o->kept[0] = o->kept[1] = nullptr;
 }
 
 // Whether a product is worth fp16 pairs. They save about half of the 2 M N K / 200 TFLOP/s that TF32 pairs
@@ -1131,46 +1138,51 @@ static int gemm_f32_f16(b200_engine *e, bool a_mn, bool b_mn, long long M, long 
                         const F32Operand &A, const F32Operand &B, void *C, long long ldc, long long batch,
                         long long strideC, const Epilogue &ep, float *C_hi = nullptr, float *C_lo = nullptr,
                         long long ld_split = 0) {
-  TcOperand a, b;
-  SplitJob ja, jb;
-  F16Rec *ra = nullptr, *rb = nullptr;
-  void *blk[4] = {nullptr, nullptr, nullptr, nullptr};
-  int rc = plan_split_f16(e, A, e->f16_recs, &a, &ja, &ra, &blk[0]);
-  if (rc == B200_OK) rc = plan_split_f16(e, B, e->f16_recs + 1, &b, &jb, &rb, &blk[2]);
+  F16Operand a, b;
+  const F32Operand *xs[2] = {&A, &B};
+  F16Operand *ops[2] = {&a, &b};
+  int rc = plan_split_f16(e, A, e->f16_recs, &a);
+  if (rc == B200_OK) rc = plan_split_f16(e, B, e->f16_recs + 1, &b);
+  for (F16Operand *o : ops)
+    if (rc == B200_OK && o->kept[0] && cudaMemsetAsync(o->rec, 0, sizeof(F16Rec), e->stream) != cudaSuccess)
+      rc = set_error(e, B200_ERR_CUDA, "b200_gemm: clearing a record failed");
   const unsigned la = f16_small_limit(A.rows * A.cols * A.batch), lb = f16_small_limit(B.rows * B.cols * B.batch);
-  if (rc == B200_OK && ja.src) rc = launch_split_f16(e, ja, jb);
-  else if (rc == B200_OK && jb.src) rc = launch_split_f16(e, jb, SplitJob());
+  if (rc == B200_OK && a.job.src) rc = launch_split_f16(e, a.job, b.job);
+  else if (rc == B200_OK && b.job.src) rc = launch_split_f16(e, b.job, SplitJob());
+  if (rc == B200_OK)
+    for (int i = 0; i < 2; ++i) keep_split_f16(e, *xs[i], ops[i]);
   F16Gate gate;
-  gate.rec_a = ra;
-  gate.rec_b = rb;
+  gate.rec_a = a.rec;
+  gate.rec_b = b.rec;
   gate.limit_a = la;
   gate.limit_b = lb;
-  if (rc == B200_OK) rc = gemm_tc_core(e, 2, a_mn, b_mn, M, N, K, a, b, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split, gate);
+  if (rc == B200_OK)
+    rc = gemm_tc_core(e, 2, a_mn, b_mn, M, N, K, a.op, b.op, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split, gate);
   if (rc == B200_OK) {
-    TcOperand ta, tb;
-    SplitJob *jobs[2] = {&ja, &jb};
-    TcOperand *ops[2] = {&ta, &tb};
-    const F32Operand *xs[2] = {&A, &B};
+    TcOperand t[2];
     for (int i = 0; i < 2; ++i) {
-      jobs[i]->src = xs[i]->src;
-      jobs[i]->hi = blk[2 * i];
-      jobs[i]->lo = blk[2 * i + 1];
-      jobs[i]->ldo = (xs[i]->cols + 3) / 4 * 4;
-      ops[i]->p0 = blk[2 * i];
-      ops[i]->p1 = blk[2 * i + 1];
-      ops[i]->ld = jobs[i]->ldo;
-      ops[i]->batch_stride = xs[i]->rows * jobs[i]->ldo;
+      SplitJob &j = ops[i]->job;
+      j.src = xs[i]->src;
+      j.hi = ops[i]->blk[0];
+      j.lo = ops[i]->blk[1];
+      j.ldo = (xs[i]->cols + 3) / 4 * 4;
+      t[i].p0 = j.hi;
+      t[i].p1 = j.lo;
+      t[i].ld = j.ldo;
+      t[i].batch_stride = xs[i]->rows * j.ldo;
     }
     F16Gate redo;
     redo.redo = (int *)(e->f16_recs + 2);
-    redo.clear_a = ra == e->f16_recs ? ra : nullptr;
-    redo.clear_b = rb == e->f16_recs + 1 ? rb : nullptr;
-    rc = launch_split_tf32_redo(e, ja, jb, ra, la, rb, lb, (int *)(e->f16_recs + 2));
-    if (rc == B200_OK) rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, ta, tb, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split,
-                                       redo);
+    redo.clear_a = a.rec == e->f16_recs ? a.rec : nullptr;
+    redo.clear_b = b.rec == e->f16_recs + 1 ? b.rec : nullptr;
+    rc = launch_split_tf32_redo(e, a.job, b.job, a.rec, la, b.rec, lb, (int *)(e->f16_recs + 2));
+    if (rc == B200_OK)
+      rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, t[0], t[1], C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split, redo);
   }
-  for (void *s2 : blk)
-    if (s2) b200_put(e, s2, 0);
+  // stream order makes handing the blocks back safe, also those whose kernels are queued
+  for (F16Operand *o : ops)
+    for (void *s2 : {o->blk[0], o->blk[1], o->kept[0], o->kept[1]})
+      if (s2) b200_put(e, s2, 0);
   return rc;
 }
 

@@ -128,3 +128,27 @@ def test_all_zero_and_recorded(fresh):
         row = np.linalg.norm(tc.numpy() - want, axis=1) / np.linalg.norm(want, axis=1)
         assert row.max() < 2e-6
     e.tape_destroy(tape)
+
+
+@pytest.mark.parametrize("which", ["a", "b", "both"])
+def test_constant_met_in_a_full_arena(which):
+    # at its first use the arena holds the TF32 pairs but not all that fp16 pairs need; with room again, the
+    # second product must not find anything that was never made
+    from gorgonia_b200 import Engine
+    e = Engine(0, 256 << 20)
+    a, b = util.normal(31, (2048, 2048)), util.normal(32, (2048, 2048), scale=0.02)
+    ta, tb, tc = e.tensor(a), e.tensor(b), e.empty((2048, 2048))
+    for t in {"a": [ta], "b": [tb], "both": [ta, tb]}[which]:
+        e.constant(t)
+    filler = e.Get(e.arena_stats()["largest_free"] - (70 << 20))
+    want = _want(a, b)
+    e.MatMul(ta, tb, tc)
+    assert_gemm_close(tc.numpy(), want, 1e-5)
+    free = e.arena_stats()["free"]
+    e.Put(filler)
+    for _ in range(2):
+        e.MatMul(ta, tb, tc)
+        assert_gemm_close(tc.numpy(), want, 1e-5)
+    e.Close()
+    # nothing but the constants' TF32 pairs (two blocks of 16 MB each) had stayed behind
+    assert free == (70 << 20) - (32 << 20) * (2 if which == "both" else 1)
