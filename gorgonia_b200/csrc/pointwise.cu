@@ -65,6 +65,8 @@ struct PwDev {
   uint8_t kb[B200_PW_MAX_INSTR], xb[B200_PW_MAX_INSTR];
   uint8_t keep_slot[B200_PW_MAX_INSTR];  // file slot that keeps the result for later, or 0xFF
   uint8_t out_of[B200_PW_MAX_INSTR];     // output index this instruction's result is stored to, or 0xFF
+  uint8_t out_next[B200_PW_MAX_OUT];     // the next output of the same instruction, or 0xFF
+  uint8_t shared_result;                 // some instruction feeds several outputs: not for pw_stream_kernel
   uint2 code[B200_PW_MAX_INSTR];         // the six above in one load: op, ka | kb << 4, xa, xb; keep, out
 };
 
@@ -549,8 +551,9 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
         sts128(file_s + (uint32_t)keep * SLOT_BYTES + u * USTRIDE, raw);
       }
     }
-    const int o = (now.y >> 8) & 0xFF;
-    if (o != 0xFF) {
+    // Whole tiles are pw_stream_kernel's alone, which gets one output per instruction; the others store a result
+    // to each of its outputs.
+    for (int o = (now.y >> 8) & 0xFF; o != 0xFF; o = INSIDE ? 0xFF : p.out_next[o]) {
       unsigned char *op_ = reinterpret_cast<unsigned char *>(p.out[o]) + (c_tile + tid) * 16;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -884,7 +887,9 @@ static int launch_stream(b200_engine *e, const PwDev &d) {
 template <typename T, int V>
 static int launch_loop(b200_engine *e, const PwDev &d) {
   constexpr int VV = Vec<T>::N;
-  const size_t smem = (size_t)(d.n_full + d.n_file) * PW_LOOP_THREADS * 16;  // at most 6 + 7 slots of 2 KB
+  // slots of 2 KB: at most six sources and a kept result per instruction but the last two
+  static_assert((B200_PW_MAX_SRC + B200_PW_MAX_INSTR) * PW_LOOP_THREADS * 16 <= 48 * 1024, "slots of pw_loop_kernel");
+  const size_t smem = (size_t)(d.n_full + d.n_file) * PW_LOOP_THREADS * 16;
   const long long tiles = ((d.n + VV - 1) / VV + PW_LOOP_THREADS - 1) / PW_LOOP_THREADS;
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, (long long)e->sm_count * 16));
   launch_kernel(e, pw_loop_kernel<T, VV, (V > 1)>, blocks, PW_LOOP_THREADS, smem, d);
@@ -898,7 +903,7 @@ static int launch_sized(b200_engine *e, const PwDev &d, int ns, int ni) {
   // Large, 16-byte aligned tensors take the streaming kernel. Below ~2 tiles per SM the ring
   // never fills and the plain kernel, with its many small blocks, spreads the work better.
   if constexpr (V > 1) {
-    if (d.n_full >= 1 && nchunks >= (long long)e->sm_count * PW_STREAM_THREADS * 2 * 2) {
+    if (d.n_full >= 1 && !d.shared_result && nchunks >= (long long)e->sm_count * PW_STREAM_THREADS * 2 * 2) {
       const int rc = launch_stream<T, V>(e, d);
       if (rc >= 0) return rc;
     }
@@ -1023,9 +1028,9 @@ static int run_program(b200_engine *e, int dtype, const b200_pw_prog *prog, void
       classify(d.rb[k], (int)k, &d.kb[k], &d.xb[k]);
     }
     for (uint32_t o = 0; o < prog->n_out; ++o) {
-      // one instruction may feed several outputs only through the plain kernel; the streaming
-      // kernel stores each result once, which is all the engine's own planner ever asks for
-      if (d.out_of[d.out_ins[o]] != 0xFF) d.n_full = 0;
+      // the streaming kernel stores each result once, which is all the engine's own planner ever asks for
+      d.out_next[o] = d.out_of[d.out_ins[o]];
+      if (d.out_next[o] != 0xFF) d.shared_result = 1;
       d.out_of[d.out_ins[o]] = (uint8_t)o;
     }
   }

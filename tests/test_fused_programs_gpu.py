@@ -120,3 +120,29 @@ def test_broadcast_index(fresh, n, dt, div, mod):
     e.BroadcastBinary("add", y, e.tensor(b), div, mod, unsafe=True)
     at = np.arange(n) // div % mod
     assert_bits_equal(y.numpy(), oracle.binary("add", oracle.binary("mul", x, g[at]), b[at]))
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [5, 1000, 3_000_001])
+@pytest.mark.parametrize("start", [0, 1])
+@pytest.mark.parametrize("n_src,n_instr", [(1, 2), (3, 4), (4, 4), (2, 5), (6, 8)])
+def test_one_result_to_several_outputs(fresh, n, dt, start, n_src, n_instr):
+    # programs of the register kernel and of the loop kernel, on small, unaligned and large tensors: the result of
+    # the first instruction (kept for the last one) goes to two outputs, the last one's to two as well
+    e = fresh
+    xs = [util.normal(60 + k, n, dt) for k in range(n_src)]
+    srcs = [_at(e, x, start) for x in xs]
+    outs = [_at(e, np.zeros(n, dt), start) for _ in range(4)]
+    SRC, INS = 0x00, 0x80
+    instr, vals = [("neg", SRC | 0, SRC | 0)], [-xs[0]]
+    for k in range(1, n_instr - 1):
+        instr.append(("add" if k % 2 else "mul", INS | (k - 1), SRC | (k % n_src)))
+        vals.append(oracle.binary("add" if k % 2 else "mul", vals[-1], xs[k % n_src]))
+    instr.append(("sub", INS | (n_instr - 2), INS | 0))
+    vals.append(oracle.binary("sub", vals[-1], vals[0]))
+    last = n_instr - 1
+    e.Pointwise({"instr": instr, "out": [0, last, 0, last]}, outs, srcs, n, dt)
+    for o, k in zip(outs, (0, last, 0, last)):
+        assert_bits_equal(o.numpy(), vals[k])
+    for s, x in zip(srcs, xs):      # nothing was written where it does not belong
+        assert_bits_equal(s.numpy(), x)
