@@ -592,6 +592,8 @@ static int conv2d_eager_pairs(b200_engine *e, int path, const float *x, const fl
              ? conv2d_win(e, x, w, y, B, C, H, W, K, kh, kw, padH, padW, dH, dW, Ho, Wo, ep, pool2, nullptr, nullptr, nullptr, nullptr)
              : conv2d_tma(e, x, w, y, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho, Wo, ep, nullptr, nullptr, nullptr, nullptr);
     e->only_if = nullptr;
+  } else {
+    clear_f16_recs(e);  // the check, which clears them, was not launched
   }
   return rc;
 }

@@ -1179,6 +1179,7 @@ static int gemm_f32_f16(b200_engine *e, bool a_mn, bool b_mn, long long M, long 
     if (rc == B200_OK)
       rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, t[0], t[1], C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split, redo);
   }
+  if (rc != B200_OK) clear_f16_recs(e);
   // stream order makes handing the blocks back safe, also those whose kernels are queued
   for (F16Operand *o : ops)
     for (void *s2 : {o->blk[0], o->blk[1], o->kept[0], o->kept[1]})

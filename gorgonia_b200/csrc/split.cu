@@ -237,5 +237,8 @@ int launch_pairs_check(b200_engine *e, F16Rec *recs, const unsigned *limits, int
   B200_CHECK_LAUNCH(e, "pairs_check_kernel");
   return B200_OK;
 }
+void clear_f16_recs(b200_engine *e) {
+  if (cudaMemsetAsync(e->f16_recs, 0, 256, e->stream) != cudaSuccess) cudaGetLastError();  // the call's own error is told
+}
 
 }  // namespace b200

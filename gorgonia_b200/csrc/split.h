@@ -45,6 +45,9 @@ int launch_magnitude(b200_engine *e, const float *x, long long n, int step, F16R
 // Whether any of k <= kMaxPairsRecs records, one after the other in memory, says that its tensor is unusable
 // goes to *verdict; the records are cleared.
 constexpr int kMaxPairsRecs = 32;
+// The engine's own records are zero between calls: a call that gave up before the launch that clears them puts
+// them back with this.
+void clear_f16_recs(b200_engine *e);
 int launch_pairs_check(b200_engine *e, F16Rec *recs, const unsigned *limits, int k, int *verdict);
 
 #ifdef __CUDACC__

@@ -23,6 +23,8 @@ engine call per reference instruction and leaves fusing to the engine's deferred
 Weights are seeded draws (Glorot-uniform / He-normal formulas of weights.go:397-479); nothing is
 computed on the host.
 """
+import contextlib
+
 import numpy as np
 
 
@@ -84,6 +86,15 @@ class _Records:
 
     def check(self):
         self.e.pairs_check(self.buf.ptr, self.counts, self.verdict)
+
+    @contextlib.contextmanager
+    def chain(self):
+        """Around the links of a chain: checked at its end, and also where a link fails (the check clears the
+        records, which are zero between chains)."""
+        try:
+            yield
+        finally:
+            self.check()
 
 
 class _ConvChain:
@@ -327,8 +338,8 @@ class LeNet(_Tape):
     def forward(self):
         e, a = self.e, self.x
         if self.fused and self.records is not None:
-            self.chain.forward_pairs(a)
-            self.records.check()
+            with self.records.chain():
+                self.chain.forward_pairs(a)
             with e.only_if(self.records.verdict):
                 a = self.chain.forward(a)
         elif self.fused:
@@ -424,12 +435,12 @@ class TinyYolo(_Tape):
 
     def _forward_pairs(self):
         e, a, b = self.e, self.chain_a, self.chain_b
-        a.forward_pairs(self.x)
-        last = a.layers[-1]
-        # chain_b's record of its input is written by the pool in front of it
-        e.MaxPool2DPairs(last["y"], last["rec"], self.pool5_split[0], b.x_rec, (2, 2), (1, 0, 1, 0), (1, 1))
-        b.forward_pairs(None, self.pool5_split[0], b.x_rec)
-        self.records.check()
+        with self.records.chain():
+            a.forward_pairs(self.x)
+            last = a.layers[-1]
+            # chain_b's record of its input is written by the pool in front of it
+            e.MaxPool2DPairs(last["y"], last["rec"], self.pool5_split[0], b.x_rec, (2, 2), (1, 0, 1, 0), (1, 1))
+            b.forward_pairs(None, self.pool5_split[0], b.x_rec)
         with e.only_if(self.records.verdict):
             return self._forward_tf32()
 

@@ -152,3 +152,24 @@ def test_constant_met_in_a_full_arena(which):
     e.Close()
     # nothing but the constants' TF32 pairs (two blocks of 16 MB each) had stayed behind
     assert free == (70 << 20) - (32 << 20) * (2 if which == "both" else 1)
+
+
+def test_failed_convolution_leaves_no_trace():
+    # the pairs' records are the engine's: a call that runs out of room must hand them back clear
+    from gorgonia_b200 import B200Error, Engine
+    B, C, H, W, K = 48, 128, 26, 26, 256
+    x, w = util.normal(33, (B, C, H, W)), util.normal(34, (K, C, 3, 3), scale=0.05)
+    out = []
+    for fail in (False, True):
+        e = Engine(0, 512 << 20)
+        tx, tw, y = e.tensor(x * np.float32(1e6)), e.tensor(w), e.empty((B, K, H, W))
+        if fail:
+            filler = e.Get(e.arena_stats()["largest_free"] - x.nbytes - (256 << 10))
+            with pytest.raises(B200Error):
+                e.Conv2d(tx, tw, y, pad=(1, 1))
+            e.Put(filler)
+        tx.set(x)
+        e.Conv2d(tx, tw, y, pad=(1, 1))
+        out.append(y.numpy())
+        e.Close()
+    util.assert_bits_equal(out[0], out[1])

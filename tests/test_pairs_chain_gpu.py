@@ -212,3 +212,27 @@ def test_only_if_refuses_other_calls(fresh):
             e.DoWork()
     e.MatMul(a, a, e.empty((64, 64)))
     e.Signal()
+
+
+@pytest.mark.parametrize("make", [_lenet, _yolo])
+def test_failed_chain_leaves_its_records_clear(fresh, monkeypatch, make):
+    e = fresh
+    m = make(e, monkeypatch, 0)
+    x = util.uniform(82, m.x.shape)
+    m.x.set(x)
+    want = m.forward().numpy()
+    m.x.set(x * np.float32(1e6))
+    links = []
+
+    def fail(*a, **kw):
+        links.append(0)
+        if len(links) == 3:
+            raise B200Error(2, "no room")
+        return type(e).Conv2dPairs(e, *a, **kw)
+    monkeypatch.setattr(e, "Conv2dPairs", fail, raising=False)
+    with pytest.raises(B200Error):
+        m.forward()
+    monkeypatch.delattr(e, "Conv2dPairs")
+    assert not m.records.buf.numpy()[:-4].any()
+    m.x.set(x)
+    assert_bits_equal(m.forward().numpy(), want)
