@@ -33,11 +33,11 @@ int set_error(b200_engine *e, int code, const char *fmt, ...) {
 bool is_constant(b200_engine *e, const void *ptr) { return e->constants.count(ptr) != 0; }
 
 CachedSplit *find_cached(b200_engine *e, const void *ptr, int kind, long long d0, long long d1, long long d2,
-                         long long ld_in) {
+                         long long ld_in, long long stride) {
   auto it = e->constants.find(ptr);
   if (it == e->constants.end()) return nullptr;
   for (auto &c : it->second.derived)
-    if (c.kind == kind && c.d0 == d0 && c.d1 == d1 && c.d2 == d2 && c.ld_in == ld_in) {
+    if (c.kind == kind && c.d0 == d0 && c.d1 == d1 && c.d2 == d2 && c.ld_in == ld_in && c.stride == stride) {
       pin_cached(e, c);  // whoever asks is about to launch a kernel that reads it
       return &c;
     }

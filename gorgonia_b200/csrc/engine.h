@@ -25,6 +25,7 @@ struct CachedSplit {
   long long d0, d1, d2, ld_in;  // the shape it was made for
   void *hi, *lo;                // arena blocks
   long long ld_out;
+  long long stride = 0;         // elements between the slices of a batch; 0 where there is one slice
 };
 struct ConstantEntry {
   std::vector<CachedSplit> derived;
@@ -178,7 +179,7 @@ inline size_t dtype_size(int dtype) {
 
 // constants (engine.cu)
 CachedSplit *find_cached(b200_engine *e, const void *ptr, int kind, long long d0, long long d1, long long d2,
-                         long long ld_in);
+                         long long ld_in, long long stride = 0);
 bool is_constant(b200_engine *e, const void *ptr);
 void add_cached(b200_engine *e, const void *ptr, const CachedSplit &c);
 void drop_constant(b200_engine *e, const void *ptr);

@@ -955,6 +955,9 @@ int gemm_tc_core(b200_engine *e, int terms, bool a_mn, bool b_mn, long long M, l
   return rc;
 }
 
+// What a constant's split is kept under besides its extents: which slices of the buffer a batch reads.
+static long long slice_stride(long long batch, long long stride) { return batch > 1 ? stride : 0; }
+
 // Finds or makes room for the TF32 head and tail of a row-major fp32 matrix (rows x cols, pitch ld,
 // `batch` of them), with a pitch that is a multiple of 4 elements. What is left to do is put into *job
 // (job->src stays null if a constant's split was there already); blk_hi / blk_lo are the blocks that the
@@ -971,7 +974,7 @@ static int plan_split_tf32(b200_engine *e, const float *src, long long rows, lon
   // a buffer declared constant (weights) is split once; the split is kept until the buffer is
   // released or un-declared, and the caller gets no blocks to hand back
   if (is_constant(e, src)) {
-    if (CachedSplit *c = find_cached(e, src, 0, rows, cols, batch, ld)) {
+    if (CachedSplit *c = find_cached(e, src, 0, rows, cols, batch, ld, slice_stride(batch, batch_stride))) {
       out->p0 = c->hi;
       out->p1 = c->lo;
       out->ld = c->ld_out;
@@ -1002,7 +1005,8 @@ static int plan_split_tf32(b200_engine *e, const float *src, long long rows, lon
 // Once the split has been launched: a constant's is kept, and the blocks are no longer the caller's.
 static void keep_split_tf32(b200_engine *e, const SplitJob &job, void **blk_hi, void **blk_lo) {
   if (!job.src || !is_constant(e, job.src)) return;
-  add_cached(e, job.src, CachedSplit{0, job.rows, job.cols, job.batch, job.ld, *blk_hi, *blk_lo, job.ldo});
+  add_cached(e, job.src, CachedSplit{0, job.rows, job.cols, job.batch, job.ld, *blk_hi, *blk_lo, job.ldo,
+                                   slice_stride(job.batch, job.stride)});
   *blk_hi = *blk_lo = nullptr;
 }
 
@@ -1052,7 +1056,7 @@ static int gemm_f32_tf32(b200_engine *e, bool a_mn, bool b_mn, long long M, long
   if (rc == B200_OK) {
     keep_split_tf32(e, ja, &blk[0], &blk[1]);
     // one matrix as both operands: only one of two equal entries is kept
-    if (!(jb.src && is_constant(e, jb.src) && find_cached(e, jb.src, 0, jb.rows, jb.cols, jb.batch, jb.ld)))
+    if (!(jb.src && is_constant(e, jb.src) && find_cached(e, jb.src, 0, jb.rows, jb.cols, jb.batch, jb.ld, slice_stride(jb.batch, jb.stride))))
       keep_split_tf32(e, jb, &blk[2], &blk[3]);
     rc = gemm_tc_core(e, 3, a_mn, b_mn, M, N, K, a, b, C, ldc, batch, strideC, ep, C_hi, C_lo, ld_split);
   }
@@ -1082,7 +1086,7 @@ static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_r
   int rc = B200_OK;
   const bool constant = is_constant(e, x.src);
   if (constant) {
-    if (CachedSplit *c = find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld)) {
+    if (CachedSplit *c = find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld, slice_stride(x.batch, x.stride))) {
       o->rec = (F16Rec *)c->hi;
       o->op.p1 = c->lo;
     } else {
@@ -1118,8 +1122,9 @@ static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_r
 // Once its split has been launched: a constant's pairs are kept, unless an equal entry (one matrix as both
 // operands) is there already.
 static void keep_split_f16(b200_engine *e, const F32Operand &x, F16Operand *o) {
-  if (!o->kept[0] || find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld)) return;
-  add_cached(e, x.src, CachedSplit{2, x.rows, x.cols, x.batch, x.ld, o->kept[0], o->kept[1], o->op.ld});
+  if (!o->kept[0] || find_cached(e, x.src, 2, x.rows, x.cols, x.batch, x.ld, slice_stride(x.batch, x.stride))) return;
+  add_cached(e, x.src, CachedSplit{2, x.rows, x.cols, x.batch, x.ld, o->kept[0], o->kept[1], o->op.ld,
+                                 slice_stride(x.batch, x.stride)});
   o->kept[0] = o->kept[1] = nullptr;
 }
 

@@ -173,3 +173,17 @@ def test_failed_convolution_leaves_no_trace():
         out.append(y.numpy())
         e.Close()
     util.assert_bits_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("size", [256, 1024])
+def test_constant_read_with_two_strides(fresh, size):
+    # one constant as a batch of slices, as every second one of them, and as one slice for the whole batch (the
+    # sizes take TF32 and fp16 pairs)
+    from gorgonia_b200 import _lib
+    e, n, batch = fresh, size, 4
+    a, b = util.normal(35, (batch, n, n)), util.normal(36, (2 * batch, n, n), scale=0.05)
+    ta, tb, tc = e.tensor(a), e.constant(e.tensor(b)), e.empty((batch, n, n))
+    for step in (1, 2, 0, 1):
+        _lib.check(_lib.lib.b200_gemm(e.h, _lib.F32, 0, 0, n, n, n, ta.ptr, n, tb.ptr, n, tc.ptr, n, batch, n * n,
+                                      step * n * n, n * n, None), e.h)
+        assert_gemm_close(tc.numpy(), _want(a, b[[step * i for i in range(batch)]]), 1e-5)
