@@ -405,6 +405,28 @@ __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float 
       }
     }
   }
+  if (F16 && stats.small) {
+    // Small results, rare: harmless where an input that they were made from is within 2^-21 of the largest (the sum
+    // of magnitudes is then far above what the pairs add), else the place marks the tensor (pairs.cuh). This thread
+    // looks at its places' inputs once more here, and not where it stored the result, for want of registers there.
+    const float least = __uint_as_float(x_rec->amax) * 4.76837158e-7f, floor = act_floor(ACT, alpha);
+    for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g < groups && !stats.bad; g += stride) {
+      const long long b = g / per_image;
+      const int rem = (int)(g - b * per_image);
+      const int ph = rem / Wg, og = rem - ph * Wg;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        float most = 0.f;
+#pragma unroll 1
+        for (int q = 0; q < C * 16; ++q) {
+          const int ih = 2 * ph - 1 + ((q >> 2) & 3), iw = 4 * og + 2 * half - 1 + (q & 3);
+          if ((unsigned)ih < (unsigned)H && (unsigned)iw < (unsigned)W)
+            most = fmaxf(most, fabsf(__ldg(x + ((b * C + (q >> 4)) * H + ih) * (long long)W + iw)));
+        }
+        if (most != 0.f && most * floor < least) stats.bad = 1;
+      }
+    }
+  }
   if (F16) stats.deliver(out16.rec);
 }
 
@@ -466,16 +488,18 @@ __global__ void __launch_bounds__(256) filter_pairs_kernel(const float *__restri
                                                            __half *__restrict__ lo, int C, int taps, F16Filters *f) {
   ptx::grid_begin();
   __shared__ float red[8];
+  __shared__ unsigned red_max[8];
   const int crs = C * taps;
   const float *in = w + (long long)blockIdx.x * crs;
   const int ex = f16_scale_exp(*(volatile const unsigned *)&f->rec.amax);
   const float scale = pow2(ex);
-  unsigned small = 0;
+  unsigned small = 0, largest = 0;
   float sum = 0.f;
   for (int i = threadIdx.x; i < crs; i += 256) {  // consecutive threads: consecutive channels of a tap
     const int tap = i / C, c = i - tap * C;
     const float v = __ldg(in + c * taps + tap);
     sum += fabsf(v);
+    largest = max(largest, __float_as_uint(v) & 0x7FFFFFFFu);
     __half h, l;
     small += f16_pair(v, scale, h, l) ? 1u : 0u;
     hi[(long long)blockIdx.x * crs + i] = h;
@@ -483,11 +507,20 @@ __global__ void __launch_bounds__(256) filter_pairs_kernel(const float *__restri
   }
   if (small) atomicAdd(&f->rec.small, small);
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  largest = __reduce_max_sync(0xffffffffu, largest);
+  if ((threadIdx.x & 31) == 0) {
+    red[threadIdx.x >> 5] = sum;
+    red_max[threadIdx.x >> 5] = largest;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int k = 1; k < 8; ++k) sum += red[k];
+    for (int k = 1; k < 8; ++k) {
+      sum += red[k];
+      largest = max(largest, red_max[k]);
+    }
     atomicMax(&f->l1, __float_as_uint(sum));  // a NaN: above every number
+    // a filter that is small as a whole: its channel of the output would be left with few bits (split.cu)
+    if (largest != 0 && __uint_as_float(largest) * scale < kFullPair) atomicOr(&f->rec.bad, 1u);
     if (blockIdx.x == 0) f->rec.scale_exp = ex;
   }
 }

@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
       if (F16) {
 #pragma unroll
         for (int j = 0; j < HALF; ++j) acc[j] = __fmul_rn(__fmul_rn(acc[j], unscale1), unscale2);
-        finish_channels<HALF>(acc, has_bias ? bias_s[warp - 2] : nullptr, p.ep.act, (float)p.ep.alpha);
+        const float largest = finish_channels<HALF>(acc, has_bias ? bias_s[warp - 2] : nullptr, p.ep.act, (float)p.ep.alpha);
         const int valid = p.K - n0;
         if (m < p.Mtot) {
           if (p.out16.rec) {
@@ -383,7 +383,10 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
             for (int j = 0; j < HALF; ++j)
               if (j < valid) stats.see(acc[j]);
           }
-          if (p.out16.h) store_pairs<HALF>(acc, valid, out_scale, p.out16.h + m * p.K + n0, p.out16.l + m * p.K + n0, stats);
+          if (p.out16.h) {
+            stats.see_place(largest, out_scale);
+            store_pairs<HALF>(acc, valid, out_scale, p.out16.h + m * p.K + n0, p.out16.l + m * p.K + n0, stats);
+          }
           if (yb) {
 #pragma unroll
             for (int j = 0; j < HALF; ++j)
@@ -415,8 +418,18 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
 struct NhwcOut {
   void *hi, *lo;
   F16Rec *rec;         // F16: in: the largest magnitude; out: the exponent used, and the small values
+  unsigned limit;      // F16: how many of these there may be
   const int *only_if;  // TF32: skip_launch
 };
+// F16: n small values of the place whose channels begin at `place` (pairs.cuh). Rare.
+__device__ __noinline__ void nhwc_small(F16Rec *rec, unsigned limit, unsigned n, const float *place, int C, int HW,
+                                        float scale) {
+  if (!f16_count_small(rec, limit, n)) return;
+#pragma unroll 4
+  for (int c = 0; c < C; ++c)
+    if (fabsf(__ldg(place + (long long)c * HW)) * scale >= kFullPair) return;
+  atomicOr(&rec->bad, 1u);
+}
 template <bool F16>
 __device__ __forceinline__ float nhwc_begin(const NhwcOut &out) {
   if (!F16) return 1.f;
@@ -424,14 +437,16 @@ __device__ __forceinline__ float nhwc_begin(const NhwcOut &out) {
   if (blockIdx.x == 0 && threadIdx.x == 0) out.rec->scale_exp = ex;
   return pow2(ex);
 }
-// N (4 or 1) neighbouring channels at element `at`
+// N (4 or 1) neighbouring channels at element `at`; their place's channels begin at x[place]
 template <bool F16, int N>
 __device__ __forceinline__ void nhwc_store(const NhwcOut &out, long long at, const float (&v)[N], float scale,
-                                           unsigned &small) {
+                                           const float *x, long long place, int C, int HW) {
   if (F16) {
     __align__(8) __half h[4], l[4];
+    unsigned small = 0;
 #pragma unroll
     for (int k = 0; k < N; ++k) small += f16_pair(v[k], scale, h[k], l[k]) ? 1u : 0u;
+    if (small) nhwc_small(out.rec, out.limit, small, x + place, C, HW, scale);
     __half *hp = (__half *)out.hi + at, *lp = (__half *)out.lo + at;
     if (N == 4) {
       *reinterpret_cast<uint2 *>(hp) = *reinterpret_cast<const uint2 *>(h);
@@ -467,7 +482,6 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
   ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
-  unsigned small = 0;
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int ptiles = (HW + 31) / 32, ctiles = (C + 31) / 32;
@@ -490,12 +504,11 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
       const int pp = p0 + j, c = c0 + tx;
       if (pp < HW && c < C) {
         const float v[1] = {tile[tx][j]};
-        nhwc_store<F16, 1>(out, ob + (long long)pp * C + c, v, scale, small);
+        nhwc_store<F16, 1>(out, ob + (long long)pp * C + c, v, scale, x, ob + pp, C, HW);
       }
     }
     __syncthreads();
   }
-  if (F16 && small) atomicAdd(&out.rec->small, small);  // rare
 }
 
 // The same rewrite for planes whose size is a multiple of 4 (so every channel row starts on a
@@ -509,7 +522,6 @@ __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restric
   ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
-  unsigned small = 0;
   constexpr int PT = 128, PITCH = PT + 1;
   __shared__ float tile[CT * PITCH];
   const int ptiles = (HW + PT - 1) / PT, ctiles = C / CT;
@@ -539,12 +551,11 @@ __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restric
         float v[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = tile[(4 * cg + k) * PITCH + pp];
-        nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, small);
+        nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, x, b * HW * (long long)C + p0 + pp, C, HW);
       }
     }
     __syncthreads();
   }
-  if (F16 && small) atomicAdd(&out.rec->small, small);
 }
 
 // The same rewrite for small planes of any size (7x7, 13x13): a block takes 32 channels of one
@@ -557,7 +568,6 @@ __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__rest
   ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
-  unsigned small = 0;
   extern __shared__ __align__(16) float img[];
   const int chunks = C >> 5;
   const long long total = B * chunks;
@@ -583,11 +593,10 @@ __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__rest
       float v[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) v[k] = img[(4 * cg + k) * pitch + pp];
-      nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, small);
+      nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, x, b * HW * (long long)C + pp, C, HW);
     }
     __syncthreads();
   }
-  if (F16 && small) atomicAdd(&out.rec->small, small);
 }
 
 // Rewrites x (B, C, HW) as NHWC TF32 head/tail into two fresh arena blocks xs[0], xs[1], which the
@@ -626,17 +635,17 @@ int conv_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, 
   int rc = b200_get(e, xbytes, &xs[0]);
   if (rc == B200_OK) rc = b200_get(e, xbytes, &xs[1]);
   if (rc != B200_OK) return rc;
-  return launch_nhwc_split<false>(e, x, B, C, HW, NhwcOut{xs[0], xs[1], nullptr, e->only_if});
+  return launch_nhwc_split<false>(e, x, B, C, HW, NhwcOut{xs[0], xs[1], nullptr, 0, e->only_if});
 }
 
 // The same rewrite into buffers the caller owns (B * C * HW floats each).
 int conv_nhwc_split_into(b200_engine *e, const float *x, long long B, int C, int HW, float *hi, float *lo) {
-  return launch_nhwc_split<false>(e, x, B, C, HW, NhwcOut{hi, lo, nullptr, nullptr});
+  return launch_nhwc_split<false>(e, x, B, C, HW, NhwcOut{hi, lo, nullptr, 0, nullptr});
 }
 
 // As pairs of fp16: heads, then tails, from `pairs` on. rec holds the largest magnitude of x.
 int conv_nhwc_pairs(b200_engine *e, const float *x, long long B, int C, int HW, __half *pairs, F16Rec *rec) {
-  return launch_nhwc_split<true>(e, x, B, C, HW, NhwcOut{pairs, pairs + B * C * HW, rec, nullptr});
+  return launch_nhwc_split<true>(e, x, B, C, HW, NhwcOut{pairs, pairs + B * C * HW, rec, f16_small_limit(B * C * HW), nullptr});
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

@@ -427,14 +427,17 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
         const int qh = p.pool2 ? oh >> 1 : oh, qw = p.pool2 ? ow >> 1 : ow;
         const long long plane = (long long)Hq * Wq;
         const long long pos = inside ? ((long long)b * Hq + qh) * Wq + qw : 0;
+        float largest = 0.f;  // of the sums in front of the activation
         auto store = [&](float *v, int c0, auto size) {  // channels from column c0 of this tile on
           constexpr int N = decltype(size)::value;
           const int valid = p.K - n0 - c0;
 #pragma unroll
           for (int j = 0; j < N; ++j)
             if (j < valid) stats.see(v[j]);
-          if (p.out16.h)
+          if (p.out16.h) {
+            stats.see_place(largest, out_scale);
             store_pairs<N>(v, valid, out_scale, p.out16.h + pos * p.K + n0 + c0, p.out16.l + pos * p.K + n0 + c0, stats);
+          }
           if (p.y) {
             float *yb = p.y + ((long long)b * p.K + n0 + c0) * plane + (long long)qh * Wq + qw;
 #pragma unroll
@@ -448,14 +451,14 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
           // finite are marked for the way behind this one
           float q[BN / 4];
           const bool b0 = (lane & 1) != 0, b1 = (lane & 8) != 0;
-          if (p.ep.act == B200_ACT_LEAKY && !((float)p.ep.alpha >= 0.f)) finish_channels<BN>(acc, bias_w, p.ep.act, (float)p.ep.alpha);
+          if (p.ep.act == B200_ACT_LEAKY && !((float)p.ep.alpha >= 0.f)) largest = finish_channels<BN>(acc, bias_w, p.ep.act, (float)p.ep.alpha);
           pool4_exchange<BN>(acc, q);
           const int c0 = (b0 ? BN / 2 : 0) + (b1 ? BN / 4 : 0);
           if (!(p.ep.act == B200_ACT_LEAKY && !((float)p.ep.alpha >= 0.f)))
-            finish_channels<BN / 4>(q, bias_w ? bias_w + c0 : nullptr, p.ep.act, (float)p.ep.alpha);
+            largest = finish_channels<BN / 4>(q, bias_w ? bias_w + c0 : nullptr, p.ep.act, (float)p.ep.alpha);
           if (inside) store(q, c0, std::integral_constant<int, BN / 4>());
         } else {
-          finish_channels<BN>(acc, bias_w, p.ep.act, (float)p.ep.alpha);
+          largest = finish_channels<BN>(acc, bias_w, p.ep.act, (float)p.ep.alpha);
           if (inside) store(acc, 0, std::integral_constant<int, BN>());
         }
       } else if (p.pool2) {

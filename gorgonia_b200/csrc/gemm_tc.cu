@@ -1078,7 +1078,9 @@ struct F16Operand {
 // Finds a constant's pairs or takes room for an operand's. Nothing is launched and nothing kept here: what was
 // taken is the caller's to hand back, also after an error.
 // The blocks are as large as the TF32 pairs need, which take their place if the fp16 pairs turn out unusable.
-static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_rec, F16Operand *o) {
+// along_rows: the product sums along the rows as they are stored (else down the columns). A constant's pairs are
+// kept for products of either kind.
+static int plan_split_f16(b200_engine *e, const F32Operand &x, bool along_rows, F16Rec *scratch_rec, F16Operand *o) {
   const long long ldo = (x.cols + 7) / 8 * 8, elems = x.rows * ldo * x.batch;
   o->op.ld = ldo;
   o->op.batch_stride = x.rows * ldo;
@@ -1116,6 +1118,8 @@ static int plan_split_f16(b200_engine *e, const F32Operand &x, F16Rec *scratch_r
   o->job.lo = const_cast<void *>(o->op.p1);
   o->job.ldo = ldo;
   o->job.rec = o->rec;
+  o->job.limit = f16_small_limit(x.rows * x.cols * x.batch);
+  o->job.lines = constant ? kLineRows | kLineCols : (along_rows ? kLineRows : kLineCols);
   return B200_OK;
 }
 
@@ -1146,12 +1150,12 @@ static int gemm_f32_f16(b200_engine *e, bool a_mn, bool b_mn, long long M, long 
   F16Operand a, b;
   const F32Operand *xs[2] = {&A, &B};
   F16Operand *ops[2] = {&a, &b};
-  int rc = plan_split_f16(e, A, e->f16_recs, &a);
-  if (rc == B200_OK) rc = plan_split_f16(e, B, e->f16_recs + 1, &b);
+  int rc = plan_split_f16(e, A, !a_mn, e->f16_recs, &a);
+  if (rc == B200_OK) rc = plan_split_f16(e, B, !b_mn, e->f16_recs + 1, &b);
   for (F16Operand *o : ops)
     if (rc == B200_OK && o->kept[0] && cudaMemsetAsync(o->rec, 0, sizeof(F16Rec), e->stream) != cudaSuccess)
       rc = set_error(e, B200_ERR_CUDA, "b200_gemm: clearing a record failed");
-  const unsigned la = f16_small_limit(A.rows * A.cols * A.batch), lb = f16_small_limit(B.rows * B.cols * B.batch);
+  const unsigned la = a.job.limit, lb = b.job.limit;
   if (rc == B200_OK && a.job.src) rc = launch_split_f16(e, a.job, b.job);
   else if (rc == B200_OK && b.job.src) rc = launch_split_f16(e, b.job, SplitJob());
   if (rc == B200_OK)

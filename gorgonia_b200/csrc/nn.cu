@@ -158,13 +158,16 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
 #pragma unroll
     for (int j = ty; j < 32; j += 8) {
       const int q = p0 + j, c = c0 + tx;
+      bool small = false, full = false;
       if (q < HWo && c < C) {
         const float v = tile[tx][j];
         const long long o = ob + (long long)q * C + c;
         if (F16) {
           __half hh, ll;
           stats.see(v);
-          stats.small += f16_pair(v, scale, hh, ll) ? 1u : 0u;
+          small = f16_pair(v, scale, hh, ll);
+          full = fabsf(v * scale) >= kFullPair;
+          stats.small += small ? 1u : 0u;
           if (!(fabsf(v * scale) <= 65504.f)) stats.bad = 1;
           out16.h[o] = hh;
           out16.l[o] = ll;
@@ -174,6 +177,8 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
           lo[o] = pool_tf32(__fsub_rn(v, h));
         }
       }
+      // the warp has 32 channels of one place: small ones and none of full range mark the tensor (pairs.cuh)
+      if (F16 && __any_sync(0xffffffffu, small) && !__any_sync(0xffffffffu, full)) stats.bad = 1;
     }
     __syncthreads();
   }

@@ -6,6 +6,12 @@
 // bound: largest input x largest sum of magnitudes of a filter + largest bias. For sums of a few thousand
 // products that is 2^6 to 2^8 above what occurs, which leaves results down to 2^-21 of the largest with full
 // pairs. The largest result that did occur is recorded for the next link's bound.
+//
+// Small values (split.cu) beside an ordinary one at the same place of an image are harmless: the sums they enter
+// hold that one too, and they came about by cancellation, with an error above what the pair adds. A place where
+// every channel is small is a place whose inputs are, and would be the whole of what some outputs of the next link
+// are made from, so one such place marks the tensor. Epilogues look at the sums in front of the activation
+// (Rectify leaves zeros that say nothing), in the eight or more channels that a thread has at a place.
 #pragma once
 #include "epilogue.cuh"
 #include "split.h"
@@ -60,6 +66,10 @@ struct PairStats {
     const unsigned m = __float_as_uint(v) & 0x7FFFFFFFu;
     amax = amax > m ? amax : m;
   }
+  // the largest magnitude among a place's channels, in front of the activation
+  __device__ __forceinline__ void see_place(float largest, float scale) {
+    if (largest != 0.f && largest * scale < kFullPair) bad = 1;
+  }
   // by whole warps, once
   __device__ __forceinline__ void deliver(F16Rec *rec) {
     const unsigned a = __reduce_max_sync(0xffffffffu, amax), s = __reduce_add_sync(0xffffffffu, small);
@@ -92,13 +102,21 @@ __device__ __forceinline__ void store_pairs(const float *v, int valid, float sca
   }
 }
 
-// acc -> act(acc + bias), the activation chosen outside the loop
+// What an activation leaves at least of a magnitude, unless it leaves nothing.
+__device__ __forceinline__ float act_floor(int act, float alpha) {
+  return act == B200_ACT_LEAKY && alpha != 0.f ? fminf(1.f, fabsf(alpha)) : 1.f;
+}
+// acc -> act(acc + bias), the activation chosen outside the loop. Returns the largest magnitude in front of it, by
+// what the activation leaves of it at least (see_place).
 template <int N>
-__device__ __forceinline__ void finish_channels(float (&acc)[N], const float *bias, int act, float alpha) {
+__device__ __forceinline__ float finish_channels(float (&acc)[N], const float *bias, int act, float alpha) {
   if (bias) {
 #pragma unroll
     for (int j = 0; j < N; ++j) acc[j] = __fadd_rn(acc[j], bias[j]);
   }
+  float largest = 0.f;
+#pragma unroll
+  for (int j = 0; j < N; ++j) largest = fmaxf(largest, fabsf(acc[j]));
   if (act == B200_ACT_RECTIFY) {
 #pragma unroll
     for (int j = 0; j < N; ++j) acc[j] = apply_act<float>(acc[j], B200_ACT_RECTIFY, alpha);
@@ -106,6 +124,7 @@ __device__ __forceinline__ void finish_channels(float (&acc)[N], const float *bi
 #pragma unroll
     for (int j = 0; j < N; ++j) acc[j] = apply_act<float>(acc[j], B200_ACT_LEAKY, alpha);
   }
+  return largest * act_floor(act, alpha);
 }
 #endif
 

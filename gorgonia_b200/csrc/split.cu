@@ -5,12 +5,15 @@
 // fp16 pairs: the whole operand is scaled by the power of two that brings its largest magnitude into
 // [2^14, 2^15); then x * 2^e = head + tail * 2^-11 with head = fp16(x * 2^e) and tail = fp16 of the (exact)
 // remainder times 2^11. fp16 has the 11 significant bits of TF32, so the pair carries x as closely as the
-// TF32 pair does, in half the bytes and at twice the tensor-core rate. What fp16 lacks is range: a value
-// below 2^-14 after scaling (2^-29 of the largest) keeps an absolute error of 2^-36 instead of a relative
-// one. Such values are counted, and infinities and NaNs are noted, in the operand's F16Rec. A product whose
-// operands hold more than n / 65536 of them, or any infinity or NaN, is made from TF32 pairs instead: the
-// kernels of both ways are launched, and one of them returns at once (the host never waits to find out).
-// N(0, 1) draws hold about one such value in 10^8.
+// TF32 pair does, in half the bytes and at twice the tensor-core rate. What fp16 lacks is range: a small
+// value, below 2^-14 after scaling (2^-29 of the largest), keeps an absolute error of 2^-36 instead of a
+// relative one. Beside a value of the full range in the same sum that is no more than that one's rounding
+// (2^-22 of at least 2^-14); where every value along k is small, a whole row or column of the product would
+// lose its bits. Small values are therefore counted in the operand's F16Rec, which also notes infinities and
+// NaNs, and each of them looks for a value of full range in its line along k. A product whose operands hold
+// more than n / 65536 small values, one that is alone, an infinity or a NaN, is made from TF32 pairs instead:
+// the kernels of both ways are launched, and one of them returns at once (the host never waits to find out).
+// N(0, 1) draws hold about one small value in 10^8, and its neighbour is an ordinary one: looking costs nothing.
 //
 // All of these passes are bound by HBM: 4 bytes read and 4 (fp16) or 8 (TF32) written per value. A thread
 // takes eight (four) neighbouring columns, 16 bytes per store; both operands of a product share a launch.
@@ -37,6 +40,53 @@ __device__ __forceinline__ float split_tf32(float x) {
   uint32_t r;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return __uint_as_float(r);
+}
+
+// Whether the line through element (row, col) of a slice holds a value of full range among the kLineReach
+// nearest after it (the line taken as a ring). By a whole warp.
+constexpr int kLineReach = 4096;
+__device__ bool line_has_full(const float *first, long long step, long long len, long long at, float scale) {
+  const int lane = threadIdx.x & 31;
+  const long long reach = len < kLineReach ? len : kLineReach;
+  for (long long o = 0; o < reach; o += 128) {
+    bool full = false;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long d = o + q * 32 + lane;
+      if (d < reach) {
+        const long long i = at + d < len ? at + d : at + d - len;
+        full |= fabsf(__ldg(first + i * step)) * scale >= kFullPair;
+      }
+    }
+    if (__any_sync(0xffffffffu, full)) return true;
+  }
+  return false;
+}
+
+// The rare end of SPLIT_F16's step: `mine` marks the small ones of this lane's eight values, which begin at
+// column c0 of row r of the slice at `slice`. By a whole warp.
+__device__ __noinline__ void note_small(const SplitJob &j, unsigned mine, const float *slice, long long r, long long c0,
+                                        float scale) {
+  const int lane = threadIdx.x & 31;
+  const unsigned n = __reduce_add_sync(0xffffffffu, (unsigned)__popc(mine));
+  bool look = false;
+  if (lane == 0) look = f16_count_small(j.rec, j.limit, n);
+  if (!__shfl_sync(0xffffffffu, look, 0)) return;
+  for (unsigned lanes = __ballot_sync(0xffffffffu, mine != 0); lanes; lanes &= lanes - 1) {
+    const int src = __ffs(lanes) - 1;
+    const long long lr = __shfl_sync(0xffffffffu, r, src), lc0 = __shfl_sync(0xffffffffu, c0, src);
+    const float *ls = (const float *)__shfl_sync(0xffffffffu, (unsigned long long)slice, src);
+    for (unsigned m = __shfl_sync(0xffffffffu, mine, src); m; m &= m - 1) {
+      const long long lc = lc0 + __ffs(m) - 1;
+      bool alone = false;
+      if (j.lines & kLineRows) alone = !line_has_full(ls + lr * j.ld, 1, j.cols, lc, scale);
+      if (!alone && (j.lines & kLineCols)) alone = !line_has_full(ls + lc, j.ld, j.rows, lr, scale);
+      if (alone) {
+        if (lane == 0) atomicOr(&j.rec->bad, 1u);
+        return;
+      }
+    }
+  }
 }
 
 template <int MODE>
@@ -69,60 +119,66 @@ __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ Spli
     scale = pow2(ex);
     if (blk == 0 && threadIdx.x == 0) j.rec->scale_exp = ex;
   }
-  unsigned amax = 0, bad = 0;  // SPLIT_F16: `bad` counts the small values
-  for (long long t = (long long)blk * 256 + threadIdx.x; t < total; t += (long long)nblk * 256) {
-    long long row, g, b, r;
-    if (narrow) {
-      const uint32_t rr = (uint32_t)t / (uint32_t)per_row, bb = rr / (uint32_t)rows;
-      row = rr;
-      g = (uint32_t)t - rr * (uint32_t)per_row;
-      b = bb;
-      r = rr - bb * (uint32_t)rows;
-    } else {
-      row = t / per_row;
-      g = t - row * per_row;
-      b = row / rows;
-      r = row - b * rows;
-    }
-    const long long c0 = g * V;
-    const float *p = src + b * stride + r * ld + c0;
-    float x[V];
-    if (vec && c0 + V <= cols) {
-#pragma unroll
-      for (int q = 0; q < V / 4; ++q) {
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(p) + q);
-        x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+  unsigned amax = 0, bad = 0;
+  // SPLIT_F16: warps stay whole for note_small
+  const long long lane_off = MODE == SPLIT_F16 ? threadIdx.x & 31 : 0;
+  for (long long t = (long long)blk * 256 + threadIdx.x; t - lane_off < total; t += (long long)nblk * 256) {
+    unsigned small = 0;
+    const float *slice = nullptr;
+    long long r = 0, c0 = 0;
+    if (MODE != SPLIT_F16 || t < total) {
+      long long row, g, b;
+      if (narrow) {
+        const uint32_t rr = (uint32_t)t / (uint32_t)per_row, bb = rr / (uint32_t)rows;
+        row = rr;
+        g = (uint32_t)t - rr * (uint32_t)per_row;
+        b = bb;
+        r = rr - bb * (uint32_t)rows;
+      } else {
+        row = t / per_row;
+        g = t - row * per_row;
+        b = row / rows;
+        r = row - b * rows;
       }
-    } else {
+      c0 = g * V;
+      slice = src + b * stride;
+      const float *p = slice + r * ld + c0;
+      float x[V];
+      if (vec && c0 + V <= cols) {
 #pragma unroll
-      for (int q = 0; q < V; ++q) x[q] = c0 + q < cols ? __ldg(p + q) : 0.f;
-    }
-    if (MODE == SPLIT_AMAX) {
+        for (int q = 0; q < V / 4; ++q) {
+          const float4 v = __ldg(reinterpret_cast<const float4 *>(p) + q);
+          x[4 * q] = v.x; x[4 * q + 1] = v.y; x[4 * q + 2] = v.z; x[4 * q + 3] = v.w;
+        }
+      } else {
 #pragma unroll
-      for (int q = 0; q < V; ++q) {
-        const unsigned m = __float_as_uint(x[q]) & 0x7FFFFFFFu;
-        if (m >= 0x7F800000u) bad = 1;
-        else amax = amax > m ? amax : m;
+        for (int q = 0; q < V; ++q) x[q] = c0 + q < cols ? __ldg(p + q) : 0.f;
       }
-    } else if (MODE == SPLIT_F16) {
-      __align__(16) __half h[V], l[V];
+      if (MODE == SPLIT_AMAX) {
 #pragma unroll
-      for (int q = 0; q < V; ++q) bad += f16_pair(x[q], scale, h[q], l[q]) ? 1u : 0u;
-      reinterpret_cast<uint4 *>(j.hi)[t] = *reinterpret_cast<const uint4 *>(h);
-      reinterpret_cast<uint4 *>(j.lo)[t] = *reinterpret_cast<const uint4 *>(l);
-    } else {
-      float h[4], l[4];
+        for (int q = 0; q < V; ++q) {
+          const unsigned m = __float_as_uint(x[q]) & 0x7FFFFFFFu;
+          if (m >= 0x7F800000u) bad = 1;
+          else amax = amax > m ? amax : m;
+        }
+      } else if (MODE == SPLIT_F16) {
+        __align__(16) __half h[V], l[V];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        h[q] = split_tf32(x[q]);
-        l[q] = split_tf32(__fsub_rn(x[q], h[q]));
+        for (int q = 0; q < V; ++q) small |= f16_pair(x[q], scale, h[q], l[q]) ? 1u << q : 0u;
+        reinterpret_cast<uint4 *>(j.hi)[t] = *reinterpret_cast<const uint4 *>(h);
+        reinterpret_cast<uint4 *>(j.lo)[t] = *reinterpret_cast<const uint4 *>(l);
+      } else {
+        float h[4], l[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          h[q] = split_tf32(x[q]);
+          l[q] = split_tf32(__fsub_rn(x[q], h[q]));
+        }
+        reinterpret_cast<float4 *>(j.hi)[t] = make_float4(h[0], h[1], h[2], h[3]);
+        reinterpret_cast<float4 *>(j.lo)[t] = make_float4(l[0], l[1], l[2], l[3]);
       }
-      reinterpret_cast<float4 *>(j.hi)[t] = make_float4(h[0], h[1], h[2], h[3]);
-      reinterpret_cast<float4 *>(j.lo)[t] = make_float4(l[0], l[1], l[2], l[3]);
     }
-  }
-  if (MODE == SPLIT_F16) {
-    if (bad) atomicAdd(&j.rec->small, bad);  // rare
+    if (MODE == SPLIT_F16 && __any_sync(0xffffffffu, small != 0)) note_small(j, small, slice, r, c0, scale);
   }
   if (MODE == SPLIT_AMAX) {
     amax = __reduce_max_sync(0xffffffffu, amax);

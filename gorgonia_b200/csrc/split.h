@@ -14,7 +14,7 @@ namespace b200 {
 struct F16Rec {
   unsigned amax;   // bits of the largest magnitude among the finite values
   unsigned small;  // values that are too small for a full pair (nonzero, below 2^-14 after scaling)
-  unsigned bad;    // nonzero: an infinity or NaN is among the values
+  unsigned bad;    // nonzero: an infinity or NaN is among the values, or a line of small values (split.cu)
   int scale_exp;   // the values were scaled by 2^scale_exp
 };
 // A tensor of n values may hold this many that are too small for a full pair.
@@ -28,8 +28,12 @@ struct SplitJob {
   long long ld = 0, stride = 0, rows = 0, cols = 0, batch = 0;
   void *hi = nullptr, *lo = nullptr;
   long long ldo = 0;
-  F16Rec *rec = nullptr;  // fp16 pairs only
+  // fp16 pairs only: the record, how many small values it allows, and along what they are summed
+  F16Rec *rec = nullptr;
+  unsigned limit = 0;
+  unsigned lines = 0;  // kLineRows and / or kLineCols
 };
+constexpr unsigned kLineRows = 1, kLineCols = 2;
 
 // Each takes one or two operands in one launch (b.src == null: one).
 int launch_split_tf32(b200_engine *e, const SplitJob &a, const SplitJob &b);
@@ -68,12 +72,19 @@ __device__ __forceinline__ void f16_unscale(int exp_a, int exp_b, float &s1, flo
 __device__ __forceinline__ bool f16_unusable(const F16Rec *r, unsigned limit) {
   return *(volatile const unsigned *)&r->bad != 0 || *(volatile const unsigned *)&r->small > limit;
 }
+constexpr float kFullPair = 6.103515625e-05f;  // 2^-14, fp16's smallest normal number
 // x * 2^e -> head and tail; true if the value is too small for a full pair
 __device__ __forceinline__ bool f16_pair(float x, float scale, __half &h, __half &l) {
   const float xs = x * scale;
   h = __float2half_rn(xs);
   l = __float2half_rn((xs - __half2float(h)) * 2048.f);
-  return x != 0.f && fabsf(xs) < 6.103515625e-05f;
+  return x != 0.f && fabsf(xs) < kFullPair;
+}
+// n small values more. Whether it is still worth looking what they lie among: not once the record says that
+// the tensor is unusable.
+__device__ __forceinline__ bool f16_count_small(F16Rec *r, unsigned limit, unsigned n) {
+  if (f16_unusable(r, limit)) return false;
+  return atomicAdd(&r->small, n) + n <= limit;
 }
 #endif
 

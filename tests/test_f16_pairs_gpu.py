@@ -187,3 +187,59 @@ def test_constant_read_with_two_strides(fresh, size):
         _lib.check(_lib.lib.b200_gemm(e.h, _lib.F32, 0, 0, n, n, n, ta.ptr, n, tb.ptr, n, tc.ptr, n, batch, n * n,
                                       step * n * n, n * n, None), e.h)
         assert_gemm_close(tc.numpy(), _want(a, b[[step * i for i in range(batch)]]), 1e-5)
+
+
+@pytest.mark.parametrize("tiny", [1e-14, 1e-16])
+@pytest.mark.parametrize("count", [1, 64])
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, True)])
+def test_small_values_that_are_alone_in_their_line(fresh, count, tiny, transA, transB):
+    # a diagonal factor of ones and a few tiny entries: each of these is the largest of its row and column
+    n = 2048
+    diag = np.ones(n, np.float32)
+    diag[np.linspace(0, n - 1, count).astype(int)] = np.float32(tiny)
+    d, x = np.diag(diag), util.normal(21, (n, n))
+    for a, b in ((d, x), (x, d)):
+        want = _want(a, b, transA, transB)
+        got = _product(fresh, a, b, transA, transB)
+        for axis in (0, 1):
+            assert (np.linalg.norm(got - want, axis=axis) / np.linalg.norm(want, axis=axis)).max() < 1e-6
+
+
+def test_small_row_of_a_tall_matrix(fresh):
+    # one row in 131072 far below the others: fewer values than a 65536th of the matrix
+    e, M, n = fresh, 131072, 1024
+    a, b = util.normal(22, (M, n)), util.normal(23, (n, n), scale=0.05)
+    rows = [0, 77_777, M - 1]
+    a[77_777] *= np.float32(1e-20)
+    want = _want(a[rows], b)
+    ta, tb, tc = e.tensor(a), e.tensor(b), e.empty((M, n))
+    e.MatMul(ta, tb, tc)
+    got = tc.numpy()[rows]
+    assert (np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)).max() < 1e-6
+
+
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True), (True, True)])
+def test_small_values_among_ordinary_ones_stay_with_fp16(fresh, transA, transB):
+    # harmless along k: no line is made of them, and the product is made once
+    e, n = fresh, 2048
+    a, b = util.normal(24, (n, n)), util.normal(25, (n, n), scale=0.02)
+    for k in range(60):
+        a[(31 * k) % n, (57 * k) % n] = np.float32(1e-13)
+        b[(17 * k) % n, (91 * k) % n] = np.float32(1e-15)
+    want = _want(a, b, transA, transB)
+    assert_gemm_close(_product(e, a, b, transA, transB), want, 1e-5)
+    # the word behind the two records says whether the product was made over
+    ta, tb, tc = e.tensor(a), e.tensor(b), e.empty((n, n))
+    fp16, tf32 = [], []
+    for spread in (False, True):
+        if spread:
+            ta.set(a * (10.0 ** np.linspace(0, 20, n)).astype(np.float32)[:, None])
+        ev = [e.event() for _ in range(2)]
+        for _ in range(3):
+            e.MatMul(ta, tb, tc, transA, transB)
+        e.record(ev[0])
+        for _ in range(20):
+            e.MatMul(ta, tb, tc, transA, transB)
+        e.record(ev[1])
+        (tf32 if spread else fp16).append(e.elapsed_ms(*ev))
+    assert fp16[0] < 0.8 * tf32[0]

@@ -236,3 +236,135 @@ def test_failed_chain_leaves_its_records_clear(fresh, monkeypatch, make):
     assert not m.records.buf.numpy()[:-4].any()
     m.x.set(x)
     assert_bits_equal(m.forward().numpy(), want)
+
+
+# ---- values that are small but alone ---------------------------------------------------------------------------------
+BIG = [(48, 128, 26, 26, 256, 3, 1), (96, 64, 32, 32, 128, 5, 2)]     # the im2col and the window kernel, 19 GFLOP and more
+
+
+def _conv64(x, w, pad):
+    import torch
+    y = torch.nn.functional.conv2d(torch.from_numpy(x).cuda().double(), torch.from_numpy(w).cuda().double(), padding=pad)
+    return y.cpu().numpy()
+
+
+@pytest.mark.parametrize("case", BIG)
+def test_large_single_convolutions_are_made_from_pairs(fresh, case):
+    # ordinary values, to float64; constant filters, whose pairs are kept from the first call on, so that the second
+    # launches the magnitude, the rewrite, the convolution and the check, and two of TF32 that find nothing to do
+    e = fresh
+    B, C, H, W, K, k, pad = case
+    x, w = util.normal(91, (B, C, H, W)), util.normal(92, (K, C, k, k), scale=0.05)
+    want = _conv64(x, w, pad)
+    tx, tw, y = e.tensor(x), e.tensor(w), e.empty(want.shape)
+    e.Conv2d(tx, tw, y, pad=(pad, pad))
+    assert_gemm_close(y.numpy(), want, 1e-5)
+    e.constant(tw)
+    for _ in range(2):
+        before = e.launches
+        e.Conv2d(tx, tw, y, pad=(pad, pad))
+        made = e.launches - before
+    assert made == 6
+    assert_gemm_close(y.numpy(), want, 1e-5)
+    # a sprinkling of small values among ordinary ones changes nothing of that
+    x.reshape(-1)[::x.size // 50] = np.float32(1e-13)
+    tx.set(x)
+    e.Conv2d(tx, tw, y, pad=(pad, pad))
+    assert_gemm_close(y.numpy(), _conv64(x, w, pad), 1e-5)
+
+
+@pytest.mark.parametrize("case", BIG)
+@pytest.mark.parametrize("where", ["filter", "pixel", "corner"])
+def test_small_values_alone_in_a_window_or_a_filter(fresh, case, where):
+    # fewer of them than the allowance: a filter of one tap, an image of a few pixels
+    e = fresh
+    B, C, H, W, K, k, pad = case
+    x, w = util.normal(93, (B, C, H, W)), util.normal(94, (K, C, k, k), scale=0.05)
+    if where == "filter":
+        w[5] = 0.0
+        w[5, 0, 1, 1] = np.float32(1e-15)
+        part = (slice(None), 5)
+    else:
+        x[1] = 0.0
+        if where == "pixel":
+            x[1, :20, 9, 7] = util.normal(95, 20) * np.float32(1e-14)
+        else:
+            x[1, C - 1, H - 1, W - 1] = np.float32(1e-16)
+        part = (1,)
+    want = _conv64(x, w, pad)
+    y = e.empty(want.shape)
+    e.Conv2d(e.tensor(x), e.tensor(w), y, pad=(pad, pad))
+    got = y.numpy()
+    assert_gemm_close(got, want, 1e-5)
+    assert np.linalg.norm(got[part] - want[part]) <= 2e-6 * np.linalg.norm(want[part])
+
+
+@pytest.mark.parametrize("case", [c for c in LINKS if c[4] % 8 == 0 and c[0] > 1])
+def test_link_marks_a_place_where_every_channel_is_small(fresh, case):
+    # the input is within range, the output's pairs (scaled by a bound) are not where all channels are small
+    e = fresh
+    B, C, H, W, K, k, pad, act, alpha, pool = case
+    x = util.normal(96, (B, C, H, W))
+    w = util.normal(97, (K, C, k, k), scale=0.05)
+    marks = []
+    for far in (False, True):
+        z = x.copy()
+        if far:
+            z[1, :, H // 2 - k:H // 2 + k, W // 2 - k:W // 2 + k] *= np.float32(2.0 ** -26)
+        tx, rx = _pairs(e, z)
+        Ho, Wo = H + 2 * pad - k + 1, W + 2 * pad - k + 1
+        shape = (B, K, Ho // 2, Wo // 2) if pool else (B, K, Ho, Wo)
+        ry, yp = e.tensor(np.zeros(4, np.int32)), e.empty((int(np.prod(shape)),))
+        e.Conv2dPairs(None, e.tensor(w), None, x.shape, rx.ptr, ry.ptr, pad=(pad, pad), act=act, alpha=alpha, pool2=pool,
+                      x_pairs=tx, y_pairs=yp)
+        marks.append(int(ry.numpy()[2]))
+    assert marks == [0, 1]
+
+
+def test_first_link_and_pool_mark_small_places(fresh):
+    e = fresh
+    w = util.normal(98, (16, 1, 3, 3), scale=0.3)
+    for far in (False, True):
+        x = util.uniform(99, (3, 1, 28, 28)) + np.float32(0.1)
+        x[1, :, 20:] = 0.0      # nothing at all is not small
+        if far:
+            x[1, 0, 24, 13] = np.float32(1e-12)
+        recs, yp = e.tensor(np.zeros(8, np.int32)), e.empty((3 * 16 * 14 * 14,))
+        tx = e.tensor(x)
+        e.pairs_magnitude(tx, recs.ptr)
+        e.Conv2dPairs(tx, e.tensor(w), None, x.shape, recs.ptr, recs.ptr + 16, pad=(1, 1), act="rectify", pool2=True,
+                      y_pairs=yp)
+        assert recs.numpy()[6] == (1 if far else 0)
+        z = util.normal(100, (2, 40, 12, 12))
+        z[:, :, 4:6, 4:6] = 0.0
+        if far:
+            z[1, 3, 4, 5] = np.float32(1e-12)
+        rz, ry = e.tensor(np.array([np.abs(z).max().view(np.int32), 0, 0, 0], np.int32)), e.tensor(np.zeros(4, np.int32))
+        e.MaxPool2DPairs(e.tensor(z), rz.ptr, e.empty((2 * 40 * 36,)), ry.ptr, (2, 2), (0, 0), (2, 2))
+        assert ry.numpy()[2] == (1 if far else 0)
+
+
+def test_dark_image_of_a_large_batch(fresh):
+    # one image in 8192 holds a single pixel of 1e-13: too few small values for the allowance at any link
+    from gorgonia_b200 import Engine
+    B = 8192
+    x = util.uniform(101, (B, 1, 28, 28))
+    x[7] = 0.0
+    x[7, 0, 13, 13] = np.float32(1e-13)
+    pooled, redo = [], []
+    for flops in (0, 1e30):
+        e = Engine(0, 4 << 30)
+        with pytest.MonkeyPatch.context() as mp:
+            m = _lenet(e, mp, flops, B)
+        m.x.set(x)
+        m.forward()
+        a = m.chain.layers[-1]
+        pooled.append((a["pooled"] or a["y"]).numpy()[7])
+        if m.records is not None:
+            redo.append(int(m.records.buf.numpy()[-4]))
+            m.x.set(util.uniform(102, x.shape))
+            m.forward()
+            redo.append(int(m.records.buf.numpy()[-4]))
+        e.Close()
+    assert np.linalg.norm(pooled[0] - pooled[1]) <= 4e-6 * np.linalg.norm(pooled[1])
+    assert redo == [1, 0]
