@@ -943,13 +943,16 @@ int b200_pairs_check(b200_engine *e, void *recs, const int64_t *counts, int k, i
 int b200_only_if(b200_engine *e, const int *flag) {
   if (!e) return B200_ERR_INVALID;
   std::lock_guard<std::recursive_mutex> lk(e->mu);
-  if (flag) {
-    B200_REQUIRE(e, !e->only_if, "b200_only_if: already in effect");
-    DeviceGuard g(e);
-    int rc = flush_pending(e);
-    if (rc != B200_OK) return rc;
+  const std::thread::id me = std::this_thread::get_id();
+  if (!flag) {
+    e->only_if_of.erase(me);
+    return B200_OK;
   }
-  e->only_if = flag;
+  B200_REQUIRE(e, !only_if_word(e), "b200_only_if: already in effect");
+  DeviceGuard g(e);
+  int rc = flush_pending(e);
+  if (rc != B200_OK) return rc;
+  e->only_if_of[me] = flag;
   return B200_OK;
 }
 

@@ -9,6 +9,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -68,10 +69,12 @@ struct b200_engine {
   // Records of the operands that a float32 product splits into pairs of fp16 (split.h): two for the
   // operands, zero between products, and a word that says whether the product has to be made over.
   b200::F16Rec *f16_recs = nullptr;
-  // While set, launches run only if the device word it names is not zero (b200_only_if): the way that stands
-  // behind one of fp16 pairs. Only entry points that say so can be called then (allow_only_if, flush_pending).
+  // The device words that threads have named with b200_only_if: the launches each of them makes run only if its
+  // word is not zero (the way that stands behind one of fp16 pairs). Only entry points that say so can be called
+  // by such a thread (OnlyIfAllowed, flush_pending); other threads' calls are as ever.
+  std::map<std::thread::id, const int *> only_if_of;
+  // What the launches of the call in progress are made under.
   const int *only_if = nullptr;
-  bool allow_only_if = false;
 
   // lazily created resources of other translation units (gemm.cu etc.)
   void *gemm_state = nullptr;
@@ -188,11 +191,18 @@ void arena_release(b200_engine *e, int64_t off);
 // Called with a derived form that a launch is about to read: a recording keeps it alive.
 void pin_cached(b200_engine *e, const CachedSplit &c);
 
+// The word the calling thread has named with b200_only_if, or null.
+inline const int *only_if_word(const b200_engine *e) {
+  if (e->only_if_of.empty()) return nullptr;
+  const auto it = e->only_if_of.find(std::this_thread::get_id());
+  return it == e->only_if_of.end() ? nullptr : it->second;
+}
+
 // In the entry points whose launches honour b200_only_if.
 struct OnlyIfAllowed {
   b200_engine *e;
-  explicit OnlyIfAllowed(b200_engine *e_) : e(e_) { e->allow_only_if = true; }
-  ~OnlyIfAllowed() { e->allow_only_if = false; }
+  explicit OnlyIfAllowed(b200_engine *e_) : e(e_) { e->only_if = only_if_word(e); }
+  ~OnlyIfAllowed() { e->only_if = nullptr; }
 };
 
 // Waits for the engine's stream; B200_ERR_TIMEOUT if a kernel launched since the last check gave

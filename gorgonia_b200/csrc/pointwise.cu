@@ -1404,7 +1404,7 @@ int plan_pending(b200_engine *e, int *n_kernels) {
 }
 
 int flush_pending(b200_engine *e) {
-  if (e->only_if && !e->allow_only_if)
+  if (!e->only_if && only_if_word(e))  // e->only_if: an entry point that honours it
     return set_error(e, B200_ERR_STATE, "this call cannot be made while b200_only_if is in effect");
   if (e->pending.empty()) {
     e->dead.clear();
@@ -1424,6 +1424,7 @@ int flush_pending(b200_engine *e) {
 }
 
 static int enqueue(b200_engine *e, const b200_pw_call &c) {
+  if (only_if_word(e)) return set_error(e, B200_ERR_STATE, "this call cannot be made while b200_only_if is in effect");
   e->pending.push_back(c);
   if (e->flags & B200_ENGINE_NO_DEFER) return flush_pending(e);
   // keep the queue bounded: a tape that never flushes would otherwise grow without limit

@@ -488,9 +488,11 @@ int b200_conv2d_chain_fwd(b200_engine *e, const void *x, const void *x_hi, const
  *   b200_pairs_magnitude: the record of a network's input: its largest magnitude (a sample's for large n).
  *   b200_pairs_check: *verdict (on the device) = 1 if any of k <= 32 adjacent records says that its tensor
  *     (of counts[i] values) was unusable, else 0; clears the records.
- *   b200_only_if: until it is called with NULL, launches are made that run only if *flag is not zero.
+ *   b200_only_if: until the calling thread calls it with NULL, this thread's launches on the engine run only
+ *     if *flag is not zero.
  *     b200_conv2d_chain_fwd (shapes of the tensor-core and first-layer kernels), b200_maxpool2d_split_fwd and
- *     b200_maxpool2d_fwd (2x2, no mask) can be called then; everything else answers B200_ERR_STATE. */
+ *     b200_maxpool2d_fwd (2x2, no mask) can be called then; everything else that launches or queues a kernel
+ *     answers B200_ERR_STATE. Other threads' calls on the engine are neither refused nor made conditional. */
 int b200_conv2d_pairs_fwd(b200_engine *e, const void *x, const void *x_pairs, const void *x_rec,
                           const void *w, void *y, void *y_pairs, void *y_rec, int64_t B, int64_t C, int64_t H,
                           int64_t W, int64_t K, int kh, int kw, int pad_h, int pad_w, const b200_epilogue *ep,

@@ -368,3 +368,45 @@ def test_dark_image_of_a_large_batch(fresh):
         e.Close()
     assert np.linalg.norm(pooled[0] - pooled[1]) <= 4e-6 * np.linalg.norm(pooled[1])
     assert redo == [1, 0]
+
+
+def test_only_if_is_the_calling_threads(fresh):
+    # another thread's calls on the same engine are neither refused nor made conditional, and a pointwise call
+    # inside is refused like every other
+    import threading
+    e = fresh
+    z = util.normal(103, (2, 16, 32, 32))
+    flag, tz, ty = e.tensor(np.zeros(4, np.int32)), e.tensor(z), e.tensor(np.zeros((2, 16, 16, 16), np.float32))
+    w = e.tensor(util.normal(104, (32, 16, 3, 3), scale=0.05))
+    ts = tuple(e.tensor(np.zeros((2, 16, 16, 16), np.float32)) for _ in range(2))
+    conv, inner, s = e.tensor(np.zeros((2, 32, 32, 32), np.float32)), e.tensor(np.zeros((2, 16, 16, 16), np.float32)), e.empty(z.shape)
+    second, failed = e.tensor(np.zeros(4, np.int32)), []
+
+    def other():
+        try:
+            e.MaxPool2D(tz, ty, (2, 2), (0, 0), (2, 2))
+            e.MaxPool2DSplit(tz, None, ts, (2, 2), (0, 0), (2, 2))
+            e.Conv2dChain(tz, w, conv, z.shape, pad=(1, 1))
+            e.Unary("neg", tz, reuse=s)
+            e.Signal()
+            with e.only_if(second.ptr):     # a condition of its own at the same time
+                e.MaxPool2D(tz, inner, (2, 2), (0, 0), (2, 2))
+        except Exception as err:            # noqa: BLE001 - handed to the test's thread
+            failed.append(err)
+
+    with e.only_if(flag.ptr):
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        e.MaxPool2D(tz, inner, (2, 2), (0, 0), (2, 2))
+        with pytest.raises(B200Error):
+            e.Unary("neg", tz, reuse=s)
+        with pytest.raises(B200Error):
+            e.Add(tz, tz, reuse=s)
+    assert not failed
+    want = oracle.maxpool2d(z, (2, 2), (0, 0), (2, 2))[0]
+    assert_bits_equal(ty.numpy(), want)
+    assert np.abs(ts[0].numpy() + ts[1].numpy() - want.transpose(0, 2, 3, 1).reshape(ts[0].shape)).max() <= 2.0 ** -21 * np.abs(z).max()
+    assert np.abs(conv.numpy()).max() > 0
+    assert_bits_equal(s.numpy(), -z)
+    assert not inner.numpy().any()
