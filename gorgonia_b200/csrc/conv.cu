@@ -596,7 +596,7 @@ static int conv2d_pairs(b200_engine *e, int path, const __half *x16, const F16Re
 static bool conv_pairs_pay(b200_engine *e, const float *w, long long B, int C, int H, int W, int K, int taps, int Ho, int Wo) {
   const double saves = 0.35 * 2.0 * B * Ho * Wo * K * (double)C * taps / 160e12;
   const double costs = 4.0 * B * C * H * (double)W / 5e12 + (is_constant(e, w) ? 20e-6 : 27e-6);
-  return C % 16 == 0 && saves > 1.2 * costs;
+  return C % 16 == 0 && saves > 1.2 * costs && !(e->flags & B200_ENGINE_NO_STREAMK);  // as f16_pays (gemm_tc.cu)
 }
 
 // x (NCHW) through pairs of fp16, with the TF32 launches behind it that run only if the pairs are unusable.

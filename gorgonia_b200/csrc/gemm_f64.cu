@@ -222,9 +222,10 @@ int gemm_f64(b200_engine *e, int transA, int transB, long long M, long long N, l
   if (tiles >= (1LL << 31) || batch > 65535)
     return set_error(e, B200_ERR_UNSUPPORTED, "b200_gemm: %lld output tiles in %lld slices are more than one launch takes", tiles, batch);
   // k is cut until there are two blocks per SM, in pieces of at least 8 slabs: below that, leaving and
-  // gathering the parts (T x T doubles each, about a microsecond per part) outweighs the shorter loop
+  // gathering the parts (T x T doubles each, about a microsecond per part) outweighs the shorter loop. The number
+  // of tiles, and with it the cut, depends on M: not with B200_ENGINE_NO_STREAMK.
   long long splits = 1;
-  if (tiles * batch < 2LL * e->sm_count)
+  if (tiles * batch < 2LL * e->sm_count && !(e->flags & B200_ENGINE_NO_STREAMK))
     splits = std::max<long long>(1, std::min<long long>({(2LL * e->sm_count + tiles * batch - 1) / (tiles * batch), slabs / 8, 16}));
   void *ws = nullptr;
   if (splits > 1 && b200_get(e, tiles * batch * splits * T * T * (long long)sizeof(double), &ws) != B200_OK)

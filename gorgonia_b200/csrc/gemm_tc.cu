@@ -1134,9 +1134,11 @@ static void keep_split_f16(b200_engine *e, const F32Operand &x, F16Operand *o) {
 
 // Whether a product is worth fp16 pairs. They save about half of the 2 M N K / 200 TFLOP/s that TF32 pairs
 // take; finding the largest magnitudes reads both operands once more (5 TB/s), and the launches that find
-// nothing to do cost 8 us.
+// nothing to do cost 8 us. Not where a result may not depend on the batch: this rule, the scale and the way back
+// all do.
 static bool f16_pays(b200_engine *e, long long M, long long N, long long K, long long batch, const F32Operand &A,
                      const F32Operand &B) {
+  if (e->flags & B200_ENGINE_NO_STREAMK) return false;
   const double saves = (double)M * N * K * batch / 200e12;
   const double reads = ((is_constant(e, A.src) ? 0.0 : (double)M * K) + (is_constant(e, B.src) ? 0.0 : (double)N * K)) * 4.0 * batch / 5e12;
   return saves > 1.3 * (reads + 8e-6);

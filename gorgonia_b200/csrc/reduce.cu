@@ -439,9 +439,11 @@ static int launch_mode(b200_engine *e, const T *x, T *y, long long outer, long l
     const int blocks = (int)std::max<long long>(1, std::min(outer, cap));
     launch_kernel(e, long_row_kernel<T, MODE>, blocks, threads, 0, x, y, outer, len);
     B200_CHECK_LAUNCH(e, "long_row_kernel");
-  } else if ((MODE == 2 || MODE == 3) && len >= 32 && outer * inner < e->sm_count * 2048LL) {
+  } else if ((MODE == 2 || MODE == 3) && len >= 32 && outer * inner < e->sm_count * 2048LL &&
+             !(MODE == 2 && (e->flags & B200_ENGINE_NO_STREAMK))) {
     // Fewer columns than threads the GPU holds (2048 per SM): split the axis. With more columns the walk
-    // below keeps every SM busy, and folding rows through shared memory would only add work.
+    // below keeps every SM busy, and folding rows through shared memory would only add work. `outer` may be a
+    // batch: a sum's order then depends on it, which that flag rules out.
     constexpr int M = MODE == 2 ? 2 : 3;
     if (inner > 16) return launch_col_split<T, M, 32>(e, x, y, outer, len, inner);
     if (inner > 8) return launch_col_split<T, M, 16>(e, x, y, outer, len, inner);

@@ -112,6 +112,7 @@ class Engine:
             raise B200Error(rc, (lib.b200_last_error(None) or b"").decode())
         self.h = h
         self.device = device
+        self.streamk = streamk
 
     # ---- lifecycle -------------------------------------------------------------------
     def Close(self):

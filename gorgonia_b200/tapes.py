@@ -160,6 +160,10 @@ class _ConvChain:
     # microsecond or two each.
     PAIRS_FLOPS = 12e9
 
+    def worth_pairs(self, flops):
+        """Not on engines whose results may not depend on the batch, as this rule does."""
+        return flops >= self.PAIRS_FLOPS and self.e.streamk
+
     @property
     def flops(self):
         f = 0
@@ -325,7 +329,7 @@ class LeNet(_Tape):
             {"w": self.wc[i], "pad": (1, 1), "bias": None, "act": "rectify", "alpha": 0.0, "pool": "2x2/2"}
             for i in range(3)]) if fused else None
         self.records = None
-        if fused and self.chain.can_pairs() and self.chain.flops >= self.chain.PAIRS_FLOPS:
+        if fused and self.chain.can_pairs() and self.chain.worth_pairs(self.chain.flops):
             self.records = _Records(e)
             self.chain.plan_pairs(self.records)
         self.dense = _DenseChain(e, batch, [{"w": self.wd[0], "bias": None, "act": "rectify"},
@@ -405,7 +409,7 @@ class TinyYolo(_Tape):
             self.out = self.chain_b.layers[-1]["y"]
             a, b = self.chain_a, self.chain_b
             self.records = None
-            if self.pool5_split is not None and a.can_pairs() and b.can_pairs() and a.flops + b.flops >= a.PAIRS_FLOPS:
+            if self.pool5_split is not None and a.can_pairs() and b.can_pairs() and a.worth_pairs(a.flops + b.flops):
                 self.records = _Records(e)
                 a.plan_pairs(self.records)
                 b.plan_pairs(self.records)

@@ -70,9 +70,11 @@ enum {
   B200_ENGINE_NO_DEFER = 2u, /* launch each pointwise call at once instead of queueing it   */
   B200_ENGINE_CONV_GATHER = 4u, /* tensor-core convolutions build their col operand with gather *
                                  * warps even where the TMA unit could (tests, comparisons)    */
-  B200_ENGINE_NO_STREAMK = 8u,  /* tensor-core kernels never share a tile's k range between    *
-                                 * CTAs: every output element is then summed in one fixed      *
-                                 * order whatever the batch size (tests, comparisons)          */
+  B200_ENGINE_NO_STREAMK = 8u,  /* matrix products, convolutions and sums along an axis never   *
+                                 * share a result's terms between CTAs, and float32 ones are    *
+                                 * always made from pairs of TF32: every output element is then *
+                                 * summed in one fixed order from the same pairs whatever the   *
+                                 * batch size (tests, comparisons)                              */
   B200_ENGINE_NO_PAIRS = 16u    /* tensor-core kernels never run as pairs of CTAs on one       *
                                  * 256-row tile (tests, comparisons); results are the same     *
                                  * bits either way                                             */

@@ -243,3 +243,49 @@ def test_small_values_among_ordinary_ones_stay_with_fp16(fresh, transA, transB):
         e.record(ev[1])
         (tf32 if spread else fp16).append(e.elapsed_ms(*ev))
     assert fp16[0] < 0.8 * tf32[0]
+
+
+def test_one_summation_order_whatever_the_batch():
+    # streamk=False promises that a shard of a batch and the whole batch agree to the bit, at sizes where the
+    # choice of pairs or of a cut along k would depend on the batch
+    from gorgonia_b200 import Engine, tapes
+    e = Engine(0, 8 << 30, streamk=False)
+    x = util.uniform(41, (1024, 1, 28, 28))
+    out = []
+    for lo, hi in ((0, 1024), (0, 512), (512, 1024)):
+        m = tapes.LeNet(e, hi - lo)
+        m.x.set(x[lo:hi])
+        out.append(m.forward().numpy())
+        e.Signal()
+        e.ResetAllocator()
+    util.assert_bits_equal(out[0], np.concatenate(out[1:]))
+
+    def shards(make, rows, parts):
+        whole = make(0, rows)
+        cut = [make(rows * k // parts, rows * (k + 1) // parts) for k in range(parts)]
+        util.assert_bits_equal(whole, np.concatenate(cut))
+        e.Signal()
+        e.ResetAllocator()
+
+    a, w = util.normal(42, (4096, 2048)), util.normal(43, (2048, 2048), scale=0.02)
+    a[0, 0] = 1e-14
+
+    def product(dt):
+        def make(lo, hi):
+            c = e.empty((hi - lo, w.shape[1]), dt)
+            return e.MatMul(e.tensor(a[lo:hi].astype(dt)), e.constant(e.tensor(w.astype(dt))), c).numpy()
+        return make
+    shards(product(np.float32), 4096, 4)
+    a, w = a[:256, :784], w[:784, :300]
+    shards(product(np.float64), 256, 4)
+    img, f = util.normal(44, (64, 128, 26, 26)), util.normal(45, (256, 128, 3, 3), scale=0.05)
+
+    def conv(lo, hi):
+        return e.Conv2d(e.tensor(img[lo:hi]), e.constant(e.tensor(f)), e.empty((hi - lo, 256, 26, 26)), pad=(1, 1)).numpy()
+    shards(conv, 64, 4)
+    s = util.normal(46, (512, 1000, 12))
+
+    def total(lo, hi):
+        return e.Reduce("sum", e.tensor(s[lo:hi]), e.empty((hi - lo, 12)), 1).numpy()
+    shards(total, 512, 8)
+    e.Close()
