@@ -282,29 +282,32 @@ __global__ void __launch_bounds__(256) maxpool2x2_any_kernel(const float *__rest
 // a 3x3 window span stay in L1 from one position to the next. Four positions are in flight per lane.
 // Bound by HBM (col is written once, nine times the image for 3x3); with an index division per element it
 // was bound by integer arithmetic: 100 x 32 x 14 x 14, 3x3 float32 57 -> 13 us.
-// grid: blockIdx.x walks groups of `rows` output rows of all images.
+// grid: blockIdx.x walks groups of `rows` lines (a line is one of `segs` runs of `seg_len` positions of an output
+// row of an image), and gridDim.y blocks share a group's (line, 32 entries) tasks.
 template <typename T>
-__global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T *__restrict__ col, long long out_rows,
+__global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T *__restrict__ col, long long lines,
                                                      int C, int H, int W, int Ho, int Wo, int kh, int kw, int padH,
-                                                     int padW, int sH, int sW, int dH, int dW, int rows) {
+                                                     int padW, int sH, int sW, int dH, int dW, int rows, int segs,
+                                                     int seg_len) {
   ptx::grid_begin();
   const int crs = C * kh * kw, pieces = (crs + 31) / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (long long g0 = (long long)blockIdx.x * rows; g0 < out_rows; g0 += (long long)gridDim.x * rows) {
-    const int here = (int)(out_rows - g0 < rows ? out_rows - g0 : rows);
-    for (int t = warp; t < pieces * here; t += 8) {
+  for (long long g0 = (long long)blockIdx.x * rows; g0 < lines; g0 += (long long)gridDim.x * rows) {
+    const int here = (int)(lines - g0 < rows ? lines - g0 : rows);
+    for (int t = warp + 8 * blockIdx.y; t < pieces * here; t += 8 * gridDim.y) {
       const int rr = t / pieces, q = (t - rr * pieces) * 32 + lane;
-      const long long row = g0 + rr, b = row / Ho;
+      const long long line = g0 + rr, row = line / segs, b = row / Ho;
+      const int ow0 = (int)(line - row * segs) * seg_len, ow1 = min(Wo, ow0 + seg_len);
       const int oh = (int)(row - b * Ho);
       if (q >= crs) continue;
       const int c = q / (kh * kw), tap = q - c * kh * kw, r = tap / kw, s = tap - r * kw;
       const int ih = oh * sH - padH + r * dH;
-      int iw = s * dW - padW;
+      int iw = ow0 * sW + s * dW - padW;
       const T *in = x + ((b * C + c) * H + ih) * (long long)W;
-      T *out = col + row * Wo * (long long)crs + q;
+      T *out = col + (row * Wo + ow0) * (long long)crs + q;
       const bool inside = ih >= 0 && ih < H;
-      int ow = 0;
-      for (; ow + 3 < Wo; ow += 4) {
+      int ow = ow0;
+      for (; ow + 3 < ow1; ow += 4) {
         T v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T 
         for (int j = 0; j < 4; ++j) out[(long long)j * crs] = v[j];
         out += 4LL * crs;
       }
-      for (; ow < Wo; ++ow) {
+      for (; ow < ow1; ++ow) {
         *out = inside && iw >= 0 && iw < W ? __ldg(in + iw) : T(0);
         iw += sW;
         out += crs;
@@ -1115,6 +1118,27 @@ static int grid_for(b200_engine *e, long long work) {
   return (int)std::max<long long>(1, std::min<long long>((work + 255) / 256, (long long)e->sm_count * 16));
 }
 
+// How an im2col is cut into blocks. A block takes `rows` whole output rows where that gives two blocks per SM: enough
+// (row, 32 entries) tasks to keep its eight warps evenly busy. With fewer rows (few images) the tasks of a group are
+// shared between `share` blocks, down to one per warp, and then rows are cut into `segs` runs of eight or more positions.
+// 3 x 3 windows, float32: one 3 x 224 x 224 image 72 -> 10 us, 256 x 13 x 13 20 -> 8.
+struct Im2colSplit {
+  int rows, share, segs, seg_len;
+};
+static Im2colSplit im2col_split(const b200_engine *e, long long out_rows, long long Wo, int crs) {
+  const int pieces = (crs + 31) / 32;
+  const long long want = 2LL * e->sm_count;
+  Im2colSplit s;
+  s.rows = std::max(1, 32 / pieces);
+  const long long groups = (out_rows + s.rows - 1) / s.rows, tasks = (long long)pieces * std::min<long long>(s.rows, out_rows);
+  s.share = (int)std::max<long long>(1, std::min((want + groups - 1) / groups, (tasks + 7) / 8));
+  const long long have = groups * s.share;
+  const long long cuts = std::max<long long>(1, std::min((want + have - 1) / have, Wo / 8));
+  s.seg_len = (int)(((Wo + cuts - 1) / cuts + 3) / 4 * 4);
+  s.segs = (int)((Wo + s.seg_len - 1) / s.seg_len);
+  return s;
+}
+
 // Groups of samples a channel's sums are cut into: about eight blocks per SM over all channels.
 static int bn_groups(const b200_engine *e, long long B, int channels) {
   return (int)std::max<long long>(1, std::min<long long>({(8LL * e->sm_count + channels - 1) / channels, B, BN_GROUPS}));
@@ -1551,17 +1575,16 @@ int b200_im2col(b200_engine *e, int dtype, const void *x, void *col, int64_t B, 
   int rc = flush_pending(e);
   if (rc != B200_OK) return rc;
   const int crs = (int)(C * kh * kw);
-  // image rows per block: enough (row, 32 entries) pieces to keep its eight warps evenly busy
-  const int rows = std::max(1, 32 / ((crs + 31) / 32));
-  const int blocks = (int)std::min<long long>((B * Ho + rows - 1) / rows, 1LL << 30);
+  const Im2colSplit sp = im2col_split(e, B * Ho, Wo, crs);
+  const dim3 grid((unsigned)std::min<long long>((B * Ho * sp.segs + sp.rows - 1) / sp.rows, 1LL << 30), (unsigned)sp.share);
   if (dtype == B200_F32)
-    launch_kernel(e, im2col_kernel<float>, blocks, 256, 0, (const float *)x, (float *)col, B * Ho, (int)C, (int)H, (int)W,
-                                                       (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h, stride_w,
-                                                       dil_h, dil_w, rows);
+    launch_kernel(e, im2col_kernel<float>, grid, 256, 0, (const float *)x, (float *)col, B * Ho * sp.segs, (int)C, (int)H,
+                  (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, sp.rows, sp.segs,
+                  sp.seg_len);
   else
-    launch_kernel(e, im2col_kernel<double>, blocks, 256, 0, (const double *)x, (double *)col, B * Ho, (int)C, (int)H,
-                                                        (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h,
-                                                        stride_w, dil_h, dil_w, rows);
+    launch_kernel(e, im2col_kernel<double>, grid, 256, 0, (const double *)x, (double *)col, B * Ho * sp.segs, (int)C,
+                  (int)H, (int)W, (int)Ho, (int)Wo, kh, kw, pad_h, pad_w, stride_h, stride_w, dil_h, dil_w, sp.rows,
+                  sp.segs, sp.seg_len);
   B200_CHECK_LAUNCH(e, "im2col_kernel");
   return B200_OK;
 }

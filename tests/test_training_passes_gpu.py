@@ -35,6 +35,16 @@ def test_im2col_pieces(fresh, case, dt):
     assert_bits_equal(col.numpy(), want.reshape(col.shape))
 
 
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("case", [
+    # few images: rows cut into runs of positions, and the channels of a row shared between blocks
+    (1, 3, 224, 224, (3, 3), (1, 1), (1, 1), (1, 1)), (1, 1, 3, 1001, (1, 3), (0, 1), (1, 2), (1, 3)),
+    (1, 256, 13, 13, (3, 3), (1, 1), (1, 1), (1, 1)), (1, 40, 1, 9, (1, 2), (0, 0), (1, 1), (1, 1)),
+    (2, 5, 31, 47, (3, 3), (2, 2), (2, 2), (1, 2))])
+def test_im2col_few_images(fresh, case, dt):
+    test_im2col_pieces(fresh, case, dt)
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 2, 2), (3, 5, 14, 14), (2, 7, 13, 6), (2, 3, 9, 8), (100, 64, 14, 14)])
 def test_maxpool2x2_gradient(fresh, shape):
     e = fresh
