@@ -168,3 +168,37 @@ def test_plan_limits_program_length():
     calls = [_call("neg", X, X, form=UN) for _ in range(20)]
     koc, nk, _, _ = _plan(calls)
     assert nk == 3 and koc.count(0) == 8
+
+
+def test_plan_time_grows_with_the_queue_not_its_square():
+    # a chain whose temporaries are all released at its end
+    import time
+    best = {}
+    for n in (500, 4000):
+        calls = [_call("add", X + 0x10000 * (k + 1), X + 0x10000 * k, 0x8000) for k in range(n)]
+        arr, rel = (_lib.PwCall * n)(*calls), (C.c_int * n)(*([n] * (n - 1) + [-1]))
+        koc, loads, stores, nk = (C.c_int * n)(), (C.c_int * n)(), (C.c_int * n)(), C.c_int()
+        times = []
+        for _ in range(5):
+            t = time.perf_counter()
+            assert lib.b200_fusion_plan(arr, n, rel, koc, C.byref(nk), loads, stores) == 0
+            times.append(time.perf_counter() - t)
+        best[n] = min(times)
+        assert nk.value == (n + 7) // 8 and set(stores[:nk.value]) == {1}
+    assert best[4000] < 24 * best[500]      # eight times the calls: 8 with sorting, 64 if each looked at all others
+
+
+def test_plan_looks_at_every_read_in_front_of_a_release():
+    # T1 is read behind the point where its kernel ends (another element count), by parts of it and as a scalar
+    for reader in (_call("neg", T3, T1, form=UN, n=512), _call("neg", T3, T1 + 1024, form=UN, n=512),
+                   _call("neg", T3, T1 - 1024, form=UN, n=512), _call("add", T3, X, T1 + 64, n=2048, bcast=1, bdiv=1, bmod=8)):
+        calls = [_call("neg", T1, X, form=UN), _call("square", T2, T1, form=UN), reader]
+        koc, nk, _, stores = _plan(calls, [3, -1, -1])
+        assert nk == 2 and stores == [2, 1]
+        koc, nk, _, stores = _plan(calls, [2, -1, -1])      # released in front of that read: somebody else's buffer by then
+        assert nk == 2 and stores == [1, 1]
+    # the address is written anew in between: only the second value is read
+    calls = [_call("neg", T1, X, form=UN), _call("square", T2, T1, form=UN), _call("neg", T1, X, form=UN, n=512),
+             _call("square", T3, T1, form=UN, n=512)]
+    koc, nk, _, stores = _plan(calls, [2, -1, 4, -1])
+    assert nk == 2 and stores == [1, 1]
