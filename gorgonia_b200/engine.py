@@ -67,10 +67,18 @@ class Tensor:
     def __init__(self, engine, ptr, shape, dtype, owned=True):
         self.engine = engine
         self.ptr = ptr
-        self.shape = tuple(int(s) for s in shape)
+        self.shape = shape
         self.dtype = np.dtype(dtype)
         self.owned = owned
-        self.size = _count(self.shape)
+
+    @property
+    def shape(self):
+        return self._shape
+
+    @shape.setter
+    def shape(self, shape):
+        self._shape = tuple(int(s) for s in shape)
+        self.size = _count(self._shape)     # kept: a call asks for it several times
 
     @property
     def nbytes(self):

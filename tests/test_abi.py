@@ -202,3 +202,14 @@ def test_plan_looks_at_every_read_in_front_of_a_release():
              _call("square", T3, T1, form=UN, n=512)]
     koc, nk, _, stores = _plan(calls, [2, -1, 4, -1])
     assert nk == 2 and stores == [1, 1]
+
+
+def test_tensor_size_follows_its_shape():
+    import numpy as np
+    from gorgonia_b200.engine import Tensor
+    t = Tensor(None, 0x1000, (4, 6), np.float32, owned=False)
+    assert t.size == 24 and t.nbytes == 96
+    t.shape = (2, 6)
+    assert t.shape == (2, 6) and t.size == 12 and t.nbytes == 48
+    t.shape = ()
+    assert t.size == 1
