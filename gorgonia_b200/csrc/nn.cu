@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(256) maxpool2x2_any_kernel(const float *__rest
 // grid: blockIdx.x walks groups of `rows` lines (a line is one of `segs` runs of `seg_len` positions of an output
 // row of an image), and gridDim.y blocks share a group's (line, 32 entries) tasks.
 template <typename T>
-__global__ void __launch_bounds__(256) im2col_kernel(const T *__restrict__ x, T *__restrict__ col, long long lines,
+__global__ void __launch_bounds__(256, 8) im2col_kernel(const T *__restrict__ x, T *__restrict__ col, long long lines,
                                                      int C, int H, int W, int Ho, int Wo, int kh, int kw, int padH,
                                                      int padW, int sH, int sW, int dH, int dW, int rows, int segs,
                                                      int seg_len) {
