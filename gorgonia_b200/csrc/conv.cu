@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(256, 2) conv3x3_first_pool_kernel(const float 
         for (int half = 0; half < 2; ++half) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) stats.see(pooled[half][k]);
-          store_pairs<8>(pooled[half], 8, out_scale, out16.h + (pos + half) * K + k0, out16.l + (pos + half) * K + k0, stats);
+          store_pairs<8>(pooled[half], 8, out_scale, out16.h + (pos + half) * K + k0, out16.l + (pos + half) * K + k0, stats, 3.402823466e+38f);
         }
       } else if (y_hi) {  // the same values as NHWC TF32 head / tail for the next convolution (K a multiple of 4)
         const long long pos = (b * Hq + ph) * (long long)Wq + (ow >> 1);

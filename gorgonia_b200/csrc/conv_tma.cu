@@ -384,8 +384,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
               if (j < valid) stats.see(acc[j]);
           }
           if (p.out16.h) {
-            stats.see_place(largest, out_scale);
-            store_pairs<HALF>(acc, valid, out_scale, p.out16.h + m * p.K + n0, p.out16.l + m * p.K + n0, stats);
+            store_pairs<HALF>(acc, valid, out_scale, p.out16.h + m * p.K + n0, p.out16.l + m * p.K + n0, stats, largest);
           }
           if (yb) {
 #pragma unroll
@@ -421,14 +420,20 @@ struct NhwcOut {
   unsigned limit;      // F16: how many of these there may be
   const int *only_if;  // TF32: skip_launch
 };
-// F16: n small values of the place whose channels begin at `place` (pairs.cuh). Rare.
-__device__ __noinline__ void nhwc_small(F16Rec *rec, unsigned limit, unsigned n, const float *place, int C, int HW,
+// F16: n small values of the place whose channels begin at `place` (pairs.cuh). Rare. The lanes that come here together
+// ask with one access for all. Returns whether the tensor is known to be of no use, so that nobody need ask again.
+__device__ __noinline__ bool nhwc_small(F16Rec *rec, unsigned limit, unsigned n, const float *place, int C, int HW,
                                         float scale) {
-  if (!f16_count_small(rec, limit, n)) return;
+  const unsigned here = __activemask(), total = __reduce_add_sync(here, n);
+  const int leader = __ffs(here) - 1;
+  bool look = false;
+  if ((threadIdx.x & 31) == leader) look = f16_count_small(rec, limit, total);
+  if (!__shfl_sync(here, look, leader)) return true;
 #pragma unroll 4
   for (int c = 0; c < C; ++c)
-    if (fabsf(__ldg(place + (long long)c * HW)) * scale >= kFullPair) return;
+    if (fabsf(__ldg(place + (long long)c * HW)) * scale >= kFullPair) return false;
   atomicOr(&rec->bad, 1u);
+  return true;
 }
 template <bool F16>
 __device__ __forceinline__ float nhwc_begin(const NhwcOut &out) {
@@ -440,13 +445,13 @@ __device__ __forceinline__ float nhwc_begin(const NhwcOut &out) {
 // N (4 or 1) neighbouring channels at element `at`; their place's channels begin at x[place]
 template <bool F16, int N>
 __device__ __forceinline__ void nhwc_store(const NhwcOut &out, long long at, const float (&v)[N], float scale,
-                                           const float *x, long long place, int C, int HW) {
+                                           const float *x, long long place, int C, int HW, bool &useless) {
   if (F16) {
     __align__(8) __half h[4], l[4];
     unsigned small = 0;
 #pragma unroll
     for (int k = 0; k < N; ++k) small += f16_pair(v[k], scale, h[k], l[k]) ? 1u : 0u;
-    if (small) nhwc_small(out.rec, out.limit, small, x + place, C, HW, scale);
+    if (small && !useless) useless = nhwc_small(out.rec, out.limit, small, x + place, C, HW, scale);
     __half *hp = (__half *)out.hi + at, *lp = (__half *)out.lo + at;
     if (N == 4) {
       *reinterpret_cast<uint2 *>(hp) = *reinterpret_cast<const uint2 *>(h);
@@ -482,6 +487,7 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
   ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
+  bool useless = false;  // F16: the record has been seen to say so
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int ptiles = (HW + 31) / 32, ctiles = (C + 31) / 32;
@@ -504,7 +510,7 @@ __global__ void __launch_bounds__(256) nhwc_split_kernel(const float *__restrict
       const int pp = p0 + j, c = c0 + tx;
       if (pp < HW && c < C) {
         const float v[1] = {tile[tx][j]};
-        nhwc_store<F16, 1>(out, ob + (long long)pp * C + c, v, scale, x, ob + pp, C, HW);
+        nhwc_store<F16, 1>(out, ob + (long long)pp * C + c, v, scale, x, ob + pp, C, HW, useless);
       }
     }
     __syncthreads();
@@ -522,6 +528,7 @@ __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restric
   ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
+  bool useless = false;  // F16: the record has been seen to say so
   constexpr int PT = 128, PITCH = PT + 1;
   __shared__ float tile[CT * PITCH];
   const int ptiles = (HW + PT - 1) / PT, ctiles = C / CT;
@@ -551,7 +558,7 @@ __global__ void __launch_bounds__(256) nhwc_split4_kernel(const float *__restric
         float v[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = tile[(4 * cg + k) * PITCH + pp];
-        nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, x, b * HW * (long long)C + p0 + pp, C, HW);
+        nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, x, b * HW * (long long)C + p0 + pp, C, HW, useless);
       }
     }
     __syncthreads();
@@ -568,6 +575,7 @@ __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__rest
   ptx::grid_begin();
   if (!F16 && skip_launch(out.only_if)) return;
   const float scale = nhwc_begin<F16>(out);
+  bool useless = false;  // F16: the record has been seen to say so
   extern __shared__ __align__(16) float img[];
   const int chunks = C >> 5;
   const long long total = B * chunks;
@@ -593,7 +601,7 @@ __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__rest
       float v[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) v[k] = img[(4 * cg + k) * pitch + pp];
-      nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, x, b * HW * (long long)C + pp, C, HW);
+      nhwc_store<F16, 4>(out, o0 + (long long)pp * C + 4 * cg, v, scale, x, b * HW * (long long)C + pp, C, HW, useless);
     }
     __syncthreads();
   }

@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
         const int qh = p.pool2 ? oh >> 1 : oh, qw = p.pool2 ? ow >> 1 : ow;
         const long long plane = (long long)Hq * Wq;
         const long long pos = inside ? ((long long)b * Hq + qh) * Wq + qw : 0;
-        float largest = 0.f;  // of the sums in front of the activation
+        float largest = -1.f;  // of the sums in front of the activation (store_pairs)
         auto store = [&](float *v, int c0, auto size) {  // channels from column c0 of this tile on
           constexpr int N = decltype(size)::value;
           const int valid = p.K - n0 - c0;
@@ -435,8 +435,8 @@ __global__ void __launch_bounds__(CW_THREADS, 1)
           for (int j = 0; j < N; ++j)
             if (j < valid) stats.see(v[j]);
           if (p.out16.h) {
-            stats.see_place(largest, out_scale);
-            store_pairs<N>(v, valid, out_scale, p.out16.h + pos * p.K + n0 + c0, p.out16.l + pos * p.K + n0 + c0, stats);
+            store_pairs<N>(v, valid, out_scale, p.out16.h + pos * p.K + n0 + c0, p.out16.l + pos * p.K + n0 + c0, stats,
+                           largest);
           }
           if (p.y) {
             float *yb = p.y + ((long long)b * p.K + n0 + c0) * plane + (long long)qh * Wq + qw;

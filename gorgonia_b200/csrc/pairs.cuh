@@ -66,10 +66,6 @@ struct PairStats {
     const unsigned m = __float_as_uint(v) & 0x7FFFFFFFu;
     amax = amax > m ? amax : m;
   }
-  // the largest magnitude among a place's channels, in front of the activation
-  __device__ __forceinline__ void see_place(float largest, float scale) {
-    if (largest != 0.f && largest * scale < kFullPair) bad = 1;
-  }
   // by whole warps, once
   __device__ __forceinline__ void deliver(F16Rec *rec) {
     const unsigned a = __reduce_max_sync(0xffffffffu, amax), s = __reduce_add_sync(0xffffffffu, small);
@@ -83,10 +79,13 @@ struct PairStats {
   }
 };
 
-// N values (a multiple of 8) to N / 8 16-byte pieces of heads and tails; `valid` is a multiple of 8.
+// N values (a multiple of 8) of one place to N / 8 16-byte pieces of heads and tails; `valid` is a multiple of 8.
+// sums: the largest magnitude of the sums in front of Rectify; negative if the values themselves tell. Looked at only
+// where some value is small.
 template <int N>
 __device__ __forceinline__ void store_pairs(const float *v, int valid, float scale, __half *h, __half *l,
-                                            PairStats &st) {
+                                            PairStats &st, float sums) {
+  const unsigned before = st.small;
 #pragma unroll
   for (int j0 = 0; j0 < N; j0 += 8) {
     if (j0 < valid) {
@@ -100,23 +99,34 @@ __device__ __forceinline__ void store_pairs(const float *v, int valid, float sca
       *reinterpret_cast<uint4 *>(l + j0) = *reinterpret_cast<const uint4 *>(ll);
     }
   }
+  if (st.small != before) {
+    if (sums < 0.f) {
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        if (j < valid) sums = fmaxf(sums, fabsf(v[j]));
+    }
+    if (sums * scale < kFullPair) st.bad = 1;
+  }
 }
 
 // What an activation leaves at least of a magnitude, unless it leaves nothing.
 __device__ __forceinline__ float act_floor(int act, float alpha) {
   return act == B200_ACT_LEAKY && alpha != 0.f ? fminf(1.f, fabsf(alpha)) : 1.f;
 }
-// acc -> act(acc + bias), the activation chosen outside the loop. Returns the largest magnitude in front of it, by
-// what the activation leaves of it at least (see_place).
+// acc -> act(acc + bias), the activation chosen outside the loop. Returns what store_pairs wants to know of the sums
+// in front of it: of an activation that leaves zeros, the largest magnitude. (Found for every activation it took 25 us
+// of tiny-YOLO's 1690 at 64 images.)
 template <int N>
 __device__ __forceinline__ float finish_channels(float (&acc)[N], const float *bias, int act, float alpha) {
   if (bias) {
 #pragma unroll
     for (int j = 0; j < N; ++j) acc[j] = __fadd_rn(acc[j], bias[j]);
   }
-  float largest = 0.f;
+  float largest = -1.f;
+  if (act == B200_ACT_RECTIFY || (act == B200_ACT_LEAKY && alpha == 0.f)) {
 #pragma unroll
-  for (int j = 0; j < N; ++j) largest = fmaxf(largest, fabsf(acc[j]));
+    for (int j = 0; j < N; ++j) largest = fmaxf(largest, fabsf(acc[j]));
+  }
   if (act == B200_ACT_RECTIFY) {
 #pragma unroll
     for (int j = 0; j < N; ++j) acc[j] = apply_act<float>(acc[j], B200_ACT_RECTIFY, alpha);
@@ -124,7 +134,7 @@ __device__ __forceinline__ float finish_channels(float (&acc)[N], const float *b
 #pragma unroll
     for (int j = 0; j < N; ++j) acc[j] = apply_act<float>(acc[j], B200_ACT_LEAKY, alpha);
   }
-  return largest * act_floor(act, alpha);
+  return largest;
 }
 #endif
 

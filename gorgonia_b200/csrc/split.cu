@@ -64,29 +64,33 @@ __device__ bool line_has_full(const float *first, long long step, long long len,
 }
 
 // The rare end of SPLIT_F16's step: `mine` marks the small ones of this lane's eight values, which begin at
-// column c0 of row r of the slice at `slice`. By a whole warp.
-__device__ __noinline__ void note_small(const SplitJob &j, unsigned mine, const float *slice, long long r, long long c0,
+// column c0 of row r of the slice at `slice`. By a whole warp. Returns whether the operand is known to be of no use, so
+// that the warp need not ask again.
+__device__ __noinline__ bool note_small(const SplitJob &j, unsigned mine, const float *slice, long long r, long long c0,
                                         float scale) {
   const int lane = threadIdx.x & 31;
   const unsigned n = __reduce_add_sync(0xffffffffu, (unsigned)__popc(mine));
   bool look = false;
   if (lane == 0) look = f16_count_small(j.rec, j.limit, n);
-  if (!__shfl_sync(0xffffffffu, look, 0)) return;
+  if (!__shfl_sync(0xffffffffu, look, 0)) return true;
   for (unsigned lanes = __ballot_sync(0xffffffffu, mine != 0); lanes; lanes &= lanes - 1) {
     const int src = __ffs(lanes) - 1;
     const long long lr = __shfl_sync(0xffffffffu, r, src), lc0 = __shfl_sync(0xffffffffu, c0, src);
     const float *ls = (const float *)__shfl_sync(0xffffffffu, (unsigned long long)slice, src);
     for (unsigned m = __shfl_sync(0xffffffffu, mine, src); m; m &= m - 1) {
+      // others may have found out meanwhile: one warp that went on through 256 values took 470 us
+      if (__shfl_sync(0xffffffffu, (int)f16_unusable(j.rec, j.limit), 0)) return true;
       const long long lc = lc0 + __ffs(m) - 1;
       bool alone = false;
       if (j.lines & kLineRows) alone = !line_has_full(ls + lr * j.ld, 1, j.cols, lc, scale);
       if (!alone && (j.lines & kLineCols)) alone = !line_has_full(ls + lc, j.ld, j.rows, lr, scale);
       if (alone) {
         if (lane == 0) atomicOr(&j.rec->bad, 1u);
-        return;
+        return true;
       }
     }
   }
+  return false;
 }
 
 template <int MODE>
@@ -120,6 +124,7 @@ __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ Spli
     if (blk == 0 && threadIdx.x == 0) j.rec->scale_exp = ex;
   }
   unsigned amax = 0, bad = 0;
+  bool useless = false;  // SPLIT_F16: the record has been seen to say so
   // SPLIT_F16: warps stay whole for note_small
   const long long lane_off = MODE == SPLIT_F16 ? threadIdx.x & 31 : 0;
   for (long long t = (long long)blk * 256 + threadIdx.x; t - lane_off < total; t += (long long)nblk * 256) {
@@ -178,7 +183,8 @@ __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ Spli
         reinterpret_cast<float4 *>(j.lo)[t] = make_float4(l[0], l[1], l[2], l[3]);
       }
     }
-    if (MODE == SPLIT_F16 && __any_sync(0xffffffffu, small != 0)) note_small(j, small, slice, r, c0, scale);
+    if (MODE == SPLIT_F16 && !useless && __any_sync(0xffffffffu, small != 0))
+      useless = note_small(j, small, slice, r, c0, scale);
   }
   if (MODE == SPLIT_AMAX) {
     amax = __reduce_max_sync(0xffffffffu, amax);
