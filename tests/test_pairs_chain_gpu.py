@@ -110,7 +110,8 @@ def test_first_link_and_pool(fresh, C):
 @pytest.mark.parametrize("case", [(32, 128, 26, 26, 256, 3, 1, 1), (128, 64, 32, 32, 64, 3, 1, 1), (32, 96, 40, 41, 250, 3, 2, 1),
                                   (48, 256, 13, 13, 256, 3, 1, 1)])
 def test_single_convolutions(fresh, case, constant):
-    # large enough for pairs; then with values that are not: the TF32 launches behind them answer
+    # TF32 pairs, but the first case with constant filters: fp16 (the larger ones are further down); then values that
+    # are out of fp16's range, which the TF32 launches behind it answer
     e = fresh
     B, C, H, W, K, k, stride, pad = case
     x, w, bias = util.normal(61, (B, C, H, W)), util.normal(62, (K, C, k, k), scale=0.05), util.normal(63, K)
@@ -268,6 +269,25 @@ def test_large_single_convolutions_are_made_from_pairs(fresh, case):
     assert_gemm_close(y.numpy(), want, 1e-5)
     # a sprinkling of small values among ordinary ones changes nothing of that
     x.reshape(-1)[::x.size // 50] = np.float32(1e-13)
+    tx.set(x)
+    e.Conv2d(tx, tw, y, pad=(pad, pad))
+    assert_gemm_close(y.numpy(), _conv64(x, w, pad), 1e-5)
+    # an image far below the others and a value far above; then infinities and NaNs; then ordinary values again
+    wide = x.copy()
+    wide[1] *= np.float32(1e-25)
+    wide[2, :, 3, 3] = np.float32(1e20)
+    tx.set(wide)
+    e.Conv2d(tx, tw, y, pad=(pad, pad))
+    got, ref = y.numpy(), _conv64(wide, w, pad)
+    for b in range(3):
+        assert_gemm_close(got[b], ref[b], 1e-5)
+    bad = x.copy()
+    bad[0, 0, 0, 0], bad[3, 1, 5, 5] = np.inf, np.nan
+    tx.set(bad)
+    e.Conv2d(tx, tw, y, pad=(pad, pad))
+    got, ref = y.numpy(), _conv64(bad, w, pad)
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref)) and not np.isfinite(got[0]).all()
+    assert_gemm_close(got[1], ref[1], 1e-5)
     tx.set(x)
     e.Conv2d(tx, tw, y, pad=(pad, pad))
     assert_gemm_close(y.numpy(), _conv64(x, w, pad), 1e-5)
