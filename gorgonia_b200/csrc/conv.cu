@@ -567,7 +567,7 @@ static int conv_filters_pairs(b200_engine *e, const float *w, int K, int C, int 
 }
 
 // One convolution of a chain on pairs of fp16 (path: a tensor-core kernel). x16: the input in pairs form.
-static int conv2d_pairs(b200_engine *e, int path, const __half *x16, const F16Rec *x_rec, const float *w, float *y,
+static int conv2d_pairs(b200_engine *e, int path, const __half *x16, const F16Rec *x_rec, unsigned limit_x, const float *w, float *y,
                         const PairsOut &out, long long B, int C, int H, int W, int K, int kh, int kw, int padH,
                         int padW, int sH, int sW, int dH, int dW, int Ho, int Wo, const Epilogue &ep, bool pool2) {
   TcOperand wf;
@@ -578,7 +578,7 @@ static int conv2d_pairs(b200_engine *e, int path, const __half *x16, const F16Re
   PairsIn in;
   in.x = x_rec;
   in.w = f;
-  in.limit_x = f16_small_limit(B * C * H * W);
+  in.limit_x = limit_x;
   in.limit_w = f16_small_limit((long long)K * C * kh * kw);
   if (path == B200_CONV_TC_WINDOW)
     rc = conv2d_win_pairs(e, x16, wf, y, B, C, H, W, K, kh, kw, padH, padW, dH, dW, Ho, Wo, ep, pool2, in, out);
@@ -614,7 +614,7 @@ static int conv2d_eager_pairs(b200_engine *e, int path, const float *x, const fl
   PairsOut out;
   out.rec = ry;
   if (rc == B200_OK)
-    rc = conv2d_pairs(e, path, (const __half *)x16, rx, w, y, out, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho,
+    rc = conv2d_pairs(e, path, (const __half *)x16, rx, f16_small_limit(n), w, y, out, B, C, H, W, K, kh, kw, padH, padW, sH, sW, dH, dW, Ho,
                       Wo, ep, pool2);
   b200_put(e, x16, 0);  // stream order; the TF32 pairs may take its place
   const unsigned limits[2] = {f16_small_limit(n), 0xFFFFFFFFu};
@@ -913,7 +913,7 @@ int b200_conv2d_pairs_fwd(b200_engine *e, const void *x, const void *x_pairs, co
     if (C == 2) return launch_conv3x3_first_pool<2, true>(e, xf, wf, nullptr, B, (int)H, (int)W, (int)K, ep, nullptr, nullptr, rx, out);
     return launch_conv3x3_first_pool<3, true>(e, xf, wf, nullptr, B, (int)H, (int)W, (int)K, ep, nullptr, nullptr, rx, out);
   }
-  return conv2d_pairs(e, path, (const __half *)x_pairs, rx, wf, (float *)y, out, B, (int)C, (int)H, (int)W, (int)K, kh,
+  return conv2d_pairs(e, path, (const __half *)x_pairs, rx, pairs_small_limit(B * C * H * W), wf, (float *)y, out, B, (int)C, (int)H, (int)W, (int)K, kh,
                       kw, pad_h, pad_w, 1, 1, 1, 1, (int)Ho, (int)Wo, ep, pool2 != 0);
 }
 
@@ -936,7 +936,7 @@ int b200_pairs_check(b200_engine *e, void *recs, const int64_t *counts, int k, i
   int rc = flush_pending(e);
   if (rc != B200_OK) return rc;
   unsigned limits[kMaxPairsRecs];
-  for (int i = 0; i < k; ++i) limits[i] = f16_small_limit(counts[i]);
+  for (int i = 0; i < k; ++i) limits[i] = pairs_small_limit(counts[i]);
   return launch_pairs_check(e, (F16Rec *)recs, limits, k, verdict);
 }
 

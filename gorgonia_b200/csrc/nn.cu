@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) maxpool_split_kernel(const float *__restr
           __half hh, ll;
           stats.see(v);
           small = f16_pair(v, scale, hh, ll);
-          full = fabsf(v * scale) >= kFullPair;
+          full = fabsf(v * scale) >= kOrdinary;
           stats.small += small ? 1u : 0u;
           if (!(fabsf(v * scale) <= 65504.f)) stats.bad = 1;
           out16.h[o] = hh;

@@ -11,7 +11,12 @@
 // hold that one too, and they came about by cancellation, with an error above what the pair adds. A place where
 // every channel is small is a place whose inputs are, and would be the whole of what some outputs of the next link
 // are made from, so one such place marks the tensor. Epilogues look at the sums in front of the activation
-// (Rectify leaves zeros that say nothing), in the eight or more channels that a thread has at a place.
+// (Rectify leaves zeros that say nothing), in the eight or more channels that a thread has at a place, and "ordinary"
+// keeps 2^7 from where pairs stop being full (kOrdinary): what 2^14 small values beside one ordinary one can add up to
+// is then below that one's own rounding, so it does not matter how many small ones a tensor holds. (With at most
+// n / 65536 of them, as a matrix may hold, tiny-YOLO came to 94 % of the allowance at two images and went over it at
+// one, and smaller slopes leave more of them in proportion.) pairs_small_limit only keeps tensors away that consist of
+// them.
 #pragma once
 #include "epilogue.cuh"
 #include "split.h"
@@ -34,7 +39,10 @@ struct PairsOut {
   F16Rec *rec = nullptr;  // null: nobody asks about the output
 };
 
+inline unsigned pairs_small_limit(long long n) { return (unsigned)(n >> 4 > 0x7FFFFFFF ? 0x7FFFFFFF : n >> 4); }
+
 #ifdef __CUDACC__
+constexpr float kOrdinary = 0.0078125f;  // 2^-7, of values scaled into fp16's range
 // Kernels of the TF32 way that stand behind one of fp16 pairs run only if that turned out unusable.
 __device__ __forceinline__ bool skip_launch(const int *only_if) { return only_if && __ldg(only_if) == 0; }
 
@@ -105,7 +113,7 @@ __device__ __forceinline__ void store_pairs(const float *v, int valid, float sca
       for (int j = 0; j < N; ++j)
         if (j < valid) sums = fmaxf(sums, fabsf(v[j]));
     }
-    if (sums * scale < kFullPair) st.bad = 1;
+    if (sums * scale < kOrdinary) st.bad = 1;
   }
 }
 

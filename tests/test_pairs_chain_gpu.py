@@ -430,3 +430,28 @@ def test_only_if_is_the_calling_threads(fresh):
     assert np.abs(conv.numpy()).max() > 0
     assert_bits_equal(s.numpy(), -z)
     assert not inner.numpy().any()
+
+
+@pytest.mark.parametrize("alpha", [0.1, 0.001, 0.0003])
+def test_many_small_values_among_ordinary_ones(fresh, alpha):
+    # a slope that leaves many small values, each beside ordinary ones: the chain is not made over, and agrees with
+    # the TF32 one
+    e = fresh
+    ch, g = (3, 16, 32, 64, 128), util.rng(105)
+    ws = [e.constant(e.tensor((g.standard_normal((ch[i + 1], ch[i], 3, 3)) * np.sqrt(2 / (9 * ch[i]))).astype(np.float32)))
+          for i in range(4)]
+    chain = tapes._ConvChain(e, 8, (3, 128, 128), [
+        {"w": ws[i], "pad": (1, 1), "bias": None, "act": "leaky", "alpha": alpha, "pool": "2x2/2" if i < 2 else None}
+        for i in range(4)])
+    assert chain.can_pairs()
+    rec = tapes._Records(e)
+    chain.plan_pairs(rec)
+    tx = e.tensor(g.random((8, 3, 128, 128), dtype=np.float32) - np.float32(0.5))
+    with rec.chain():
+        got = chain.forward_pairs(tx).numpy()
+        small = rec.buf.numpy().reshape(-1, 4)[:len(rec.counts), 1]
+    assert rec.buf.numpy()[-4] == 0
+    assert alpha > 0.05 or (small > np.array(rec.counts) >> 16).any()     # more than a matrix may hold
+    want = chain.forward(tx).numpy()
+    # both chains' sums end in float32 roundings: as the chains of the tapes
+    assert np.abs(got - want).max() <= 4e-5 * np.abs(want).max()
