@@ -607,8 +607,7 @@ __global__ void __launch_bounds__(256) nhwc_split_img_kernel(const float *__rest
   }
 }
 
-// Rewrites x (B, C, HW) as NHWC TF32 head/tail into two fresh arena blocks xs[0], xs[1], which the
-// caller releases.
+// Rewrites x (B, C, HW) as NHWC pairs with the kernel that its plane and alignment allow.
 template <bool F16>
 static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, const NhwcOut &out) {
   if (HW % 4 == 0 && C % 16 == 0 && (uintptr_t)x % 16 == 0) {
@@ -637,6 +636,7 @@ static int launch_nhwc_split(b200_engine *e, const float *x, long long B, int C,
   B200_CHECK_LAUNCH(e, "nhwc_split_kernel");
   return B200_OK;
 }
+// As TF32 head/tail into two fresh arena blocks xs[0], xs[1], which the caller releases.
 int conv_nhwc_split(b200_engine *e, const float *x, long long B, int C, int HW, void **xs) {
   const long long xbytes = B * C * HW * 4;
   xs[0] = xs[1] = nullptr;

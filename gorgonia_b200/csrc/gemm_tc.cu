@@ -526,10 +526,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           }
           ptx::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) {
-            if (PAIR) ptx::mbar_arrive_cluster(at_leader(&acc_empty[buf]));
-            else ptx::mbar_arrive(&acc_empty[buf]);
-          }
+          if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
         }
         if (kb0 != 0 || kb1 != p.num_k) {
           // part of a tile: leave it in the workspace; the CTA that delivers the last part finishes the tile

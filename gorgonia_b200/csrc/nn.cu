@@ -1163,7 +1163,7 @@ static int batchnorm_fwd_t(b200_engine *e, const T *x, T *y, long long B, int C,
   if (training) {
     for (int c0 = 0; c0 < C && le == cudaSuccess; c0 += b200_engine::kSkCounters) {
       const int nc = std::min(C - c0, (int)b200_engine::kSkCounters);
-      launch_kernel(e, bn_sums_kernel<T>, dim3(nc, bn_groups(e, B, nc)), 256, 0, 
+      launch_kernel(e, bn_sums_kernel<T>, dim3(nc, bn_groups(e, B, nc)), 256, 0,
           c0, x, B, C, S, (double *)part, e->sk_counters, (T)momentum, (T)eps, running_mean, running_var, save_mean,
           save_var, (T *)ab);
       le = cudaGetLastError();
@@ -1209,7 +1209,7 @@ static int batchnorm_bwd_t(b200_engine *e, const T *x, const T *dy, T *dx, long 
   cudaError_t le = cudaSuccess;
   for (int c0 = 0; c0 < C && le == cudaSuccess; c0 += b200_engine::kSkCounters) {
     const int nc = std::min(C - c0, (int)b200_engine::kSkCounters);
-    launch_kernel(e, bn_bwd_sums_kernel<T>, dim3(nc, bn_groups(e, B, nc)), 256, 0, 
+    launch_kernel(e, bn_bwd_sums_kernel<T>, dim3(nc, bn_groups(e, B, nc)), 256, 0,
         c0, x, dy, B, C, S, (double *)part, e->sk_counters, training, (T)eps, running_var, save_mean, save_var, (T *)coef);
     le = cudaGetLastError();
     e->launches++;
@@ -1291,11 +1291,11 @@ int b200_maxpool2d_pairs_fwd(b200_engine *e, const void *x, const void *x_rec, v
   out.l = out.h + B * C * Ho * Wo;
   out.rec = (F16Rec *)y_rec;
   if (kh == 2 && kw == 2)
-    launch_kernel(e, maxpool_split_kernel<true, true>, blocks, 256, 0, 
+    launch_kernel(e, maxpool_split_kernel<true, true>, blocks, 256, 0,
         (const float *)x, nullptr, nullptr, nullptr, nullptr, (const F16Rec *)x_rec, out, B, (int)C, (int)H, (int)W,
         (int)Ho, (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   else
-    launch_kernel(e, maxpool_split_kernel<false, true>, blocks, 256, 0, 
+    launch_kernel(e, maxpool_split_kernel<false, true>, blocks, 256, 0,
         (const float *)x, nullptr, nullptr, nullptr, nullptr, (const F16Rec *)x_rec, out, B, (int)C, (int)H, (int)W,
         (int)Ho, (int)Wo, kh, kw, stride_h, stride_w, oh0, ow0);
   B200_CHECK_LAUNCH(e, "maxpool_split_kernel");
@@ -1426,20 +1426,20 @@ int b200_maxpool2d_bwd(b200_engine *e, int dtype, const void *dy, const int64_t 
       pad_west == 0 && pad_east == 0 && W % 2 == 0 && (uintptr_t)dx % 8 == 0) {
     const long long lines = B * C * ((H + 1) / 2);
     if (W % 4 == 0 && (uintptr_t)dx % 16 == 0 && (uintptr_t)dy % 8 == 0 && (uintptr_t)mask % 16 == 0)
-      launch_kernel(e, maxpool2x2_bwd_kernel<2>, grid_for(e, lines * (Wo / 2)), 256, 0, 
+      launch_kernel(e, maxpool2x2_bwd_kernel<2>, grid_for(e, lines * (Wo / 2)), 256, 0,
           (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo);
     else
-      launch_kernel(e, maxpool2x2_bwd_kernel<1>, grid_for(e, lines * Wo), 256, 0, 
+      launch_kernel(e, maxpool2x2_bwd_kernel<1>, grid_for(e, lines * Wo), 256, 0,
           (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo);
     B200_CHECK_LAUNCH(e, "maxpool2x2_bwd_kernel");
     return B200_OK;
   }
   if (dtype == B200_F32)
-    launch_kernel(e, maxpool_bwd_kernel<float>, grid_for(e, total), 256, 0, 
+    launch_kernel(e, maxpool_bwd_kernel<float>, grid_for(e, total), 256, 0,
         (const float *)dy, (const long long *)mask, (float *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw,
         stride_h, stride_w, oh0, ow0);
   else
-    launch_kernel(e, maxpool_bwd_kernel<double>, grid_for(e, total), 256, 0, 
+    launch_kernel(e, maxpool_bwd_kernel<double>, grid_for(e, total), 256, 0,
         (const double *)dy, (const long long *)mask, (double *)dx, B * C, (int)H, (int)W, (int)Ho, (int)Wo, kh, kw,
         stride_h, stride_w, oh0, ow0);
   B200_CHECK_LAUNCH(e, "maxpool_bwd_kernel");
@@ -1687,14 +1687,14 @@ int b200_gather_axis(b200_engine *e, const void *x, const int64_t *idx, void *y,
   const bool w4 = row_bytes % 4 == 0 && (uintptr_t)x % 4 == 0 && (uintptr_t)y % 4 == 0;
   if (w16) {
     const long long words = row_bytes / 16;
-    launch_kernel(e, gather_rows_kernel<uint4>, grid_for(e, outer * n_idx * words), 256, 0, 
+    launch_kernel(e, gather_rows_kernel<uint4>, grid_for(e, outer * n_idx * words), 256, 0,
         (const uint4 *)x, (const long long *)idx, (uint4 *)y, outer, n_idx, words, n_rows, bad);
   } else if (w4) {
     const long long words = row_bytes / 4;
-    launch_kernel(e, gather_rows_kernel<uint32_t>, grid_for(e, outer * n_idx * words), 256, 0, 
+    launch_kernel(e, gather_rows_kernel<uint32_t>, grid_for(e, outer * n_idx * words), 256, 0,
         (const uint32_t *)x, (const long long *)idx, (uint32_t *)y, outer, n_idx, words, n_rows, bad);
   } else {
-    launch_kernel(e, gather_rows_kernel<unsigned char>, grid_for(e, outer * n_idx * row_bytes), 256, 0, 
+    launch_kernel(e, gather_rows_kernel<unsigned char>, grid_for(e, outer * n_idx * row_bytes), 256, 0,
         (const unsigned char *)x, (const long long *)idx, (unsigned char *)y, outer, n_idx, row_bytes, n_rows, bad);
   }
   B200_CHECK_LAUNCH(e, "gather_rows_kernel");

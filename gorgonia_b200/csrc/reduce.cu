@@ -407,7 +407,7 @@ static int launch_col_split(b200_engine *e, const T *x, T *y, long long outer, l
     chunks = 1;  // no room for the parts: whole columns
   const long long per = (len + chunks - 1) / chunks;
   chunks = (len + per - 1) / per;
-  launch_kernel(e, col_split_kernel<T, MODE, CX>, dim3((unsigned)blocks, (unsigned)chunks), 256, 0, 
+  launch_kernel(e, col_split_kernel<T, MODE, CX>, dim3((unsigned)blocks, (unsigned)chunks), 256, 0,
       x, y, len, inner, (int)groups, per, (T *)ws, e->sk_counters);
   if (ws) b200_put(e, ws, 0);  // stream order: whoever gets the block next runs after this kernel
   B200_CHECK_LAUNCH(e, "col_split_kernel");
