@@ -590,9 +590,11 @@ static int conv2d_pairs(b200_engine *e, int path, const __half *x16, const F16Re
 }
 
 // Whether a single convolution is worth pairs of fp16. They save about 0.35 of what TF32 pairs take (160
-// TFLOP/s); finding the input's largest magnitude reads it once more, and the four more launches cost 20 us
-// (16 x 128 x 26 x 26 to 256 channels, 6.4 GFLOP: 45 us with TF32 pairs, 55 with fp16), two more with filters
-// that are not constant.
+// TFLOP/s); finding the input's largest magnitude reads it once more, and the four more launches are set down
+// with 20 us, two more with filters that are not constant. Measured both ways (TF32 / fp16, us; 3x3, 128 -> 256
+// channels on 26 x 26): 16 images, 6.4 GFLOP, 41 / 41 with constant filters and 45 / 52 with others; 24 images
+// 51 / 43 and 55 / 54; 32 images 66 / 57 and 70 / 68; 48 images 95 / 71 and 98 / 83. The rule turns to fp16 at 31
+// images and 42: dependent launches cost about half of what it sets down, so it stays on the safe side.
 static bool conv_pairs_pay(b200_engine *e, const float *w, long long B, int C, int H, int W, int K, int taps, int Ho, int Wo) {
   const double saves = 0.35 * 2.0 * B * Ho * Wo * K * (double)C * taps / 160e12;
   const double costs = 4.0 * B * C * H * (double)W / 5e12 + (is_constant(e, w) ? 20e-6 : 27e-6);

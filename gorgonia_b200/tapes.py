@@ -157,7 +157,9 @@ class _ConvChain:
 
     # Convolutions of this much work per pass are worth pairs of fp16: they save about 0.45 of what TF32 pairs
     # take at 160 TFLOP/s, and the launches of the TF32 chain behind them, which find nothing to do, cost a
-    # microsecond or two each.
+    # microsecond or two each. Measured both ways (TF32 / fp16, us): LeNet at 128 images (1.9 GFLOP) 76 / 78, 256
+    # 84 / 82, 512 (7.6) 125 / 107, 1024 (15.3) 176 / 148; tiny-YOLO at 2 images (13.9) 241 / 221, 8 452 / 341, but at
+    # one (7.0) 211 / 381: its tensors are allowed a small value or two (n / 65536), and the chain is made over.
     PAIRS_FLOPS = 12e9
 
     def worth_pairs(self, flops):
