@@ -13,7 +13,7 @@ Prints ONE JSON line (rank 0). Workloads (--workload):
                tanh(x*w+b) (16 B/elem). Metric: GB/s of algorithmic bytes. N GPUs = N replicas.
                As the headline it also reports the sweep at 2^20, 2^24 and 2^27 elements, the
                broadcast Add for B = 4096 .. 262144 and the chain with (1,1024) rows for w and b.
-  gemm         MatMul M=N=K=8192, float32 (3xTF32). Metric: TFLOP/s (2*M*N*K). Replicas.
+  gemm         MatMul M=N=K=8192, float32 (pairs of fp16, or of TF32). Metric: TFLOP/s (2*M*N*K). Replicas.
   linalg       the whole GEMM/GEMV sweep: MatMul 1024^3, 4096^3, 8192^3 in float32 and bfloat16, a
                batch of 64 products of 512^3, MatVecMul 16384^2 in both orientations, Outer 8192^2,
                each with its own roofline. Headline value: the 8192^3 float32 product.
@@ -34,6 +34,7 @@ restatement of gorgonia's CPU engine; the Go reference itself cannot be built he
 sample of the workload.
 """
 import argparse
+import contextlib
 import ctypes as C
 import json
 import os
@@ -53,6 +54,7 @@ ELEMENTWISE_OPS = [  # (name, kind, algorithmic bytes per element)
     ("bcast_add", "bcast", 8), ("chain_tanh_xw_b", "chain", 16),
 ]
 BYTES_PER_ELEM_STEP = sum(b for _, _, b in ELEMENTWISE_OPS)
+F32_METRIC = "MatMul float32 throughput, 2*M*N*K"
 MODEL_BATCH = {"mlp": 256, "lenet": 8192, "yolo": 64}
 REF_NOTE = ("CPU restatement of gorgonia's CPU-engine semantics (oracle/); the Go reference cannot be built here "
             "(no Go toolchain, dependencies not vendored)")
@@ -569,6 +571,21 @@ def read_columns(e, t, base, cols, M, N):
     return strip
 
 
+def f32_pairs(e, product):
+    """What a float32 product is made from: a split and a product of pairs of TF32, or, of fp16, two passes for the
+    split, the product, and the two TF32 launches behind it that find nothing to do."""
+    before = e.launches
+    product()
+    return "fp16" if e.launches - before > 2 else "TF32"
+
+
+def f32_peak(e, pk, pairs):
+    """The rate at which the tensor core issues the three products of a pair: measured TF32, or 16-bit."""
+    if pairs == "TF32":
+        return tf32_peak(e, pk)
+    return pk["bf16_tflops"], f"{pk['source']}: 16-bit library product, burst"
+
+
 def wl_gemm(ctx, args, main):
     n = 8192
     steps, warmup = (args.steps, args.warmup) if main else (5, 3)
@@ -588,20 +605,20 @@ def wl_gemm(ctx, args, main):
     flops = 2.0 * n ** 3
     pk = peaks()
     tf = flops / step_s / 1e12
-    peak32, peak32_src = tf32_peak(e, pk)
+    pairs = f32_pairs(e, lambda: e.MatMul(ta, tb, tc))
+    peak32, peak32_src = f32_peak(e, pk, pairs)
     parity = None
     if ctx.rank == 0 and not args.profile:
         parity = parity_product(e, tc, a, b, 1e-5)
-    res = {"metric": "MatMul float32 (3xTF32) throughput, 2*M*N*K", "unit": "TFLOP/s", "value": ctx.world * tf,
-           "ms_per_step": step_s * 1e3, "dtype": "f32 (3xTF32 on tensor cores, fp32 accumulate)",
+    res = {"metric": F32_METRIC, "unit": "TFLOP/s", "value": ctx.world * tf,
+           "ms_per_step": step_s * 1e3, "dtype": f"f32 (pairs of {pairs} on tensor cores, fp32 accumulate)",
            "config": {"workload": "gemm_f32_8192", "M": n, "N": n, "K": n, "l2": "operands larger than L2",
                       "parallelism": f"replicas x{ctx.world}" if ctx.world > 1 else "single GPU"},
            "gpu_launches": launches, "clocks": clocks, "steps": steps, "warmup": warmup,
            "parity_checked": parity,
-           "roofline": {"bound": "tensor", "kernel": "gemm_tc_kernel<3,128>", "achieved": 3 * tf,
-                        "peak": peak32, "unit": "TFLOP/s (TF32 issued = 3 x algorithmic)",
-                        "frac": 3 * tf / peak32, "peak_source": peak32_src,
-                        "frac_of_bf16_burst_over_2": 3 * tf / (pk["bf16_tflops"] / 2), "traffic": None}}
+           "roofline": {"bound": "tensor", "kernel": f"gemm_tc_kernel<{2 if pairs == 'fp16' else 3},128> and its split passes",
+                        "achieved": 3 * tf, "peak": peak32, "unit": f"TFLOP/s ({pairs} issued = 3 x algorithmic)",
+                        "frac": 3 * tf / peak32, "peak_source": peak32_src, "traffic": None}}
     if not main or args.profile:
         # bf16 beside it, same shape
         tab, tbb = e.tensor_bf16(a), e.tensor_bf16(b)
@@ -647,10 +664,9 @@ def wl_linalg(ctx, args, main):
     e.ResetAllocator()
     ctx._flush = None
     pk = peaks()
-    peak32, peak32_src = tf32_peak(e, pk)
     steps = 5
     items = {"matmul_f32_8192": {"tflops": round(res["value"] / ctx.world, 1), "frac": round(res["roofline"]["frac"], 4),
-                                 "bound": "tensor (3 x TF32 issued)", "parity_checked": res.get("parity_checked")}}
+                                 "bound": f"tensor, {res['roofline']['unit']}", "parity_checked": res.get("parity_checked")}}
     g = np.random.Generator(np.random.Philox(31 + ctx.rank))
 
     def normal(shape):
@@ -665,8 +681,9 @@ def wl_linalg(ctx, args, main):
             ta, tb = e.tensor(a), e.tensor(b)
             s_ = ctx.timed_flushed(lambda: e.MatMul(ta, tb, tc), steps, 3)
             tf = flops / s_ / 1e12
-            items[f"matmul_f32_{n}"] = {"tflops": round(tf, 1), "frac": round(3 * tf / peak32, 4),
-                                        "bound": "tensor (3 x TF32 issued)",
+            pairs = f32_pairs(e, lambda: e.MatMul(ta, tb, tc))
+            items[f"matmul_f32_{n}"] = {"tflops": round(tf, 1), "frac": round(3 * tf / f32_peak(e, pk, pairs)[0], 4),
+                                        "bound": f"tensor (3 x {pairs} issued)",
                                         "parity_checked": parity_product(e, tc, a, b, 1e-5) if ctx.rank == 0 else None}
             ta.free(); tb.free()
         ab, bb = from_bf16(to_bf16(a)), from_bf16(to_bf16(b))
@@ -684,8 +701,9 @@ def wl_linalg(ctx, args, main):
     tA, tB, tC = e.tensor(A), e.tensor(Bm), e.empty((64, 512, 512))
     s_ = ctx.timed_flushed(lambda: e.MatMul(tA, tB, tC), steps, 3)
     tf = 64 * 2.0 * 512 ** 3 / s_ / 1e12
-    items["matmul_f32_64x512"] = {"tflops": round(tf, 1), "frac": round(3 * tf / peak32, 4),
-                                  "bound": "tensor (3 x TF32 issued)",
+    pairs = f32_pairs(e, lambda: e.MatMul(tA, tB, tC))
+    items["matmul_f32_64x512"] = {"tflops": round(tf, 1), "frac": round(3 * tf / f32_peak(e, pk, pairs)[0], 4),
+                                  "bound": f"tensor (3 x {pairs} issued)",
                                   "parity_checked": parity_product(e, tC, A[37], Bm[37], 1e-5, batch_index=37)
                                   if ctx.rank == 0 else None}
     e.Signal()
@@ -724,8 +742,7 @@ def wl_linalg(ctx, args, main):
     res["config"]["workload"] = "linalg_sweep (headline: gemm_f32_8192)"
     res["config"]["l2"] = "8192^3 operands larger than L2; every other item flushes L2 before each timed step"
     res["roofline"]["items"] = items
-    res["roofline"]["tf32_peak"] = peak32
-    res["roofline"]["tf32_peak_source"] = peak32_src
+    res["roofline"]["tf32_peak"], res["roofline"]["tf32_peak_source"] = tf32_peak(e, pk)
     return res
 
 
@@ -830,30 +847,42 @@ def dominant_kernel(ctx, name, m, b):
     if name == "mlp":
         return None
     e = ctx.engine
+    pairs = "fp16" if m.records is not None else "TF32"
     if name == "yolo":
-        chain, i, kern = m.chain_b, 1, "conv_tma_kernel<128, 32> (layer 7: 1024 -> 1024 channels, 3x3, 13x13)"
+        chain, i = m.chain_b, 1
+        kern = f"conv_tma_kernel on pairs of {pairs} (layer 7: 1024 -> 1024 channels, 3x3, 13x13)"
     else:
-        chain, i, kern = m.chain, 1, "conv_win_kernel<64, 32> (conv1 + pool: 32 -> 64 channels, 3x3, 14x14)"
+        chain, i, kern = m.chain, 1, f"conv_win_kernel on pairs of {pairs} (conv1 + pool: 32 -> 64 channels, 3x3, 14x14)"
     L, prev = chain.layers[i], chain.layers[i - 1]
     x_split = prev["pool_split"] if prev.get("pool_split") is not None else prev["split"]
     x_plain = prev["pooled"] if prev.get("pooled") is not None else prev["y"]
+    x_rec = prev.get("pool_rec", prev.get("rec"))
 
     def launch():
-        e.Conv2dChain(x_plain if x_split is None else None, L["w"], L["y"], L["in_shape"], pad=L["pad"], bias=L["bias"],
-                      act=L["act"], alpha=L["alpha"], pool2=L["fuse_pool"], x_split=x_split, y_split=L["split"])
-    launch()
-    e.Signal()
-    e.record(ctx.ev[0])
-    for _ in range(10):
+        if pairs == "fp16":     # the link's input, its record and its output as the links in front have left them
+            e.Conv2dPairs(None, L["w"], L["y"], L["in_shape"], x_rec, L["rec"], pad=L["pad"], bias=L["bias"], act=L["act"],
+                          alpha=L["alpha"], pool2=L["fuse_pool"], x_pairs=x_split[0],
+                          y_pairs=L["split"][0] if L["split"] else None)
+        else:
+            e.Conv2dChain(x_plain if x_split is None else None, L["w"], L["y"], L["in_shape"], pad=L["pad"], bias=L["bias"],
+                          act=L["act"], alpha=L["alpha"], pool2=L["fuse_pool"], x_split=x_split, y_split=L["split"])
+
+    with m.records.chain() if pairs == "fp16" else contextlib.nullcontext():
+        if pairs == "fp16":
+            m.links_pairs()
         launch()
-    e.record(ctx.ev[1])
+        e.Signal()
+        e.record(ctx.ev[0])
+        for _ in range(10):
+            launch()
+        e.record(ctx.ev[1])
     us = e.elapsed_ms(*ctx.ev) * 100.0
     B, Cc, H, W = L["in_shape"]
     K, _, kh, kw = L["w"].shape
     flops = 2.0 * B * H * W * K * Cc * kh * kw        # stride 1, same padding
     out = {"kernel": kern, "us": us, "flops": flops, "tflops": flops / (us * 1e-6) / 1e12}
-    if name == "yolo" and b == 64:
-        out["traffic"] = 754.3e6
+    if name == "yolo" and b == 64 and pairs == "fp16":
+        out["traffic"] = 129.95e6
         out["traffic_source"] = ("dram__bytes_read.sum + dram__bytes_write.sum of this launch under ncu "
                                  "(profiles/conv_tma_kernel_yolo_layer7.txt)")
     return out
@@ -903,13 +932,14 @@ def wl_model(ctx, args, name, main):
     clocks = sampler.stop() if ctx.rank == 0 else None
     pk = peaks()
     tf = m.flops_per_sample * b / step_s / 1e12
-    peak32, peak32_src = tf32_peak(e, pk)
+    pairs = "fp16" if getattr(m, "records", None) is not None else "TF32"
+    peak32, peak32_src = f32_peak(e, pk, pairs)
     parity = None
     if ctx.rank == 0 and not args.profile:
         parity = parity_model(name, m, x)
     dom = dominant_kernel(ctx, name, m, b) if not args.profile else None
     res = {"metric": f"{name} forward throughput", "unit": "samples/s", "value": total / step_s,
-           "ms_per_step": step_s * 1e3, "dtype": "f32 (matrix products as 3xTF32, fp32 accumulate)",
+           "ms_per_step": step_s * 1e3, "dtype": f"f32 ({'convolutions' if name != 'mlp' else 'products'} on pairs of {pairs}, fp32 accumulate)",
            "config": {"workload": f"{name}_forward", "global_batch": total, "batch_per_gpu": b,
                       "parallelism": f"batch-sharded x{ctx.world}, weights replicated, no collective",
                       "l2": "activations larger than L2" if name != "mlp" else "flush not needed: launch-bound"},
@@ -920,9 +950,8 @@ def wl_model(ctx, args, name, main):
                                    "lenet": "conv_win_kernel + conv_tma_kernel + gemm_tc_kernel (whole step)",
                                    "yolo": "conv_tma_kernel + conv_win_kernel (whole step)"}[name],
                         "achieved": 3 * tf,
-                        "peak": peak32, "unit": "TFLOP/s (TF32 issued = 3 x algorithmic)",
-                        "frac": 3 * tf / peak32, "peak_source": peak32_src,
-                        "frac_of_bf16_burst_over_2": 3 * tf / (pk["bf16_tflops"] / 2), "traffic": None}}
+                        "peak": peak32, "unit": f"TFLOP/s ({pairs} issued = 3 x algorithmic)",
+                        "frac": 3 * tf / peak32, "peak_source": peak32_src, "traffic": None}}
     if dom is not None:
         # the dominant kernel of the step, timed alone: its own launches between CUDA events
         whole = {k: res["roofline"][k] for k in ("kernel", "achieved", "frac")}
@@ -1075,9 +1104,8 @@ def run_reference(args):
                                        "d2h_bytes_per_step": 0}, "note": REF_NOTE}
     line["metric"] = {"elementwise": "elementwise sweep throughput (algorithmic bytes)",
                       "backward": "backward ops throughput (algorithmic bytes)",
-                      "gemm": "MatMul float32 (3xTF32) throughput, 2*M*N*K",
-                      "linalg": "MatMul float32 (3xTF32) throughput, 2*M*N*K"}.get(args.workload,
-                                                                         f"{args.workload} forward throughput")
+                      "gemm": F32_METRIC,
+                      "linalg": F32_METRIC}.get(args.workload, f"{args.workload} forward throughput")
     print(json.dumps(line), flush=True)
 
 

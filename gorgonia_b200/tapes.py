@@ -341,11 +341,15 @@ class LeNet(_Tape):
         self.logits = e.empty((batch, 10))
         self.out = e.empty((batch, 10))
 
+    def links_pairs(self):
+        """The links on pairs of fp16 (within records.chain())."""
+        self.chain.forward_pairs(self.x)
+
     def forward(self):
         e, a = self.e, self.x
         if self.fused and self.records is not None:
             with self.records.chain():
-                self.chain.forward_pairs(a)
+                self.links_pairs()
             with e.only_if(self.records.verdict):
                 a = self.chain.forward(a)
         elif self.fused:
@@ -439,20 +443,21 @@ class TinyYolo(_Tape):
             self.record()
         return self
 
-    def _forward_pairs(self):
+    def links_pairs(self):
+        """The links on pairs of fp16 (within records.chain())."""
         e, a, b = self.e, self.chain_a, self.chain_b
-        with self.records.chain():
-            a.forward_pairs(self.x)
-            last = a.layers[-1]
-            # chain_b's record of its input is written by the pool in front of it
-            e.MaxPool2DPairs(last["y"], last["rec"], self.pool5_split[0], b.x_rec, (2, 2), (1, 0, 1, 0), (1, 1))
-            b.forward_pairs(None, self.pool5_split[0], b.x_rec)
-        with e.only_if(self.records.verdict):
-            return self._forward_tf32()
+        a.forward_pairs(self.x)
+        last = a.layers[-1]
+        # chain_b's record of its input is written by the pool in front of it
+        e.MaxPool2DPairs(last["y"], last["rec"], self.pool5_split[0], b.x_rec, (2, 2), (1, 0, 1, 0), (1, 1))
+        b.forward_pairs(None, self.pool5_split[0], b.x_rec)
 
     def forward(self):
         if self.fused and self.records is not None:
-            return self._forward_pairs()
+            with self.records.chain():
+                self.links_pairs()
+            with self.e.only_if(self.records.verdict):
+                return self._forward_tf32()
         return self._forward_tf32()
 
     def _forward_tf32(self):
