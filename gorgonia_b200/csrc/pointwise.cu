@@ -448,7 +448,12 @@ __device__ __forceinline__ void sts128(uint32_t addr, const uint4 &v) {
 // ring_s / file_s: shared-memory addresses of this stage's ring slots and of the file slots,
 // already offset by this thread's lane (tid * 16).
 // ALIGNED: every tensor starts on a 16-byte boundary (else its elements are moved one at a time).
-template <typename T, int V, int U, int THREADS, bool INSIDE, bool ALIGNED>
+// DIVS: some broadcast source's element is found by division (SRC_CHUNK, SRC_GENERAL). PACKED: instructions are decoded
+// from one load each, which pays where one CTA per SM runs long programs (a gated unit on 2^24 float32: 139 us) and not
+// with two. Code that a program does not reach costs it registers and instruction fetches all the same: with the
+// divisions and the packed form in every kernel, tanh(x * w + b) on 2^27 float32 took 283 us and a row added to a
+// matrix 196; without them 256 and 176.
+template <typename T, int V, int U, int THREADS, bool INSIDE, bool ALIGNED, bool DIVS, bool PACKED>
 __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_t file_s, long long c_tile,
                                         int tid) {
   constexpr int W = U * V;
@@ -491,6 +496,9 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
             const T x = sp[0];
 #pragma unroll
             for (int j = 0; j < V; ++j) v[j] = x;
+          } else if (!DIVS) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) v[j] = T(0);  // not reached
           } else if (mode == SRC_CHUNK) {
             const T x = valid[u] > 0 ? sp[bcast_index(p, s, i)] : T(0);
 #pragma unroll
@@ -511,8 +519,9 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
 #pragma unroll
   for (int j = 0; j < W; ++j) acc[j] = T(0);
   const int n_instr = p.n_instr;
-  // One 8-byte load decodes an instruction; the one after it is fetched while this one runs.
-  uint2 code = p.code[0];
+  // PACKED: one 8-byte load decodes an instruction; the one after it is fetched while this one runs.
+  uint2 code = make_uint2(0, 0);
+  if (PACKED) code = p.code[0];
 #pragma unroll 1
   for (int q = 0; q < n_instr; ++q) {
     T a[W], b[W];
@@ -534,17 +543,17 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
       }
     };
     const uint2 now = code;
-    code = p.code[q + 1 < n_instr ? q + 1 : q];
-    const int op = now.x & 0xFF;
-    fetch_op(a, (now.x >> 8) & 15, (now.x >> 16) & 0xFF);
+    if (PACKED) code = p.code[q + 1 < n_instr ? q + 1 : q];
+    const int op = PACKED ? now.x & 0xFF : p.op[q];
+    fetch_op(a, PACKED ? (now.x >> 8) & 15 : p.ka[q], PACKED ? (now.x >> 16) & 0xFF : p.xa[q]);
     if (op < B200_OP_ABS) {
-      fetch_op(b, (now.x >> 12) & 15, now.x >> 24);
+      fetch_op(b, PACKED ? (now.x >> 12) & 15 : p.kb[q], PACKED ? now.x >> 24 : p.xb[q]);
     } else {
 #pragma unroll
       for (int j = 0; j < W; ++j) b[j] = a[j];
     }
     pw_apply<T, W>(op, a, b, acc);
-    const int keep = now.y & 0xFF;
+    const int keep = PACKED ? now.y & 0xFF : p.keep_slot[q];
     if (keep != 0xFF) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -555,7 +564,7 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
     }
     // Whole tiles are pw_stream_kernel's alone, which gets one output per instruction; the others store a result
     // to each of its outputs.
-    for (int o = (now.y >> 8) & 0xFF; o != 0xFF; o = INSIDE ? 0xFF : p.out_next[o]) {
+    auto store = [&](int o) {
       unsigned char *op_ = reinterpret_cast<unsigned char *>(p.out[o]) + (c_tile + tid) * 16;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -575,6 +584,12 @@ __device__ __forceinline__ void pw_tile(const PwDev &p, uint32_t ring_s, uint32_
           }
         }
       }
+    };
+    const int o0 = PACKED ? (now.y >> 8) & 0xFF : p.out_of[q];
+    if (INSIDE && !PACKED) {
+      if (o0 != 0xFF) store(o0);
+    } else {
+      for (int o = o0; o != 0xFF; o = INSIDE ? 0xFF : p.out_next[o]) store(o);
     }
   }
 }
@@ -620,7 +635,7 @@ __global__ void __launch_bounds__(PW_LOOP_THREADS) pw_loop_kernel(const __grid_c
   const long long ntiles = ((p.n + V - 1) / V + PW_LOOP_THREADS - 1) / PW_LOOP_THREADS;
   for (long long k = blockIdx.x; k < ntiles; k += gridDim.x) {
     pw_fill<T, V, 1, PW_LOOP_THREADS, false, ALIGNED>(p, ring_s, k * PW_LOOP_THREADS, tid);
-    pw_tile<T, V, 1, PW_LOOP_THREADS, false, ALIGNED>(p, ring_s, file_s, k * PW_LOOP_THREADS, tid);
+    pw_tile<T, V, 1, PW_LOOP_THREADS, false, ALIGNED, true, true>(p, ring_s, file_s, k * PW_LOOP_THREADS, tid);
   }
 }
 
@@ -665,11 +680,19 @@ __device__ __forceinline__ void pw_tile_single(int op, bool a_imm, bool b_imm, b
   }
 }
 
+// The end of a tensor in a SINGLE kernel, out of line: with this code among that of the whole tiles, tanh and the
+// logistic function on 2^27 float32 took 199 and 201 us, and 177 each this way (exp 189 either way).
+template <typename T, int V, int U>
+__device__ __noinline__ void pw_ragged(const PwDev &p, uint32_t ring_s, uint32_t file_s, long long c_tile, int tid) {
+  pw_fill<T, V, U, PW_STREAM_THREADS, true, true>(p, ring_s, c_tile, tid);
+  pw_tile<T, V, U, PW_STREAM_THREADS, false, true, true, true>(p, ring_s, file_s, c_tile, tid);
+}
+
 // SINGLE: the program is one instruction over ring slots and immediates (decided on the host), and
 // full tiles take the lean path above. A separate instantiation, so that the general kernel's code
 // and register allocation are not touched by it (measured: sharing one kernel cost the fused
 // chains 5 %).
-template <typename T, int V, int U, bool SINGLE, int CTAS>
+template <typename T, int V, int U, bool SINGLE, int CTAS, bool DIVS>
 __global__ void __launch_bounds__(PW_STREAM_THREADS, CTAS)
     pw_stream_kernel(const __grid_constant__ PwDev p, int stages, int *err_flag) {
   ptx::grid_begin();
@@ -735,11 +758,13 @@ __global__ void __launch_bounds__(PW_STREAM_THREADS, CTAS)
     if (SINGLE && c_tile + TILE_CHUNKS <= nchunks_full)
       pw_tile_single<T, V, U>(s_op, s_a_imm, s_b_imm, s_unary, s_imm_a, s_imm_b, ring_s + s_a_off, ring_s + s_b_off,
                               s_out + c_tile * 16);
-    else if (c_tile + TILE_CHUNKS <= nchunks_full) {
-      pw_tile<T, V, U, PW_STREAM_THREADS, true, true>(p, ring_s, file_s, c_tile, tid);
+    else if (!SINGLE && c_tile + TILE_CHUNKS <= nchunks_full) {
+      pw_tile<T, V, U, PW_STREAM_THREADS, true, true, DIVS, CTAS == 1>(p, ring_s, file_s, c_tile, tid);
+    } else if (SINGLE) {
+      pw_ragged<T, V, U>(p, ring_s, file_s, c_tile, tid);
     } else {
       pw_fill<T, V, U, PW_STREAM_THREADS, true, true>(p, ring_s, c_tile, tid);  // the ragged last chunk
-      pw_tile<T, V, U, PW_STREAM_THREADS, false, true>(p, ring_s, file_s, c_tile, tid);
+      pw_tile<T, V, U, PW_STREAM_THREADS, false, true, DIVS, CTAS == 1>(p, ring_s, file_s, c_tile, tid);
     }
     __syncthreads();    // every thread is done reading this ring stage
     if (s_fail) break;  // uniform: s_fail was written before the barrier
@@ -815,7 +840,7 @@ static int launch_stream_wide(b200_engine *e, const PwDev &d, size_t budget, int
   const size_t smem = (size_t)stages * TILE_CHUNKS * 16;
   const int blocks = (int)std::min<long long>(ntiles, 2LL * e->sm_count);
   static std::atomic<int> attr_dev_mask{0};
-  auto kern = pw_stream_kernel<T, V, U, true, 2>;
+  auto kern = pw_stream_kernel<T, V, U, true, 2, false>;
   if (!(attr_dev_mask & (1 << (e->device & 31)))) {
     B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
     attr_dev_mask |= 1 << (e->device & 31);
@@ -826,8 +851,8 @@ static int launch_stream_wide(b200_engine *e, const PwDev &d, size_t budget, int
   return B200_OK;
 }
 
-template <typename T, int V, int U, int CTAS>
-static int launch_stream_u(b200_engine *e, const PwDev &d, size_t budget, int stages) {
+template <typename T, int V, int U, int CTAS, bool DIVS>
+static int launch_stream_d(b200_engine *e, const PwDev &d, size_t budget, int stages) {
   constexpr int TILE_CHUNKS = PW_STREAM_THREADS * U;
   constexpr int SLOT_BYTES = TILE_CHUNKS * 16;
   const long long nchunks = (d.n + V - 1) / V;
@@ -837,14 +862,14 @@ static int launch_stream_u(b200_engine *e, const PwDev &d, size_t budget, int st
   const int blocks = (int)std::min<long long>(ntiles, (long long)CTAS * e->sm_count);
   static std::atomic<int> attr_dev_mask[2];  // per instantiation: devices on which the attribute is set
   if (single) {
-    auto kern = pw_stream_kernel<T, V, U, true, 2>;
+    auto kern = pw_stream_kernel<T, V, U, true, 2, false>;
     if (!(attr_dev_mask[1] & (1 << (e->device & 31)))) {
       B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
       attr_dev_mask[1] |= 1 << (e->device & 31);
     }
     launch_kernel(e, kern, blocks, PW_STREAM_THREADS, smem, d, stages, e->d_flags + 2);
   } else {
-    auto kern = pw_stream_kernel<T, V, U, false, CTAS>;
+    auto kern = pw_stream_kernel<T, V, U, false, CTAS, DIVS>;
     if (!(attr_dev_mask[0] & (1 << (e->device & 31)))) {
       B200_CHECK_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
       attr_dev_mask[0] |= 1 << (e->device & 31);
@@ -854,6 +879,14 @@ static int launch_stream_u(b200_engine *e, const PwDev &d, size_t budget, int st
   B200_CHECK_LAUNCH(e, "pw_stream_kernel");
   e->flags_dirty = true;
   return B200_OK;
+}
+
+template <typename T, int V, int U, int CTAS>
+static int launch_stream_u(b200_engine *e, const PwDev &d, size_t budget, int stages) {
+  bool divs = CTAS == 1;
+  for (int s = 0; s < d.n_src; ++s) divs |= d.src_mode[s] == SRC_CHUNK || d.src_mode[s] == SRC_GENERAL;
+  return divs ? launch_stream_d<T, V, U, CTAS, true>(e, d, budget, stages)
+              : launch_stream_d<T, V, U, CTAS, CTAS == 1>(e, d, budget, stages);
 }
 
 // Picks the tile width and ring depth that fit shared memory; -1 if the program does not fit.

@@ -146,3 +146,26 @@ def test_one_result_to_several_outputs(fresh, n, dt, start, n_src, n_instr):
         assert_bits_equal(o.numpy(), vals[k])
     for s, x in zip(srcs, xs):      # nothing was written where it does not belong
         assert_bits_equal(s.numpy(), x)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [4096, 3_000_001])
+@pytest.mark.parametrize("chunk", [None, (784, 32), (3, 5)])
+@pytest.mark.parametrize("instr", [3, 7])
+def test_rows_and_scalars_with_and_without_divided_sources(fresh, n, dt, chunk, instr):
+    # rows and scalars alone take the kernels without index divisions, a third kind of source the others
+    e, SRC, INS = fresh, 0x00, 0x80
+    x, row, one = util.normal(71, n, dt), util.normal(72, 64, dt), util.normal(73, 1, dt)
+    srcs, bcast, third = [x, row, one], {1: (1, 64), 2: (1, 1)}, None
+    if chunk:
+        third = util.normal(74, chunk[1], dt)
+        srcs, bcast = srcs + [third], {**bcast, 3: chunk}
+    full = [x, row[np.arange(n) % 64], np.full(n, one[0], dt)] + ([third[np.arange(n) // chunk[0] % chunk[1]]] if chunk else [])
+    prog, val = [("mul", SRC | 0, SRC | 1)], oracle.binary("mul", full[0], full[1])
+    for k in range(1, instr):
+        s = k % len(srcs) if k > 1 else 2
+        prog.append(("add" if k % 2 else "mul", INS | (k - 1), SRC | s))
+        val = oracle.binary("add" if k % 2 else "mul", val, full[s])
+    out = e.empty((n,), dt)
+    e.Pointwise({"instr": prog, "out": [instr - 1], "bcast": bcast}, [out], [e.tensor(a) for a in srcs], n, dt)
+    assert_bits_equal(out.numpy(), val)
